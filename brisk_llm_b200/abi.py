@@ -77,6 +77,7 @@ SIGNATURES = {
     "brisk_cuda_max_context": (C.c_uint64, [C.c_void_p]),
     "brisk_cuda_last_error": (C.c_char_p, [C.c_void_p]),
     "brisk_cuda_generate_greedy": (C.c_int, [C.c_void_p, C.c_int32, C.c_uint64, C.POINTER(C.c_int32), _FP]),
+    "brisk_cuda_log_likelihood": (C.c_int, [C.c_void_p, C.POINTER(C.c_int32), C.c_uint64, C.c_uint32, C.POINTER(C.c_double)]),
     "brisk_cuda_get_stats": (C.c_int, [C.c_void_p, C.POINTER(Stats)]),
     "brisk_cuda_matmul": (C.c_int, [C.c_int32, C.c_void_p, C.c_uint64, C.c_uint64, _FP, C.c_uint64, _FP, C.c_char_p, C.c_size_t]),
     "brisk_cuda_matmul_seconds": (C.c_int, [C.c_int32, C.c_void_p, C.c_uint64, C.c_uint64, C.c_uint64, C.c_uint32,

@@ -270,6 +270,10 @@ size_t topk_scratch_keys(uint32_t vocab, uint32_t k);
 void launch_topk(const float* logits, uint32_t vocab, uint32_t k, unsigned long long* scratch, int32_t* out_ids, float* out_values, cudaStream_t s,
                  uint64_t* launches = nullptr);
 
+// ---- log-probability of each row's next token (score.cu) -------------------------------------------------------------
+// out[i] = logits[i][targets[i]] - max - log(sum exp(logits[i][:] - max)) for `rows` rows of logits[rows][vocab].
+void launch_row_logp(const float* logits, uint32_t vocab, uint32_t rows, const int32_t* targets, double* out, cudaStream_t s);
+
 // Tensor parallel re-layout: gathered[rank][t][rows_l] -> dst[t][rank*rows_l + r] (add: dst += ...), tp ranks.
 void launch_tp_unpack(const float* gathered, float* dst, uint32_t n, uint32_t rows_l, uint32_t tp, bool add, cudaStream_t s);
 

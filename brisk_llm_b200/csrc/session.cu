@@ -177,11 +177,12 @@ struct Session {
 
     // state and scratch
     DevBuffer kv, rope, rope_local, rope_none, proj_b, tanh_table, tokens_dev, scalars, hidden_b, q_b, k_b, v_b, attended_b, ffn_b, up_b, logits_b, tp_local, tp_gathered, full_b, actf, actq0, actd0, acts0, actqk,
-        actdk, actbs, partial, am_val, am_idx, history, logit_history, trace, topk_keys, topk_out;
+        actdk, actbs, partial, am_val, am_idx, history, logit_history, trace, topk_keys, topk_out, score_dev;
     DevActMut act;
     float* logits_host = nullptr;     // pinned [64][vocab]
     int32_t* tokens_host = nullptr;   // pinned [kMaxBatch + 4]
     int32_t* topk_host = nullptr;     // pinned [2 * kMaxTopK]: ids, then the values' bits
+    double* score_host = nullptr;     // pinned [kMaxBatch] log-probabilities
     uint64_t position = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -275,6 +276,7 @@ struct Session {
         if (logits_host) cudaFreeHost(logits_host);
         if (tokens_host) cudaFreeHost(tokens_host);
         if (topk_host) cudaFreeHost(topk_host);
+        if (score_host) cudaFreeHost(score_host);
         if (step_error_host) cudaFreeHost(step_error_host);
     }
 
@@ -536,6 +538,8 @@ struct Session {
         BK_CUDA(cudaMallocHost(&logits_host, size_t(kMaxScored) * vocab * sizeof(float)));
         BK_CUDA(cudaMallocHost(&tokens_host, (kMaxBatch + 4) * sizeof(int32_t)));
         BK_CUDA(cudaMallocHost(&topk_host, 2 * kMaxTopK * sizeof(int32_t)));
+        score_dev.alloc(kMaxBatch * sizeof(double));
+        BK_CUDA(cudaMallocHost(&score_host, kMaxBatch * sizeof(double)));
         BK_CUDA(cudaMallocHost(&step_error_host, 4 * sizeof(unsigned int)));  // [0] the persistent kernel's word, [1] the peer exchange's, [2] the few-token attention's
         step_error_host[0] = step_error_host[1] = step_error_host[2] = step_error_host[3] = 0;  // [3]: the tcgen05 prompt multiply's
         chain_error_dev = attn_chain_error_word();
@@ -738,7 +742,8 @@ struct Session {
 
     // The layers of one batch. n tokens are in tokens_dev, their first position in d_position(); max_visible bounds
     // position + n. single = true takes the fused single-token kernels (n == 1).
-    void run_layers(uint32_t n, bool all_logits, uint32_t max_visible, bool single) {
+    enum Logits { NO_LOGITS, LAST_LOGITS, ALL_LOGITS };  // which rows go through the output head
+    void run_layers(uint32_t n, Logits logits, uint32_t max_visible, bool single) {
         float* hid = hidden_b.as<float>();
         if (variant_layers) single = false;
         {
@@ -891,17 +896,38 @@ struct Session {
                 }
             }
         }
-        const uint32_t rows = all_logits ? n : 1;
-        const float* last = all_logits ? hid : hid + size_t(n - 1) * hidden;
+        if (logits == NO_LOGITS) return;
+        const uint32_t rows = logits == ALL_LOGITS ? n : 1;
+        if (!single) {
+            head_rows(n - rows, rows);
+            return;
+        }
         if (tp) {
             {
                 Scope sc(this, PH_HEAD);
-                apply({{head, tp_local.as<float>(), vocab_l}}, last, hidden, output_norm, hidden, EPI_STORE, rows);
+                apply({{head, tp_local.as<float>(), vocab_l}}, hid, hidden, output_norm, hidden, EPI_STORE);
+            }
+            exchange(tp_local.as<float>(), logits_b.as<float>(), 1, vocab_l, false);
+        } else {
+            Scope sc(this, PH_HEAD);
+            apply({{head, logits_b.as<float>(), vocab}}, hid, hidden, output_norm, hidden, EPI_STORE);
+        }
+    }
+
+    // Output norm and head of rows [first, first + rows) of the residual stream, at most kMaxScored of them, into logits_b.
+    void head_rows(uint32_t first, uint32_t rows) {
+        Needs nd;
+        need(nd, head.type);
+        const float* x = hidden_b.as<float>() + size_t(first) * hidden;
+        if (tp_size > 1) {
+            {
+                Scope sc(this, PH_HEAD);
+                multiply({{head, tp_local.as<float>(), vocab_l}}, prepare(x, hidden, output_norm, rows, hidden, nd), rows, EPI_STORE);
             }
             exchange(tp_local.as<float>(), logits_b.as<float>(), rows, vocab_l, false);
         } else {
             Scope sc(this, PH_HEAD);
-            apply({{head, logits_b.as<float>(), vocab}}, last, hidden, output_norm, hidden, EPI_STORE, rows);
+            multiply({{head, logits_b.as<float>(), vocab}}, prepare(x, hidden, output_norm, rows, hidden, nd), rows, EPI_STORE);
         }
         if (final_softcap != 0.0f) {  // src/model.cpp:1206-1209
             launch_softcap(logits_b.as<float>(), size_t(rows) * vocab, final_softcap, tanh_table.as<uint8_t>(), stream);
@@ -909,12 +935,12 @@ struct Session {
         }
     }
 
-    void forward(uint32_t n, bool all_logits, uint32_t max_visible) { run_layers(n, all_logits, max_visible, false); }
+    void forward(uint32_t n, Logits logits, uint32_t max_visible) { run_layers(n, logits, max_visible, false); }
     bool step_active() const { return (step_enabled || token_enabled) && !profiling; }
     bool token_active() const { return token_enabled && !profiling; }
     void forward_decode() {
         if (!step_active()) {
-            run_layers(1, false, uint32_t(max_context), true);
+            run_layers(1, LAST_LOGITS, uint32_t(max_context), true);
             return;
         }
         if (token_enabled) {
@@ -1015,7 +1041,7 @@ struct Session {
         const bool too_long = !step_active() && !variant_layers &&
                               !dec_attention_fits(uint32_t(max_context), heads_l, head_dim, sms);
         if ((flags & BRISK_CUDA_FLAG_NO_MEGAKERNEL) || too_long) {
-            forward(1, false, uint32_t(max_context));  // the batched kernels, one token
+            forward(1, LAST_LOGITS, uint32_t(max_context));  // the batched kernels, one token
         } else if ((flags & BRISK_CUDA_FLAG_NO_GRAPH) || profiling || (step_active() && !step_in_graph())) {
             forward_decode();
         } else {
@@ -1060,10 +1086,8 @@ struct Session {
             BK_CUDA(cudaMemcpyAsync(tokens_dev.p, tokens_host, cnt * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
             BK_CUDA(cudaMemcpyAsync(d_position(), tokens_host + kMaxBatch, sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
             stats.h2d_bytes += cnt * sizeof(int32_t) + sizeof(uint32_t);
-            const bool last = begin + cnt == n;
             if (cnt == 1 && (!all || n == 1)) step_on_device();  // one token: its one row of logits is all there is, with or without `all`
-            else forward(cnt, all, uint32_t(position + cnt));
-            (void)last;
+            else forward(cnt, all ? ALL_LOGITS : begin + cnt == n ? LAST_LOGITS : NO_LOGITS, uint32_t(position + cnt));
             position += cnt;
         }
         if (topk != 0) {
@@ -1089,6 +1113,80 @@ struct Session {
             throw;
         }
         return logits_host;
+    }
+
+    // Engine::log_likelihood (src/engine.cpp:10-33). The reference's chunks only bound its row buffer: the tokens go through
+    // the layers in prompt-sized batches, the head takes kMaxScored rows at a time, and each position's log-probability is
+    // all that leaves the device.
+    double log_likelihood(const int32_t* tokens, uint64_t n, uint32_t chunk) {
+        if (n < 2) throw CudaError("cuda: need at least two tokens to score");
+        // an error of a later chunk is raised after the chunks before it were appended, as a walk by chunks does
+        uint64_t good = 0;
+        const uint64_t before = position;
+        while (good < n) {
+            const uint64_t cnt = std::min<uint64_t>(chunk, n - good);
+            position = before + good;
+            try {
+                check_tokens(tokens + good, cnt, true);
+            } catch (...) {
+                position = before;
+                if (good > 0) score(tokens, good, good);
+                throw;
+            }
+            good += cnt;
+        }
+        position = before;
+        return score(tokens, n, n - 1);
+    }
+
+    // Appends n tokens and returns the summed log-probability of tokens[1 .. rows]; rows < n unless only the appending matters.
+    double score(const int32_t* tokens, uint64_t n, uint64_t rows) {
+        rows = std::min<uint64_t>(rows, n - 1);
+        begin_call();
+        BK_CUDA(cudaEventRecord(ev0, stream));
+        double total = 0.0;
+        uint32_t pending = 0;  // log-probabilities on their way to score_host
+        auto collect = [&] {
+            BK_CUDA(cudaStreamSynchronize(stream));
+            for (uint32_t i = 0; i < pending; ++i) total += score_host[i];
+            pending = 0;
+        };
+        const uint64_t start = position;
+        for (uint64_t begin = 0; begin < n; begin += kMaxBatch) {
+            const uint32_t cnt = uint32_t(std::min<uint64_t>(kMaxBatch, n - begin));
+            const uint32_t scored = begin < rows ? uint32_t(std::min<uint64_t>(cnt, rows - begin)) : 0;
+            collect();  // also: tokens_host is reused
+            const uint32_t staged = cnt + (begin + cnt < n ? 1 : 0);  // the next batch's first token is this batch's last target
+            std::memcpy(tokens_host, tokens + begin, staged * sizeof(int32_t));
+            tokens_host[kMaxBatch + 3] = int32_t(uint32_t(position));
+            BK_CUDA(cudaMemcpyAsync(tokens_dev.p, tokens_host, staged * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
+            BK_CUDA(cudaMemcpyAsync(d_position(), tokens_host + kMaxBatch + 3, sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
+            stats.h2d_bytes += staged * sizeof(int32_t) + sizeof(uint32_t);
+            forward(cnt, NO_LOGITS, uint32_t(position + cnt));
+            for (uint32_t first = 0; first < scored; first += kMaxScored) {
+                const uint32_t part = std::min(kMaxScored, scored - first);
+                head_rows(first, part);
+                launch_row_logp(logits_b.as<float>(), vocab, part, tokens_dev.as<int32_t>() + first + 1, score_dev.as<double>() + first, stream);
+                ++launches;
+            }
+            if (scored != 0) BK_CUDA(cudaMemcpyAsync(score_host, score_dev.p, scored * sizeof(double), cudaMemcpyDeviceToHost, stream));
+            stats.d2h_bytes += scored * sizeof(double);
+            pending = scored;
+            position += cnt;
+        }
+        BK_CUDA(cudaEventRecord(ev1, stream));
+        queue_step_check();
+        collect();
+        float ms = 0;
+        BK_CUDA(cudaEventElapsedTime(&ms, ev0, ev1));
+        end_call(ms);
+        try {
+            finish_step_check();
+        } catch (...) {
+            position = start;
+            throw;
+        }
+        return total;
     }
 
     void generate_greedy(int32_t first, uint64_t steps, int32_t* out_tokens, float* out_logits) {
@@ -1222,6 +1320,14 @@ int brisk_cuda_eval_topk(brisk_cuda_session* session, const int32_t* tokens, uin
         session->s.eval(tokens, n, false, k);
         std::memcpy(out_ids, session->s.topk_host, k * sizeof(int32_t));
         std::memcpy(out_values, session->s.topk_host + bk::kMaxTopK, k * sizeof(float));
+    });
+}
+
+int brisk_cuda_log_likelihood(brisk_cuda_session* session, const int32_t* tokens, uint64_t n, uint32_t chunk, double* out) {
+    return guarded(session, [&] {
+        if (chunk == 0 || chunk > bk::kMaxScored || out == nullptr) throw bk::CudaError("cuda: scoring takes chunks of 1 to 64 tokens and an output");
+        BK_CUDA(cudaSetDevice(session->s.device));
+        *out = session->s.log_likelihood(tokens, n, chunk);
     });
 }
 

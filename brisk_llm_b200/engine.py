@@ -9,7 +9,6 @@ no other implementation behind this class.
 from __future__ import annotations
 
 import ctypes as C
-import math
 
 import numpy as np
 
@@ -127,17 +126,10 @@ class CudaSession:
         if len(tokens) < 2:
             raise RuntimeError("need at least two tokens to score")
         chunk = max(1, min(int(chunk), MAX_SCORED_TOKENS))
-        total = 0.0
-        for begin in range(0, len(tokens), chunk):
-            part = tokens[begin:begin + chunk]
-            logits = self.eval_all(part)
-            for t in range(len(part)):
-                if begin + t + 1 >= len(tokens):
-                    break
-                row = logits[t]
-                mx = row.max()
-                total += float(row[tokens[begin + t + 1]] - mx) - math.log(np.exp((row - mx).astype(np.float64)).sum())
-        return total
+        total = C.c_double()
+        if self._lib.brisk_cuda_log_likelihood(self._h, tokens.ctypes.data_as(C.POINTER(C.c_int32)), len(tokens), chunk, C.byref(total)) != 0:
+            self._fail()
+        return total.value
 
     def generate_greedy(self, first_token: int, steps: int, want_logits: bool = False):
         """`steps` greedy tokens without a host round trip per token (arg-max on the device, lowest id on ties)."""

@@ -227,6 +227,12 @@ int brisk_cuda_generate_greedy(brisk_cuda_session* session, int32_t first_token,
  * from vocab * 4 bytes to k * 8. k: 1..64 (and at most the vocabulary size); k = 1 is the greedy pick. */
 int brisk_cuda_eval_topk(brisk_cuda_session* session, const int32_t* tokens, uint64_t n, uint32_t k, int32_t* out_ids, float* out_values);
 
+/* Engine::log_likelihood (src/engine.cpp:10-33): appends the n >= 2 tokens and returns, in *out, the sum over i >= 1 of
+ * log p(tokens[i] | tokens[..i]). The logits stay on the device; each position sends back its log-probability. The
+ * reference walks the text in eval_all chunks of `chunk` (1 to 64) tokens: an id out of range or a context that runs out
+ * fails here too with the chunks before the failing one appended. */
+int brisk_cuda_log_likelihood(brisk_cuda_session* session, const int32_t* tokens, uint64_t n, uint32_t chunk, double* out);
+
 int brisk_cuda_get_stats(const brisk_cuda_session* session, brisk_cuda_stats* out);
 
 /* Test hook, the counterpart of metal_matmul (src/metal/metal_session.h:39-47): out[t*rows + r] =

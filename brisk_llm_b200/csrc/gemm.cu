@@ -1,230 +1,372 @@
-// Batched multiply for prompt processing: int8 tensor-core MMA on Q8_0-quantised activations, with the reference's
-// per-block arithmetic kept intact.
+// Multiply of a few to many tokens by Q4_0 / Q8_0 matrices: int8 tensor-core MMA on Q8_0-quantised activations, with the
+// reference's per-block arithmetic kept intact.
 //
-// For Q4_0 / Q8_0 weights the reference computes, per (row, token), sum over 32-value blocks IN ORDER of
-// float(int_dot) * d_w * d_x (src/quant.cpp:445-482). Here one m16n8k32 s8 MMA yields the 16x8 integer block dots of
-// a tile; each thread then scales its four results (two separate f32 multiplies) and adds them to f32 accumulators it
-// alone owns, walking the blocks in order - the same sequence of roundings as the CPU, so results are bit-identical
-// and the next 8-bit re-quantisation sees the same values. K is never split across threads. Q4_0's nibbles are
-// widened in registers (the low nibbles of a 4-byte word are exactly the MMA fragment for k = 4t..4t+3, the high
-// nibbles the fragment for k = 16+4t..) and its -8 offset is taken off the fragment once, four bytes at a time, so the
-// integer block dot comes out of the MMA complete. The MMA's C operand is the constant 0x4B400000 - the bit pattern of
-// the float 1.5 * 2^23 - so that each result, read as a float, is exactly 1.5 * 2^23 + dot (|dot| <= 32 * 127 * 127 <
-// 2^22): one exact f32 subtraction stands in for the integer-to-float conversion and nothing is zeroed between MMAs.
+// The reference computes, per (row, token), the sum over 32-value blocks IN ORDER of float(int_dot) * d_w * d_x
+// (src/quant.cpp:445-482). One m16n8k32 s8 MMA yields the integer block dots of 16 tokens x 8 rows; each thread scales
+// the dots it holds and adds them to f32 accumulators it alone owns, walking the blocks in order - the same sequence of
+// roundings as the CPU, so results are bit-identical and the next 8-bit re-quantisation sees the same values. K is never
+// split across threads.
 //
-// Tiling: CTA = 128 rows x 64 tokens, 8 warps of 32 x 32 - or, for matrices with so few rows that such tiles would leave
-// half of the SMs idle, 64 rows x 64 tokens with warps of 16 x 32; weights, activations and their scales are staged through
-// shared memory with cp.async, two stages of 8 blocks (256 columns). Padding of 16 bytes per row keeps the fragment
-// reads bank-conflict free. The per-block rescale (5 ALU instructions per output and block) bounds the kernel, not the
-// tensor pipe: that is the price of integer-exact semantics.
+// Bound: the f32 pipe. A term costs three roundings the reference makes (dot * d_w, * d_x, + sum), and nothing else may
+// go through that pipe if the rest is to keep out of the way:
+//   - the MMA's C operand is the bit pattern of 1.5 * 2^23, so a result read as a float is 1.5 * 2^23 + dot exactly, and
+//     fma(result, d_w, -1.5 * 2^23 * d_w) is dot * d_w rounded once (the addend has 13 significant bits: it is exact) -
+//     conversion and first multiply in one instruction;
+//   - packed f32x2 instructions work on two outputs each. They do not raise the f32 rate (measured: 0.49 of them per
+//     cycle and scheduler against 0.98 scalar ones) but halve the issue slots, which the fragment loads and MMAs need. The
+//     sum is an fma by 1.0 taken from the kernel's parameters: a packed multiply feeding a packed add is contracted into
+//     one fused multiply-add by the assembler, and the reference does not fuse;
+//   - tokens are the MMA's M side and weight rows its N side, so a thread's packed pair is two rows of one token: the pair
+//     of weight scales is what two adjacent scale rows hold, and the token's scale is one value twice;
+//   - Q4_0 nibbles become signed bytes as 16 * (q - 8) - the nibble in the byte's upper half with its top bit flipped: one
+//     logic operation for four weights. Sums come out 16 times as large, exactly, and are scaled once at the end.
+//
+// Tiling: a CTA of four warps side by side along the rows; a warp covers 16 MI tokens x 8 NI rows (big tiles reuse
+// fragments, small ones fill the GPU; the rule is at pick_tile). Weights, activations and their scales come through a ring
+// of cp.async stages of four blocks. Row pitches carry 16 bytes of padding: fragment reads are conflict-free. For a
+// gate/up pair half of a warp's rows are gate rows and half the up rows at the same place, and the activation is applied
+// in the epilogue. Measured: 4096 x 14336 Q4_0 at 512 tokens 282 -> 225 us (134 TMAC/s), 1024 x 3072 25 -> 19 us; at 9
+// tokens 43 -> 30 us (and 14336 x 4096 35 -> 23 us) against a kernel whose warps split a stage and add terms up through
+// shared memory.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 
+#include "formats.cuh"
 #include "kernels.h"
 
 namespace bk {
 namespace {
 
-constexpr int GN = 64, KB = 8, GWARPS = 8;  // GM, the rows of a CTA tile, is 64 * MI (MI = 16-row MMA tiles per warp)
+constexpr int KB = 4, GWARPS = 4;  // blocks per stage, warps per CTA
 
-template <int WBYTES, int GM>  // bytes of quants per block and row: 16 (Q4_0) or 32 (Q8_0); rows of the CTA tile
+// One stage of a CTA tile of RT rows x TT tokens; WB: bytes of quants per block and row, 16 (Q4_0) or 32 (Q8_0).
+template <int WB, int RT, int TT>
 struct Stage {
-    static constexpr int kARow = KB * WBYTES + 16;
-    static constexpr int kBRow = KB * 32 + 16;
-    static constexpr int kA = GM * kARow;         // weight quants
-    static constexpr int kAd = GM * KB * 2;       // weight scales (f16)
-    static constexpr int kB = GN * kBRow;         // activation quants
-    static constexpr int kBd = GN * KB * 4;       // activation scales (f32)
-    static constexpr int kBytes = kA + kAd + kB + kBd;
+    static constexpr int kWRow = KB * WB + 16;
+    static constexpr int kXRow = KB * 32 + 16;
+    static constexpr int kW = RT * kWRow;
+    static constexpr int kWd = RT * KB * 2;  // weight scales [row][block], f16
+    static constexpr int kX = TT * kXRow;
+    static constexpr int kXd = TT * KB * 4;  // activation scales [token][block], f32
+    static constexpr int kBytes = kW + kWd + kX + kXd;
 };
 
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem) {
-    const uint32_t a = uint32_t(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(a), "l"(gmem) : "memory");
+struct GemmParams {
+    DevMatrix m[3];
+    float* out[3];
+    uint32_t ldo[3];
+    uint32_t first_tile[4];  // row tiles of target i: [first_tile[i], first_tile[i + 1])
+    DevAct act;
+    uint32_t n;
+    int count, epi;
+    float one;  // 1.0f
+};
+
+__device__ __forceinline__ void cp_async8(uint32_t smem, const void* gmem) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async16(uint32_t smem, const void* gmem) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem), "l"(gmem) : "memory");
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-    const uint32_t a = uint32_t(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(a), "l"(gmem) : "memory");
-}
-
-constexpr int kMagicBits = 0x4B400000;     // 1.5 * 2^23 as a float
+constexpr int kMagicBits = 0x4B400000;  // 1.5 * 2^23 as a float; |dot| <= 16 * 32 * 8 * 127 or 32 * 128 * 127, both < 2^22
 constexpr float kMagic = 12582912.0f;
 
 // d = a x b + kMagicBits in every element
-__device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+__device__ __forceinline__ void mma_s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
         : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(kMagicBits));
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(kMagicBits));
+}
+__device__ __forceinline__ void ldmatrix4(uint32_t (&r)[4], uint32_t addr) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+template <class T> __device__ __forceinline__ T lds(uint32_t addr);
+template <> __device__ __forceinline__ uint32_t lds<uint32_t>(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
+}
+template <> __device__ __forceinline__ float lds<float>(uint32_t addr) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(addr) : "memory");
+    return v;
+}
+template <> __device__ __forceinline__ uint4 lds<uint4>(uint32_t addr) {
+    uint4 v;
+    asm volatile("ld.shared.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+    return v;
 }
 
-// Two f32 operations per instruction (packed f32x2, IEEE round-to-nearest in each half: the same results as two scalar
-// instructions). Not used for the final addition: a mul.rn.f32x2 whose only use is an add.rn.f32x2 is contracted into a
-// fused multiply-add by the assembler (measured), and the reference does not fuse.
 using f32x2 = unsigned long long;
 __device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
 __device__ __forceinline__ f32x2 pack2(int a, int b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
 __device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { f32x2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 __device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
-// Two outputs of one row (token columns 2t and 2t + 1): each block's term added to its running sum in the reference's order,
-// (float(dot) * d_w) * d_x, then the add.
-__device__ __forceinline__ void add_terms(float& acc0, float& acc1, int biased0, int biased1, f32x2 dw2, f32x2 dx2) {
-    float t0, t1;
-    unpack2(mul2(mul2(sub2(pack2(biased0, biased1), pack2(kMagic, kMagic)), dw2), dx2), t0, t1);
-    acc0 = __fadd_rn(acc0, t0);
-    acc1 = __fadd_rn(acc1, t1);
-}
-
-struct GemmParams {
-    DevMatrix m;
-    DevAct act;
-    float* out;
-    uint32_t ldo, n;
-    int epi;  // EPI_STORE or EPI_ADD
-};
-
-template <int WBYTES, int MI>
-__global__ void __launch_bounds__(GWARPS * 32, 2) gemm_q8_kernel(const GemmParams p) {
-    constexpr int GM = 64 * MI;
-    using S = Stage<WBYTES, GM>;
+template <int WB, int MI, int NI, bool PAIR, int STAGES, int MINB>
+__global__ void __launch_bounds__(GWARPS * 32, MINB) gemm_q8_kernel(const __grid_constant__ GemmParams p) {
+    constexpr int RT = GWARPS * 8 * NI, TT = 16 * MI, THREADS = GWARPS * 32;
+    using S = Stage<WB, RT, TT>;
     extern __shared__ __align__(16) unsigned char smem[];
+    const uint32_t sbase = uint32_t(__cvta_generic_to_shared(smem));
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t g = lane >> 2, t = lane & 3;
-    const uint32_t row_base = blockIdx.x * GM, tok_base = blockIdx.y * GN;
-    const uint32_t wr = (warp & 3) * (16 * MI), wt = (warp >> 2) * 32;  // this warp's (16 MI) x 32 corner inside the CTA tile
-    const uint32_t nb = p.m.blocks;                              // 32-value blocks per row
-    // Rows are walked in chunks of KB blocks. A row whose block count is a multiple of 4 but not of 8 (1152 or 896 values)
-    // ends in a chunk of 4 blocks: its other 4 are neither loaded nor multiplied, so every output is still the sum over
-    // its own blocks in order.
-    const uint32_t chunks = (nb + KB - 1) / KB;
-    const bool aligned8 = nb % KB == 0;  // else the f16 scale rows start on 8-byte, not 16-byte, boundaries
+    const uint32_t tok_base = blockIdx.x * TT;
+    int target = 0;
+    if (!PAIR) {
+        if (p.count > 1 && blockIdx.y >= p.first_tile[1]) target = 1;
+        if (p.count > 2 && blockIdx.y >= p.first_tile[2]) target = 2;
+    }
+    const DevMatrix& m = p.m[target];
+    const uint32_t nb = m.blocks, chunks = nb / KB;
+    // Rows of the tile: RT of one matrix, or (pair) RT / 2 of the gate matrix and the same RT / 2 of the up matrix.
+    const uint32_t row_base = (blockIdx.y - p.first_tile[target]) * (PAIR ? RT / 2 : RT);
 
-    auto stage_ptr = [&](int s) { return smem + size_t(s) * S::kBytes; };
-    auto load_stage = [&](int s, uint32_t chunk) {
-        unsigned char* base = stage_ptr(s);
-        const uint32_t b0 = chunk * KB;
-        const uint32_t valid = min(uint32_t(KB), nb - b0);  // blocks of this chunk that exist: KB, or 4 in a short last chunk
-        // weights: GM rows x KB*WBYTES bytes, 16-byte pieces
-        constexpr int kPiecesA = KB * WBYTES / 16;
-        for (uint32_t i = tid; i < GM * kPiecesA; i += GWARPS * 32) {
-            const uint32_t r = i / kPiecesA, piece = i % kPiecesA;
-            if (piece * 16 >= valid * WBYTES) continue;
-            const uint32_t row = min(row_base + r, p.m.rows - 1);
-            cp_async16(base + r * S::kARow + piece * 16, p.m.qa + (size_t(row) * nb + b0) * WBYTES + piece * 16);
+    // What this thread copies into every stage: 16-byte pieces of quants, an 8-byte run of weight scales, 16 bytes of
+    // activation scales. The places are worked out once; a stage advances them by a constant.
+    constexpr int kWParts = KB * WB / 16;                                      // pieces per row and stage
+    constexpr int kWPieces = (RT * kWParts + THREADS - 1) / THREADS, kXPieces = TT * 8 / THREADS;
+    static_assert(RT * kWParts % THREADS == 0 && TT * 8 % THREADS == 0 && RT <= THREADS && TT <= THREADS, "whole pieces per thread");
+    const uint8_t* wsrc[kWPieces];
+    const int8_t* xsrc[kXPieces];
+    auto row_of = [&](uint32_t r, const DevMatrix*& mat) {  // tile row r -> its matrix and row there (clamped)
+        mat = &m;
+        uint32_t row = row_base + r;
+        if (PAIR && r >= RT / 2) {
+            mat = &p.m[1];
+            row -= RT / 2;
         }
-        for (uint32_t r = tid; r < GM; r += GWARPS * 32) {
-            const uint32_t row = min(row_base + r, p.m.rows - 1);
-            const __half* src = p.m.d + size_t(row) * nb + b0;
-            unsigned char* dst = base + S::kA + r * KB * 2;
-            if (aligned8) {
-                cp_async16(dst, src);
-            } else {
-                cp_async8(dst, src);
-                if (valid > 4) cp_async8(dst + 8, src + 4);
-            }
+        return min(row, m.rows - 1);
+    };
+#pragma unroll
+    for (int i = 0; i < kWPieces; ++i) {
+        const uint32_t at = tid + i * THREADS, r = at / kWParts;
+        const DevMatrix* mat;
+        const uint32_t row = row_of(r, mat);
+        wsrc[i] = mat->qa + size_t(row) * nb * WB + (at % kWParts) * 16;
+    }
+#pragma unroll
+    for (int i = 0; i < kXPieces; ++i) {
+        const uint32_t at = tid + i * THREADS, tok = min(tok_base + at / 8, p.n - 1);
+        xsrc[i] = p.act.q0 + size_t(tok) * p.act.cols + (at % 8) * 16;
+    }
+    const __half* dsrc = nullptr;
+    if (tid < RT) {
+        const DevMatrix* mat;
+        const uint32_t row = row_of(tid, mat);
+        dsrc = mat->d + size_t(row) * nb;
+    }
+    const float* xdsrc = p.act.d0 + size_t(min(tok_base + tid % TT, p.n - 1)) * nb;
+    auto load_stage = [&](uint32_t slot, uint32_t chunk) {
+        const uint32_t at = sbase + slot * S::kBytes;
+#pragma unroll
+        for (int i = 0; i < kWPieces; ++i) {
+            const uint32_t piece = tid + i * THREADS;
+            cp_async16(at + piece / kWParts * S::kWRow + piece % kWParts * 16, wsrc[i] + size_t(chunk) * (KB * WB));
         }
-        unsigned char* bq = base + S::kA + S::kAd;
-        for (uint32_t i = tid; i < GN * (KB * 2); i += GWARPS * 32) {
-            const uint32_t r = i / (KB * 2), piece = i % (KB * 2);
-            if (piece >= valid * 2) continue;
-            const uint32_t tok = min(tok_base + r, p.n - 1);
-            cp_async16(bq + r * S::kBRow + piece * 16, p.act.q0 + size_t(tok) * p.act.cols + b0 * 32 + piece * 16);
+        if (tid < RT) cp_async8(at + S::kW + tid * (KB * 2), dsrc + size_t(chunk) * KB);
+#pragma unroll
+        for (int i = 0; i < kXPieces; ++i) {
+            const uint32_t piece = tid + i * THREADS;
+            cp_async16(at + S::kW + S::kWd + piece / 8 * S::kXRow + piece % 8 * 16, xsrc[i] + size_t(chunk) * (KB * 32));
         }
-        unsigned char* bd = bq + S::kB;
-        for (uint32_t i = tid; i < GN * 2; i += GWARPS * 32) {
-            const uint32_t r = i >> 1, piece = i & 1;
-            if (piece * 4 >= valid) continue;
-            const uint32_t tok = min(tok_base + r, p.n - 1);
-            cp_async16(bd + r * KB * 4 + piece * 16, p.act.d0 + size_t(tok) * nb + b0 + piece * 4);
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
+        if (tid < TT) cp_async16(at + S::kW + S::kWd + S::kX + tid * (KB * 4), xdsrc + size_t(chunk) * KB);
     };
 
-    float acc[MI][4][4];
+    f32x2 acc[MI][NI][2];  // [..][0]: rows 2t, 2t + 1 of token g, [..][1]: of token g + 8
 #pragma unroll
     for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
-#pragma unroll
-            for (int j = 0; j < 4; ++j) acc[mi][ni][j] = 0.0f;
+        for (int ni = 0; ni < NI; ++ni) acc[mi][ni][0] = acc[mi][ni][1] = 0ull;
+    const f32x2 one2 = pack2(p.one, p.one), minus_magic2 = pack2(-kMagic, -kMagic);
+    // first tile row of this warp's row tile ni
+    auto tile_row = [&](int ni) -> uint32_t {
+        if constexpr (PAIR) return (ni / (NI / 2)) * (RT / 2) + warp * (4 * NI) + (ni % (NI / 2)) * 8;
+        else return warp * (8 * NI) + ni * 8;
+    };
 
-    load_stage(0, 0);
+#pragma unroll
+    for (int s = 0; s < STAGES - 1; ++s) {
+        if (uint32_t(s) < chunks) load_stage(s, s);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    uint32_t slot = 0, fill = STAGES - 1;
     for (uint32_t chunk = 0; chunk < chunks; ++chunk) {
-        if (chunk + 1 < chunks) {
-            load_stage((chunk + 1) & 1, chunk + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();
-        const unsigned char* base = stage_ptr(chunk & 1);
-        const unsigned char* aq = base;
-        const __half* ad = reinterpret_cast<const __half*>(base + S::kA);
-        const unsigned char* bq = base + S::kA + S::kAd;
-        const float* bd = reinterpret_cast<const float*>(bq + S::kB);
-        const int valid = int(min(uint32_t(KB), nb - chunk * KB));
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        __syncthreads();  // the stage has landed for every thread, and the slot filled next is no longer read
+        if (chunk + STAGES - 1 < chunks) load_stage(fill, chunk + STAGES - 1);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        fill = fill + 1 == STAGES ? 0 : fill + 1;
+        const uint32_t at = sbase + slot * S::kBytes;
+        slot = slot + 1 == STAGES ? 0 : slot + 1;
+
+        uint4 dw[NI];  // scales of rows 2t and 2t + 1, four blocks each
+#pragma unroll
+        for (int ni = 0; ni < NI; ++ni) dw[ni] = lds<uint4>(at + S::kW + (tile_row(ni) + 2 * t) * (KB * 2));
+        const uint32_t xfrag = at + S::kW + S::kWd + ((lane & 7) + ((lane >> 3) & 1) * 8) * S::kXRow + (lane >> 4) * 16;
+        const uint32_t xscale = at + S::kW + S::kWd + S::kX + g * (KB * 4);
+        const uint32_t wfrag = at + g * S::kWRow + 4 * t;
 #pragma unroll
         for (int b = 0; b < KB; ++b) {
-            if (b >= 4 && valid <= 4) continue;  // the short last chunk of a row of 8k + 4 blocks
             uint32_t a[MI][4];
-            f32x2 dw2[MI][2];  // each row's weight scale, twice (for the row's two token columns)
+            f32x2 dx2[MI][2];
 #pragma unroll
             for (int mi = 0; mi < MI; ++mi) {
-                const uint32_t r0 = wr + mi * 16 + g, r1 = r0 + 8;
-                if (WBYTES == 16) {
-                    const uint32_t w0 = *reinterpret_cast<const uint32_t*>(aq + r0 * S::kARow + b * 16 + 4 * t);
-                    const uint32_t w1 = *reinterpret_cast<const uint32_t*>(aq + r1 * S::kARow + b * 16 + 4 * t);
-                    a[mi][0] = __vsub4(w0 & 0x0F0F0F0Fu, 0x08080808u);
-                    a[mi][1] = __vsub4(w1 & 0x0F0F0F0Fu, 0x08080808u);
-                    a[mi][2] = __vsub4((w0 >> 4) & 0x0F0F0F0Fu, 0x08080808u);
-                    a[mi][3] = __vsub4((w1 >> 4) & 0x0F0F0F0Fu, 0x08080808u);
-                } else {
-                    a[mi][0] = *reinterpret_cast<const uint32_t*>(aq + r0 * S::kARow + b * 32 + 4 * t);
-                    a[mi][1] = *reinterpret_cast<const uint32_t*>(aq + r1 * S::kARow + b * 32 + 4 * t);
-                    a[mi][2] = *reinterpret_cast<const uint32_t*>(aq + r0 * S::kARow + b * 32 + 16 + 4 * t);
-                    a[mi][3] = *reinterpret_cast<const uint32_t*>(aq + r1 * S::kARow + b * 32 + 16 + 4 * t);
-                }
-                const float d0 = __half2float(ad[r0 * KB + b]), d1 = __half2float(ad[r1 * KB + b]);
-                dw2[mi][0] = pack2(d0, d0);
-                dw2[mi][1] = pack2(d1, d1);
+                ldmatrix4(a[mi], xfrag + mi * 16 * S::kXRow + b * 32);
+                const float d0 = lds<float>(xscale + (mi * 16) * (KB * 4) + b * 4), d1 = lds<float>(xscale + (mi * 16 + 8) * (KB * 4) + b * 4);
+                dx2[mi][0] = pack2(d0, d0);
+                dx2[mi][1] = pack2(d1, d1);
             }
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni) {
-                const uint32_t tb = wt + ni * 8;
-                const uint32_t b0 = *reinterpret_cast<const uint32_t*>(bq + (tb + g) * S::kBRow + b * 32 + 4 * t);
-                const uint32_t b1 = *reinterpret_cast<const uint32_t*>(bq + (tb + g) * S::kBRow + b * 32 + 16 + 4 * t);
-                const uint32_t c0 = tb + 2 * t, c1 = c0 + 1;  // the two token columns this thread's results belong to
-                const f32x2 dx2 = pack2(bd[c0 * KB + b], bd[c1 * KB + b]);
+            for (int ni = 0; ni < NI; ++ni) {
+                uint32_t b0, b1;
+                if (WB == 16) {
+                    const uint32_t w = lds<uint32_t>(wfrag + tile_row(ni) * S::kWRow + b * 16);
+                    b0 = ((w << 4) ^ 0x80808080u) & 0xF0F0F0F0u;
+                    b1 = (w ^ 0x80808080u) & 0xF0F0F0F0u;
+                } else {
+                    b0 = lds<uint32_t>(wfrag + tile_row(ni) * S::kWRow + b * 32);
+                    b1 = lds<uint32_t>(wfrag + tile_row(ni) * S::kWRow + b * 32 + 16);
+                }
+                const uint32_t lo = b < 2 ? dw[ni].x : dw[ni].y, hi = b < 2 ? dw[ni].z : dw[ni].w;
+                const f32x2 dw2 = pack2(__half2float(__ushort_as_half(uint16_t(b & 1 ? lo >> 16 : lo & 0xFFFF))),
+                                        __half2float(__ushort_as_half(uint16_t(b & 1 ? hi >> 16 : hi & 0xFFFF))));
+                const f32x2 off2 = mul2(dw2, minus_magic2);
 #pragma unroll
                 for (int mi = 0; mi < MI; ++mi) {
                     int c[4];
-                    mma_s8(c, a[mi][0], a[mi][1], a[mi][2], a[mi][3], b0, b1);
-                    // (row g, col 2t) (row g, col 2t+1) (row g+8, col 2t) (row g+8, col 2t+1)
-                    add_terms(acc[mi][ni][0], acc[mi][ni][1], c[0], c[1], dw2[mi][0], dx2);
-                    add_terms(acc[mi][ni][2], acc[mi][ni][3], c[2], c[3], dw2[mi][1], dx2);
+                    mma_s8(c, a[mi], b0, b1);
+                    acc[mi][ni][0] = fma2(mul2(fma2(pack2(c[0], c[1]), dw2, off2), dx2[mi][0]), one2, acc[mi][ni][0]);
+                    acc[mi][ni][1] = fma2(mul2(fma2(pack2(c[2], c[3]), dw2, off2), dx2[mi][1]), one2, acc[mi][ni][1]);
                 }
             }
         }
-        __syncthreads();  // the stage is free for the load issued two iterations from now
     }
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
 
+    constexpr float kScale = WB == 16 ? 0.0625f : 1.0f;  // exact
+    float* const out = p.out[target];
+    const uint32_t ldo = p.ldo[target];
+    const bool even = (ldo & 1) == 0;
 #pragma unroll
     for (int mi = 0; mi < MI; ++mi) {
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni) {
+        for (int half = 0; half < 2; ++half) {
+            const uint32_t tok = tok_base + mi * 16 + half * 8 + g;
+            if (tok >= p.n) continue;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const uint32_t row = row_base + wr + mi * 16 + g + (j >= 2 ? 8 : 0);
-                const uint32_t tok = tok_base + wt + ni * 8 + 2 * t + (j & 1);
-                if (row < p.m.rows && tok < p.n) {
-                    float* o = p.out + size_t(tok) * p.ldo + row;
-                    *o = p.epi == EPI_ADD ? __fadd_rn(*o, acc[mi][ni][j]) : acc[mi][ni][j];
+            for (int ni = 0; ni < (PAIR ? NI / 2 : NI); ++ni) {
+                const uint32_t row = row_base + tile_row(ni) + 2 * t;
+                if (row >= m.rows) continue;
+                float v0, v1;
+                unpack2(acc[mi][ni][half], v0, v1);
+                v0 *= kScale;
+                v1 *= kScale;
+                if constexpr (PAIR) {
+                    float u0, u1;
+                    unpack2(acc[mi][ni + NI / 2][half], u0, u1);
+                    u0 *= kScale;
+                    u1 *= kScale;
+                    v0 = p.epi == EPI_SILU_MUL ? silu_mul(v0, u0) : relu2_mul(v0, u0);
+                    v1 = p.epi == EPI_SILU_MUL ? silu_mul(v1, u1) : relu2_mul(v1, u1);
+                }
+                float* o = out + size_t(tok) * ldo + row;
+                if (even && row + 1 < m.rows) {
+                    float2 v = make_float2(v0, v1);
+                    if (p.epi == EPI_ADD) {
+                        const float2 old = *reinterpret_cast<const float2*>(o);
+                        v = make_float2(__fadd_rn(old.x, v0), __fadd_rn(old.y, v1));
+                    }
+                    *reinterpret_cast<float2*>(o) = v;
+                } else {
+                    o[0] = p.epi == EPI_ADD ? __fadd_rn(o[0], v0) : v0;
+                    if (row + 1 < m.rows) o[1] = p.epi == EPI_ADD ? __fadd_rn(o[1], v1) : v1;
                 }
             }
         }
     }
+}
+
+// A tile shape and what it costs: cycles of one block of its K loop when nothing shares the scheduler (the dependent
+// chain fragment - MMA - three roundings) and when the scheduler is full (issue and f32 pipe), measured on B200 with the
+// 4096 x 14336 Q4_0 matrix at 9 to 512 tokens.
+struct Tile {
+    int mi, ni, alone, shared, resident;
+    void (*kernel)(GemmParams);
+    uint32_t smem;
+    uint32_t rows() const { return uint32_t(GWARPS * 8 * ni); }
+    uint32_t tokens() const { return uint32_t(16 * mi); }
+};
+
+template <int WB, bool PAIR, int MI, int NI, int STAGES, int RESIDENT>
+Tile tile_of(int alone, int shared) {
+    return Tile{MI, NI, alone, shared, RESIDENT, gemm_q8_kernel<WB, MI, NI, PAIR, STAGES, RESIDENT>, uint32_t(STAGES * Stage<WB, GWARPS * 8 * NI, 16 * MI>::kBytes)};
+}
+template <int WB, bool PAIR>
+const std::vector<Tile>& tiles_of() {
+    static const std::vector<Tile> list = [] {
+        std::vector<Tile> v = {tile_of<WB, PAIR, 4, 2, 3, 3>(305, 240), tile_of<WB, PAIR, 2, 2, 5, 4>(210, 135), tile_of<WB, PAIR, 1, 2, 6, 6>(166, 90)};
+        if constexpr (!PAIR) {
+            v.push_back(tile_of<WB, PAIR, 2, 1, 5, 4>(186, 79));
+            v.push_back(tile_of<WB, PAIR, 1, 1, 8, 5>(127, 52));
+        }
+        return v;
+    }();
+    return list;
+}
+
+// The tile whose busiest SM is done first: it runs ceil(tiles / SMs) CTAs, `resident` of them at a time, and a round of
+// CTAs takes the longer of one warp's chain and what the scheduler's warps need together. Few rows or tokens favour small
+// tiles (1024 x 2048 at 23 tokens: 6.4 us against 14.6 with the largest), a full GPU large ones (4096 x 14336 at 512
+// tokens: 225 us against 351 with the smallest).
+const Tile& pick_tile(const std::vector<Tile>& list, const GemmParams& p, bool pair, uint32_t sms) {
+    const Tile* best = nullptr;
+    uint64_t best_cost = 0;
+    for (const Tile& tile : list) {
+        uint64_t tiles = 0;
+        const uint32_t rows = pair ? tile.rows() / 2 : tile.rows();
+        for (int i = 0; i < (pair ? 1 : p.count); ++i) tiles += (p.m[i].rows + rows - 1) / rows;
+        tiles *= (p.n + tile.tokens() - 1) / tile.tokens();
+        const uint64_t per_sm = (tiles + sms - 1) / sms, rounds = (per_sm + tile.resident - 1) / tile.resident;
+        const uint64_t cost = std::max<uint64_t>(rounds * uint64_t(tile.alone), per_sm * uint64_t(tile.shared));
+        if (best == nullptr || cost < best_cost) {
+            best = &tile;
+            best_cost = cost;
+        }
+    }
+    return *best;
+}
+
+template <int WB, bool PAIR>
+void launch_q8(GemmParams& p, uint32_t sms, cudaStream_t s) {
+    static DeviceOnce once;
+    if (once.first()) {
+        for (const Tile& tile : tiles_of<WB, PAIR>()) {
+            BK_CUDA(cudaFuncSetAttribute(tile.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile.smem)));
+            BK_CUDA(cudaFuncSetAttribute(tile.kernel, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
+        }
+    }
+    const Tile& tile = pick_tile(tiles_of<WB, PAIR>(), p, PAIR, sms);
+    uint32_t tiles = 0;
+    const uint32_t rows = PAIR ? tile.rows() / 2 : tile.rows();
+    for (int i = 0; i < (PAIR ? 1 : p.count); ++i) {
+        p.first_tile[i] = tiles;
+        tiles += (p.m[i].rows + rows - 1) / rows;
+    }
+    tile.kernel<<<dim3((p.n + tile.tokens() - 1) / tile.tokens(), tiles), GWARPS * 32, tile.smem, s>>>(p);
+    BK_CUDA(cudaGetLastError());
+}
+
+uint32_t sm_count() {
+    static const uint32_t sms = [] {
+        int dev = 0, count = 148;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+        return uint32_t(count);
+    }();
+    return sms;
 }
 
 }  // namespace
@@ -240,57 +382,41 @@ static bool gemm_tc_on() {
 bool gemm_k_supports(int type);  // gemm_k.cu: the 256-value super-block formats
 void launch_gemm_k(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s);
 
-// Q4_0 / Q8_0 rows of a multiple of 4 blocks (128 values): whole chunks of 8 blocks plus, at most, one chunk of 4.
-bool gemm_supports(int type, uint32_t cols) { return ((type == T_Q4_0 || type == T_Q8_0) && cols % 128 == 0) || gemm_k_supports(type); }
-
-// out = weights x activations for one target (EPI_STORE / EPI_ADD).
-template <int WBYTES, int MI>
-static void launch_gemm_tile(const GemmParams& p, cudaStream_t s) {
-    constexpr int GM = 64 * MI;
-    constexpr size_t smem = 2 * Stage<WBYTES, GM>::kBytes;
-    static DeviceOnce once;
-    if (once.first()) {
-        BK_CUDA(cudaFuncSetAttribute(gemm_q8_kernel<WBYTES, MI>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-        BK_CUDA(cudaFuncSetAttribute(gemm_q8_kernel<WBYTES, MI>, cudaFuncAttributePreferredSharedMemoryCarveout, 100));
-    }
-    const dim3 grid((p.m.rows + GM - 1) / GM, (p.n + GN - 1) / GN);
-    gemm_q8_kernel<WBYTES, MI><<<grid, GWARPS * 32, smem, s>>>(p);
-    BK_CUDA(cudaGetLastError());
+// Q4_0 / Q8_0 rows of a multiple of 4 blocks (128 values) from 2 tokens on; the super-block formats from 16 on.
+static bool gemm_supports(int type, uint32_t cols, uint32_t n) {
+    if (type == T_Q4_0 || type == T_Q8_0) return cols % (32 * KB) == 0 && n >= 2;
+    return gemm_k_supports(type) && n >= kGemmMinTokens;
 }
 
-static void launch_gemm_one(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s) {
-    if (n >= 32 && gemm_tc_on() && gemm_tc_supports(tg.m.type, tg.m.cols)) {
-        launch_gemm_tc(tg, act, n, epi, s);
-        return;
+int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s) {
+    const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
+    for (int i = 0; i < count; ++i) {
+        if (!gemm_supports(targets[i].m.type, targets[i].m.cols, n)) return 0;
     }
-    const GemmParams p{tg.m, act, tg.out, tg.ldo, n, int(epi)};
-    static const int sms = [] {
-        int dev = 0, count = 148;
-        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+    const int type = targets[0].m.type;
+    if (type != T_Q4_0 && type != T_Q8_0) {
+        if (pair) return 0;
+        for (int i = 0; i < count; ++i) launch_gemm_k(targets[i], act, n, epi, s);
         return count;
-    }();
-    // 128-row tiles unless they would leave SMs without a CTA: then 64-row tiles, twice as many CTAs
-    const uint32_t big_tiles = ((tg.m.rows + 127) / 128) * ((n + GN - 1) / GN);
-    const bool small = big_tiles < uint32_t(sms);
-    if (tg.m.type == T_Q4_0) {
-        if (small) launch_gemm_tile<16, 1>(p, s);
-        else launch_gemm_tile<16, 2>(p, s);
-    } else {
-        if (small) launch_gemm_tile<32, 1>(p, s);
-        else launch_gemm_tile<32, 2>(p, s);
     }
-}
-
-bool launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s) {
-    if (epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL) return false;  // the caller runs gate and up separately, then launch_gate_mul
+    if (!pair && n >= 32 && gemm_tc_on() && gemm_tc_supports(type, targets[0].m.cols)) {
+        for (int i = 0; i < count; ++i) launch_gemm_tc(targets[i], act, n, epi, s);
+        return count;
+    }
+    GemmParams p{};
     for (int i = 0; i < count; ++i) {
-        if (!gemm_supports(targets[i].m.type, targets[i].m.cols)) return false;
+        p.m[i] = targets[i].m;
+        p.out[i] = targets[i].out;
+        p.ldo[i] = targets[i].ldo;
     }
-    for (int i = 0; i < count; ++i) {
-        if (gemm_k_supports(targets[i].m.type)) launch_gemm_k(targets[i], act, n, epi, s);
-        else launch_gemm_one(targets[i], act, n, epi, s);
-    }
-    return true;
+    p.act = act;
+    p.n = n;
+    p.count = count;
+    p.epi = int(epi);
+    p.one = 1.0f;
+    if (type == T_Q4_0) pair ? launch_q8<16, true>(p, sm_count(), s) : launch_q8<16, false>(p, sm_count(), s);
+    else pair ? launch_q8<32, true>(p, sm_count(), s) : launch_q8<32, false>(p, sm_count(), s);
+    return 1;
 }
 
 }  // namespace bk

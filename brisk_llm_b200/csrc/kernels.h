@@ -58,12 +58,6 @@ struct MatTarget {
 // goes to targets[0].out. n may exceed 8: the launcher walks token tiles.
 void launch_matvec(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s);
 
-// ---- 2..16 tokens on the int8 tensor path, weights streamed once (smallbatch.cu) ---------------------
-// Same contract as launch_matvec; returns false (nothing launched) unless the targets are Q4_0 / Q8_0 with rows of a
-// multiple of 8 blocks and 2 <= n <= kSmallBatchMax.
-constexpr uint32_t kSmallBatchMax = 16;
-bool launch_smallbatch(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s);
-
 // ---- tensor-parallel exchange of one token by peer stores (tp_peer.cu) ---------------------------------
 // bufs_dev: device array of the tp ranks' exchange buffers (2 slots of slot_pairs tagged pairs each) as mapped here;
 // this rank's [rows_l] slice goes to every rank, dst receives (or is added) the whole [rows_l * tp] vector.
@@ -72,13 +66,14 @@ void launch_tp_peer_exchange(uint2* const* bufs_dev, uint32_t* epoch, unsigned i
                              const float* local, float* dst, uint32_t rows_l, bool add, cudaStream_t s);
 
 // ---- batched multiply on the int8 tensor path (gemm.cu) ----------------------------------------
-// Same contract as launch_matvec for n >= 16 tokens; returns false when this type/shape has no tensor kernel
-// (the caller then uses launch_matvec).
-bool launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s);
+// Same contract as launch_matvec; returns the number of kernels launched, 0 when these types, shapes or token counts have
+// no tensor kernel (the caller then uses launch_matvec). The super-block formats have none for the pair epilogues: the
+// caller multiplies gate and up separately and runs launch_gate_mul.
+constexpr uint32_t kGemmMinTokens = 16;  // super-block formats: fewer tokens go through the streaming kernel
+int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s);
 // The Q4_0 / Q8_0 prompt multiply on tcgen05 / tensor memory (gemm_tc.cu; BRISK_CUDA_GEMM=tc): its waits are bounded, and this
 // word is non-zero on the device after a launch whose wait ran out.
 unsigned int* gemm_tc_error_word();
-bool gemm_supports(int type, uint32_t cols);
 // The activation after separate gate and up multiplies. mode 0: gate[i] = silu(gate[i]) * up[i]; 1: max(gate[i],0)^2 * up[i];
 // 2: tanh-GELU(gate[i]) * up[i] (gelu_mul_f32, src/kernels_f32.cpp:291-296), its tanh corrected by tanh_table (see
 // build_tanh_table) when one is given.

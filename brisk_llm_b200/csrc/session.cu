@@ -626,19 +626,16 @@ struct Session {
     // One multiply of the batched path: targets of one weight type share a launch of the streaming kernel; prompt
     // batches go to the tensor-core kernel where the type has one.
     void multiply(std::vector<MatTarget> targets, const DevAct& a, uint32_t n, Epilogue epi) {
-        const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
-        if (pair) {
-            if (small_batch_on() && launch_smallbatch(targets.data(), int(targets.size()), a, n, epi, stream)) {  // 2..16 tokens
-                ++launches;
+        if (epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL) {
+            if (const int ran = launch_gemm(targets.data(), int(targets.size()), a, n, epi, stream)) {
+                launches += ran;
                 return;
             }
-            if (n >= 16 && gemm_supports(targets[0].m.type, targets[0].m.cols)) {
-                // prompt batches: gate and up as two tensor-core multiplies, then the activation elementwise
-                MatTarget gate{targets[0].m, targets[0].out, targets[0].ldo}, up{targets[1].m, up_b.as<float>(), targets[0].ldo};
-                launch_gemm(&gate, 1, a, n, EPI_STORE, stream);
-                launch_gemm(&up, 1, a, n, EPI_STORE, stream);
+            // formats whose tensor kernel has no fused activation: gate and up as two multiplies, then the activation elementwise
+            const MatTarget both[2] = {{targets[0].m, targets[0].out, targets[0].ldo}, {targets[1].m, up_b.as<float>(), targets[0].ldo}};
+            if (const int ran = launch_gemm(both, 2, a, n, EPI_STORE, stream)) {
                 launch_gate_mul(targets[0].out, up_b.as<float>(), size_t(n) * targets[0].ldo, epi == EPI_RELU2_MUL, stream);
-                launches += 3;
+                launches += ran + 1;
                 return;
             }
             launch_matvec(targets.data(), int(targets.size()), a, n, epi, stream);
@@ -648,13 +645,11 @@ struct Session {
         while (!targets.empty()) {
             std::vector<MatTarget> same, rest;
             for (const MatTarget& t : targets) (t.m.type == targets[0].m.type ? same : rest).push_back(t);
-            if (small_batch_on() && launch_smallbatch(same.data(), int(same.size()), a, n, epi, stream)) {  // 2..16 tokens
-                ++launches;
-            } else if (!(n >= 16 && launch_gemm(same.data(), int(same.size()), a, n, epi, stream))) {
+            if (const int ran = launch_gemm(same.data(), int(same.size()), a, n, epi, stream)) {
+                launches += ran;
+            } else {
                 launch_matvec(same.data(), int(same.size()), a, n, epi, stream);
                 launches += (n + kMaxSmallBatch - 1) / kMaxSmallBatch;
-            } else {
-                launches += same.size();
             }
             targets.swap(rest);
         }
@@ -962,11 +957,6 @@ struct Session {
         ++persistent_steps;
     }
     // After the call's final synchronisation: did a barrier wait of the persistent kernel run out?
-    // BRISK_CUDA_SMALLBATCH=0 keeps the streaming kernel for 2..16 tokens (a comparison aid); read at every call
-    static bool small_batch_on() {
-        const char* env = std::getenv("BRISK_CUDA_SMALLBATCH");
-        return env == nullptr || std::atoi(env) != 0;
-    }
     void queue_step_check() {
         // the few-token attention kernel waits for bulk copies (every wait bounded): its error word, read with the call's results
         BK_CUDA(cudaMemcpyAsync(step_error_host + 2, chain_error_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));

@@ -63,57 +63,63 @@ __device__ __forceinline__ void cta_quantize_q8_0(const float* row, uint32_t col
     }
 }
 
+// One Q8_K super-block by one warp: lane l holds values 8l .. 8l + 7. `qk` and `bs` are this lane's own places (its values, the
+// sums of 16 its pair of lanes forms), `dk` the super-block's.
+__device__ __forceinline__ void warp_quantize_q8_k(const float (&vals)[8], int8_t* qk, float* dk, int16_t* bs) {
+    const uint32_t lane = threadIdx.x & 31;
+    float amax = 0.0f, ext = 0.0f;
+    uint32_t idx = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float ax = fabsf(vals[i]);
+        if (ax > amax) {
+            amax = ax;
+            ext = vals[i];
+            idx = lane * 8 + i;
+        }
+    }
+    // Largest magnitude, the earliest element on ties - what a sequential strict '>' scan finds.
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float oa = __shfl_xor_sync(0xffffffffu, amax, o);
+        const float oe = __shfl_xor_sync(0xffffffffu, ext, o);
+        const uint32_t oi = __shfl_xor_sync(0xffffffffu, idx, o);
+        if (oa > amax || (oa == amax && oi < idx)) {
+            amax = oa;
+            ext = oe;
+            idx = oi;
+        }
+    }
+    if (amax == 0.0f) {
+        *reinterpret_cast<uint2*>(qk) = make_uint2(0u, 0u);
+        if ((lane & 1) == 0) *bs = 0;
+        if (lane == 0) *dk = 0.0f;
+        return;
+    }
+    const float inv = __fdiv_rn(-127.0f, ext);
+    uint32_t w[2] = {0u, 0u};
+    int sum = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int qi = int(fminf(127.0f, rintf(__fmul_rn(inv, vals[i]))));
+        sum += qi;
+        w[i >> 2] |= uint32_t(uint8_t(int8_t(qi))) << (8 * (i & 3));
+    }
+    *reinterpret_cast<uint2*>(qk) = make_uint2(w[0], w[1]);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    if ((lane & 1) == 0) *bs = int16_t(sum);
+    if (lane == 0) *dk = __fdiv_rn(1.0f, inv);
+}
+
 // row[0..cols) -> qk (int8), dk (f32 scale per 256), bs (int16 sums of 16). One warp per 256-value super-block.
 __device__ __forceinline__ void cta_quantize_q8_k(const float* row, uint32_t cols, int8_t* qk, float* dk, int16_t* bs) {
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
     const uint32_t nb = cols / 256;
     for (uint32_t b = warp; b < nb; b += warps) {
-        const float* v = row + b * 256 + lane * 8;
         float vals[8];
-        float amax = 0.0f, ext = 0.0f;
-        uint32_t idx = 0;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            vals[i] = v[i];
-            const float ax = fabsf(vals[i]);
-            if (ax > amax) {
-                amax = ax;
-                ext = vals[i];
-                idx = lane * 8 + i;
-            }
-        }
-        // Largest magnitude, the earliest element on ties - what a sequential strict '>' scan finds.
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            const float oa = __shfl_xor_sync(0xffffffffu, amax, o);
-            const float oe = __shfl_xor_sync(0xffffffffu, ext, o);
-            const uint32_t oi = __shfl_xor_sync(0xffffffffu, idx, o);
-            if (oa > amax || (oa == amax && oi < idx)) {
-                amax = oa;
-                ext = oe;
-                idx = oi;
-            }
-        }
-        int8_t* qo = qk + b * 256 + lane * 8;
-        if (amax == 0.0f) {
-            *reinterpret_cast<uint2*>(qo) = make_uint2(0u, 0u);
-            if ((lane & 1) == 0) bs[b * 16 + (lane >> 1)] = 0;
-            if (lane == 0) dk[b] = 0.0f;
-            continue;
-        }
-        const float inv = __fdiv_rn(-127.0f, ext);
-        uint32_t w[2] = {0u, 0u};
-        int sum = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int qi = int(fminf(127.0f, rintf(__fmul_rn(inv, vals[i]))));
-            sum += qi;
-            w[i >> 2] |= uint32_t(uint8_t(int8_t(qi))) << (8 * (i & 3));
-        }
-        *reinterpret_cast<uint2*>(qo) = make_uint2(w[0], w[1]);
-        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-        if ((lane & 1) == 0) bs[b * 16 + (lane >> 1)] = int16_t(sum);
-        if (lane == 0) dk[b] = __fdiv_rn(1.0f, inv);
+        for (int i = 0; i < 8; ++i) vals[i] = row[b * 256 + lane * 8 + i];
+        warp_quantize_q8_k(vals, qk + b * 256 + lane * 8, dk + b, bs + b * 16 + (lane >> 1));
     }
 }
 

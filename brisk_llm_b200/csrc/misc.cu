@@ -211,214 +211,6 @@ __global__ void __launch_bounds__(128) qk_norm_rope_store_kernel(const RopeArgs 
     }
 }
 
-// ---- attention --------------------------------------------------------------------------------------------
-// Causal attention of token t (absolute position P + t) over cached positions 0..P+t, in the reference's own
-// order of float operations (src/model.cpp:1050-1093 over src/kernels_f32.cpp:231-284), so that the result is
-// bit-identical to the CPU engine's and the 8-bit re-quantisation that follows sees the same values:
-//   scores   s[p] = dot_f32(q, k_p) * scale, dot_f32 = 16 interleaved partial sums, then their sum in order
-//   softmax  e[p] = expf(s[p] - max) (glibc's expf, see exact_math.h), sum in f64, p[p] = e[p] * float(1/sum)
-//   output   out[i] = ((p[0]*v_0[i] + p[1]*v_1[i]) + p[2]*v_2[i]) + ...   one position after the other
-// Three kernels: scores (a thread per position, all query heads of one K/V head), softmax (a CTA per row),
-// weighted sum (a thread per output value, walking the positions in order).
-constexpr uint32_t kMaxGroup = 16;  // query heads per K/V head, at most (kMaxHeadsPerKv, src/model.h:34)
-
-// Tokens of a batch that share one pass over the cached K (or V) rows: 16 for long contexts (every tile re-reads all
-// visible rows, so fewer, larger tiles win: measured 1436 -> 956 ms of attention in an 8192-token prefill of the 7B-class
-// model), 8 for short ones (more CTAs to fill the GPU: 512-token prefill of the 0.6B-class model 50.8 k vs 49.4 k tok/s).
-constexpr uint32_t kLongContext = 1024;
-
-// grid (position chunks of 128, K/V heads, token tiles). A thread owns one cached position: it reads that K row once
-// and scores it against every (token, query head) of the tile, each score in dot_f32's order.
-template <int GROUP, int DIM, uint32_t kTokTile>
-__global__ void __launch_bounds__(128) attn_scores_kernel(const AttnArgs a) {
-    extern __shared__ float qs[];  // [kTokTile][GROUP][DIM]
-    const uint32_t kvh = blockIdx.y, t0 = blockIdx.z * kTokTile;
-    const uint32_t tn = min(kTokTile, a.n - t0);
-    const uint32_t base_visible = *a.position + t0 + 1;        // positions the tile's first token sees
-    const uint32_t last_visible = base_visible + tn - 1;       // ... and its last
-    const uint32_t p = blockIdx.x * 128 + threadIdx.x;
-    if (blockIdx.x * 128 >= last_visible) return;
-    for (uint32_t i = threadIdx.x; i < tn * GROUP * DIM; i += 128) {
-        const uint32_t j = i / (GROUP * DIM), rest = i % (GROUP * DIM);
-        qs[i] = a.q[size_t(t0 + j) * a.heads * DIM + size_t(kvh) * GROUP * DIM + rest];
-    }
-    __syncthreads();
-    if (p >= last_visible) return;
-    const uint4* kr = reinterpret_cast<const uint4*>(a.k_cache + (size_t(kvh) * a.max_context + p) * DIM);
-    // The K row stays in registers: widened to f32 up to 128 values; a 256-wide row is kept as packed halves (128 registers)
-    // and widened sixteen values at a time where it is used.
-    constexpr bool kPacked = DIM > 128;
-    float kf[kPacked ? 1 : DIM];
-    uint4 kraw[kPacked ? DIM / 8 : 1];
-#pragma unroll
-    for (int i = 0; i < DIM / 8; ++i) {
-        const uint4 raw = kr[i];
-        if constexpr (kPacked) {
-            kraw[i] = raw;
-        } else {
-            const __half2* h = reinterpret_cast<const __half2*>(&raw);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float2 f = __half22float2(h[j]);
-                kf[8 * i + 2 * j] = f.x;
-                kf[8 * i + 2 * j + 1] = f.y;
-            }
-        }
-    }
-    for (uint32_t j = 0; j < tn; ++j) {
-        if (p >= base_visible + j) continue;  // token j does not see this position
-#pragma unroll
-        for (int g = 0; g < GROUP; ++g) {
-            const float4* q4 = reinterpret_cast<const float4*>(qs + (j * GROUP + g) * DIM);
-            float lanes[16];
-#pragma unroll
-            for (int l = 0; l < 16; ++l) lanes[l] = 0.0f;
-#pragma unroll
-            for (int i = 0; i < DIM; i += 16) {
-                float kk[16];
-                if constexpr (kPacked) {
-#pragma unroll
-                    for (int u = 0; u < 2; ++u) {
-                        const uint4 raw = kraw[i / 8 + u];
-                        const __half2* h = reinterpret_cast<const __half2*>(&raw);
-#pragma unroll
-                        for (int x = 0; x < 4; ++x) {
-                            const float2 f = __half22float2(h[x]);
-                            kk[8 * u + 2 * x] = f.x;
-                            kk[8 * u + 2 * x + 1] = f.y;
-                        }
-                    }
-                } else {
-#pragma unroll
-                    for (int x = 0; x < 16; ++x) kk[x] = kf[i + x];
-                }
-#pragma unroll
-                for (int l = 0; l < 4; ++l) {
-                    const float4 q = q4[i / 4 + l];
-                    lanes[4 * l + 0] = __fadd_rn(lanes[4 * l + 0], __fmul_rn(q.x, kk[4 * l + 0]));
-                    lanes[4 * l + 1] = __fadd_rn(lanes[4 * l + 1], __fmul_rn(q.y, kk[4 * l + 1]));
-                    lanes[4 * l + 2] = __fadd_rn(lanes[4 * l + 2], __fmul_rn(q.z, kk[4 * l + 2]));
-                    lanes[4 * l + 3] = __fadd_rn(lanes[4 * l + 3], __fmul_rn(q.w, kk[4 * l + 3]));
-                }
-            }
-            float sum = 0.0f;
-#pragma unroll
-            for (int l = 0; l < 16; ++l) sum = __fadd_rn(sum, lanes[l]);
-            a.scores[(size_t(t0 + j) * a.heads + kvh * GROUP + g) * a.max_context + p] = __fmul_rn(sum, a.scale);
-        }
-    }
-}
-
-__global__ void __launch_bounds__(256) attn_softmax_kernel(const AttnArgs a) {
-    const uint32_t h = blockIdx.x, t = blockIdx.y, tid = threadIdx.x;
-    const uint32_t visible = *a.position + t + 1;
-    // a sliding-window layer normalises over the last `window` positions only (src/model.cpp:1084-1088)
-    const uint32_t start = a.window != 0 && visible > a.window ? visible - a.window : 0;
-    float* s = a.scores + (size_t(t) * a.heads + h) * a.max_context;
-    __shared__ float redf[8];
-    __shared__ double redd[8];
-    float mx = -INFINITY;
-    for (uint32_t p = start + tid; p < visible; p += 256) mx = fmaxf(mx, s[p]);
-    mx = warp_max(mx);
-    if ((tid & 31) == 0) redf[tid >> 5] = mx;
-    __syncthreads();
-    mx = redf[0];
-#pragma unroll
-    for (int w = 1; w < 8; ++w) mx = fmaxf(mx, redf[w]);
-    double part = 0.0;
-    for (uint32_t p = start + tid; p < visible; p += 256) {
-        const float e = exact_expf(__fsub_rn(s[p], mx));
-        s[p] = e;
-        part += double(e);
-    }
-    part = warp_sum(part);
-    if ((tid & 31) == 0) redd[tid >> 5] = part;
-    __syncthreads();
-    double total = 0.0;
-#pragma unroll
-    for (int w = 0; w < 8; ++w) total += redd[w];
-    const float inv = float(1.0 / total);
-    for (uint32_t p = start + tid; p < visible; p += 256) s[p] = __fmul_rn(s[p], inv);
-}
-
-// grid (heads x parts, token tiles), one thread per value of the head; a 256-wide head is summed as two independent
-// 128-wide parts (every output value is its own sum over the positions). V rows and the tile's probabilities are staged through
-// shared memory in chunks of 64 positions, so every cached row is read once per kTokTile tokens; each thread keeps one
-// accumulator per token and adds p * v position after position, as weighted_sum_f32 does.
-constexpr uint32_t kWChunk = 64;
-
-template <uint32_t kTokTile>
-__global__ void __launch_bounds__(128) attn_weighted_kernel(const AttnArgs a) {
-    extern __shared__ __align__(16) unsigned char wraw[];  // V chunk [kWChunk][dim] f16 | probabilities [kTokTile][kWChunk] f32
-    const uint32_t parts = (a.dim + 127) / 128, dim = a.dim / parts;  // dim: the 64 or 128 values this CTA sums
-    const uint32_t h = blockIdx.x / parts, doff = blockIdx.x % parts * dim, t0 = blockIdx.y * kTokTile, tid = threadIdx.x;
-    const uint32_t row_shift = dim == 128 ? 4 : 3;  // 16-byte pieces per staged row: dim / 8
-    const uint32_t tn = min(kTokTile, a.n - t0);
-    const uint32_t kvh = h / (a.heads / a.kv_heads);
-    const uint32_t base_visible = *a.position + t0 + 1, last_visible = base_visible + tn - 1;
-    __half* vs = reinterpret_cast<__half*>(wraw);
-    float* ws = reinterpret_cast<float*>(wraw + size_t(kWChunk) * dim * sizeof(__half));
-    const __half* vbase = a.v_cache + size_t(kvh) * a.max_context * a.dim + doff;
-    float acc[kTokTile];
-#pragma unroll
-    for (int j = 0; j < int(kTokTile); ++j) acc[j] = 0.0f;
-    // Sliding-window layer: token j sums positions [start_j, visible_j) with start_j = max(0, visible_j - window), in order
-    // (src/model.cpp:1085-1091). Chunks below the first token's start are skipped; chunks at or above the last token's start
-    // are seen in full by every token of the tile.
-    const uint32_t win = a.window;
-    const uint32_t start_first = win != 0 && base_visible > win ? base_visible - win : 0;
-    const uint32_t start_last = win != 0 && last_visible > win ? last_visible - win : 0;
-    for (uint32_t c0 = start_first / kWChunk * kWChunk; c0 < last_visible; c0 += kWChunk) {
-        const uint32_t cn = min(kWChunk, last_visible - c0);
-        __syncthreads();  // the previous chunk is fully consumed
-        for (uint32_t i = tid; i < cn * dim / 8; i += 128) {
-            const uint32_t row = i >> row_shift, piece = i & ((1u << row_shift) - 1);
-            reinterpret_cast<uint4*>(vs)[i] = *reinterpret_cast<const uint4*>(vbase + size_t(c0 + row) * a.dim + piece * 8);
-        }
-        for (uint32_t i = tid; i < tn * kWChunk; i += 128) {
-            const uint32_t j = i / kWChunk, pp = c0 + i % kWChunk;
-            const uint32_t vis = base_visible + j, st = win != 0 && vis > win ? vis - win : 0;
-            ws[i] = pp < vis && pp >= st ? a.scores[(size_t(t0 + j) * a.heads + h) * a.max_context + pp] : 0.0f;
-        }
-        __syncthreads();
-        if (tid < dim) {
-            if (c0 + cn <= base_visible && c0 >= start_last && tn == kTokTile && cn % 4 == 0) {
-                // Every token of the tile sees the whole chunk (all chunks but the last one or two): no causal tests, and the
-                // probabilities of four positions come in one 16-byte read per token. Per token the products are still added
-                // in position order.
-                for (uint32_t pp = 0; pp < cn; pp += 4) {
-                    const float v0 = __half2float(vs[(pp + 0) * dim + tid]), v1 = __half2float(vs[(pp + 1) * dim + tid]);
-                    const float v2 = __half2float(vs[(pp + 2) * dim + tid]), v3 = __half2float(vs[(pp + 3) * dim + tid]);
-#pragma unroll
-                    for (int j = 0; j < int(kTokTile); ++j) {
-                        const float4 w = *reinterpret_cast<const float4*>(ws + j * kWChunk + pp);
-                        acc[j] = __fadd_rn(acc[j], __fmul_rn(w.x, v0));
-                        acc[j] = __fadd_rn(acc[j], __fmul_rn(w.y, v1));
-                        acc[j] = __fadd_rn(acc[j], __fmul_rn(w.z, v2));
-                        acc[j] = __fadd_rn(acc[j], __fmul_rn(w.w, v3));
-                    }
-                }
-            } else {
-                for (uint32_t pp = 0; pp < cn; ++pp) {
-                    const float v = __half2float(vs[pp * dim + tid]);
-#pragma unroll
-                    for (int j = 0; j < int(kTokTile); ++j) {
-                        // a position past token j's causal limit must not touch its sum at all (adding 0*v could turn -0 into +0)
-                        const uint32_t vis = base_visible + j, st = win != 0 && vis > win ? vis - win : 0;
-                        if (c0 + pp < vis && c0 + pp >= st && j < int(tn)) acc[j] = __fadd_rn(acc[j], __fmul_rn(ws[j * kWChunk + pp], v));
-                    }
-                }
-            }
-        }
-    }
-    if (tid < dim) {
-#pragma unroll
-        for (int j = 0; j < int(kTokTile); ++j) {
-            if (j < int(tn)) a.out[size_t(t0 + j) * a.heads * a.dim + size_t(h) * a.dim + doff + tid] = acc[j];
-        }
-    }
-}
-
 }  // namespace
 
 // ---- greedy arg-max -------------------------------------------------------------------------------------
@@ -531,68 +323,21 @@ int chain_mode() {  // read at every call: the tests switch it between sessions 
 
 size_t attn_scratch_floats(uint32_t n, uint32_t heads, uint32_t max_context) { return size_t(n) * heads * max_context; }
 
+// attn_prompt.cu
+void launch_attn_scores(const AttnArgs& a, uint32_t sms, cudaStream_t s);
+void launch_attn_softmax_weighted(const AttnArgs& a, uint32_t sms, cudaStream_t s);
+
 void launch_attention(const AttnArgs& a, cudaStream_t s) {
-    const uint32_t group = a.heads / a.kv_heads;
-    if ((a.dim != 64 && a.dim != 128 && a.dim != 256) || group > kMaxGroup) throw CudaError("cuda: attention takes head sizes 64, 128 and 256 and at most 16 query heads per K/V head");
-    const uint32_t tile = a.max_visible > kLongContext ? 16u : 8u;
-    const uint32_t tiles = (a.n + tile - 1) / tile;
-    const dim3 grid((a.max_visible + 127) / 128, a.kv_heads, tiles);
-    const size_t smem = size_t(tile) * group * a.dim * sizeof(float);
-#define BK_SCORES_T(G, D, T)                                                                                                                  \
-    do {                                                                                                                                      \
-        if (smem > 48 * 1024) BK_CUDA(cudaFuncSetAttribute(attn_scores_kernel<G, D, T>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem))); \
-        attn_scores_kernel<G, D, T><<<grid, 128, smem, s>>>(a);                                                                               \
-    } while (0)
-#define BK_SCORES(G)                                                            \
-    if (a.dim == 128) {                                                         \
-        if (tile == 16) BK_SCORES_T(G, 128, 16);                                \
-        else BK_SCORES_T(G, 128, 8);                                            \
-    } else if (a.dim == 64) {                                                   \
-        if (tile == 16) BK_SCORES_T(G, 64, 16);                                 \
-        else BK_SCORES_T(G, 64, 8);                                             \
-    } else {                                                                    \
-        if (tile == 16) BK_SCORES_T(G, 256, 16);                                \
-        else BK_SCORES_T(G, 256, 8);                                            \
-    }
-    switch (group) {
-        case 1: BK_SCORES(1); break;
-        case 2: BK_SCORES(2); break;
-        case 3: BK_SCORES(3); break;
-        case 4: BK_SCORES(4); break;
-        case 5: BK_SCORES(5); break;
-        case 6: BK_SCORES(6); break;
-        case 7: BK_SCORES(7); break;
-        case 8: BK_SCORES(8); break;
-        default: throw CudaError("cuda: query heads per K/V head must be 1 to 8");
-    }
-#undef BK_SCORES
-#undef BK_SCORES_T
-    BK_CUDA(cudaGetLastError());
-    {
-        static const int sms = [] {
-            int dev = 0, count = 148;
-            if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
-            return count;
-        }();
-        const int mode = chain_mode();
-        if (mode != 0 && (a.n <= kChainMaxTokens || mode == 1) && attn_chain_fits(a.n, a.heads, a.kv_heads, a.dim, a.max_visible, uint32_t(sms))) {
-            launch_attn_chain(a, uint32_t(sms), s);
-            return;
-        }
-    }
-    attn_softmax_kernel<<<dim3(a.heads, a.n), 256, 0, s>>>(a);
-    BK_CUDA(cudaGetLastError());
-    const uint32_t parts = (a.dim + 127) / 128;
-    if (a.n == 1) {  // a single token (models that take these kernels for their decode steps too): no tile to share V rows with
-        const size_t smem_1 = size_t(kWChunk) * (a.dim / parts) * sizeof(__half) + size_t(kWChunk) * sizeof(float);
-        attn_weighted_kernel<1><<<dim3(a.heads * parts, 1), 128, smem_1, s>>>(a);
-        BK_CUDA(cudaGetLastError());
-        return;
-    }
-    const size_t smem_w = size_t(kWChunk) * (a.dim / parts) * sizeof(__half) + size_t(tile) * kWChunk * sizeof(float);
-    if (tile == 16) attn_weighted_kernel<16><<<dim3(a.heads * parts, tiles), 128, smem_w, s>>>(a);
-    else attn_weighted_kernel<8><<<dim3(a.heads * parts, tiles), 128, smem_w, s>>>(a);
-    BK_CUDA(cudaGetLastError());
+    if ((a.dim != 64 && a.dim != 128 && a.dim != 256) || a.heads / a.kv_heads > 8) throw CudaError("cuda: attention takes head sizes 64, 128 and 256 and at most 8 query heads per K/V head");
+    static const uint32_t sms = [] {
+        int dev = 0, count = 148;
+        if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&count, cudaDevAttrMultiProcessorCount, dev);
+        return uint32_t(count);
+    }();
+    launch_attn_scores(a, sms, s);
+    const int mode = chain_mode();
+    if (mode != 0 && (a.n <= kChainMaxTokens || mode == 1) && attn_chain_fits(a.n, a.heads, a.kv_heads, a.dim, a.max_visible, sms)) launch_attn_chain(a, sms, s);
+    else launch_attn_softmax_weighted(a, sms, s);
 }
 
 size_t argmax_scratch_elems(uint32_t) { return size_t(kArgmaxBlocks) * 64; }

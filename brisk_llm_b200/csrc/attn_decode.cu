@@ -1,0 +1,398 @@
+// Attention of the single new token in two kernels, bit-identical to the CPU engine's (src/model.cpp:1022-1093; the orders
+// of the float operations are those of attn_prompt.cu). Both are launched with programmatic dependent launch and request
+// the K rows and V tiles of earlier positions before the results they depend on are complete.
+//
+//   scores  a CTA takes 256 positions of one K/V head and all of its query heads: per-head norm and RoPE of q (and, where the
+//           token's own position lies, of the new k, with the f16 cache store), then the dots. Two lanes share two positions,
+//           each with half of the 16 partial sums, and two heads share every widened K value.
+//   sum     a CTA takes 32 values of one head: softmax of the head's scores, then the position-ordered weighted sum - a
+//           chain of dependent f32 additions (src/kernels_f32.cpp:265-273), 4.1 cycles each at best, that bounds the kernel.
+//           One warp runs the 32 chains; four warps on the other schedulers produce p[pos] * v[pos][i] into a pair of
+//           tiles, four positions of a value side by side, so that a chain lane reads them with one 16-byte load and adds
+//           them one after the other. A producer warp asks for its own pieces of V three tiles ahead with cp.async; chain
+//           and producers meet at named barriers. Shared-memory traffic, 3.5 wavefronts a position, is what keeps it at 5.4
+//           cycles (one load a position, and loads that queue behind a producer on the same scheduler, made it 8.3).
+//
+// Measured, one layer of the 7B shape at 8000 positions: 13.6 + 44.6 -> 11.5 + 32.5 us; 1B shape at 1024 positions
+// 5.1 + 9.9 -> 5.2 + 8.3 us. One kernel for both, a cluster of CTAs per K/V head that exchanges the softmax through
+// distributed shared memory, was measured too: 46-64 us and 14.5 us. Three cluster barriers cost it about 3 us, and this
+// GPU places only 7 clusters of 16 (15 of 8) at a CTA per SM, so one of the 7B shape's has to share its SMs.
+#include <algorithm>
+
+#include "attn_decode.h"
+#include "decode_body.cuh"
+#include "exact_math.h"
+
+namespace bk {
+namespace {
+
+constexpr uint32_t kScoreThreads = 256, kSumThreads = 512, kSumWarps = kSumThreads / 32;
+constexpr uint32_t kTileFloats = 4096;                  // 128 positions of 32 values
+constexpr uint32_t kProducers = 4;                      // warps
+constexpr uint32_t kPieces = 16, kDepth = 4;            // pieces of 8 positions x 32 values per tile; tiles in flight
+constexpr uint32_t kItems = kPieces / kProducers;       // pieces per producer warp and tile
+constexpr uint32_t kPieceBytes = 9 * 64;                // a staged piece: rows of 64 bytes, the second four shifted by one row (banks)
+constexpr uint32_t kRingBytes = kDepth * kPieces * kPieceBytes;
+
+constexpr uint32_t kTile = kTileFloats / 32, kBatch = 32;  // positions per tile, and that a chain lane loads ahead
+
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
+__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
+// the packed sum: an addition the assembler does not contract with the multiplication before it (see attn_prompt.cu)
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
+
+template <int DIM>
+__global__ void __launch_bounds__(kScoreThreads, 2) decode_scores_kernel(const DecAttnParams a, float one) {
+    constexpr int kSteps = DIM / 16;
+    constexpr int POS = DIM > 128 ? 1 : 2;  // positions of a pair of lanes: a 256-wide row takes the registers of two
+    constexpr uint32_t kPositions = kScoreThreads / 2 * POS;
+    extern __shared__ __align__(16) float qs[];  // [group][DIM], then the new k [DIM]
+    const uint32_t group = a.heads / a.kv_heads, kvh = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t pos = *a.position, visible = pos + 1, first = blockIdx.x * kPositions;
+    if (first >= visible) return;
+    const uint32_t mine = min(kPositions, visible - first);
+    const bool owner = pos - first < mine;
+    // Half a warp apart, so that the halves of a row's 32-byte sectors are asked for by one instruction.
+    const uint32_t half = lane >> 4, in_cta = warp * 16 + (lane & 15);
+    const __half* kbase = a.k_cache + (size_t(kvh) * a.max_context + first) * DIM + half * 8;
+    uint4 raw[POS][kSteps];
+#pragma unroll
+    for (int j = 0; j < POS; ++j) {
+        const uint32_t i = in_cta + j * (kScoreThreads / 2);
+        if (i < mine && first + i != pos) {
+            const uint4* kr = reinterpret_cast<const uint4*>(kbase + size_t(i) * DIM);
+#pragma unroll
+            for (int s = 0; s < kSteps; ++s) raw[j][s] = kr[2 * s];
+        }
+    }
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    const float* rope = a.rope + size_t(pos) * DIM;
+    for (uint32_t task = warp; task <= group; task += kScoreThreads / 32) {
+        if (task < group) {
+            const uint32_t h = kvh * group + task;
+            warp_norm_rope_head<DIM / 32>(a.q + size_t(h) * DIM, a.q_bias ? a.q_bias + size_t(h) * DIM : nullptr, a.q_norm, rope, a.eps, a.neox, qs + task * DIM);
+        } else if (owner) {
+            float* knew = qs + group * DIM;
+            warp_norm_rope_head<DIM / 32>(a.k + size_t(kvh) * DIM, a.k_bias ? a.k_bias + size_t(kvh) * DIM : nullptr, a.k_norm, rope, a.eps, a.neox, knew);
+            __syncwarp();
+            warp_store_new_kv(a, kvh, pos, knew);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < POS; ++j) {
+        const uint32_t i = in_cta + j * (kScoreThreads / 2);
+        if (i < mine && first + i == pos) {  // the token's own row: the f16 values just stored
+            const float* knew = qs + group * DIM + half * 8;
+#pragma unroll
+            for (int s = 0; s < kSteps; ++s) {
+                __half2 h[4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) h[k] = __floats2half2_rn(knew[s * 16 + 2 * k], knew[s * 16 + 2 * k + 1]);
+                raw[j][s] = *reinterpret_cast<const uint4*>(h);
+            }
+        }
+    }
+    const f32x2 one2 = pack2(one, one);
+#pragma unroll 1
+    for (uint32_t g = 0; g < group; g += 2) {  // two heads at a time share a widened value (the last of an odd group goes twice)
+        const uint32_t g1 = min(g + 1, group - 1);
+        // widened again for every pair of heads: hoisted out of this loop the rows would take twice the registers
+#pragma unroll
+        for (int j = 0; j < POS; ++j)
+#pragma unroll
+            for (int k = 0; k < kSteps; ++k) asm volatile("" : "+r"(raw[j][k].x), "+r"(raw[j][k].y), "+r"(raw[j][k].z), "+r"(raw[j][k].w));
+        const ulonglong2* qa = reinterpret_cast<const ulonglong2*>(qs + g * DIM + half * 8);
+        const ulonglong2* qb = reinterpret_cast<const ulonglong2*>(qs + g1 * DIM + half * 8);
+        f32x2 part[2][POS][4];
+#pragma unroll
+        for (int j = 0; j < POS; ++j)
+#pragma unroll
+            for (int k = 0; k < 4; ++k) part[0][j][k] = part[1][j][k] = 0ull;
+#pragma unroll
+        for (int s = 0; s < kSteps; ++s) {
+            const ulonglong2 a0 = qa[s * 4], a1 = qa[s * 4 + 1], b0 = qb[s * 4], b1 = qb[s * 4 + 1];
+            const f32x2 va[4] = {a0.x, a0.y, a1.x, a1.y}, vb[4] = {b0.x, b0.y, b1.x, b1.y};
+#pragma unroll
+            for (int j = 0; j < POS; ++j) {
+                const __half2* h = reinterpret_cast<const __half2*>(&raw[j][s]);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 f = __half22float2(h[k]);
+                    const f32x2 k2 = pack2(f.x, f.y);
+                    part[0][j][k] = fma2(mul2(va[k], k2), one2, part[0][j][k]);
+                    part[1][j][k] = fma2(mul2(vb[k], k2), one2, part[1][j][k]);
+                }
+            }
+        }
+        float sum[2][POS];
+        auto add_parts = [&] {
+#pragma unroll
+            for (int k = 0; k < 4; ++k)
+#pragma unroll
+                for (int hd = 0; hd < 2; ++hd)
+#pragma unroll
+                    for (int j = 0; j < POS; ++j) {
+                        float x, y;
+                        unpack2(part[hd][j][k], x, y);
+                        sum[hd][j] = __fadd_rn(__fadd_rn(sum[hd][j], x), y);
+                    }
+        };
+#pragma unroll
+        for (int j = 0; j < POS; ++j) sum[0][j] = sum[1][j] = 0.0f;
+        add_parts();
+#pragma unroll
+        for (int j = 0; j < POS; ++j) {  // the upper half-warp goes on from its partner's sums of the first eight
+            sum[0][j] = __shfl_sync(0xffffffffu, sum[0][j], lane & 15);
+            sum[1][j] = __shfl_sync(0xffffffffu, sum[1][j], lane & 15);
+        }
+        if (half == 1) {
+            add_parts();
+#pragma unroll
+            for (int j = 0; j < POS; ++j) {
+                const uint32_t i = in_cta + j * (kScoreThreads / 2);
+                if (i < mine) {
+                    a.scores[size_t(kvh * group + g) * a.max_context + first + i] = __fmul_rn(sum[0][j], a.scale);
+                    a.scores[size_t(kvh * group + g1) * a.max_context + first + i] = __fmul_rn(sum[1][j], a.scale);
+                }
+            }
+        }
+    }
+}
+
+// Producer warps leave the chain warp's scheduler (warp mod 4) to it: its loads would queue behind theirs.
+__device__ __forceinline__ uint32_t producer_number(uint32_t warp) { return warp == 5 ? 3 : warp < 4 ? warp - 1 : kProducers; }  // kProducers and above: none
+__device__ __forceinline__ void tile_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kProducers * 32 + 32) : "memory"); }
+__device__ __forceinline__ void tile_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kProducers * 32 + 32) : "memory"); }
+
+// grid: heads x dim / 32. ps_floats: room for the visible positions' probabilities, a multiple of 4.
+__global__ void __launch_bounds__(kSumThreads, 1) decode_sum_kernel(const DecAttnParams a, uint32_t window, uint32_t ps_floats) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    float* ps = reinterpret_cast<float*>(smem);
+    float* tiles = ps + ps_floats;
+    unsigned char* ring = reinterpret_cast<unsigned char*>(tiles + 2 * kTileFloats);
+    __shared__ float redf[kSumWarps];
+    __shared__ double redd[kSumWarps];
+    __shared__ uint64_t exp_table[32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, dim = a.dim, slices = dim / 32;
+    const uint32_t h = blockIdx.x / slices, col0 = blockIdx.x % slices * 32, kvh = h / (a.heads / a.kv_heads);
+    const uint32_t visible = *a.position + 1, start = window != 0 && visible > window ? visible - window : 0, cnt = visible - start;
+    const __half* vbase = a.v_cache + (size_t(kvh) * a.max_context + start) * dim + col0;
+
+    const uint32_t producer = producer_number(warp);
+    auto piece_at = [&](uint32_t tile, uint32_t i) { return ring + (tile % kDepth * kPieces + i * kProducers + producer) * kPieceBytes; };
+    auto request = [&](uint32_t tile, uint32_t from, uint32_t to) {  // rows [from, to) of the sequence that lie in `tile`
+        const uint32_t r = lane >> 2, c = lane & 3;
+#pragma unroll
+        for (uint32_t i = 0; i < kItems; ++i) {
+            const uint32_t piece = i * kProducers + producer, p = tile * kTile + piece * 8 + r;
+            if (p >= from && p < to) {
+                const uint32_t dst = uint32_t(__cvta_generic_to_shared(piece_at(tile, i) + r * 64 + (r >> 2) * 64 + c * 16));
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(vbase + size_t(p) * dim + c * 8) : "memory");
+            }
+        }
+    };
+    if (producer < kProducers) {
+        for (uint32_t t = 0; t + 1 < kDepth; ++t) {
+            request(t, 0, cnt - 1);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        }
+    }
+    if (tid < 32) exp_table[tid] = exp2_table_device()[tid];
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+
+    // ---- softmax (src/kernels_f32.cpp:275-284): e = expf(s - max), f64 sum, p = e * float(1 / sum) ----
+    const float* s = a.scores + size_t(h) * a.max_context + start;
+    float m = -INFINITY;
+    for (uint32_t p0 = tid; p0 < cnt; p0 += 8 * kSumThreads) {  // eight loads in flight
+        float v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = p0 + u * kSumThreads < cnt ? __ldcg(s + p0 + u * kSumThreads) : -INFINITY;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            if (p0 + u * kSumThreads < cnt) ps[p0 + u * kSumThreads] = v[u];
+            m = fmaxf(m, v[u]);
+        }
+    }
+    m = warp_max(m);
+    if (lane == 0) redf[warp] = m;
+    __syncthreads();
+    m = warp_max(redf[lane & (kSumWarps - 1)]);
+    double part = 0.0;
+    {
+        uint32_t p = tid;
+        for (; p + 3 * kSumThreads < cnt; p += 4 * kSumThreads) {  // four at a time: one exp is a long chain of f64 operations
+            float e[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) e[u] = exact_expf_flat(__fsub_rn(ps[p + u * kSumThreads], m), exp_table);
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                ps[p + u * kSumThreads] = e[u];
+                part += double(e[u]);
+            }
+        }
+        for (; p < cnt; p += kSumThreads) {
+            const float e = exact_expf_flat(__fsub_rn(ps[p], m), exp_table);
+            ps[p] = e;
+            part += double(e);
+        }
+    }
+    part = warp_sum(part);
+    if (lane == 0) redd[warp] = part;
+    __syncthreads();
+    const double total = warp_sum(lane < kSumWarps ? redd[lane] : 0.0);
+    const float inv = float(1.0 / total);
+    for (uint32_t p = tid; p < cnt; p += kSumThreads) ps[p] = __fmul_rn(ps[p], inv);
+    __syncthreads();
+
+    // ---- weighted sum ----
+    const uint32_t chunks = (cnt + kTile - 1) / kTile;
+    if (producer < kProducers) {
+        if ((cnt - 1) / kTile + 1 < kDepth) {  // a short context: the own row belongs to a tile requested above
+            request((cnt - 1) / kTile, cnt - 1, cnt);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+#pragma unroll 1
+        for (uint32_t c = 0; c < chunks; ++c) {
+            const uint32_t b = c & 1, dp = lane & 15, pg = lane >> 4;  // this lane: values 2 dp, 2 dp + 1 of positions 4 pg .. 4 pg + 3
+            request(c + kDepth - 1, 0, cnt);
+            asm volatile("cp.async.commit_group;" ::: "memory");
+            asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
+            __syncwarp();  // tile c's pieces of this warp have landed
+            uint32_t v[kItems][4];
+            float4 pr[kItems];
+#pragma unroll
+            for (uint32_t i = 0; i < kItems; ++i) {
+                const unsigned char* at = piece_at(c, i) + pg * 5 * 64 + dp * 4;
+#pragma unroll
+                for (int j = 0; j < 4; ++j) v[i][j] = *reinterpret_cast<const uint32_t*>(at + j * 64);
+                pr[i] = *reinterpret_cast<const float4*>(ps + min(c * kTile + (i * kProducers + producer) * 8 + pg * 4, ps_floats - 4));
+            }
+            if (c >= 2) tile_sync(3 + b);  // the chains are done with this buffer's previous tile
+            float* tile = tiles + size_t(b) * kTileFloats;
+#pragma unroll
+            for (uint32_t i = 0; i < kItems; ++i) {
+                const uint32_t piece = i * kProducers + producer;
+                float2 f[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) f[j] = __half22float2(*reinterpret_cast<const __half2*>(&v[i][j]));
+                const float4 lo = make_float4(__fmul_rn(pr[i].x, f[0].x), __fmul_rn(pr[i].y, f[1].x), __fmul_rn(pr[i].z, f[2].x), __fmul_rn(pr[i].w, f[3].x));
+                const float4 hi = make_float4(__fmul_rn(pr[i].x, f[0].y), __fmul_rn(pr[i].y, f[1].y), __fmul_rn(pr[i].z, f[2].y), __fmul_rn(pr[i].w, f[3].y));
+                float4* at = reinterpret_cast<float4*>(tile) + (piece * 2 + pg) * 32 + 2 * dp;
+                const bool swap = (dp & 4) != 0;  // every other quad of lanes stores its values the other way round: no bank conflict
+                at[swap ? 1 : 0] = swap ? hi : lo;
+                at[swap ? 0 : 1] = swap ? lo : hi;
+            }
+            __syncwarp();  // the pieces may be overwritten
+            tile_arrive(1 + b);
+        }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
+    } else if (warp == 0) {
+        float acc = 0.0f;
+        const float4* tile0 = reinterpret_cast<const float4*>(tiles) + lane;
+        constexpr uint32_t kTileVecs = kTileFloats / 4, kVecs = kBatch / 4;
+        // Two register sets: while one set's products are added, one load between every four additions fills the other. The
+        // order is written down because the compiler left to itself moves the loads behind the additions that hide them.
+        float4 s0[kVecs], s1[kVecs];
+        auto load = [&](const float4* src, float4& v) {
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                         : "r"(uint32_t(__cvta_generic_to_shared(src)))
+                         : "memory");
+        };
+        auto add4 = [&](const float4& v) {
+            asm volatile("add.rn.f32 %0, %0, %1;\n\tadd.rn.f32 %0, %0, %2;\n\tadd.rn.f32 %0, %0, %3;\n\tadd.rn.f32 %0, %0, %4;"
+                         : "+f"(acc)
+                         : "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w));
+        };
+        auto load_and_add = [&](const float4* src, float4 (&dst)[kVecs], const float4 (&sum)[kVecs]) {
+#pragma unroll
+            for (uint32_t u = 0; u < kVecs; ++u) {
+                load(src + u * 32, dst[u]);
+                add4(sum[u]);
+            }
+        };
+        uint32_t waited = 0;  // tiles 0 .. waited - 1 have been waited for
+        if (cnt >= 2 * kBatch) {
+            tile_sync(1);
+            waited = 1;
+#pragma unroll
+            for (uint32_t u = 0; u < kVecs; ++u) load(tile0 + u * 32, s0[u]);
+        }
+        uint32_t done = 0;
+#pragma unroll 1
+        for (uint32_t c = 0; c < chunks; ++c) {
+            const uint32_t rows = min(kTile, cnt - c * kTile), pairs = rows / (2 * kBatch);
+            if (pairs == 0) break;  // a last tile of fewer positions: below
+            const float4* src = tile0 + (c & 1) * kTileVecs;  // s0 holds its first batch
+#pragma unroll 1
+            for (uint32_t i = 0; i + 1 < pairs; ++i) {
+                load_and_add(src + (2 * i + 1) * kVecs * 32, s1, s0);
+                load_and_add(src + (2 * i + 2) * kVecs * 32, s0, s1);
+            }
+            load_and_add(src + (2 * pairs - 1) * kVecs * 32, s1, s0);
+            if (c + 1 < chunks && min(kTile, cnt - (c + 1) * kTile) >= 2 * kBatch) {  // the next tile's first batch, before this tile's last additions
+                tile_sync(1 + ((c + 1) & 1));
+                waited = c + 2;
+                load_and_add(tile0 + ((c + 1) & 1) * kTileVecs, s0, s1);
+            } else {
+#pragma unroll
+                for (uint32_t u = 0; u < kVecs; ++u) add4(s1[u]);
+            }
+            done = c * kTile + 2 * kBatch * pairs;
+            if (rows == kTile && c + 2 < chunks) tile_arrive(3 + (c & 1));  // a producer waits for exactly these
+        }
+        if (done < cnt) {  // what is left of the last tile
+            const uint32_t c = done / kTile;
+            if (waited <= c) tile_sync(1 + (c & 1));
+            const float* src = reinterpret_cast<const float*>(tile0 + (c & 1) * kTileVecs);
+            for (; done < cnt; ++done) acc = __fadd_rn(acc, src[(done % kTile) / 4 * 128 + done % 4]);
+        }
+        a.out[size_t(h) * dim + col0 + lane] = acc;
+    }
+}
+
+template <class... Params, class... Args>
+void launch(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t smem, bool pdl, cudaStream_t s, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = pdl ? 1 : 0;
+    BK_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
+}
+
+template <int DIM>
+void launch_scores(const DecAttnParams& a, uint32_t max_visible, cudaStream_t s) {
+    constexpr uint32_t kPositions = DIM > 128 ? 128 : 256;
+    launch(decode_scores_kernel<DIM>, dim3((max_visible + kPositions - 1) / kPositions, a.kv_heads), kScoreThreads,
+           size_t(a.heads / a.kv_heads + 1) * DIM * sizeof(float), a.pdl != 0, s, a, 1.0f);
+}
+
+size_t sum_smem(uint32_t positions) { return size_t((positions + 3) & ~3u) * 4 + 2 * kTileFloats * 4 + kRingBytes; }
+
+}  // namespace
+
+bool attn_decode_fits(uint32_t dim, uint32_t positions) { return (dim == 64 || dim == 128 || dim == 256) && sum_smem(positions) <= 200 * 1024; }
+
+void launch_attn_decode(const DecAttnParams& a, uint32_t window, cudaStream_t s) {
+    if (a.dim == 64) launch_scores<64>(a, a.max_context, s);
+    else if (a.dim == 128) launch_scores<128>(a, a.max_context, s);
+    else launch_scores<256>(a, a.max_context, s);
+    static DeviceOnce once;
+    if (once.first()) BK_CUDA(cudaFuncSetAttribute(decode_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    const uint32_t positions = window != 0 ? std::min(window, a.max_context) : a.max_context;
+    launch(decode_sum_kernel, dim3(a.heads * (a.dim / 32)), kSumThreads, sum_smem(positions), a.pdl != 0, s, a, window, (positions + 3) & ~3u);
+}
+
+}  // namespace bk

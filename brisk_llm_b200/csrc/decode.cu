@@ -1,18 +1,20 @@
-// Fused kernels of the single-token step (batch-1 decode), six per layer:
+// Fused kernels of the single-token step (batch-1 decode), five per layer:
 //
 //   multiply   norm+quantise prologue -> q/k/v | o (+residual) | gate,up (+activation) | down (+residual) | head
-//   scores     per-head norm + RoPE of q and of the new k, f16 K/V store, q.k for every visible position
-//   attend     softmax + position-ordered weighted sum of V
+//   attention  norm, RoPE, cache store, scores, softmax and position-ordered weighted sum: attn_decode.cu (or, past the
+//              contexts that kernel takes, a scores kernel and a softmax + weighted-sum kernel below)
 //
-// Every kernel can be launched with programmatic dependent launch (it then starts while its predecessor drains, issues
-// the loads that do not depend on it - its first weight units - and only then waits, griddepcontrol.wait, for the
-// predecessor's results); see pdl_mode() for why that is off by default. The activation vector a multiply needs (RMS
+// Every kernel is launched with programmatic dependent launch (it starts while its predecessor drains, issues the loads
+// that do not depend on it - its first weight units - and only then waits, griddepcontrol.wait, for the predecessor's
+// results); see pdl_mode(). The activation vector a multiply needs (RMS
 // norm, 8-bit quantisation) is recomputed by every CTA in shared memory instead of by a separate one-CTA kernel. All arithmetic is the reference's, in the
 // reference's order (see formats.cuh, rowops.cuh, exact_math.h), so the step stays bit-identical to the CPU engine.
+#include <algorithm>
 #include <cstdlib>
 #include <cstring>
 #include <type_traits>
 
+#include "attn_decode.h"
 #include "decode_body.cuh"
 
 namespace bk {
@@ -21,15 +23,16 @@ namespace {
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// How the step's kernels overlap: 0 = plain stream order (default); 1 = programmatic dependent launch, dependents
-// released as soon as a kernel starts (several later kernels may sit resident, waiting); 2 = dependents released
-// after a kernel's prologue (only the next kernel runs ahead). Measured on B200 with the 0.6B-shaped model, 8
-// layers: 411 / 482 / 452 us per token for modes 0 / 1 / 2 - the resident waiting CTAs cost more than the weight
-// prefetch gains, so the default is 0. BRISK_CUDA_PDL selects another mode for experiments.
+// How the step's kernels overlap: 2 (default) = programmatic dependent launch, dependents released after a kernel's
+// prologue, so that only the next kernel runs ahead: its CTAs are resident with their first weights (or K rows and V tiles)
+// on the way when the last results arrive. 1 = released as soon as a kernel starts, 0 = plain stream order. Measured, us
+// per token for modes 0 / 1 / 2: 1B Q4_K_M shape at 1024 positions 818 / 767 / 755, ternary 2B at 517 1403 / 1330 / 1330,
+// 7B Q4_0 at 8192 3320 / 3200 / 3210. What a kernel reads ahead of its wait must be older than the kernel before it;
+// mode 1 may run several kernels ahead and is for measurements only. BRISK_CUDA_PDL selects the mode.
 int pdl_mode() {
     static const int mode = [] {
         const char* env = std::getenv("BRISK_CUDA_PDL");
-        return env != nullptr ? std::atoi(env) : 0;
+        return env != nullptr ? std::atoi(env) : 2;
     }();
     return mode;
 }
@@ -336,6 +339,13 @@ void launch_dec_attention(const RopeArgs& r, const AttnArgs& at, uint32_t sms, c
     a.pdl = pdl_mode();
     const uint32_t group = a.heads / a.kv_heads;
     if (a.dim % 16 != 0 || a.dim > 256) throw CudaError("cuda: head size must be a multiple of 16 up to 256");
+    if (chain_mode() != 0 && !relaxed("attention") && attn_decode_fits(a.dim, at.window != 0 ? std::min(at.window, a.max_context) : a.max_context)) {
+        launch_attn_decode(a, at.window, s);
+        return;
+    }
+    if (at.window != 0) throw CudaError("cuda: a sliding-window layer needs the kernels of attn_decode.cu for single tokens");
+    // Contexts whose probabilities do not fit beside that kernel's tiles (and BRISK_CUDA_CHAIN=0, for comparison): a slice of a
+    // head's values per CTA, products and chain in turns.
     const dim3 grid((a.max_context + 127) / 128, a.kv_heads);
     const size_t smem = size_t(group + 1) * a.dim * sizeof(float);
 #define BK_SCORES(G)                                                                                       \
@@ -362,19 +372,6 @@ void launch_dec_attention(const RopeArgs& r, const AttnArgs& at, uint32_t sms, c
         dec_attn_combine_kernel<<<a.heads, 128, 0, s>>>(a, partial);
         BK_CUDA(cudaGetLastError());
         return;
-    }
-    {
-        // Long contexts (and BRISK_CUDA_CHAIN=1): the single-token kernel of attn_chain.cu instead of the fused one below -
-        // same results; at 8192 positions ~43 us per layer against ~75.
-        const int mode = chain_mode();
-        if ((mode == 1 || (mode != 0 && a.max_context >= kChainOneMinContext)) && attn_chain_one_fits(a.dim, a.max_context)) {
-            AttnArgs one = at;
-            one.n = 1;
-            one.max_visible = a.max_context;
-            one.window = 0;
-            launch_attn_chain_one(one, s);
-            return;
-        }
     }
     a.slice_width = dec_attn_slice_width(a.heads, a.dim, sms);
     const size_t smem2 = dec_attn_out_smem(a.max_context, a.slice_width);

@@ -135,13 +135,8 @@ void launch_attention(const AttnArgs& a, cudaStream_t s);
 // two query heads, slice of the head), chain warps and product warps; same results as the kernels above.
 bool attn_chain_fits(uint32_t n, uint32_t heads, uint32_t kv_heads, uint32_t dim, uint32_t max_visible, uint32_t sms);
 void launch_attn_chain(const AttnArgs& a, uint32_t sms, cudaStream_t s);
-// The single-token form (product warps and a chain warp; same file): a.n is taken as 1.
-bool attn_chain_one_fits(uint32_t dim, uint32_t max_visible);
-void launch_attn_chain_one(const AttnArgs& a, cudaStream_t s);
-constexpr uint32_t kChainOneMinContext = 2048;  // single tokens of sessions with at least this context take it
 constexpr uint32_t kChainMaxTokens = 24;      // more tokens than this share V rows through the tiled kernel instead
-// BRISK_CUDA_CHAIN: 0 never, 1 wherever it fits, unset: 2..kChainMaxTokens tokens, and single tokens (their own form of the
-// kernel, below) in sessions whose context is at least kChainOneMinContext.
+// BRISK_CUDA_CHAIN: 0 never (nor the single-token kernel of attn_decode.cu), 1 wherever it fits, unset: 2..kChainMaxTokens tokens.
 int chain_mode();
 unsigned int* attn_chain_error_word();        // non-zero on the device after a launch whose wait for a bulk copy ran out
 
@@ -151,8 +146,8 @@ unsigned int* attn_chain_error_word();        // non-zero on the device after a 
 // dependent launch: weights are prefetched while the previous kernel drains. `sms` sizes the persistent grid.
 void launch_dec_multiply(const MatTarget* targets, int count, const float* x, const float* norm_weight, float eps, uint32_t cols, Epilogue epi,
                          uint32_t sms, cudaStream_t s, unsigned long long* trace = nullptr);
-// Attention of the single new token: scores kernel (per-head norm + RoPE of q and the new k, f16 K/V store in its
-// prologue) and softmax + weighted-sum kernel. Takes the same argument structs as the batched kernels (n is 1).
+// Attention of the single new token: per-head norm + RoPE of q and the new k, f16 K/V store, scores, softmax and weighted sum.
+// Takes the same argument structs as the batched kernels (n is 1).
 void launch_dec_attention(const RopeArgs& r, const AttnArgs& at, uint32_t sms, cudaStream_t s);
 // Whether a context of max_context positions fits the shared memory of that attention's weighted-sum kernel.
 bool dec_attention_fits(uint32_t max_context, uint32_t heads, uint32_t dim, uint32_t sms);

@@ -14,6 +14,7 @@
 // 9 tokens: the 9-token step of the 7B shape 6.32 -> 6.08 ms against one CTA per row with the row in shared
 // memory, the 512-token prompt of the 0.6B shape 7.40 -> 7.16 ms.
 #include "kernels.h"
+#include "pdl.cuh"
 #include "rowops.cuh"
 
 namespace bk {
@@ -24,6 +25,8 @@ constexpr uint32_t kThreads = 256, kSegment = kThreads * 8;
 __global__ void __launch_bounds__(kThreads) norm_quant_kernel(const float* __restrict__ x, uint32_t ldx, const float* __restrict__ weight,
                                                               float eps, uint32_t cols, DevActMut act, int want0, int wantk) {
     __shared__ double red[32];
+    wait_for_previous();
+    release_next();
     const uint32_t t = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const float* xr = x + size_t(t) * ldx;
     const float scale = weight != nullptr ? cta_rms_scale(xr, cols, eps, red) : 1.0f;
@@ -86,8 +89,7 @@ void launch_norm_quant(const float* x, uint32_t ldx, const float* weight, float 
                        const DevActMut& act, bool want0, bool wantk, cudaStream_t s) {
     // x may be act.f32: then one CTA takes the whole row, so that nobody still sums what another has overwritten
     const uint32_t segments = x == act.f32 ? 1u : (cols + kSegment - 1) / kSegment;
-    norm_quant_kernel<<<dim3(n, segments), kThreads, 0, s>>>(x, ldx, weight, eps, cols, act, want0 ? 1 : 0, wantk ? 1 : 0);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(norm_quant_kernel, dim3(n, segments), dim3(kThreads), 0, s, x, ldx, weight, eps, cols, act, want0 ? 1 : 0, wantk ? 1 : 0);
 }
 
 }  // namespace bk

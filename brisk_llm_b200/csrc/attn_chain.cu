@@ -27,6 +27,7 @@
 // the other they cost 850 cycles each and, at 8192 positions, as much as the chains.
 #include "exact_math.h"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace bk {
 namespace {
@@ -95,6 +96,8 @@ __global__ void __launch_bounds__(256) attn_chain_kernel(const ChainParams a) {
     const uint32_t wph = nt / 32 / HQ;  // warps per head
     const uint32_t tok = blockIdx.y, h0 = blockIdx.x * HQ;
     const uint32_t kvh = h0 / (a.heads / a.kv_heads);
+    wait_for_previous();
+    release_next();
     const uint32_t visible = *a.position + tok + 1;
     // a sliding-window layer attends to the last `window` positions only (src/model.cpp:1084-1091)
     const uint32_t start = a.window != 0 && visible > a.window ? visible - a.window : 0;
@@ -291,8 +294,7 @@ void launch_variant(const ChainParams& p, cudaStream_t s) {
     static DeviceOnce once;
     if (once.first()) BK_CUDA(cudaFuncSetAttribute(attn_chain_kernel<C, HQ>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     const uint32_t threads = HQ * (p.dim / (32 * C)) * 32;
-    attn_chain_kernel<C, HQ><<<dim3(p.heads / HQ, p.n), threads, smem, s>>>(p);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(attn_chain_kernel<C, HQ>, dim3(p.heads / HQ, p.n), dim3(threads), smem, s, p);
 }
 
 }  // namespace

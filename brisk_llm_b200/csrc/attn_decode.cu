@@ -22,6 +22,7 @@
 #include "attn_decode.h"
 #include "decode_body.cuh"
 #include "exact_math.h"
+#include "pdl.cuh"
 
 namespace bk {
 namespace {
@@ -67,8 +68,8 @@ __global__ void __launch_bounds__(kScoreThreads, 2) decode_scores_kernel(const D
             for (int s = 0; s < kSteps; ++s) raw[j][s] = kr[2 * s];
         }
     }
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    wait_for_previous();
+    release_next();
     const float* rope = a.rope + size_t(pos) * DIM;
     for (uint32_t task = warp; task <= group; task += kScoreThreads / 32) {
         if (task < group) {
@@ -202,8 +203,8 @@ __global__ void __launch_bounds__(kSumThreads, 1) decode_sum_kernel(const DecAtt
         }
     }
     if (tid < 32) exp_table[tid] = exp2_table_device()[tid];
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    wait_for_previous();
+    release_next();
 
     // ---- softmax (src/kernels_f32.cpp:275-284): e = expf(s - max), f64 sum, p = e * float(1 / sum) ----
     const float* s = a.scores + size_t(h) * a.max_context + start;
@@ -357,26 +358,11 @@ __global__ void __launch_bounds__(kSumThreads, 1) decode_sum_kernel(const DecAtt
     }
 }
 
-template <class... Params, class... Args>
-void launch(void (*kernel)(Params...), dim3 grid, uint32_t threads, size_t smem, bool pdl, cudaStream_t s, Args... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(threads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    BK_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
-}
-
 template <int DIM>
 void launch_scores(const DecAttnParams& a, uint32_t max_visible, cudaStream_t s) {
     constexpr uint32_t kPositions = DIM > 128 ? 128 : 256;
-    launch(decode_scores_kernel<DIM>, dim3((max_visible + kPositions - 1) / kPositions, a.kv_heads), kScoreThreads,
-           size_t(a.heads / a.kv_heads + 1) * DIM * sizeof(float), a.pdl != 0, s, a, 1.0f);
+    launch_dependent(decode_scores_kernel<DIM>, dim3((max_visible + kPositions - 1) / kPositions, a.kv_heads), dim3(kScoreThreads),
+                     size_t(a.heads / a.kv_heads + 1) * DIM * sizeof(float), s, a, 1.0f);
 }
 
 size_t sum_smem(uint32_t positions) { return size_t((positions + 3) & ~3u) * 4 + 2 * kTileFloats * 4 + kRingBytes; }
@@ -392,7 +378,7 @@ void launch_attn_decode(const DecAttnParams& a, uint32_t window, cudaStream_t s)
     static DeviceOnce once;
     if (once.first()) BK_CUDA(cudaFuncSetAttribute(decode_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     const uint32_t positions = window != 0 ? std::min(window, a.max_context) : a.max_context;
-    launch(decode_sum_kernel, dim3(a.heads * (a.dim / 32)), kSumThreads, sum_smem(positions), a.pdl != 0, s, a, window, (positions + 3) & ~3u);
+    launch_dependent(decode_sum_kernel, dim3(a.heads * (a.dim / 32)), dim3(kSumThreads), sum_smem(positions), s, a, window, (positions + 3) & ~3u);
 }
 
 }  // namespace bk

@@ -18,6 +18,7 @@
 
 #include "exact_math.h"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace bk {
 namespace {
@@ -43,6 +44,7 @@ __global__ void __launch_bounds__(128) attn_scores_kernel(const AttnArgs a, uint
     extern __shared__ __align__(16) float qs[];  // [tile_rows][DIM]
     const uint32_t group = a.heads / a.kv_heads, kvh = blockIdx.y, rows = a.n * group, tid = threadIdx.x;
     const uint32_t r0 = (gridDim.z - 1 - blockIdx.z) * tile_rows, rn = min(tile_rows, rows - r0);
+    wait_for_previous();
     const uint32_t position = *a.position;
     const uint32_t last_visible = position + (r0 + rn - 1) / group + 1;
     if (blockIdx.x * 128 >= last_visible) return;
@@ -97,6 +99,7 @@ __global__ void __launch_bounds__(128) attn_scores_kernel(const AttnArgs a, uint
             ++token;
         }
     }
+    release_next();
 }
 
 // Heads of 256 values: a K row does not fit a thread's registers. Four lanes share two cached positions: lane k of a quad
@@ -109,6 +112,7 @@ __global__ void __launch_bounds__(128) attn_scores_wide_kernel(const AttnArgs a,
     extern __shared__ __align__(16) float qs[];  // [tile_rows][DIM]
     const uint32_t group = a.heads / a.kv_heads, kvh = blockIdx.y, rows = a.n * group;
     const uint32_t r0 = (gridDim.z - 1 - blockIdx.z) * tile_rows, rn = min(tile_rows, rows - r0);
+    wait_for_previous();
     const uint32_t position = *a.position;
     const uint32_t last_visible = position + (r0 + rn - 1) / group + 1;
     if (blockIdx.x * kPositions >= last_visible) return;
@@ -177,6 +181,7 @@ __global__ void __launch_bounds__(128) attn_scores_wide_kernel(const AttnArgs a,
             ++token;
         }
     }
+    release_next();
 }
 
 // ---- softmax ------------------------------------------------------------------------------------------------------
@@ -186,6 +191,7 @@ __global__ void __launch_bounds__(128) attn_scores_wide_kernel(const AttnArgs a,
 template <int THREADS, int HELD>
 __global__ void __launch_bounds__(256) attn_softmax_kernel(const AttnArgs a) {
     constexpr uint32_t kRows = 256 / THREADS;
+    wait_for_previous();
     __shared__ float redf[8];
     __shared__ double redd[8];
     const uint32_t row = blockIdx.x * kRows + threadIdx.x / THREADS, tid = threadIdx.x % THREADS;
@@ -236,6 +242,7 @@ __global__ void __launch_bounds__(256) attn_softmax_kernel(const AttnArgs a) {
         for (int w = 0; w < 8; ++w) total += redd[w];
     }
     const float inv = float(1.0 / total);
+    release_next();
 #pragma unroll
     for (int i = 0; i < HELD; ++i) {
         const uint32_t p = tid + i * THREADS;
@@ -266,6 +273,7 @@ __global__ void __launch_bounds__(128) attn_weighted_kernel(const AttnArgs a, fl
     const uint32_t group = a.heads / a.kv_heads, kvh = blockIdx.y, doff = blockIdx.x * width, tid = threadIdx.x;
     const uint32_t rows = a.n * group, r0 = (gridDim.z - 1 - blockIdx.z) * tile_rows, rn = min(tile_rows, rows - r0);
     const uint32_t col = tid % lanes * 4, mine = tid / lanes * R;  // this lane's first value, the first of its rows
+    wait_for_previous();
     const uint32_t position = *a.position, win = a.window;
     const uint32_t base_visible = position + r0 / group + 1, last_visible = position + (r0 + rn - 1) / group + 1;
     const uint32_t start_first = win != 0 && base_visible > win ? base_visible - win : 0;
@@ -382,6 +390,7 @@ __global__ void __launch_bounds__(128) attn_weighted_kernel(const AttnArgs a, fl
         }
         edge(max(lo, hi), cn);
     }
+    release_next();
 #pragma unroll
     for (int i = 0; i < R; ++i) {
         if (mine + i >= rn) continue;
@@ -411,16 +420,14 @@ void launch_scores(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
     while (tile > 8 && uint64_t(chunks) * a.kv_heads * ((rows + tile - 1) / tile) < 4ull * sms) tile /= 2;
     static DeviceOnce once;
     if (once.first()) BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(64 * DIM * sizeof(float))));
-    kernel<<<dim3(chunks, a.kv_heads, (rows + tile - 1) / tile), 128, size_t(tile) * DIM * sizeof(float), s>>>(a, tile, 1.0f);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(kernel, dim3(chunks, a.kv_heads, (rows + tile - 1) / tile), dim3(128), size_t(tile) * DIM * sizeof(float), s, a, tile, 1.0f);
 }
 
 template <int R>
 void launch_weighted(const AttnArgs& a, uint32_t tiles, uint32_t parts, cudaStream_t s) {
     const uint32_t width = a.dim / parts, tile_rows = R * (512 / width);
     const size_t smem = size_t(2) * kChunk * width * sizeof(__half) + size_t(kChunk) * (tile_rows + 4) * sizeof(float);
-    attn_weighted_kernel<R><<<dim3(parts, a.kv_heads, tiles), 128, smem, s>>>(a, 1.0f);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(attn_weighted_kernel<R>, dim3(parts, a.kv_heads, tiles), dim3(128), smem, s, a, 1.0f);
 }
 
 }  // namespace
@@ -433,10 +440,9 @@ void launch_attn_scores(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
 
 void launch_attn_softmax_weighted(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
     const uint32_t softmax_rows = a.n * a.heads, widest = a.window != 0 ? std::min(a.window, a.max_visible) : a.max_visible;
-    if (widest <= 512) attn_softmax_kernel<32, 16><<<(softmax_rows + 7) / 8, 256, 0, s>>>(a);
-    else if (widest <= 1024) attn_softmax_kernel<32, 32><<<(softmax_rows + 7) / 8, 256, 0, s>>>(a);
-    else attn_softmax_kernel<256, 16><<<softmax_rows, 256, 0, s>>>(a);
-    BK_CUDA(cudaGetLastError());
+    if (widest <= 512) launch_dependent(attn_softmax_kernel<32, 16>, dim3((softmax_rows + 7) / 8), dim3(256), 0, s, a);
+    else if (widest <= 1024) launch_dependent(attn_softmax_kernel<32, 32>, dim3((softmax_rows + 7) / 8), dim3(256), 0, s, a);
+    else launch_dependent(attn_softmax_kernel<256, 16>, dim3(softmax_rows), dim3(256), 0, s, a);
     // More rows per lane reuse the V row it has widened (16 rows: 736 us for the case above, 8: 921), fewer fill the GPU: the
     // most that still leave one and a half CTAs an SM.
     const uint32_t rows = a.n * (a.heads / a.kv_heads), parts = (a.dim + 127) / 128, groups = 512 / (a.dim / parts);

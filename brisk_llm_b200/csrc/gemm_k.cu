@@ -13,6 +13,7 @@
 // Everything before the float expression is exact integer work, so results are bit-identical to the CPU kernels.
 // Tiling as in gemm.cu: CTA = 128 rows x 64 tokens, 8 warps of 32 x 32, two cp.async stages of one super-block each.
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace bk {
 namespace {
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[mi][ni][j] = 0.0f;
 
+    wait_for_previous();
     load_stage(0, 0);
     for (uint32_t sb = 0; sb < nsb; ++sb) {
         if (sb + 1 < nsb) {
@@ -321,6 +323,7 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
         }
         __syncthreads();
     }
+    release_next();
 
 #pragma unroll
     for (int mi = 0; mi < 2; ++mi)
@@ -343,8 +346,7 @@ void launch_one(const KParams& p, cudaStream_t s) {
     static DeviceOnce once;
     if (once.first()) BK_CUDA(cudaFuncSetAttribute(gemm_k_kernel<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     const dim3 grid((p.m.rows + KM - 1) / KM, (p.n + KN - 1) / KN);
-    gemm_k_kernel<TYPE><<<grid, KWARPS * 32, smem, s>>>(p);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(gemm_k_kernel<TYPE>, grid, dim3(KWARPS * 32), smem, s, p);
 }
 
 }  // namespace

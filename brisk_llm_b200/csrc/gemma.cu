@@ -13,12 +13,15 @@
 #include "common.cuh"
 #include "formats.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 #include "rowops.cuh"
 
 namespace bk {
 namespace {
 
 __global__ void __launch_bounds__(256) scale_rows_kernel(float* x, size_t count, float scale) {
+    wait_for_previous();
+    release_next();
     const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < count) x[i] = __fmul_rn(x[i], scale);
 }
@@ -26,6 +29,8 @@ __global__ void __launch_bounds__(256) scale_rows_kernel(float* x, size_t count,
 // One CTA per token row: p = proj * scale * weight (rms_norm's order, src/model.cpp:87-97), then hidden += p.
 __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restrict__ proj, const float* __restrict__ weight,
                                                             float* __restrict__ hidden, uint32_t cols, float eps) {
+    wait_for_previous();
+    release_next();
     __shared__ double red[32];
     const float* p = proj + size_t(blockIdx.x) * cols;
     float* h = hidden + size_t(blockIdx.x) * cols;
@@ -36,6 +41,8 @@ __global__ void __launch_bounds__(256) post_norm_add_kernel(const float* __restr
 }
 
 __global__ void __launch_bounds__(256) softcap_kernel(float* logits, size_t count, float cap, const uint8_t* tanh_table) {
+    wait_for_previous();
+    release_next();
     const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < count) logits[i] = __fmul_rn(cap, tanh_like_host(__fdiv_rn(logits[i], cap), tanh_table));
 }
@@ -49,18 +56,15 @@ __global__ void __launch_bounds__(256) tanh_base_kernel(uint32_t first, uint32_t
 }  // namespace
 
 void launch_scale_rows(float* x, size_t count, float scale, cudaStream_t s) {
-    scale_rows_kernel<<<unsigned((count + 255) / 256), 256, 0, s>>>(x, count, scale);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(scale_rows_kernel, dim3(unsigned((count + 255) / 256)), dim3(256), 0, s, x, count, scale);
 }
 
 void launch_post_norm_add(const float* proj, const float* weight, float* hidden, uint32_t n, uint32_t cols, float eps, cudaStream_t s) {
-    post_norm_add_kernel<<<n, 256, 0, s>>>(proj, weight, hidden, cols, eps);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(post_norm_add_kernel, dim3(n), dim3(256), 0, s, proj, weight, hidden, cols, eps);
 }
 
 void launch_softcap(float* logits, size_t count, float cap, const uint8_t* tanh_table, cudaStream_t s) {
-    softcap_kernel<<<unsigned((count + 255) / 256), 256, 0, s>>>(logits, count, cap, tanh_table);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(softcap_kernel, dim3(unsigned((count + 255) / 256)), dim3(256), 0, s, logits, count, cap, tanh_table);
 }
 
 size_t tanh_table_bytes() { return size_t(kTanhTableHi - kTanhTableLo) / 2; }

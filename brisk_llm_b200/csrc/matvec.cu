@@ -16,6 +16,7 @@
 
 #include "formats.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace bk {
 namespace {
@@ -42,6 +43,7 @@ __global__ void __launch_bounds__(kWarps * 32) matvec_kernel(const Params p) {
     static_assert(CHAINS <= 32, "one lane per chain");
     __shared__ float tile[F::kExact ? kWarps : 1][F::kExact ? CHAINS : 1][33];
 
+    wait_for_previous();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t group = blockIdx.x * kWarps + warp;
     if (group >= p.first_group[PAIR ? 1 : p.count]) return;
@@ -130,7 +132,7 @@ __global__ void __launch_bounds__(kWarps * 32) matvec_kernel(const Params p) {
 template <class F, int NTOK, int RW, bool PAIR>
 void launch_one(const Params& p, uint32_t groups, cudaStream_t s) {
     const unsigned grid = (groups + kWarps - 1) / kWarps;
-    matvec_kernel<F, NTOK, RW, PAIR><<<grid, kWarps * 32, 0, s>>>(p);
+    launch_dependent(matvec_kernel<F, NTOK, RW, PAIR>, dim3(grid), dim3(kWarps * 32), 0, s, p);
 }
 
 // Rows per warp: as many as keep one lane per chain (<= 32 chains) and divide every target's row count.
@@ -179,6 +181,8 @@ void dispatch(Params& p, bool pair, uint32_t n, cudaStream_t s) {
 }
 
 __global__ void gate_mul_kernel(float* gate, const float* up, size_t count, int mode, const uint8_t* tanh_table) {
+    wait_for_previous();
+    release_next();
     const size_t i = size_t(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i < count) gate[i] = mode == 2 ? gelu_mul(gate[i], up[i], tanh_table) : mode == 1 ? relu2_mul(gate[i], up[i]) : silu_mul(gate[i], up[i]);
 }
@@ -186,8 +190,7 @@ __global__ void gate_mul_kernel(float* gate, const float* up, size_t count, int 
 }  // namespace
 
 void launch_gate_mul(float* gate, const float* up, size_t count, int mode, cudaStream_t s, const uint8_t* tanh_table) {
-    gate_mul_kernel<<<unsigned((count + 255) / 256), 256, 0, s>>>(gate, up, count, mode, tanh_table);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(gate_mul_kernel, dim3(unsigned((count + 255) / 256)), dim3(256), 0, s, gate, up, count, mode, tanh_table);
 }
 
 void launch_matvec(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s) {

@@ -9,6 +9,7 @@
 #include <cstdlib>
 
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace bk {
 namespace {
@@ -145,6 +146,8 @@ __global__ void embed_kernel(const DevMatrix m, const int32_t* tokens, float* __
 
 // ---- per-head RMS norm (optional) + RoPE on q and k, K/V -> f16 cache (src/model.cpp:1022-1046) ----
 __global__ void __launch_bounds__(128) qk_norm_rope_store_kernel(const RopeArgs a) {
+    wait_for_previous();
+    release_next();
     __shared__ float head[512];
     __shared__ double red[4];
     // `half` pairs rotate: all dim / 2 of them, or (partial rotary, src/model.cpp:104-115, :1024) only the pairs within the
@@ -312,8 +315,7 @@ void launch_embed(const DevMatrix& embd, const int32_t* tokens_dev, uint32_t n, 
 
 void launch_qk_norm_rope_store(const RopeArgs& a, cudaStream_t s) {
     if (a.dim > 512 || a.dim % 2 != 0) throw CudaError("cuda: head size must be even and at most 512");
-    qk_norm_rope_store_kernel<<<dim3(a.n, a.heads + a.kv_heads), 128, 0, s>>>(a);
-    BK_CUDA(cudaGetLastError());
+    launch_dependent(qk_norm_rope_store_kernel, dim3(a.n, a.heads + a.kv_heads), dim3(128), 0, s, a);
 }
 
 int chain_mode() {  // read at every call: the tests switch it between sessions of one process

@@ -14,6 +14,7 @@
 #include <dlfcn.h>
 
 #include "../../include/brisk_cuda.h"
+#include "attn_decode.h"
 #include "kernels.h"
 
 namespace bk {
@@ -158,7 +159,7 @@ struct Session {
     uint64_t max_context = 0;
     float eps = 0, rope_base = 0;
     // Gemma 3 (src/model.cpp:169-176, :286): scaled embeddings, tanh-GELU gate, sliding window, soft cap of the logits.
-    // Such a model runs every step, single tokens too, through the batched kernels plus the few kernels of gemma.cu.
+    // Such a model's single tokens take one kernel per operation, plus the few of gemma.cu.
     float embedding_scale = 1.0f, final_softcap = 0.0f;
     uint32_t sliding_window = 0;
     bool gelu = false, variant_layers = false;
@@ -435,8 +436,8 @@ struct Session {
             if (d.attn_post_norm || d.ffn_post_norm || d.slides) variant_layers = true;
         }
         if (gelu || embedding_scale != 1.0f || final_softcap != 0.0f) variant_layers = true;
-        if (head_dim > 128) variant_layers = true;  // the fused single-token kernels take heads of 64 and 128
-        if (rope_dim != head_dim) variant_layers = true;  // ... and rotate whole heads
+        if (head_dim > 128) variant_layers = true;  // the persistent kernel takes heads of 64 and 128
+        if (rope_dim != head_dim) variant_layers = true;  // ... and rotates whole heads
         BK_CUDA(cudaStreamSynchronize(stream));
         if (m.output.data == nullptr) {
             // A tied head is streamed once per token as the head; the embedding lookup reads one row of it.
@@ -554,7 +555,7 @@ struct Session {
         const char* env = std::getenv("BRISK_CUDA_STEP");
         if (tp_size > 1) step_note = "off: tensor parallel steps exchange activations between the operations";
         else if (unrotated_layers) step_note = "off: layers without RoPE take the per-operation kernels (the persistent kernel rotates every layer with one table)";
-        else if (variant_layers) step_note = "off: Gemma layer variants (post-norms, GELU, sliding window), 256-wide heads and partial rotary run through the batched kernels";
+        else if (variant_layers) step_note = "off: Gemma layer variants (post-norms, GELU, sliding window), 256-wide heads and partial rotary take one kernel per operation";
         else if (flags & (BRISK_CUDA_FLAG_NO_MEGAKERNEL | BRISK_CUDA_FLAG_NO_PERSISTENT)) step_note = "off: disabled by the session's flags";
         else if (env != nullptr && std::strcmp(env, "0") == 0) step_note = "off: BRISK_CUDA_STEP=0";
         else if (trace.p != nullptr) step_note = "off: tracing the per-operation kernels";
@@ -735,12 +736,19 @@ struct Session {
         peer_on = true;
     }
 
+    // Whether single tokens take the fused kernels: partial rotary does not, and what only the kernels of attn_decode.cu cover
+    // (windows, 256-wide heads) needs a context that fits them.
+    bool single_kernels() const {
+        if (!variant_layers) return true;
+        return rope_dim == head_dim && chain_mode() != 0 && attn_decode_fits(head_dim, uint32_t(max_context));
+    }
+
     // The layers of one batch. n tokens are in tokens_dev, their first position in d_position(); max_visible bounds
     // position + n. single = true takes the fused single-token kernels (n == 1).
     enum Logits { NO_LOGITS, LAST_LOGITS, ALL_LOGITS };  // which rows go through the output head
     void run_layers(uint32_t n, Logits logits, uint32_t max_visible, bool single) {
         float* hid = hidden_b.as<float>();
-        if (variant_layers) single = false;
+        if (!single_kernels()) single = false;
         {
             Scope sc(this, PH_EMBED);
             launch_embed(embd, tokens_dev.as<int32_t>(), n, hid, stream);
@@ -907,6 +915,7 @@ struct Session {
             Scope sc(this, PH_HEAD);
             apply({{head, logits_b.as<float>(), vocab}}, hid, hidden, output_norm, hidden, EPI_STORE);
         }
+        soft_cap(1);
     }
 
     // Output norm and head of rows [first, first + rows) of the residual stream, at most kMaxScored of them, into logits_b.
@@ -924,10 +933,13 @@ struct Session {
             Scope sc(this, PH_HEAD);
             multiply({{head, logits_b.as<float>(), vocab}}, prepare(x, hidden, output_norm, rows, hidden, nd), rows, EPI_STORE);
         }
-        if (final_softcap != 0.0f) {  // src/model.cpp:1206-1209
-            launch_softcap(logits_b.as<float>(), size_t(rows) * vocab, final_softcap, tanh_table.as<uint8_t>(), stream);
-            ++launches;
-        }
+        soft_cap(rows);
+    }
+
+    void soft_cap(uint32_t rows) {
+        if (final_softcap == 0.0f) return;
+        launch_softcap(logits_b.as<float>(), size_t(rows) * vocab, final_softcap, tanh_table.as<uint8_t>(), stream);  // src/model.cpp:1206-1209
+        ++launches;
     }
 
     void forward(uint32_t n, Logits logits, uint32_t max_visible) { run_layers(n, logits, max_visible, false); }

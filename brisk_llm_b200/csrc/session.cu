@@ -177,11 +177,11 @@ struct Session {
     uint64_t weight_bytes = 0, kv_bytes = 0;
 
     // state and scratch
-    DevBuffer kv, rope, rope_local, rope_none, proj_b, tanh_table, tokens_dev, scalars, hidden_b, q_b, k_b, v_b, attended_b, ffn_b, up_b, logits_b, tp_local, tp_gathered, full_b, actf, actq0, actd0, acts0, actqk,
+    DevBuffer kv, rope, rope_local, rope_none, proj_b, tanh_table, inputs_dev, hidden_b, q_b, k_b, v_b, attended_b, ffn_b, up_b, logits_b, tp_local, tp_gathered, full_b, actf, actq0, actd0, acts0, actqk,
         actdk, actbs, partial, am_val, am_idx, history, logit_history, trace, topk_keys, topk_out, score_dev;
     DevActMut act;
     float* logits_host = nullptr;     // pinned [64][vocab]
-    int32_t* tokens_host = nullptr;   // pinned [kMaxBatch + 4]
+    int32_t* inputs_host = nullptr;   // pinned staging of inputs_dev
     int32_t* topk_host = nullptr;     // pinned [2 * kMaxTopK]: ids, then the values' bits
     double* score_host = nullptr;     // pinned [kMaxBatch] log-probabilities
     uint64_t position = 0;
@@ -206,6 +206,7 @@ struct Session {
     unsigned int* step_error_host = nullptr;  // pinned copy of the kernel's barrier-timeout word
     uint64_t persistent_steps = 0;
     uint64_t launches = 0;  // kernels launched by the current call
+    bool batched = false;   // the current call ran batched kernels
     // Per-phase device time, the counterpart of the reference's Session::Profile / BRISK_GPU_PROFILE
     // (src/model.h:242-245, src/metal/metal_session.mm:711-719). Enabled by brisk_cuda_profile_enable(): every phase is
     // then bracketed by CUDA events and the single-token step runs without its graph.
@@ -258,10 +259,21 @@ struct Session {
     brisk_cuda_stats stats{};
     std::string error;
 
-    // device scalars: [0] position (u32), [1] chosen token, [2] history length
-    uint32_t* d_position() const { return scalars.as<uint32_t>(); }
-    int32_t* d_chosen() const { return scalars.as<int32_t>() + 1; }
-    uint32_t* d_history_len() const { return scalars.as<uint32_t>() + 2; }
+    // What a call hands to the device, in one copy: [0] position (u32), [1] chosen token, [2] history length, then the tokens of
+    // a batch and the one after them.
+    static constexpr uint32_t kInputTokens = 4;
+    uint32_t* d_position() const { return inputs_dev.as<uint32_t>(); }
+    int32_t* d_chosen() const { return inputs_dev.as<int32_t>() + 1; }
+    uint32_t* d_history_len() const { return inputs_dev.as<uint32_t>() + 2; }
+    int32_t* d_tokens() const { return inputs_dev.as<int32_t>() + kInputTokens; }
+    void upload_inputs(const int32_t* tokens, uint32_t count) {  // the staging buffer is free: its last copy has completed
+        inputs_host[0] = int32_t(uint32_t(position));
+        inputs_host[1] = inputs_host[2] = inputs_host[3] = 0;
+        std::memcpy(inputs_host + kInputTokens, tokens, count * sizeof(int32_t));
+        const size_t bytes = (kInputTokens + count) * sizeof(int32_t);
+        BK_CUDA(cudaMemcpyAsync(inputs_dev.p, inputs_host, bytes, cudaMemcpyHostToDevice, stream));
+        stats.h2d_bytes += bytes;
+    }
 
     ~Session() {
         if (stream) cudaStreamSynchronize(stream);
@@ -275,7 +287,7 @@ struct Session {
         if (ev1) cudaEventDestroy(ev1);
         if (stream) cudaStreamDestroy(stream);
         if (logits_host) cudaFreeHost(logits_host);
-        if (tokens_host) cudaFreeHost(tokens_host);
+        if (inputs_host) cudaFreeHost(inputs_host);
         if (topk_host) cudaFreeHost(topk_host);
         if (score_host) cudaFreeHost(score_host);
         if (step_error_host) cudaFreeHost(step_error_host);
@@ -490,9 +502,8 @@ struct Session {
         }
 
         const uint32_t widest = std::max(std::max(hidden, q_dim), ffn);
-        tokens_dev.alloc((kMaxBatch + 4) * sizeof(int32_t));
-        scalars.alloc(64);
-        BK_CUDA(cudaMemsetAsync(scalars.p, 0, 64, stream));
+        inputs_dev.alloc((kInputTokens + kMaxBatch + 4) * sizeof(int32_t));
+        BK_CUDA(cudaMemsetAsync(inputs_dev.p, 0, inputs_dev.bytes, stream));
         hidden_b.alloc(size_t(kMaxBatch) * hidden * 4);
         q_b.alloc(size_t(kMaxBatch) * q_dim * 4);
         k_b.alloc(size_t(kMaxBatch) * kv_dim * 4);
@@ -537,7 +548,7 @@ struct Session {
             BK_CUDA(cudaMemsetAsync(trace.p, 0, trace.bytes, stream));
         }
         BK_CUDA(cudaMallocHost(&logits_host, size_t(kMaxScored) * vocab * sizeof(float)));
-        BK_CUDA(cudaMallocHost(&tokens_host, (kMaxBatch + 4) * sizeof(int32_t)));
+        BK_CUDA(cudaMallocHost(&inputs_host, (kInputTokens + kMaxBatch + 4) * sizeof(int32_t)));
         BK_CUDA(cudaMallocHost(&topk_host, 2 * kMaxTopK * sizeof(int32_t)));
         score_dev.alloc(kMaxBatch * sizeof(double));
         BK_CUDA(cudaMallocHost(&score_host, kMaxBatch * sizeof(double)));
@@ -590,7 +601,7 @@ struct Session {
         if (tok_env != nullptr && std::strcmp(tok_env, "1") == 0) {
             TokenEnds ends;
             ends.embd = embd; ends.head = head; ends.output_norm = output_norm; ends.logits = logits_b.as<float>(); ends.vocab = vocab;
-            ends.token = tokens_dev.as<int32_t>(); ends.chosen = d_chosen(); ends.history = history.as<int32_t>(); ends.history_len = d_history_len();
+            ends.token = d_tokens(); ends.chosen = d_chosen(); ends.history = history.as<int32_t>(); ends.history_len = d_history_len();
             token_enabled = token_plan.build(args, sh, ends, sms, stream, why);
             if (token_enabled) {
                 step_note = "on: " + token_plan.description();
@@ -743,7 +754,7 @@ struct Session {
         return rope_dim == head_dim && chain_mode() != 0 && attn_decode_fits(head_dim, uint32_t(max_context));
     }
 
-    // The layers of one batch. n tokens are in tokens_dev, their first position in d_position(); max_visible bounds
+    // The layers of one batch. n tokens are in d_tokens(), their first position in d_position(); max_visible bounds
     // position + n. single = true takes the fused single-token kernels (n == 1).
     enum Logits { NO_LOGITS, LAST_LOGITS, ALL_LOGITS };  // which rows go through the output head
     void run_layers(uint32_t n, Logits logits, uint32_t max_visible, bool single) {
@@ -751,7 +762,7 @@ struct Session {
         if (!single_kernels()) single = false;
         {
             Scope sc(this, PH_EMBED);
-            launch_embed(embd, tokens_dev.as<int32_t>(), n, hid, stream);
+            launch_embed(embd, d_tokens(), n, hid, stream);
             if (embedding_scale != 1.0f) {  // src/model.cpp:899-901
                 launch_scale_rows(hid, size_t(n) * hidden, embedding_scale, stream);
                 ++launches;
@@ -942,7 +953,10 @@ struct Session {
         ++launches;
     }
 
-    void forward(uint32_t n, Logits logits, uint32_t max_visible) { run_layers(n, logits, max_visible, false); }
+    void forward(uint32_t n, Logits logits, uint32_t max_visible) {
+        batched = true;
+        run_layers(n, logits, max_visible, false);
+    }
     bool step_active() const { return (step_enabled || token_enabled) && !profiling; }
     bool token_active() const { return token_enabled && !profiling; }
     void forward_decode() {
@@ -952,7 +966,7 @@ struct Session {
         }
         if (token_enabled) {
             if (!token_plan.embeds_itself()) {
-                launch_embed(embd, tokens_dev.as<int32_t>(), 1, hidden_b.as<float>(), stream);
+                launch_embed(embd, d_tokens(), 1, hidden_b.as<float>(), stream);
                 ++launches;
             }
             token_plan.launch(stream, advance_on_device);
@@ -961,7 +975,7 @@ struct Session {
             return;
         }
         // embedding | all layers in one persistent kernel | output head
-        launch_embed(embd, tokens_dev.as<int32_t>(), 1, hidden_b.as<float>(), stream);
+        launch_embed(embd, d_tokens(), 1, hidden_b.as<float>(), stream);
         step_plan.launch(stream);
         MatTarget target{head, logits_b.as<float>(), vocab};
         launch_dec_multiply(&target, 1, hidden_b.as<float>(), output_norm, eps, hidden, EPI_STORE, sms, stream, nullptr);
@@ -970,12 +984,15 @@ struct Session {
     }
     // After the call's final synchronisation: did a barrier wait of the persistent kernel run out?
     void queue_step_check() {
-        // the few-token attention kernel waits for bulk copies (every wait bounded): its error word, read with the call's results
-        BK_CUDA(cudaMemcpyAsync(step_error_host + 2, chain_error_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
-        BK_CUDA(cudaMemcpyAsync(step_error_host + 3, gemm_tc_error_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
+        // The few-token attention and the tcgen05 multiply have bounded waits: their error words, read with the results of a call
+        // that may have run them. (A word is a copy of its own, about 2 us at the end of every call.)
+        if (batched) {
+            BK_CUDA(cudaMemcpyAsync(step_error_host + 2, chain_error_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
+            BK_CUDA(cudaMemcpyAsync(step_error_host + 3, gemm_tc_error_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
+        }
         if (peer_on) BK_CUDA(cudaMemcpyAsync(step_error_host + 1, peer_state.as<unsigned int>() + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
-        if (token_enabled) BK_CUDA(cudaMemcpyAsync(step_error_host, token_plan.error_word(), sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
-        else if (step_enabled) BK_CUDA(cudaMemcpyAsync(step_error_host, step_plan.error_word(), sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
+        if (token_enabled && persistent_steps != 0) BK_CUDA(cudaMemcpyAsync(step_error_host, token_plan.error_word(), sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
+        else if (persistent_steps != 0) BK_CUDA(cudaMemcpyAsync(step_error_host, step_plan.error_word(), sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
     }
     void finish_step_check() {
         if (step_error_host[3] != 0) {
@@ -1037,7 +1054,8 @@ struct Session {
         BK_CUDA(e);
     }
 
-    void step_on_device() {  // one token whose id is tokens_dev[0] at *d_position()
+    void step_on_device() {  // one token whose id is *d_tokens() at *d_position()
+        if (!single_kernels()) batched = true;
         // The fused weighted sum keeps a head's probabilities of the whole context in shared memory; past that the batched
         // kernels, which have no such limit, take single tokens too.
         const bool too_long = !step_active() && !variant_layers &&
@@ -1054,6 +1072,7 @@ struct Session {
     }
 
     void begin_call() {
+        batched = false;
         launches = 0;
         persistent_steps = 0;
         stats.h2d_bytes = stats.d2h_bytes = 0;
@@ -1081,13 +1100,8 @@ struct Session {
         BK_CUDA(cudaEventRecord(ev0, stream));
         for (uint64_t begin = 0; begin < n; begin += kMaxBatch) {
             const uint32_t cnt = uint32_t(std::min<uint64_t>(kMaxBatch, n - begin));
-            BK_CUDA(cudaStreamSynchronize(stream));  // tokens_host is reused
-            std::memcpy(tokens_host, tokens + begin, cnt * sizeof(int32_t));
-            const uint32_t pos32 = uint32_t(position);
-            std::memcpy(tokens_host + kMaxBatch, &pos32, sizeof(pos32));
-            BK_CUDA(cudaMemcpyAsync(tokens_dev.p, tokens_host, cnt * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-            BK_CUDA(cudaMemcpyAsync(d_position(), tokens_host + kMaxBatch, sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
-            stats.h2d_bytes += cnt * sizeof(int32_t) + sizeof(uint32_t);
+            if (begin != 0) BK_CUDA(cudaStreamSynchronize(stream));  // the staging buffer is reused; calls end synchronised
+            upload_inputs(tokens + begin, cnt);
             if (cnt == 1 && (!all || n == 1)) step_on_device();  // one token: its one row of logits is all there is, with or without `all`
             else forward(cnt, all ? ALL_LOGITS : begin + cnt == n ? LAST_LOGITS : NO_LOGITS, uint32_t(position + cnt));
             position += cnt;
@@ -1157,18 +1171,14 @@ struct Session {
         for (uint64_t begin = 0; begin < n; begin += kMaxBatch) {
             const uint32_t cnt = uint32_t(std::min<uint64_t>(kMaxBatch, n - begin));
             const uint32_t scored = begin < rows ? uint32_t(std::min<uint64_t>(cnt, rows - begin)) : 0;
-            collect();  // also: tokens_host is reused
+            collect();  // also: the staging buffer is reused
             const uint32_t staged = cnt + (begin + cnt < n ? 1 : 0);  // the next batch's first token is this batch's last target
-            std::memcpy(tokens_host, tokens + begin, staged * sizeof(int32_t));
-            tokens_host[kMaxBatch + 3] = int32_t(uint32_t(position));
-            BK_CUDA(cudaMemcpyAsync(tokens_dev.p, tokens_host, staged * sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-            BK_CUDA(cudaMemcpyAsync(d_position(), tokens_host + kMaxBatch + 3, sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
-            stats.h2d_bytes += staged * sizeof(int32_t) + sizeof(uint32_t);
+            upload_inputs(tokens + begin, staged);
             forward(cnt, NO_LOGITS, uint32_t(position + cnt));
             for (uint32_t first = 0; first < scored; first += kMaxScored) {
                 const uint32_t part = std::min(kMaxScored, scored - first);
                 head_rows(first, part);
-                launch_row_logp(logits_b.as<float>(), vocab, part, tokens_dev.as<int32_t>() + first + 1, score_dev.as<double>() + first, stream);
+                launch_row_logp(logits_b.as<float>(), vocab, part, d_tokens() + first + 1, score_dev.as<double>() + first, stream);
                 ++launches;
             }
             if (scored != 0) BK_CUDA(cudaMemcpyAsync(score_host, score_dev.p, scored * sizeof(double), cudaMemcpyDeviceToHost, stream));
@@ -1201,14 +1211,7 @@ struct Session {
             logit_history.p = nullptr;
             logit_history.alloc(steps * vocab * sizeof(float));
         }
-        const uint32_t pos32 = uint32_t(position);
-        tokens_host[0] = first;
-        std::memcpy(tokens_host + kMaxBatch, &pos32, sizeof(pos32));
-        tokens_host[kMaxBatch + 1] = 0;
-        tokens_host[kMaxBatch + 2] = 0;
-        BK_CUDA(cudaMemcpyAsync(tokens_dev.p, tokens_host, sizeof(int32_t), cudaMemcpyHostToDevice, stream));
-        BK_CUDA(cudaMemcpyAsync(scalars.p, tokens_host + kMaxBatch, 3 * sizeof(uint32_t), cudaMemcpyHostToDevice, stream));
-        stats.h2d_bytes += 4 * sizeof(int32_t);
+        upload_inputs(&first, 1);
         build_step_graph();
         BK_CUDA(cudaEventRecord(ev0, stream));
         const bool fused_pick = token_active() && !(flags & BRISK_CUDA_FLAG_NO_MEGAKERNEL);
@@ -1221,7 +1224,7 @@ struct Session {
             }
             if (!fused_pick) {
                 Scope sc(this, PH_SAMPLE);
-                launch_argmax_advance(logits_b.as<float>(), vocab, d_chosen(), am_val.as<float>(), am_idx.as<int32_t>(), tokens_dev.as<int32_t>(),
+                launch_argmax_advance(logits_b.as<float>(), vocab, d_chosen(), am_val.as<float>(), am_idx.as<int32_t>(), d_tokens(),
                                       d_position(), history.as<int32_t>(), d_history_len(), stream);
             }
             launches += 2;

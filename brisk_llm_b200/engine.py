@@ -22,6 +22,7 @@ class CudaSession:
                  tp_unique_id: bytes | None = None):
         self._lib = abi.load_library()
         self._h = None
+        self._logits = None
         opts = abi.Options()
         opts.max_context, opts.device, opts.flags = max_context, device, flags
         opts.tp_rank, opts.tp_size = tp_rank, tp_size
@@ -59,11 +60,10 @@ class CudaSession:
         out = C.POINTER(C.c_float)()
         if self._lib.brisk_cuda_eval(self._h, tokens.ctypes.data_as(C.POINTER(C.c_int32)), len(tokens), int(all_logits), C.byref(out)) != 0:
             self._fail()
-        rows = len(tokens) if all_logits else 1
-        view = np.ctypeslib.as_array(out, shape=(rows, self.vocab_size))  # pinned memory of the session
-        if copy:
-            view = view.copy()
-        return view if all_logits else view[0]
+        if self._logits is None:  # the session's pinned buffer never moves
+            self._logits = np.ctypeslib.as_array(out, shape=(MAX_SCORED_TOKENS, self.vocab_size))
+        view = self._logits[:len(tokens)] if all_logits else self._logits[0]
+        return view.copy() if copy else view
 
     def eval(self, tokens, copy: bool = True) -> np.ndarray:
         """Appends the tokens; logits (vocab floats) for the token after the last one. With copy=False the result is a

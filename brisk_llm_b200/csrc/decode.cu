@@ -121,13 +121,16 @@ void dispatch_dec(DecMatParams& p, bool pair, uint32_t sms, cudaStream_t s) {
         div2 = div2 && p.m[i].rows % 2 == 0;
     }
     // Rows per warp: more rows per warp share the activation loads and the serial adds (fewer instructions per weight
-    // byte), as long as about half of all warps still get a row group.
-    const uint32_t enough = sms * kDecWarps / 2;
-    constexpr bool heavy = sizeof(typename F::W) > 32;  // K-quants: many registers per row, cap the rows per warp
+    // byte), as long as enough of all warps still get a row group: half of them, a quarter for the formats with Q8_K
+    // activations, whose loads are heavier (measured: down projections 2048 x 8192 Q6_K 14.6 -> 12.7 us, 2560 x 6912 TQ2_0
+    // 14.3 -> 13.1; Q8_0 loses by it). The K-quants stop at two rows: four spill (28672 x 4096 Q4_K: one row per warp 31 us,
+    // two 27, four 35).
+    const uint32_t enough = sms * kDecWarps / (takes_q8_k(p.m[0].type) ? 4 : 2);
+    constexpr bool heavy = sizeof(typename F::W) > 32;
     int rw = 1;
     if (relaxed("rowsum")) div4 = false;
     if (div4 && !heavy && rows / 4 >= enough) rw = 4;
-    else if (div2 && (!heavy || !pair) && rows / 2 >= enough) rw = 2;
+    else if (div2 && rows / 2 >= enough) rw = 2;
     if (pair) {
         if (rw == 4) launch_dec_one<F, 4, true>(p, sms, s);
         else if (rw == 2) launch_dec_one<F, 2, true>(p, sms, s);

@@ -152,8 +152,8 @@ __global__ void __launch_bounds__(GWARPS * 32, MINB) gemm_q8_kernel(const __grid
     }
 #pragma unroll
     for (int i = 0; i < kXPieces; ++i) {
-        const uint32_t at = tid + i * THREADS, tok = min(tok_base + at / 8, p.n - 1);
-        xsrc[i] = p.act.q0 + size_t(tok) * p.act.cols + (at % 8) * 16;
+        const uint32_t at = tid + i * THREADS, tok = tok_base + at / 8;
+        xsrc[i] = tok < p.n ? p.act.q0 + size_t(tok) * p.act.cols + (at % 8) * 16 : nullptr;
     }
     const __half* dsrc = nullptr;
     if (tid < RT) {
@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(GWARPS * 32, MINB) gemm_q8_kernel(const __grid
         const uint32_t row = row_of(tid, mat);
         dsrc = mat->d + size_t(row) * nb;
     }
-    const float* xdsrc = p.act.d0 + size_t(min(tok_base + tid % TT, p.n - 1)) * nb;
+    const bool scales = tid < TT && tok_base + tid < p.n;  // this thread copies a token's scales
+    const float* xdsrc = p.act.d0 + size_t(scales ? tok_base + tid : 0) * nb;
     auto load_weights = [&](uint32_t slot, uint32_t chunk) {
         const uint32_t at = sbase + slot * S::kBytes;
 #pragma unroll
@@ -176,9 +177,11 @@ __global__ void __launch_bounds__(GWARPS * 32, MINB) gemm_q8_kernel(const __grid
 #pragma unroll
         for (int i = 0; i < kXPieces; ++i) {
             const uint32_t piece = tid + i * THREADS;
-            cp_async16(at + S::kW + S::kWd + piece / 8 * S::kXRow + piece % 8 * 16, xsrc[i] + size_t(chunk) * (KB * 32));
+            // Tokens past the last are left out: their rows of the MMAs hold whatever was there and are never stored. (A copy
+            // of the last token in their place had every CTA read the same few lines of L2 over and over.)
+            if (xsrc[i] != nullptr) cp_async16(at + S::kW + S::kWd + piece / 8 * S::kXRow + piece % 8 * 16, xsrc[i] + size_t(chunk) * (KB * 32));
         }
-        if (tid < TT) cp_async16(at + S::kW + S::kWd + S::kX + tid * (KB * 4), xdsrc + size_t(chunk) * KB);
+        if (scales) cp_async16(at + S::kW + S::kWd + S::kX + tid * (KB * 4), xdsrc + size_t(chunk) * KB);
     };
 
     f32x2 acc[MI][NI][2];  // [..][0]: rows 2t, 2t + 1 of token g, [..][1]: of token g + 8
@@ -403,12 +406,11 @@ static bool gemm_tc_on() {
     return env == nullptr ? kGemmTcDefault : std::strcmp(env, "tc") == 0;
 }
 bool gemm_k_supports(int type);  // gemm_k.cu: the 256-value super-block formats
-void launch_gemm_k(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s);
+void launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t sms, cudaStream_t s);
 
-// Q4_0 / Q8_0 rows of a multiple of 4 blocks (128 values) from 2 tokens on; the super-block formats from 16 on.
+// From 2 tokens on: Q4_0 / Q8_0 rows of a multiple of 4 blocks (128 values), and the super-block formats.
 static bool gemm_supports(int type, uint32_t cols, uint32_t n) {
-    if (type == T_Q4_0 || type == T_Q8_0) return cols % (32 * KB) == 0 && n >= 2;
-    return gemm_k_supports(type) && n >= kGemmMinTokens;
+    return n >= 2 && (type == T_Q4_0 || type == T_Q8_0 ? cols % (32 * KB) == 0 : gemm_k_supports(type));
 }
 
 int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s) {
@@ -419,8 +421,8 @@ int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t
     const int type = targets[0].m.type;
     if (type != T_Q4_0 && type != T_Q8_0) {
         if (pair) return 0;
-        for (int i = 0; i < count; ++i) launch_gemm_k(targets[i], act, n, epi, s);
-        return count;
+        launch_gemm_k(targets, count, act, n, epi, sm_count(), s);
+        return 1;
     }
     if (!pair && n >= 32 && gemm_tc_on() && gemm_tc_supports(type, targets[0].m.cols)) {
         for (int i = 0; i < count; ++i) launch_gemm_tc(targets[i], act, n, epi, s);

@@ -18,14 +18,15 @@
 // the row's eight minimums replace eight multiply-adds per output. Measured: prompts of 777 tokens, ternary 2B shape
 // 30.0 -> 27.1 ms, Q5_K_M 1B shape (its Q5_K matrices went through the streaming kernel) 119.7 -> 18.6 ms; 1023 tokens of
 // the Q4_K_M 1B shape 21.5 -> 20.0 ms.
-// Tiling as in gemm.cu: CTA = 128 rows x 64 tokens, 8 warps of 32 x 32, two cp.async stages of one super-block each.
+// Tiling as in gemm.cu: the tile is picked from rows, tokens and row length (launch_type); stages of one super-block come
+// through a cp.async ring, and targets of one type share a launch.
+#include <algorithm>
+
 #include "kernels.h"
 #include "pdl.cuh"
 
 namespace bk {
 namespace {
-
-constexpr int KM = 128, KN = 64, KWARPS = 8;
 
 __device__ __forceinline__ void cp16(void* smem, const void* gmem) {
     const uint32_t a = uint32_t(__cvta_generic_to_shared(smem));
@@ -52,16 +53,18 @@ __device__ __forceinline__ void mma_k16_from(int (&d)[4], uint32_t a0, uint32_t 
 __device__ __forceinline__ uint32_t fifth_bits(uint32_t bits) { return (((bits & 0xFu) * 0x00204081u) & 0x01010101u) << 4; }
 
 struct KParams {
-    DevMatrix m;
+    DevMatrix m[3];
+    float* out[3];
+    uint32_t ldo[3];
+    uint32_t first_tile[4];  // row tiles of target i: [first_tile[i], first_tile[i + 1])
     DevAct act;
-    float* out;
-    uint32_t ldo, n;
-    int epi;
+    uint32_t n;
+    int count, epi;
 };
 
 // Shared-memory stage of one super-block. Row strides carry 16 bytes of padding so that the 8 rows a warp's fragment
 // loads touch fall into different banks.
-template <int TYPE>
+template <int TYPE, int KM, int KN>
 struct KStage {
     static constexpr bool kMins = TYPE == T_Q4_K || TYPE == T_Q5_K;
     static constexpr int kQ = TYPE == T_TQ2_0 ? 64 : TYPE == T_Q4_K ? 128 : TYPE == T_Q5_K ? 160 : 192;  // quant bytes per row and super-block
@@ -77,68 +80,91 @@ struct KStage {
     static constexpr int kBytes = kA + kSc + kD + kB + kBd + kBs;
 };
 
-template <int TYPE>
-__global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p) {
-    using S = KStage<TYPE>;
-    extern __shared__ __align__(16) unsigned char smem[];
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// Warps of 16 MI rows x 8 NI tokens, WR of them along the rows and WT along the tokens.
+//
+// KS > 1, for few tokens and long rows: KS warps on the same rows and tokens take every KS-th super-block, each with stages
+// of its own. Only the sum of a row's terms is serial: the terms of a round meet in shared memory and every thread adds those
+// of its outputs in super-block order. (One warp walks a super-block in 1.4 us, 2048 x 8192 Q6_K in 44 us whatever the tile.)
+template <int TYPE, int MI, int NI, int WR, int WT, int KS, int STAGES, int RESIDENT>
+__global__ void __launch_bounds__(WR * WT * KS * 32, RESIDENT) gemm_k_kernel(const __grid_constant__ KParams p) {
+    static_assert(KS == 1 || (WR == 1 && WT == 1), "a split row has one warp per share");
+    constexpr uint32_t KM = 16 * MI * WR, KN = 8 * NI * WT, ALL = WR * WT * KS * 32, THREADS = ALL / KS;  // THREADS fill a stage
+    using S = KStage<TYPE, KM, KN>;
+    static_assert(KM <= THREADS && KN <= THREADS, "a thread stages one row's and one token's scales at most");
+    extern __shared__ __align__(16) unsigned char smem_all[];
+    const uint32_t tid = threadIdx.x % THREADS, ks = threadIdx.x / THREADS, lane = tid & 31, warp = tid >> 5;
+    unsigned char* smem = smem_all + size_t(ks) * STAGES * S::kBytes;
+    constexpr uint32_t kOutputs = MI * NI * 128, kMine = KS > 1 ? kOutputs / ALL : 1;  // split rows: outputs of the CTA and of a thread
+    float* terms = reinterpret_cast<float*>(smem_all + size_t(KS) * STAGES * S::kBytes);  // [2][KS][kOutputs]
     const uint32_t g = lane >> 2, t = lane & 3;
-    const uint32_t row_base = blockIdx.x * KM, tok_base = blockIdx.y * KN;
-    const uint32_t wr = (warp & 3) * 32, wt = (warp >> 2) * 32;
-    const uint32_t nsb = p.m.blocks;  // super-blocks per row
+    int target = 0;
+    if (p.count > 1 && blockIdx.x >= p.first_tile[1]) target = 1;
+    if (p.count > 2 && blockIdx.x >= p.first_tile[2]) target = 2;
+    const DevMatrix& m = p.m[target];
+    const uint32_t row_base = (blockIdx.x - p.first_tile[target]) * KM, tok_base = blockIdx.y * KN;
+    const uint32_t wr = warp % WR * (16 * MI), wt = warp / WR * (8 * NI);
+    const uint32_t nsb = m.blocks, rounds = (nsb + KS - 1) / KS;  // super-blocks per row
+    auto block_of = [&](uint32_t round) { return round * KS + ks; };
 
-    auto load_stage = [&](int s, uint32_t sb) {
-        unsigned char* base = smem + size_t(s) * S::kBytes;
-        constexpr int kPieces = S::kQ / 16;
-        for (uint32_t i = tid; i < KM * kPieces; i += KWARPS * 32) {
+    auto load_weights = [&](uint32_t slot, uint32_t sb) {
+        unsigned char* base = smem + size_t(slot) * S::kBytes;
+        constexpr uint32_t kPieces = S::kQ / 16;
+        for (uint32_t i = tid; i < KM * kPieces; i += THREADS) {
             const uint32_t r = i / kPieces, piece = i % kPieces;
-            const uint32_t row = min(row_base + r, p.m.rows - 1);
+            const size_t at = size_t(min(row_base + r, m.rows - 1)) * nsb + sb;
             const unsigned char* src;
-            if (TYPE == T_Q6_K) {
-                // three planes of 64 bytes per super-block: qa | qb | qc
-                const uint8_t* plane = piece < 4 ? p.m.qa : piece < 8 ? p.m.qb : p.m.qc;
-                src = plane + (size_t(row) * nsb + sb) * 64 + (piece & 3) * 16;
+            if (TYPE == T_Q6_K) {  // three planes of 64 bytes per super-block: qa | qb | qc
+                const uint8_t* plane = piece < 4 ? m.qa : piece < 8 ? m.qb : m.qc;
+                src = plane + at * 64 + (piece & 3) * 16;
             } else if (TYPE == T_Q5_K && piece >= 8) {
-                src = p.m.qb + (size_t(row) * nsb + sb) * 32 + (piece - 8) * 16;  // the units' fifth bits, one u32 each
+                src = m.qb + at * 32 + (piece - 8) * 16;  // the units' fifth bits, one u32 each
             } else if (TYPE == T_Q5_K) {
-                src = p.m.qa + (size_t(row) * nsb + sb) * 128 + piece * 16;
+                src = m.qa + at * 128 + piece * 16;
             } else {
-                src = p.m.qa + (size_t(row) * nsb + sb) * S::kQ + piece * 16;
+                src = m.qa + at * S::kQ + piece * 16;
             }
             cp16(base + r * S::kARow + piece * 16, src);
         }
-        if (TYPE != T_TQ2_0) {
-            for (uint32_t r = tid; r < KM; r += KWARPS * 32) {
-                const uint32_t row = min(row_base + r, p.m.rows - 1);
-                cp16(base + S::kA + r * 16, p.m.sc + (size_t(row) * nsb + sb) * 16);
-            }
-        }
-        // d planes are 2 (TQ2_0, Q6_K) or 4 (Q4_K) bytes per super-block: too small for cp.async, plain loads
-        uint16_t* dd = reinterpret_cast<uint16_t*>(base + S::kA + S::kSc);
-        for (uint32_t r = tid; r < KM; r += KWARPS * 32) {
-            const uint32_t row = min(row_base + r, p.m.rows - 1);
-            const uint16_t* src = reinterpret_cast<const uint16_t*>(p.m.d);
-            if (S::kMins) {
-                dd[2 * r] = src[2 * (size_t(row) * nsb + sb)];
-                dd[2 * r + 1] = src[2 * (size_t(row) * nsb + sb) + 1];
-            } else {
-                dd[2 * r] = src[size_t(row) * nsb + sb];
-            }
-        }
-        unsigned char* bq = base + S::kA + S::kSc + S::kD;
-        for (uint32_t i = tid; i < KN * 16; i += KWARPS * 32) {
+        if (TYPE != T_TQ2_0 && tid < KM) cp16(base + S::kA + tid * 16, m.sc + (size_t(min(row_base + tid, m.rows - 1)) * nsb + sb) * 16);
+    };
+    auto load_tokens = [&](uint32_t slot, uint32_t sb) {
+        unsigned char* bq = smem + size_t(slot) * S::kBytes + S::kA + S::kSc + S::kD;
+        for (uint32_t i = tid; i < KN * 16; i += THREADS) {
             const uint32_t r = i >> 4, piece = i & 15;
-            const uint32_t tok = min(tok_base + r, p.n - 1);
-            cp16(bq + r * S::kBRow + piece * 16, p.act.qk + size_t(tok) * p.act.cols + sb * 256 + piece * 16);
+            // Tokens past the last are left out: their columns of the MMAs hold whatever was there and are never stored. (A copy of
+            // the last token in their place made 2 tokens slower than 16: every CTA read the same few lines over and over.)
+            if (tok_base + r < p.n) cp16(bq + r * S::kBRow + piece * 16, p.act.qk + size_t(tok_base + r) * p.act.cols + sb * 256 + piece * 16);
         }
-        float* bd = reinterpret_cast<float*>(bq + S::kB);
-        unsigned char* bs = bq + S::kB + S::kBd;
-        for (uint32_t r = tid; r < KN; r += KWARPS * 32) {
-            const uint32_t tok = min(tok_base + r, p.n - 1);
-            bd[r] = p.act.dk[size_t(tok) * nsb + sb];
-            const uint4* sums = reinterpret_cast<const uint4*>(p.act.bs + (size_t(tok) * nsb + sb) * 16);
-            const uint4 lo = sums[0], hi = sums[1];
-            const uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};  // two sums of 16 each
+    };
+    // What is too small or too raw for cp.async goes through registers, loaded a super-block before it is stored: the row's d
+    // (and dmin), the token's scale and its sums of 16.
+    const uint32_t srow = min(row_base + tid, m.rows - 1), stok = tok_base + tid;
+    uint32_t next_d = 0;
+    float next_dx = 0.0f;
+    uint4 next_lo{}, next_hi{};
+    auto fetch_row = [&](uint32_t sb) {
+        if (tid < KM && sb < nsb) {
+            if (S::kMins) next_d = reinterpret_cast<const uint32_t*>(m.d)[size_t(srow) * nsb + sb];
+            else next_d = reinterpret_cast<const uint16_t*>(m.d)[size_t(srow) * nsb + sb];
+        }
+    };
+    auto fetch_token = [&](uint32_t sb) {
+        if (tid < KN && stok < p.n && sb < nsb) {
+            next_dx = p.act.dk[size_t(stok) * nsb + sb];
+            const uint4* sums = reinterpret_cast<const uint4*>(p.act.bs + (size_t(stok) * nsb + sb) * 16);
+            next_lo = sums[0];
+            next_hi = sums[1];
+        }
+    };
+    auto store_scales = [&](uint32_t slot) {
+        unsigned char* base = smem + size_t(slot) * S::kBytes;
+        if (tid < KM) reinterpret_cast<uint32_t*>(base + S::kA + S::kSc)[tid] = next_d;
+        if (tid < KN) {
+            float* bd = reinterpret_cast<float*>(base + S::kA + S::kSc + S::kD + S::kB);
+            unsigned char* bs = reinterpret_cast<unsigned char*>(bd) + S::kBd;
+            const uint32_t r = tid;
+            bd[r] = next_dx;
+            const uint32_t w[8] = {next_lo.x, next_lo.y, next_lo.z, next_lo.w, next_hi.x, next_hi.y, next_hi.z, next_hi.w};  // two sums of 16 each
             if constexpr (TYPE == T_Q6_K) {
 #pragma unroll
                 for (int k = 0; k < 8; ++k) {
@@ -161,28 +187,55 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
                 *reinterpret_cast<uint4*>(bs + r * 16) = make_uint4(low[0], low[1], high[0], high[1]);
             }
         }
-        asm volatile("cp.async.commit_group;" ::: "memory");
     };
 
-    float acc[2][4][4];
+    float sums[kMine] = {};  // split rows
+    float acc[MI][NI][4];
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
+    for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+        for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
             for (int j = 0; j < 4; ++j) acc[mi][ni][j] = 0.0f;
 
+    // the weights of the first stages before the activations are there
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i) {
+        if (block_of(i) < nsb) load_weights(i, block_of(i));
+    }
+    fetch_row(block_of(0));
     wait_for_previous();
-    load_stage(0, 0);
-    for (uint32_t sb = 0; sb < nsb; ++sb) {
-        if (sb + 1 < nsb) {
-            load_stage((sb + 1) & 1, sb + 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (p.n <= 64) release_next();  // few CTAs will wait beside this kernel
+    fetch_token(block_of(0));
+#pragma unroll
+    for (int i = 0; i < STAGES - 1; ++i) {
+        if (block_of(i) < nsb) {
+            load_tokens(i, block_of(i));
+            store_scales(i);
         }
-        __syncthreads();
-        const unsigned char* base = smem + size_t(sb & 1) * S::kBytes;
+        fetch_row(block_of(i + 1));
+        fetch_token(block_of(i + 1));
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    }
+    uint32_t slot = 0, fill = STAGES - 1;
+    for (uint32_t round = 0; round < rounds; ++round) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
+        // the stage has landed for every thread that reads it, and the slot filled next is no longer read
+        if constexpr (KS == 1) __syncthreads();
+        else __syncwarp();
+        if (block_of(round + STAGES - 1) < nsb) {
+            load_weights(fill, block_of(round + STAGES - 1));
+            load_tokens(fill, block_of(round + STAGES - 1));
+            store_scales(fill);
+            fetch_row(block_of(round + STAGES));
+            fetch_token(block_of(round + STAGES));
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        fill = fill + 1 == STAGES ? 0 : fill + 1;
+        const unsigned char* base = smem + size_t(slot) * S::kBytes;
+        slot = slot + 1 == STAGES ? 0 : slot + 1;
+        const bool here = block_of(round) < nsb;  // the last round of a split row may leave warps without a super-block
+        if (here) {
         const unsigned char* aq = base;
         const unsigned char* asc = base + S::kA;
         const __half* ad = reinterpret_cast<const __half*>(base + S::kA + S::kSc);
@@ -191,11 +244,11 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
         const unsigned char* bs = bq + S::kB + S::kBd;
 
         // integer accumulators of this super-block: [row tile][token tile][4 results]
-        int weighted[2][4][4], offsets[2][4][4];  // offsets: Q4_K / Q5_K only
+        int weighted[MI][NI][4], offsets[MI][NI][4];  // offsets: Q4_K / Q5_K only
 #pragma unroll
-        for (int mi = 0; mi < 2; ++mi)
+        for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni)
+            for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     weighted[mi][ni][j] = 0;
@@ -205,9 +258,9 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
         if constexpr (TYPE == T_TQ2_0) {
 #pragma unroll
             for (int jj = 0; jj < 2; ++jj) {  // halves of 128 values: units 2jj (k 0..15 of each run) and 2jj+1 (k 16..31)
-                uint32_t w0[2][2], w1[2][2];
+                uint32_t w0[MI][2], w1[MI][2];
 #pragma unroll
-                for (int mi = 0; mi < 2; ++mi) {
+                for (int mi = 0; mi < MI; ++mi) {
                     const uint32_t r0 = wr + mi * 16 + g, r1 = r0 + 8;
                     w0[mi][0] = *reinterpret_cast<const uint32_t*>(aq + r0 * S::kARow + (2 * jj) * 16 + 4 * t);
                     w0[mi][1] = *reinterpret_cast<const uint32_t*>(aq + r0 * S::kARow + (2 * jj + 1) * 16 + 4 * t);
@@ -218,12 +271,12 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
                 for (int l = 0; l < 4; ++l) {  // run l: values jj*128 + 32l .. +31
                     const int kofs = jj * 128 + l * 32;
 #pragma unroll
-                    for (int ni = 0; ni < 4; ++ni) {
+                    for (int ni = 0; ni < NI; ++ni) {
                         const unsigned char* brow = bq + (wt + ni * 8 + g) * S::kBRow + kofs;
                         const uint32_t b0 = *reinterpret_cast<const uint32_t*>(brow + 4 * t);
                         const uint32_t b1 = *reinterpret_cast<const uint32_t*>(brow + 16 + 4 * t);
 #pragma unroll
-                        for (int mi = 0; mi < 2; ++mi) {
+                        for (int mi = 0; mi < MI; ++mi) {
                             mma_k32(weighted[mi][ni], (w0[mi][0] >> (2 * l)) & 0x03030303u, (w1[mi][0] >> (2 * l)) & 0x03030303u,
                                     (w0[mi][1] >> (2 * l)) & 0x03030303u, (w1[mi][1] >> (2 * l)) & 0x03030303u, b0, b1);
                         }
@@ -233,11 +286,11 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
         } else if constexpr (S::kMins) {
 #pragma unroll
             for (int ch = 0; ch < 4; ++ch) {  // 64-value chunk: sub-blocks 2ch (low nibbles) and 2ch+1 (high nibbles)
-                uint32_t w0[2][2], w1[2][2];
-                uint32_t f0[2][2], f1[2][2];   // Q5_K: the fifth bits of rows g and g + 8, this thread's four of each half
-                int sc[2][2][2];               // [row tile][row g / g+8][sub-block low / high]
+                uint32_t w0[MI][2], w1[MI][2];
+                uint32_t f0[MI][2], f1[MI][2];   // Q5_K: the fifth bits of rows g and g + 8, this thread's four of each half
+                int sc[MI][2][2];               // [row tile][row g / g+8][sub-block low / high]
 #pragma unroll
-                for (int mi = 0; mi < 2; ++mi) {
+                for (int mi = 0; mi < MI; ++mi) {
                     const uint32_t r0 = wr + mi * 16 + g, r1 = r0 + 8;
                     w0[mi][0] = *reinterpret_cast<const uint32_t*>(aq + r0 * S::kARow + (2 * ch) * 16 + 4 * t);
                     w0[mi][1] = *reinterpret_cast<const uint32_t*>(aq + r0 * S::kARow + (2 * ch + 1) * 16 + 4 * t);
@@ -259,9 +312,9 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
                     const int sbk = 2 * ch + h;
-                    uint32_t v[2][4];
+                    uint32_t v[MI][4];
 #pragma unroll
-                    for (int mi = 0; mi < 2; ++mi) {
+                    for (int mi = 0; mi < MI; ++mi) {
                         v[mi][0] = (w0[mi][0] >> (4 * h)) & 0x0F0F0F0Fu;
                         v[mi][1] = (w1[mi][0] >> (4 * h)) & 0x0F0F0F0Fu;
                         v[mi][2] = (w0[mi][1] >> (4 * h)) & 0x0F0F0F0Fu;
@@ -274,12 +327,12 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
                         }
                     }
 #pragma unroll
-                    for (int ni = 0; ni < 4; ++ni) {
+                    for (int ni = 0; ni < NI; ++ni) {
                         const unsigned char* brow = bq + (wt + ni * 8 + g) * S::kBRow + sbk * 32;
                         const uint32_t b0 = *reinterpret_cast<const uint32_t*>(brow + 4 * t);
                         const uint32_t b1 = *reinterpret_cast<const uint32_t*>(brow + 16 + 4 * t);
 #pragma unroll
-                        for (int mi = 0; mi < 2; ++mi) {
+                        for (int mi = 0; mi < MI; ++mi) {
                             int c[4] = {0, 0, 0, 0};
                             mma_k32(c, v[mi][0], v[mi][1], v[mi][2], v[mi][3], b0, b1);
                             weighted[mi][ni][0] += sc[mi][0][h] * c[0];
@@ -292,12 +345,12 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
             }
             // offsets = sum over the eight sub-blocks of min * sum(x): the minimums against both digits (k = 0 .. 7 of 16)
 #pragma unroll
-            for (int mi = 0; mi < 2; ++mi) {
+            for (int mi = 0; mi < MI; ++mi) {
                 const uint32_t r0 = wr + mi * 16 + g, r1 = r0 + 8;
                 const uint32_t m0 = t < 2 ? *reinterpret_cast<const uint32_t*>(asc + r0 * 16 + 8 + 4 * t) : 0u;
                 const uint32_t m1 = t < 2 ? *reinterpret_cast<const uint32_t*>(asc + r1 * 16 + 8 + 4 * t) : 0u;
 #pragma unroll
-                for (int ni = 0; ni < 4; ++ni) {
+                for (int ni = 0; ni < NI; ++ni) {
                     const unsigned char* digits = bs + (wt + ni * 8 + g) * 16 + 4 * (t & 1);
                     int high[4] = {0, 0, 0, 0};
                     mma_k16(high, m0, m1, *reinterpret_cast<const uint32_t*>(digits + 8));
@@ -309,9 +362,9 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
         } else {  // Q6_K
 #pragma unroll
             for (int u = 0; u < 4; ++u) {  // unit u: 64 values = four runs of 16: k-th run at (u>>1)*128 + 32k + (u&1)*16
-                uint32_t a[2][2], b[2][2], cc[2][2];
+                uint32_t a[MI][2], b[MI][2], cc[MI][2];
 #pragma unroll
-                for (int mi = 0; mi < 2; ++mi) {
+                for (int mi = 0; mi < MI; ++mi) {
 #pragma unroll
                     for (int hh = 0; hh < 2; ++hh) {
                         const uint32_t r = wr + mi * 16 + g + hh * 8;
@@ -324,10 +377,10 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
                 for (int k = 0; k < 4; ++k) {
                     const int grp = (u >> 1) * 8 + 2 * k + (u & 1);  // 16-value group inside the super-block
                     const int kofs = (u >> 1) * 128 + 32 * k + (u & 1) * 16;
-                    uint32_t v[2][2];
-                    int sc[2][2];
+                    uint32_t v[MI][2];
+                    int sc[MI][2];
 #pragma unroll
-                    for (int mi = 0; mi < 2; ++mi) {
+                    for (int mi = 0; mi < MI; ++mi) {
 #pragma unroll
                         for (int hh = 0; hh < 2; ++hh) {
                             const uint32_t L = 0x0F0F0F0Fu, H = 0x30303030u;
@@ -338,12 +391,12 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
                         }
                     }
 #pragma unroll
-                    for (int ni = 0; ni < 4; ++ni) {
+                    for (int ni = 0; ni < NI; ++ni) {
                         const uint32_t tb = wt + ni * 8;
                         const uint32_t b0 = *reinterpret_cast<const uint32_t*>(bq + (tb + g) * S::kBRow + kofs + 4 * t);
                         const int2 o = *reinterpret_cast<const int2*>(reinterpret_cast<const int*>(bs) + grp * KN + tb + 2 * t);
 #pragma unroll
-                        for (int mi = 0; mi < 2; ++mi) {
+                        for (int mi = 0; mi < MI; ++mi) {
                             int c[4];
                             mma_k16_from(c, v[mi][0], v[mi][1], b0, o.x, o.y);
                             weighted[mi][ni][0] += sc[mi][0] * c[0];
@@ -358,12 +411,12 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
 
         // the super-block's float term, added to the running sums in super-block order
 #pragma unroll
-        for (int mi = 0; mi < 2; ++mi) {
+        for (int mi = 0; mi < MI; ++mi) {
             const uint32_t r0 = wr + mi * 16 + g, r1 = r0 + 8;
             const float dw0 = __half2float(ad[2 * r0]), dw1 = __half2float(ad[2 * r1]);
             const float dm0 = S::kMins ? __half2float(ad[2 * r0 + 1]) : 0.0f, dm1 = S::kMins ? __half2float(ad[2 * r1 + 1]) : 0.0f;
 #pragma unroll
-            for (int ni = 0; ni < 4; ++ni) {
+            for (int ni = 0; ni < NI; ++ni) {
                 const uint32_t c0 = wt + ni * 8 + 2 * t, c1 = c0 + 1;
                 const float dx0 = bd[c0], dx1 = bd[c1];
                 float term[4];
@@ -384,48 +437,120 @@ __global__ void __launch_bounds__(KWARPS * 32, 1) gemm_k_kernel(const KParams p)
                     term[3] = __fmul_rn(__fmul_rn(dx1, dw1), float(weighted[mi][ni][3] - xs1));
                 }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[mi][ni][j] = __fadd_rn(acc[mi][ni][j], term[j]);
+                for (int j = 0; j < 4; ++j) {
+                    if constexpr (KS == 1) acc[mi][ni][j] = __fadd_rn(acc[mi][ni][j], term[j]);
+                    else terms[((round & 1) * KS + ks) * kOutputs + ((mi * NI + ni) * 4 + j) * 32 + lane] = term[j];
+                }
             }
         }
-        __syncthreads();
+        }
+        if constexpr (KS > 1) {
+            __syncthreads();  // the round's terms are there; those of the round before last are no longer read
+            const uint32_t valid = min(uint32_t(KS), nsb - round * KS);
+#pragma unroll
+            for (uint32_t e = 0; e < kMine; ++e) {
+                const float* mine = terms + (round & 1) * KS * kOutputs + threadIdx.x + e * ALL;
+#pragma unroll
+                for (int k = 0; k < KS; ++k) {
+                    if (uint32_t(k) < valid) sums[e] = __fadd_rn(sums[e], mine[k * kOutputs]);
+                }
+            }
+        }
     }
-    release_next();
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    if (p.n > 64) release_next();
+    auto store = [&](uint32_t row, uint32_t tok, float value) {
+        if (row < m.rows && tok < p.n) {
+            float* o = p.out[target] + size_t(tok) * p.ldo[target] + row;
+            *o = p.epi == EPI_ADD ? __fadd_rn(*o, value) : value;
+        }
+    };
+    if constexpr (KS > 1) {
+#pragma unroll
+        for (uint32_t e = 0; e < kMine; ++e) {
+            const uint32_t f = threadIdx.x + e * ALL, l = f & 31, j = (f >> 5) & 3, ni = (f >> 7) % NI, mi = (f >> 7) / NI;
+            store(row_base + mi * 16 + (l >> 2) + (j >= 2 ? 8 : 0), tok_base + ni * 8 + 2 * (l & 3) + (j & 1), sums[e]);
+        }
+        return;
+    }
 
 #pragma unroll
-    for (int mi = 0; mi < 2; ++mi)
+    for (int mi = 0; mi < MI; ++mi)
 #pragma unroll
-        for (int ni = 0; ni < 4; ++ni)
+        for (int ni = 0; ni < NI; ++ni)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
-                const uint32_t row = row_base + wr + mi * 16 + g + (j >= 2 ? 8 : 0);
-                const uint32_t tok = tok_base + wt + ni * 8 + 2 * t + (j & 1);
-                if (row < p.m.rows && tok < p.n) {
-                    float* o = p.out + size_t(tok) * p.ldo + row;
-                    *o = p.epi == EPI_ADD ? __fadd_rn(*o, acc[mi][ni][j]) : acc[mi][ni][j];
-                }
+                store(row_base + wr + mi * 16 + g + (j >= 2 ? 8 : 0), tok_base + wt + ni * 8 + 2 * t + (j & 1), acc[mi][ni][j]);
             }
 }
 
+struct KTile {
+    uint32_t rows, tokens, split, threads, resident, smem;
+    uint64_t alone, shared;  // ns of a super-block (Q4_K): of one CTA by itself, and per CTA of a full SM
+    void (*kernel)(KParams);
+};
+
+template <int TYPE, int MI, int NI, int WR, int WT, int KS, int STAGES, int RESIDENT>
+KTile tile_of(uint64_t alone, uint64_t shared) {
+    const uint32_t stages = KS * STAGES * KStage<TYPE, 16 * MI * WR, 8 * NI * WT>::kBytes, terms = KS > 1 ? 2 * KS * MI * NI * 128 * 4 : 0;
+    return KTile{16 * MI * WR, 8 * NI * WT, KS, WR * WT * KS * 32, RESIDENT, stages + terms, alone, shared, gemm_k_kernel<TYPE, MI, NI, WR, WT, KS, STAGES, RESIDENT>};
+}
+
+// The tile whose busiest SM is done first, as in gemm.cu; 800 ns for what a CTA does besides its super-blocks. The other types'
+// figures are the same within their common factor. Measured, Q4_K: 2048 x 8192 at 9 tokens 65 (128 x 64 tiles) / 25 (64 x 16)
+// / 7.9 us (16 x 16, split), 14336 x 4096 at 9 tokens 80 / 20 / 24, 2048 x 2048 at 512 tokens 18.8 / 30 / -.
 template <int TYPE>
-void launch_one(const KParams& p, cudaStream_t s) {
-    constexpr size_t smem = 2 * KStage<TYPE>::kBytes;
+void launch_type(KParams& p, uint32_t sms, cudaStream_t s) {
+    static const KTile tiles[] = {
+        tile_of<TYPE, 2, 4, 4, 2, 1, 2, 1>(2000, 2000), tile_of<TYPE, 1, 4, 4, 2, 1, 2, 2>(1250, 1060), tile_of<TYPE, 1, 2, 4, 1, 1, 4, 4>(770, 540),
+        tile_of<TYPE, 1, 2, 1, 1, 8, 2, 1>(210, 230), tile_of<TYPE, 1, 1, 1, 1, 4, 3, 3>(200, 137),
+    };
     static DeviceOnce once;
-    if (once.first()) BK_CUDA(cudaFuncSetAttribute(gemm_k_kernel<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    const dim3 grid((p.m.rows + KM - 1) / KM, (p.n + KN - 1) / KN);
-    launch_dependent(gemm_k_kernel<TYPE>, grid, dim3(KWARPS * 32), smem, s, p);
+    if (once.first()) {
+        for (const KTile& tile : tiles) BK_CUDA(cudaFuncSetAttribute(tile.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile.smem)));
+    }
+    const KTile* pick = nullptr;
+    uint64_t best = 0;
+    for (const KTile& tile : tiles) {
+        uint64_t ctas = 0;
+        for (int i = 0; i < p.count; ++i) ctas += (p.m[i].rows + tile.rows - 1) / tile.rows;
+        ctas *= (p.n + tile.tokens - 1) / tile.tokens;
+        const uint64_t per_sm = (ctas + sms - 1) / sms, rounds = (per_sm + tile.resident - 1) / tile.resident;
+        const uint64_t blocks = (p.m[0].blocks + tile.split - 1) / tile.split * tile.split;
+        const uint64_t cost = std::max(rounds * (tile.alone * blocks + 800), per_sm * tile.shared * blocks);
+        if (pick == nullptr || cost < best) {
+            pick = &tile;
+            best = cost;
+        }
+    }
+    uint32_t row_tiles = 0;
+    for (int i = 0; i < p.count; ++i) {
+        p.first_tile[i] = row_tiles;
+        row_tiles += (p.m[i].rows + pick->rows - 1) / pick->rows;
+    }
+    launch_dependent(pick->kernel, dim3(row_tiles, (p.n + pick->tokens - 1) / pick->tokens), dim3(pick->threads), pick->smem, s, p);
 }
 
 }  // namespace
 
 bool gemm_k_supports(int type) { return type == T_Q4_K || type == T_Q5_K || type == T_Q6_K || type == T_TQ2_0; }
 
-void launch_gemm_k(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s) {
-    const KParams p{tg.m, act, tg.out, tg.ldo, n, int(epi)};
-    switch (tg.m.type) {
-        case T_Q4_K: launch_one<T_Q4_K>(p, s); break;
-        case T_Q5_K: launch_one<T_Q5_K>(p, s); break;
-        case T_Q6_K: launch_one<T_Q6_K>(p, s); break;
-        case T_TQ2_0: launch_one<T_TQ2_0>(p, s); break;
+void launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t sms, cudaStream_t s) {
+    KParams p{};
+    for (int i = 0; i < count; ++i) {
+        p.m[i] = targets[i].m;
+        p.out[i] = targets[i].out;
+        p.ldo[i] = targets[i].ldo;
+    }
+    p.act = act;
+    p.n = n;
+    p.count = count;
+    p.epi = int(epi);
+    switch (targets[0].m.type) {
+        case T_Q4_K: launch_type<T_Q4_K>(p, sms, s); break;
+        case T_Q5_K: launch_type<T_Q5_K>(p, sms, s); break;
+        case T_Q6_K: launch_type<T_Q6_K>(p, sms, s); break;
+        case T_TQ2_0: launch_type<T_TQ2_0>(p, sms, s); break;
         default: throw CudaError("cuda: no super-block tensor kernel for this type");
     }
 }

@@ -19,12 +19,12 @@ def test_tiles(fmt, rows, cols):
 
 
 @pytest.mark.parametrize("fmt", (F.Q4_K, F.Q5_K, F.Q6_K, F.TQ2_0), ids=lambda f: F.NAMES[f])
-@pytest.mark.parametrize("rows,cols", [(1, 256), (127, 512), (129, 768)])
+@pytest.mark.parametrize("rows,cols", [(1, 256), (127, 512), (129, 2304), (4100, 1024)])
 def test_super_block_tiles(fmt, rows, cols):
     wb, _ = H.random_matrix(fmt, rows, cols, seed=rows)
     x = np.random.default_rng(cols).standard_normal((129, cols)).astype(np.float32)
     x[3] = 1.0  # equal values: sums of 16 and 32 at their largest
     x[4] = -1.0
     want = H.oracle_matmul(fmt, wb, rows, cols, x)
-    for n in (16, 65, 129):
+    for n in (2, 8, 9, 16, 17, 65, 129):
         assert np.array_equal(engine.matmul(fmt, wb, rows, cols, x[:n]), want[:n]), n

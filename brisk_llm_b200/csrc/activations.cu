@@ -52,27 +52,13 @@ __global__ void __launch_bounds__(kThreads) norm_quant_kernel(const float* __res
             }
         }
         if (want0) {  // four lanes per block of 32
-            float amax = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) amax = fmaxf(amax, fabsf(v[k]));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-            amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-            const float d = __fdiv_rn(amax, 127.0f);
-            const float inv = d != 0.0f ? __fdiv_rn(1.0f, d) : 0.0f;
-            uint32_t q[2] = {0u, 0u};
-            int sum = 0;
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int qk = __float2int_rn(__fmul_rn(v[k], inv));
-                sum += qk;
-                q[k >> 2] |= uint32_t(qk & 0xFF) << (8 * (k & 3));
-            }
-            sum += __shfl_xor_sync(0xffffffffu, sum, 1);
-            sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+            float d;
+            int sum;
+            const uint2 packed = quad_quantize_q8_0(v, d, sum);
             if (mine) {
-                *reinterpret_cast<uint2*>(act.q0 + size_t(t) * cols + i) = make_uint2(q[0], q[1]);
+                *reinterpret_cast<uint2*>(act.q0 + size_t(t) * cols + i) = packed;
                 if ((lane & 3) == 0) {
-                    act.d0[size_t(t) * (cols / 32) + i / 32] = __half2float(__float2half_rn(d));
+                    act.d0[size_t(t) * (cols / 32) + i / 32] = d;
                     act.s0[size_t(t) * (cols / 32) + i / 32] = sum;
                 }
             }

@@ -197,39 +197,181 @@ __device__ __forceinline__ void dec_multiply_body(const DecMatParams& p, const u
     };
 #pragma unroll
     for (int d = 0; d < kDepth; ++d) issue(wq[d]);
+    // The activation row: x, normed where there is a weight, then quantised the way F takes it.
     const uint32_t cols = p.cols;
     constexpr uint32_t kT = kDecWarps * 32;
-    const uint32_t n4 = cols / 4;
-    const float4* w4 = reinterpret_cast<const float4*>(p.weight);
-    float4 wpre[2];  // the norm weights of this thread's first two float4s (rows up to 4096 values): no dependence on the previous operation either
+    DevAct act{};
+    act.cols = cols;
+    if constexpr (!Io::kTagged) {
+        // A thread owns chunks of eight consecutive values and keeps them in registers from the load to the quantised byte:
+        // four lanes hold a Q8_0 block, a warp a Q8_K super-block. Through shared memory, one lane per Q8_0 block, as the
+        // tagged form below does it, a token of the 7B Q4_K_M shape takes 2.23 ms instead of 2.13. (There the barrier between
+        // arrival and quantisation pays: warps that quantise while others still poll slow both, 752 -> 815 us a token.)
+        // Rows of up to 16384 values stay in registers; of a longer one the norm's sum is taken first and the values are read
+        // again.
+        const uint32_t n8 = cols / 8, tid = threadIdx.x;
+        const float4* w4 = reinterpret_cast<const float4*>(p.weight);
+        float4 wpre[2];  // the norm weights of this thread's first chunk: no dependence on the previous operation
+        wpre[0] = wpre[1] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (p.weight != nullptr && tid < n8) {
+            wpre[0] = w4[2 * tid];
+            wpre[1] = w4[2 * tid + 1];
+        }
+        gate.wait();
+        dec_stamp(p.trace, cta, 1);
+        float* xf = reinterpret_cast<float*>(act_smem);  // F16 / F32 weights
+        constexpr bool kQ80 = std::is_same_v<F, FQ4_0> || std::is_same_v<F, FQ4_1> || std::is_same_v<F, FQ5_0> || std::is_same_v<F, FQ8_0>;
+        int8_t* q = reinterpret_cast<int8_t*>(act_smem);
+        float* qd = reinterpret_cast<float*>(act_smem + cols);
+        int32_t* q0s = reinterpret_cast<int32_t*>(act_smem + cols + (cols / 32) * 4);
+        int16_t* qks = reinterpret_cast<int16_t*>(act_smem + cols + ((cols / 256 + 3) / 4) * 16);
+        auto load_chunks = [&](uint32_t base, auto& v) {  // v[k]: chunk base + tid + k * kT, zeros past the end
+            constexpr int K = int(sizeof(v) / sizeof(v[0]));
+            const float4* x4 = reinterpret_cast<const float4*>(p.x);
+            float4 a[K][2];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const uint32_t i = threadIdx.x + k * kT;
-        wpre[k] = (p.weight != nullptr && i < n4) ? w4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    }
-    gate.wait();
-    dec_stamp(p.trace, cta, 1);
-    if (p.trace != nullptr && cta == 0 && threadIdx.x == 0) {  // tracing only: latency of one dependent load
-        const float probe = *reinterpret_cast<const volatile float*>(p.x);
-        if (probe == 123456.0f) p.trace[7] = 0;
-        unsigned long long t;
-        asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-        p.trace[6] = t;
-    }
+            for (int k = 0; k < K; ++k) {
+                const uint32_t c = base + tid + k * kT;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) a[k][i] = c < n8 ? __ldcg(x4 + 2 * c + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            }
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    v[k][4 * i] = a[k][i].x;
+                    v[k][4 * i + 1] = a[k][i].y;
+                    v[k][4 * i + 2] = a[k][i].z;
+                    v[k][4 * i + 3] = a[k][i].w;
+                }
+            }
+        };
+        double part = 0.0;
+        auto add_squares = [&](const auto& v) {
+            constexpr int K = int(sizeof(v) / sizeof(v[0]));
+#pragma unroll
+            for (int k = 0; k < K; ++k)
+#pragma unroll
+                for (int i = 0; i < 8; ++i) part += double(__fmul_rn(v[k][i], v[k][i]));  // padding adds exact zeros
+        };
+        float scale = 1.0f;
+        auto finish_scale = [&] {
+            part = warp_sum(part);
+            if (lane == 0) red[warp] = part;
+            __syncthreads();
+            double total = 0.0;
+            const uint32_t busy = min(uint32_t(kDecWarps), (n8 + 31) / 32);  // warps with values
+            for (uint32_t w = 0; w < busy; ++w) total += red[w];
+            // total / cols; a power-of-two length divides exactly by multiplying with its reciprocal (no f64 division)
+            const bool pow2 = (cols & (cols - 1)) == 0;
+            const double recip = __longlong_as_double((long long)(1023 - (31 - __clz(int(cols)))) << 52);
+            const float mean = float(pow2 ? total * recip : total / double(cols));
+            scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
+            dec_stamp(p.trace, cta, 2);
+        };
+        auto store_chunks = [&](uint32_t base, auto& v) {  // norm, quantise, store
+            constexpr int K = int(sizeof(v) / sizeof(v[0]));
+#pragma unroll
+            for (int k = 0; k < K; ++k) {
+                const uint32_t c = base + tid + k * kT;
+                if (c - lane >= n8) break;  // nothing left for this warp
+                const bool mine = c < n8;
+                if (p.weight != nullptr) {
+                    float4 wa = wpre[0], wb = wpre[1];
+                    if (k != 0 || base != 0) {
+                        wa = mine ? w4[2 * c] : wa;
+                        wb = mine ? w4[2 * c + 1] : wb;
+                    }
+                    const float w[8] = {wa.x, wa.y, wa.z, wa.w, wb.x, wb.y, wb.z, wb.w};
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) v[k][i] = __fmul_rn(__fmul_rn(v[k][i], scale), w[i]);
+                }
+                if constexpr (kQ80) {
+                    float d;
+                    int sum;
+                    const uint2 packed = quad_quantize_q8_0(v[k], d, sum);
+                    if (mine) {
+                        *reinterpret_cast<uint2*>(q + c * 8) = packed;
+                        if ((lane & 3) == 0) {
+                            qd[c / 4] = d;
+                            q0s[c / 4] = sum;
+                        }
+                    }
+                } else if constexpr (F::kExact) {
+                    warp_quantize_q8_k(v[k], q + c * 8, qd + c / 32, qks + c / 2);
+                } else if (mine) {
+                    float4* o = reinterpret_cast<float4*>(xf + c * 8);
+                    o[0] = make_float4(v[k][0], v[k][1], v[k][2], v[k][3]);
+                    o[1] = make_float4(v[k][4], v[k][5], v[k][6], v[k][7]);
+                }
+            }
+        };
+        auto whole_row = [&](auto kc) {  // the row in registers: kc chunks a thread
+            float v[decltype(kc)::value][8];
+            load_chunks(0, v);
+            if (p.weight != nullptr) {
+                add_squares(v);
+                finish_scale();
+            }
+            dec_stamp(p.trace, cta, 3);
+            store_chunks(0, v);
+        };
+        if (n8 <= kT) {
+            whole_row(std::integral_constant<int, 1>{});
+        } else if (n8 <= 2 * kT) {
+            whole_row(std::integral_constant<int, 2>{});
+        } else if (n8 <= 4 * kT) {
+            whole_row(std::integral_constant<int, 4>{});
+        } else {
+            float v[2][8];
+            if (p.weight != nullptr) {
+                for (uint32_t base = 0; base < n8; base += 2 * kT) {
+                    load_chunks(base, v);
+                    add_squares(v);
+                }
+                finish_scale();
+            }
+            for (uint32_t base = 0; base < n8; base += 2 * kT) {
+                load_chunks(base, v);
+                store_chunks(base, v);
+            }
+        }
+        act.f32 = xf;
+        act.q0 = act.qk = q;
+        act.d0 = act.dk = qd;
+        act.s0 = q0s;
+        act.bs = qks;
+        __syncthreads();
+    } else {
+        const uint32_t n4 = cols / 4;
+        const float4* w4 = reinterpret_cast<const float4*>(p.weight);
+        float4 wpre[2];  // the norm weights of this thread's first two float4s (rows up to 4096 values): no dependence on the previous operation either
+#pragma unroll
+        for (int k = 0; k < 2; ++k) {
+            const uint32_t i = threadIdx.x + k * kT;
+            wpre[k] = (p.weight != nullptr && i < n4) ? w4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        }
+        gate.wait();
+        dec_stamp(p.trace, cta, 1);
+        if (p.trace != nullptr && cta == 0 && threadIdx.x == 0) {  // tracing only: latency of one dependent load
+            const float probe = *reinterpret_cast<const volatile float*>(p.x);
+            if (probe == 123456.0f) p.trace[7] = 0;
+            unsigned long long t;
+            asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+            p.trace[6] = t;
+        }
 
-    // Prologue: the activation row in shared memory - f32 (normed), then the planes this format multiplies by.
-    // x as float4s (row lengths are multiples of 32), up to 8 per thread in flight so that their latencies overlap.
-    float* xf = reinterpret_cast<float*>(act_smem);
-    const float4* x4 = reinterpret_cast<const float4*>(p.x);
-    float4* xf4 = reinterpret_cast<float4*>(xf);
-    double part = 0.0;
-    constexpr int kBatch = Io::kTagged ? 4 : 8;  // float4s per thread in flight (the tagged form holds twice the registers per float4)
-    // K = how many float4s per thread this batch really has (1, 2, 4 or 8): a 1024-value row is one float4 for half of
-    // the threads, and a fixed 8-way unrolled, predicated form would have every warp issue eight times the code.
-    auto load_batch = [&](uint32_t base, auto kc) {
-        constexpr int K = decltype(kc)::value;
-        float4 xv[K];
-        if constexpr (Io::kTagged) {
+        // Prologue: the activation row in shared memory - f32 (normed), then the planes this format multiplies by.
+        // x as float4s (row lengths are multiples of 32), up to 8 per thread in flight so that their latencies overlap.
+        float* xf = reinterpret_cast<float*>(act_smem);
+        float4* xf4 = reinterpret_cast<float4*>(xf);
+        double part = 0.0;
+        constexpr int kBatch = 4;  // float4s per thread in flight, as pairs twice their registers
+        // K = how many float4s per thread this batch really has (1, 2, 4 or 8): a 1024-value row is one float4 for half of
+        // the threads, and a fixed 8-way unrolled, predicated form would have every warp issue eight times the code.
+        auto load_batch = [&](uint32_t base, auto kc) {
+            constexpr int K = decltype(kc)::value;
+            float4 xv[K];
             // float4 i = pairs 4i..4i+3 = two 16-byte loads; the whole batch is re-read until every tag is there
             const uint4* xp = reinterpret_cast<const uint4*>(p.x);
             uint4 a[K], b[K];
@@ -255,89 +397,80 @@ __device__ __forceinline__ void dec_multiply_body(const DecMatParams& p, const u
             }
 #pragma unroll
             for (int k = 0; k < K; ++k) xv[k] = make_float4(__uint_as_float(a[k].x), __uint_as_float(a[k].z), __uint_as_float(b[k].x), __uint_as_float(b[k].z));
-        } else {
 #pragma unroll
             for (int k = 0; k < K; ++k) {
                 const uint32_t i = base + threadIdx.x + k * kT;
-                xv[k] = i < n4 ? __ldcg(x4 + i) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-        }
-#pragma unroll
-        for (int k = 0; k < K; ++k) {
-            const uint32_t i = base + threadIdx.x + k * kT;
-            if (i < n4) xf4[i] = xv[k];
-            part += double(__fmul_rn(xv[k].x, xv[k].x));  // padding adds exact zeros
-            part += double(__fmul_rn(xv[k].y, xv[k].y));
-            part += double(__fmul_rn(xv[k].z, xv[k].z));
-            part += double(__fmul_rn(xv[k].w, xv[k].w));
-        }
-    };
-    for (uint32_t base = 0; base < n4; base += kBatch * kT) {
-        const uint32_t left = n4 - base;
-        if (left <= kT) load_batch(base, std::integral_constant<int, 1>{});
-        else if (left <= 2 * kT) load_batch(base, std::integral_constant<int, 2>{});
-        else if (left <= 4 * kT || kBatch == 4) load_batch(base, std::integral_constant<int, 4>{});
-        else load_batch(base, std::integral_constant<int, kBatch>{});
-    }
-    if (p.weight != nullptr) {
-        part = warp_sum(part);
-        if (lane == 0) red[warp] = part;
-        __syncthreads();
-        double total = 0.0;
-#pragma unroll
-        for (int w = 0; w < kDecWarps; ++w) total += red[w];
-        // total / cols; a power-of-two length divides exactly by multiplying with its reciprocal (no f64 division)
-        const bool pow2 = (cols & (cols - 1)) == 0;
-        const double recip = __longlong_as_double((long long)(1023 - (31 - __clz(int(cols)))) << 52);
-        const float mean = float(pow2 ? total * recip : total / double(cols));
-        const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
-        dec_stamp(p.trace, cta, 2);
-        auto scale_batch = [&](uint32_t base, auto kc) {
-            constexpr int K = decltype(kc)::value;
-            float4 wv[K];
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const uint32_t i = base + threadIdx.x + k * kT;
-                if (k < 2 && base == 0) wv[k] = wpre[k];
-                else wv[k] = i < n4 ? w4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            }
-#pragma unroll
-            for (int k = 0; k < K; ++k) {
-                const uint32_t i = base + threadIdx.x + k * kT;
-                if (i < n4) {  // the same thread wrote xf4[i] above
-                    const float4 xx = xf4[i];
-                    xf4[i] = make_float4(__fmul_rn(__fmul_rn(xx.x, scale), wv[k].x), __fmul_rn(__fmul_rn(xx.y, scale), wv[k].y),
-                                         __fmul_rn(__fmul_rn(xx.z, scale), wv[k].z), __fmul_rn(__fmul_rn(xx.w, scale), wv[k].w));
-                }
+                if (i < n4) xf4[i] = xv[k];
+                part += double(__fmul_rn(xv[k].x, xv[k].x));  // padding adds exact zeros
+                part += double(__fmul_rn(xv[k].y, xv[k].y));
+                part += double(__fmul_rn(xv[k].z, xv[k].z));
+                part += double(__fmul_rn(xv[k].w, xv[k].w));
             }
         };
-        for (uint32_t base = 0; base < n4; base += 8 * kT) {
+        for (uint32_t base = 0; base < n4; base += kBatch * kT) {
             const uint32_t left = n4 - base;
-            if (left <= kT) scale_batch(base, std::integral_constant<int, 1>{});
-            else if (left <= 2 * kT) scale_batch(base, std::integral_constant<int, 2>{});
-            else scale_batch(base, std::integral_constant<int, 8>{});
+            if (left <= kT) load_batch(base, std::integral_constant<int, 1>{});
+            else if (left <= 2 * kT) load_batch(base, std::integral_constant<int, 2>{});
+            else load_batch(base, std::integral_constant<int, kBatch>{});
         }
+        if (p.weight != nullptr) {
+            part = warp_sum(part);
+            if (lane == 0) red[warp] = part;
+            __syncthreads();
+            double total = 0.0;
+#pragma unroll
+            for (int w = 0; w < kDecWarps; ++w) total += red[w];
+            // total / cols; a power-of-two length divides exactly by multiplying with its reciprocal (no f64 division)
+            const bool pow2 = (cols & (cols - 1)) == 0;
+            const double recip = __longlong_as_double((long long)(1023 - (31 - __clz(int(cols)))) << 52);
+            const float mean = float(pow2 ? total * recip : total / double(cols));
+            const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, p.eps)));
+            dec_stamp(p.trace, cta, 2);
+            auto scale_batch = [&](uint32_t base, auto kc) {
+                constexpr int K = decltype(kc)::value;
+                float4 wv[K];
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const uint32_t i = base + threadIdx.x + k * kT;
+                    if (k < 2 && base == 0) wv[k] = wpre[k];
+                    else wv[k] = i < n4 ? w4[i] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                }
+#pragma unroll
+                for (int k = 0; k < K; ++k) {
+                    const uint32_t i = base + threadIdx.x + k * kT;
+                    if (i < n4) {  // the same thread wrote xf4[i] above
+                        const float4 xx = xf4[i];
+                        xf4[i] = make_float4(__fmul_rn(__fmul_rn(xx.x, scale), wv[k].x), __fmul_rn(__fmul_rn(xx.y, scale), wv[k].y),
+                                             __fmul_rn(__fmul_rn(xx.z, scale), wv[k].z), __fmul_rn(__fmul_rn(xx.w, scale), wv[k].w));
+                    }
+                }
+            };
+            for (uint32_t base = 0; base < n4; base += 8 * kT) {
+                const uint32_t left = n4 - base;
+                if (left <= kT) scale_batch(base, std::integral_constant<int, 1>{});
+                else if (left <= 2 * kT) scale_batch(base, std::integral_constant<int, 2>{});
+                else scale_batch(base, std::integral_constant<int, 8>{});
+            }
+        }
+        __syncthreads();
+        dec_stamp(p.trace, cta, 3);
+        act.f32 = xf;
+        unsigned char* planes = act_smem + size_t(cols) * 4;
+        if constexpr (std::is_same_v<F, FQ4_0> || std::is_same_v<F, FQ4_1> || std::is_same_v<F, FQ5_0> || std::is_same_v<F, FQ8_0>) {
+            int8_t* q = reinterpret_cast<int8_t*>(planes);
+            float* d = reinterpret_cast<float*>(planes + cols);
+            int32_t* s = reinterpret_cast<int32_t*>(planes + cols + (cols / 32) * 4);
+            cta_quantize_q8_0(xf, cols, q, d, s);
+            act.q0 = q; act.d0 = d; act.s0 = s;
+        } else if constexpr (F::kExact) {
+            int8_t* q = reinterpret_cast<int8_t*>(planes);
+            float* d = reinterpret_cast<float*>(planes + cols);
+            int16_t* bs = reinterpret_cast<int16_t*>(planes + cols + ((cols / 256 + 3) / 4) * 16);
+            cta_quantize_q8_k(xf, cols, q, d, bs);
+            act.qk = q; act.dk = d; act.bs = bs;
+        }
+        __syncthreads();
     }
-    __syncthreads();
-    dec_stamp(p.trace, cta, 3);
-    DevAct act{};
-    act.cols = cols;
-    act.f32 = xf;
-    unsigned char* planes = act_smem + size_t(cols) * 4;
-    if constexpr (std::is_same_v<F, FQ4_0> || std::is_same_v<F, FQ4_1> || std::is_same_v<F, FQ5_0> || std::is_same_v<F, FQ8_0>) {
-        int8_t* q = reinterpret_cast<int8_t*>(planes);
-        float* d = reinterpret_cast<float*>(planes + cols);
-        int32_t* s = reinterpret_cast<int32_t*>(planes + cols + (cols / 32) * 4);
-        cta_quantize_q8_0(xf, cols, q, d, s);
-        act.q0 = q; act.d0 = d; act.s0 = s;
-    } else if constexpr (F::kExact) {
-        int8_t* q = reinterpret_cast<int8_t*>(planes);
-        float* d = reinterpret_cast<float*>(planes + cols);
-        int16_t* bs = reinterpret_cast<int16_t*>(planes + cols + ((cols / 256 + 3) / 4) * 16);
-        cta_quantize_q8_k(xf, cols, q, d, bs);
-        act.qk = q; act.dk = d; act.bs = bs;
-    }
-    __syncthreads();
     gate.prologue_done();
     dec_stamp(p.trace, cta, 4);
     if (!any) return;

@@ -63,6 +63,30 @@ __device__ __forceinline__ void cta_quantize_q8_0(const float* row, uint32_t col
     }
 }
 
+// One Q8_0 block by four neighbouring lanes, eight consecutive values each: this lane's packed bytes; the block's scale (rounded
+// to f16) and sum in every lane of the four.
+__device__ __forceinline__ uint2 quad_quantize_q8_0(const float (&v)[8], float& d, int& sum) {
+    float amax = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(v[i]));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+    const float dd = __fdiv_rn(amax, 127.0f);
+    const float inv = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
+    uint32_t packed[2] = {0u, 0u};
+    sum = 0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int qi = __float2int_rn(__fmul_rn(v[i], inv));
+        sum += qi;
+        packed[i >> 2] |= uint32_t(qi & 0xFF) << (8 * (i & 3));
+    }
+    sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+    sum += __shfl_xor_sync(0xffffffffu, sum, 2);
+    d = __half2float(__float2half_rn(dd));
+    return make_uint2(packed[0], packed[1]);
+}
+
 // One Q8_K super-block by one warp: lane l holds values 8l .. 8l + 7. `qk` and `bs` are this lane's own places (its values, the
 // sums of 16 its pair of lanes forms), `dk` the super-block's.
 __device__ __forceinline__ void warp_quantize_q8_k(const float (&vals)[8], int8_t* qk, float* dk, int16_t* bs) {

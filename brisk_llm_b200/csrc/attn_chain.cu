@@ -1,4 +1,4 @@
-// Softmax + weighted sum of attention for 2..24 tokens at once (one token: attn_decode.cu), arranged around the one thing the reference's order of
+// Weighted sum of attention for 2..24 tokens at once (one token: attn_decode.cu), arranged around the one thing the reference's order of
 // operations does not let anybody parallelise: out[i] = ((p[0]*v_0[i] + p[1]*v_1[i]) + p[2]*v_2[i]) + ... is a chain of
 // dependent f32 additions per (token, head, i), one per visible position (src/kernels_f32.cpp:265-273), and the result
 // has to be that chain's, bit for bit, because the 8-bit re-quantisation that follows turns a 1-ulp difference into a
@@ -20,12 +20,8 @@
 // Products that go through shared memory (an earlier form of this kernel: product warps and chain warps) cost 8 bytes of
 // shared-memory traffic per product, 16 cycles per position with two heads on an SM; this form costs 2 bytes per value.
 //
-// Before the chains all threads compute the softmax of the CTA's HQ score rows into shared memory exactly as the other
-// attention kernels do (max, e = expf(s - max) with glibc's expf, f64 sum, p = e * float(1 / sum); src/kernels_f32.cpp:
-// 275-284) - with the same split of the f64 sum over 256 (virtual) threads, so the totals are the same doubles. The exps
-// take their 2^(i/32) table from shared memory and run four at a time: with the table in global memory and one exp after
-// the other they cost 850 cycles each and, at 8192 positions, as much as the chains.
-#include "exact_math.h"
+// The softmax is a kernel of its own (attn_prompt.cu), a CTA or a warp per row: inside this one, at one CTA per SM, its exps
+// took as long as the chains (7B shape, 9 tokens at 2064 positions: 31 us together, 6 + 25 apart).
 #include "kernels.h"
 #include "pdl.cuh"
 
@@ -34,7 +30,6 @@ namespace {
 
 constexpr uint32_t kStages = 4;
 constexpr uint32_t kStageBytes = 32 * 1024;
-constexpr uint32_t kSumThreads = 256;  // the f64 sum is split the way a 256-thread CTA splits it
 constexpr uint32_t kWaitLimit = 1u << 22;
 __device__ unsigned int g_chain_error;  // set when a wait for a bulk copy ran out (never seen; every wait is bounded all the same)
 
@@ -48,7 +43,7 @@ __device__ unsigned long long g_chain_trace[32];
 #endif
 
 struct ChainParams {
-    const float* scores;   // [n][heads][max_context] scaled scores
+    const float* scores;   // [n][heads][max_context] probabilities
     const __half* v_cache; // [kv][max_context][dim]
     float* out;            // [n][heads * dim]
     const uint32_t* position;
@@ -86,9 +81,6 @@ template <int C, int HQ>
 __global__ void __launch_bounds__(256) attn_chain_kernel(const ChainParams a) {
     using R = typename Raw<C>::T;
     extern __shared__ __align__(16) unsigned char smem[];
-    __shared__ float redf[HQ][8];
-    __shared__ double redd[HQ][8];
-    __shared__ uint64_t tab[32];
     __shared__ __align__(8) uint64_t full[kStages];
     float* ps = reinterpret_cast<float*>(smem);                                             // [HQ][ps_stride]
     unsigned char* ring = smem + size_t(HQ) * a.ps_stride * sizeof(float);                  // [kStages][stage_rows][dim] f16
@@ -129,65 +121,20 @@ __global__ void __launch_bounds__(256) attn_chain_kernel(const ChainParams a) {
         for (uint32_t st = 0; st + 1 < kStages; ++st) request(st);  // in flight while the softmax runs
     }
 
-    // ---- softmax of the HQ rows ------------------------------------------------------------------------------------
+    // ---- the HQ rows' probabilities ---------------------------------------------------------------------------------
     const long long t_begin = CHAIN_CLOCK();
-    if (tid < 32) tab[tid] = exp2_table_device()[tid];
 #pragma unroll
     for (int q = 0; q < HQ; ++q) {
         const float* s = a.scores + (size_t(tok) * a.heads + h0 + q) * a.max_context + start;
-        float m = -INFINITY;
-        uint32_t p = tid;
-        for (; p + 7 * nt < cnt; p += 8 * nt) {  // eight loads in flight per thread: one after the other they cost an L2 round trip each
+        for (uint32_t p0 = tid; p0 < cnt; p0 += 8 * nt) {  // eight loads in flight per thread: one after the other they cost an L2 round trip each
             float v[8];
 #pragma unroll
-            for (int u = 0; u < 8; ++u) v[u] = __ldcg(s + p + u * nt);
+            for (int u = 0; u < 8; ++u) v[u] = p0 + u * nt < cnt ? __ldcg(s + p0 + u * nt) : 0.0f;
 #pragma unroll
             for (int u = 0; u < 8; ++u) {
-                ps[q * a.ps_stride + p + u * nt] = v[u];
-                m = fmaxf(m, v[u]);
+                if (p0 + u * nt < cnt) ps[q * a.ps_stride + p0 + u * nt] = v[u];
             }
         }
-        for (; p < cnt; p += nt) {
-            const float v = __ldcg(s + p);
-            ps[q * a.ps_stride + p] = v;
-            m = fmaxf(m, v);
-        }
-        m = warp_max(m);
-        if (lane == 0) redf[q][warp] = m;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < HQ; ++q) {
-        float* row = ps + q * a.ps_stride;
-        float m = redf[q][0];
-        for (uint32_t w = 1; w < nt / 32; ++w) m = fmaxf(m, redf[q][w]);
-        // virtual thread vt of 256 sums positions vt, vt + 256, ... in that order, as a 256-thread CTA does
-        for (uint32_t vt = tid; vt < kSumThreads; vt += nt) {
-            double part = 0.0;
-            uint32_t p = vt;
-            for (; p + 3 * kSumThreads < cnt; p += 4 * kSumThreads) {
-                const float e0 = exact_expf_flat(__fsub_rn(row[p], m), tab), e1 = exact_expf_flat(__fsub_rn(row[p + kSumThreads], m), tab);
-                const float e2 = exact_expf_flat(__fsub_rn(row[p + 2 * kSumThreads], m), tab), e3 = exact_expf_flat(__fsub_rn(row[p + 3 * kSumThreads], m), tab);
-                row[p] = e0; row[p + kSumThreads] = e1; row[p + 2 * kSumThreads] = e2; row[p + 3 * kSumThreads] = e3;
-                part += double(e0); part += double(e1); part += double(e2); part += double(e3);
-            }
-            for (; p < cnt; p += kSumThreads) {
-                const float e = exact_expf_flat(__fsub_rn(row[p], m), tab);
-                row[p] = e;
-                part += double(e);
-            }
-            part = warp_sum(part);
-            if (lane == 0) redd[q][vt >> 5] = part;
-        }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int q = 0; q < HQ; ++q) {
-        double total = 0.0;
-#pragma unroll
-        for (int w = 0; w < 8; ++w) total += redd[q][w];
-        const float inv = float(1.0 / total);
-        for (uint32_t p = tid; p < cnt; p += nt) ps[q * a.ps_stride + p] = __fmul_rn(ps[q * a.ps_stride + p], inv);
     }
     CHAIN_ADD(0, t_begin);
     const long long t_phase = CHAIN_CLOCK();
@@ -309,7 +256,7 @@ bool attn_chain_fits(uint32_t n, uint32_t heads, uint32_t kv_heads, uint32_t dim
     return dim % 32 == 0 && dim <= 256 && heads % kv_heads == 0 && choose(n, heads, kv_heads, dim, max_visible, sms).c != 0;
 }
 
-// a.scores holds the scaled scores of the n tokens (rows of max_context floats); a.out receives the attended rows.
+// a.scores holds the probabilities of the n tokens (rows of max_context floats); a.out receives the attended rows.
 void launch_attn_chain(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
     const Choice ch = choose(a.n, a.heads, a.kv_heads, a.dim, a.max_visible, sms);
     if (ch.c == 0) throw CudaError("cuda: context too long for the chained attention kernel");

@@ -415,9 +415,12 @@ void launch_scores(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
     }();
     const uint32_t rows = a.n * (a.heads / a.kv_heads), chunks = (a.max_visible + kPerCta - 1) / kPerCta;
     // More rows per tile reuse the K row a thread has widened; fewer fill the GPU: the largest tile that leaves four CTAs
-    // an SM, half of which the causal edge may leave without work.
+    // an SM, half of which the causal edge may leave without work. Few tokens have no such edge, and re-reading the K rows is
+    // what they pay for: most of an SM's CTA each is enough (9 tokens at 2064 positions, 7B shape: tiles of 8 rows 18.9 us, of
+    // all 36 15.4).
+    const uint64_t enough = a.n <= kChainMaxTokens ? sms * 4ull / 5 : 4ull * sms;
     uint32_t tile = 64;
-    while (tile > 8 && uint64_t(chunks) * a.kv_heads * ((rows + tile - 1) / tile) < 4ull * sms) tile /= 2;
+    while (tile > 8 && uint64_t(chunks) * a.kv_heads * ((rows + tile - 1) / tile) < enough) tile /= 2;
     static DeviceOnce once;
     if (once.first()) BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(64 * DIM * sizeof(float))));
     launch_dependent(kernel, dim3(chunks, a.kv_heads, (rows + tile - 1) / tile), dim3(128), size_t(tile) * DIM * sizeof(float), s, a, tile, 1.0f);
@@ -438,11 +441,15 @@ void launch_attn_scores(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
     else launch_scores<256>(a, sms, s);
 }
 
-void launch_attn_softmax_weighted(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
+void launch_attn_softmax(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
     const uint32_t softmax_rows = a.n * a.heads, widest = a.window != 0 ? std::min(a.window, a.max_visible) : a.max_visible;
-    if (widest <= 512) launch_dependent(attn_softmax_kernel<32, 16>, dim3((softmax_rows + 7) / 8), dim3(256), 0, s, a);
-    else if (widest <= 1024) launch_dependent(attn_softmax_kernel<32, 32>, dim3((softmax_rows + 7) / 8), dim3(256), 0, s, a);
+    const bool many = softmax_rows >= 16 * sms;  // enough rows for a warp each (1000 positions, 144 rows: 8.7 us so, 4 with a CTA each)
+    if (widest <= 512 && (many || widest <= 128)) launch_dependent(attn_softmax_kernel<32, 16>, dim3((softmax_rows + 7) / 8), dim3(256), 0, s, a);
+    else if (widest <= 1024 && many) launch_dependent(attn_softmax_kernel<32, 32>, dim3((softmax_rows + 7) / 8), dim3(256), 0, s, a);
     else launch_dependent(attn_softmax_kernel<256, 16>, dim3(softmax_rows), dim3(256), 0, s, a);
+}
+
+void launch_attn_weighted(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
     // More rows per lane reuse the V row it has widened (16 rows: 736 us for the case above, 8: 921), fewer fill the GPU: the
     // most that still leave one and a half CTAs an SM.
     const uint32_t rows = a.n * (a.heads / a.kv_heads), parts = (a.dim + 127) / 128, groups = 512 / (a.dim / parts);

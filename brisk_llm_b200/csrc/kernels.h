@@ -130,7 +130,7 @@ struct AttnArgs {
 };
 size_t attn_scratch_floats(uint32_t n, uint32_t heads, uint32_t max_context);
 void launch_attention(const AttnArgs& a, cudaStream_t s);
-// Softmax + weighted sum for a few tokens (attn_chain.cu): a.scores holds their scaled scores. One CTA per (token, one or
+// Weighted sum for a few tokens (attn_chain.cu): a.scores holds their probabilities. One CTA per (token, one or
 // two query heads, slice of the head), chain warps and product warps; same results as the kernels above.
 bool attn_chain_fits(uint32_t n, uint32_t heads, uint32_t kv_heads, uint32_t dim, uint32_t max_visible, uint32_t sms);
 void launch_attn_chain(const AttnArgs& a, uint32_t sms, cudaStream_t s);

@@ -327,7 +327,8 @@ size_t attn_scratch_floats(uint32_t n, uint32_t heads, uint32_t max_context) { r
 
 // attn_prompt.cu
 void launch_attn_scores(const AttnArgs& a, uint32_t sms, cudaStream_t s);
-void launch_attn_softmax_weighted(const AttnArgs& a, uint32_t sms, cudaStream_t s);
+void launch_attn_softmax(const AttnArgs& a, uint32_t sms, cudaStream_t s);
+void launch_attn_weighted(const AttnArgs& a, uint32_t sms, cudaStream_t s);
 
 void launch_attention(const AttnArgs& a, cudaStream_t s) {
     if ((a.dim != 64 && a.dim != 128 && a.dim != 256) || a.heads / a.kv_heads > 8) throw CudaError("cuda: attention takes head sizes 64, 128 and 256 and at most 8 query heads per K/V head");
@@ -337,9 +338,10 @@ void launch_attention(const AttnArgs& a, cudaStream_t s) {
         return uint32_t(count);
     }();
     launch_attn_scores(a, sms, s);
+    launch_attn_softmax(a, sms, s);
     const int mode = chain_mode();
     if (mode != 0 && (a.n <= kChainMaxTokens || mode == 1) && attn_chain_fits(a.n, a.heads, a.kv_heads, a.dim, a.max_visible, sms)) launch_attn_chain(a, sms, s);
-    else launch_attn_softmax_weighted(a, sms, s);
+    else launch_attn_weighted(a, sms, s);
 }
 
 size_t argmax_scratch_elems(uint32_t) { return size_t(kArgmaxBlocks) * 64; }

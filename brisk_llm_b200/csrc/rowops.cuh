@@ -16,9 +16,16 @@ namespace bk {
 __device__ __forceinline__ float cta_rms_scale(const float* x, uint32_t cols, float eps, double* red) {
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
     double part = 0.0;
-    for (uint32_t i = tid; i < cols; i += blockDim.x) {
-        const float v = x[i];
-        part += double(__fmul_rn(v, v));
+    const float4* x4 = reinterpret_cast<const float4*>(x);  // rows are 16-byte aligned and a multiple of 32 long
+    for (uint32_t i0 = tid; i0 < cols / 4; i0 += 4 * blockDim.x) {  // four 16-byte loads in flight
+        float4 v[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) v[u] = i0 + u * blockDim.x < cols / 4 ? x4[i0 + u * blockDim.x] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+            part += double(__fmul_rn(v[u].x, v[u].x)) + double(__fmul_rn(v[u].y, v[u].y));
+            part += double(__fmul_rn(v[u].z, v[u].z)) + double(__fmul_rn(v[u].w, v[u].w));
+        }
     }
     part = warp_sum(part);
     __syncthreads();  // red may still be read by a previous call

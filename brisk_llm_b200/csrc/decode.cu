@@ -78,6 +78,18 @@ __global__ void __launch_bounds__(kDecWarps * 32) dec_matvec_kernel(const DecMat
     dec_multiply_body<F, RW, PAIR, kDepth, PdlGate, PlainIo, RELAX>(p, blockIdx.x, gridDim.x, smem_raw, tile, red, PdlGate{p.pdl});
 }
 
+// Two multiplies of one activation row whose weights have different types (the q, k and v projections of the "medium" mixes:
+// V in Q6_K) as one launch: the first ctas1 CTAs take the first, the others the second. A launch of its own for V costs 5 us
+// of prologue for 0.9 MB of weights; measured, the whole token of the 1B Q4_K_M shape at 1024 positions 630 -> 589 us.
+template <class F1, class F2>
+__global__ void __launch_bounds__(kDecWarps * 32) dec_matvec_two_kernel(const __grid_constant__ DecMatParams p1, const __grid_constant__ DecMatParams p2, uint32_t ctas1) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    __shared__ __align__(16) float tile[dec_tile_floats(2)];
+    __shared__ double red[32];
+    if (blockIdx.x < ctas1) dec_multiply_body<F1, 2, false, 2, PdlGate, PlainIo>(p1, blockIdx.x, ctas1, smem_raw, tile, red, PdlGate{p1.pdl});
+    else dec_multiply_body<F2, 1, false, 2, PdlGate, PlainIo>(p2, blockIdx.x - ctas1, gridDim.x - ctas1, smem_raw, tile, red, PdlGate{p2.pdl});
+}
+
 // BRISK_CUDA_RELAXED: a comma-separated list of the orders to relax in the one-kernel-per-operation single-token path -
 // "rowsum" (butterfly row sums in the multiplies), "attention" (split-position softmax and weighted sum combined afterwards,
 // with the fast exp). Off by default and never used by a parity test: the exact order is what makes the results the
@@ -326,6 +338,52 @@ void launch_dec_multiply(const MatTarget* targets, int count, const float* x, co
         case T_F32: dispatch_dec<FF32>(p, pair, sms, s); break;
         default: throw CudaError("cuda: unsupported weight type");
     }
+}
+
+bool launch_dec_multiply_two(const MatTarget* first, int count1, const MatTarget* second, int count2, const float* x, const float* norm_weight, float eps,
+                             uint32_t cols, uint32_t sms, cudaStream_t s) {
+    const int t1 = first[0].m.type, t2 = second[0].m.type;
+    if (t2 != T_Q6_K || (t1 != T_Q4_K && t1 != T_Q5_K) || relaxed("rowsum")) return false;
+    DecMatParams p[2]{};
+    const MatTarget* targets[2] = {first, second};
+    const int counts[2] = {count1, count2};
+    uint64_t groups[2], cost[2];
+    for (int i = 0; i < 2; ++i) {
+        p[i].count = counts[i];
+        p[i].epi = EPI_STORE;
+        p[i].x = x;
+        p[i].weight = norm_weight;
+        p[i].eps = eps;
+        p[i].cols = cols;
+        p[i].pdl = pdl_mode();
+        for (int k = 0; k < counts[i]; ++k) {
+            if (targets[i][k].m.cols != cols || (i == 0 && targets[i][k].m.rows % 2 != 0)) return false;
+            p[i].m[k] = targets[i][k].m;
+            p[i].out[k] = targets[i][k].out;
+        }
+        const int rw = i == 0 ? 2 : 1;
+        groups[i] = dec_assign_groups(p[i], rw, false);
+        cost[i] = uint64_t(rw) * block_bytes(targets[i][0].m.type);
+    }
+    // the split of the SMs after which the busiest warp of either side has the least to read
+    uint32_t ctas1 = 1;
+    uint64_t best = ~0ull;
+    for (uint32_t n1 = 1; n1 < sms; ++n1) {
+        const uint64_t w1 = uint64_t(n1) * kDecWarps, w2 = uint64_t(sms - n1) * kDecWarps;
+        const uint64_t worst = std::max((groups[0] + w1 - 1) / w1 * cost[0], (groups[1] + w2 - 1) / w2 * cost[1]);
+        if (worst < best) {
+            best = worst;
+            ctas1 = n1;
+        }
+    }
+    const size_t smem = dec_act_smem(cols);
+    auto go = [&](auto kernel) {
+        if (smem > 40 * 1024) BK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 160 * 1024));
+        launch_pdl(kernel, dim3(sms), dim3(kDecWarps * 32), smem, s, p[0], p[1], ctas1);
+    };
+    if (t1 == T_Q4_K) go(dec_matvec_two_kernel<FQ4_K, FQ6_K>);
+    else go(dec_matvec_two_kernel<FQ5_K, FQ6_K>);
+    return true;
 }
 
 bool dec_attention_fits(uint32_t max_context, uint32_t heads, uint32_t dim, uint32_t sms) {

@@ -145,6 +145,10 @@ unsigned int* attn_chain_error_word();        // non-zero on the device after a 
 // dependent launch: weights are prefetched while the previous kernel drains. `sms` sizes the persistent grid.
 void launch_dec_multiply(const MatTarget* targets, int count, const float* x, const float* norm_weight, float eps, uint32_t cols, Epilogue epi,
                          uint32_t sms, cudaStream_t s, unsigned long long* trace = nullptr);
+// Two groups of targets of different types (Q4_K or Q5_K, then Q6_K; EPI_STORE) over one row, as one launch; false (nothing
+// launched) for other types.
+bool launch_dec_multiply_two(const MatTarget* first, int count1, const MatTarget* second, int count2, const float* x, const float* norm_weight, float eps,
+                             uint32_t cols, uint32_t sms, cudaStream_t s);
 // Attention of the single new token: per-head norm + RoPE of q and the new k, f16 K/V store, scores, softmax and weighted sum.
 // Takes the same argument structs as the batched kernels (n is 1).
 void launch_dec_attention(const RopeArgs& r, const AttnArgs& at, uint32_t sms, cudaStream_t s);

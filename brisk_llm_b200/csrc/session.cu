@@ -787,6 +787,11 @@ struct Session {
                 while (!targets.empty()) {  // one launch per weight type among the targets
                     std::vector<MatTarget> same, rest;
                     for (const MatTarget& tg : targets) (tg.m.type == targets[0].m.type ? same : rest).push_back(tg);
+                    if (rest.size() == 1 && epi == EPI_STORE && t == nullptr &&
+                        launch_dec_multiply_two(same.data(), int(same.size()), rest.data(), 1, x, w, eps, cols, sms, stream)) {
+                        ++launches;
+                        return;
+                    }
                     launch_dec_multiply(same.data(), int(same.size()), x, w, eps, cols, epi, sms, stream, t);
                     ++launches;
                     targets.swap(rest);

@@ -170,7 +170,14 @@ __device__ __forceinline__ void tile_sync(int id) { asm volatile("bar.sync %0, %
 __device__ __forceinline__ void tile_arrive(int id) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kProducers * 32 + 32) : "memory"); }
 
 // grid: heads x dim / 32. ps_floats: room for the visible positions' probabilities, a multiple of 4.
-__global__ void __launch_bounds__(kSumThreads, 1) decode_sum_kernel(const DecAttnParams a, uint32_t window, uint32_t ps_floats) {
+// DIM = 0: the scores are there. DIM = 64, 128: every CTA computes its head's scores itself, which saves the kernel before it
+// for as long as the K rows (each read by group x dim / 32 CTAs, the first 512 positions' before the wait) cost less.
+template <int DIM>
+__global__ void __launch_bounds__(kSumThreads, 1) decode_sum_kernel(const DecAttnParams a, uint32_t window, uint32_t ps_floats, float one) {
+    constexpr bool kScores = DIM != 0;
+    constexpr int kSteps = kScores ? DIM / 16 : 1, POS = 2;  // as in the scores kernel
+    __shared__ __align__(16) float q_row[kScores ? DIM : 4], k_new[kScores ? DIM : 4];
+    __shared__ __align__(4) __half v_new[32];  // the token's own V slice: its cache row is another CTA's store
     extern __shared__ __align__(16) unsigned char smem[];
     float* ps = reinterpret_cast<float*>(smem);
     float* tiles = ps + ps_floats;
@@ -203,13 +210,99 @@ __global__ void __launch_bounds__(kSumThreads, 1) decode_sum_kernel(const DecAtt
         }
     }
     if (tid < 32) exp_table[tid] = exp2_table_device()[tid];
+    const uint32_t half = lane >> 4, in_cta = warp * 16 + (lane & 15);
+    uint4 raw[POS][kSteps];
+    auto load_k = [&](uint32_t p0) {
+        const __half* kbase = a.k_cache + (size_t(kvh) * a.max_context + start) * DIM + half * 8;
+#pragma unroll
+        for (int j = 0; j < POS; ++j) {
+            const uint32_t i = p0 + in_cta + j * (kSumThreads / 2);
+            if (i < cnt - 1) {
+                const uint4* kr = reinterpret_cast<const uint4*>(kbase + size_t(i) * DIM);
+#pragma unroll
+                for (int s = 0; s < kSteps; ++s) raw[j][s] = kr[2 * s];
+            }
+        }
+    };
+    if constexpr (kScores) load_k(0);
     wait_for_previous();
     release_next();
+    float m = -INFINITY;
+    if constexpr (kScores) {
+        const uint32_t pos = visible - 1;
+        const float* rope = a.rope + size_t(pos) * DIM;
+        if (warp == 0) {
+            warp_norm_rope_head<DIM / 32>(a.q + size_t(h) * DIM, a.q_bias ? a.q_bias + size_t(h) * DIM : nullptr, a.q_norm, rope, a.eps, a.neox, q_row);
+        } else if (warp == 1) {
+            warp_norm_rope_head<DIM / 32>(a.k + size_t(kvh) * DIM, a.k_bias ? a.k_bias + size_t(kvh) * DIM : nullptr, a.k_norm, rope, a.eps, a.neox, k_new);
+            __syncwarp();
+            if (h % (a.heads / a.kv_heads) == 0 && col0 == 0) warp_store_new_kv(a, kvh, pos, k_new);
+        } else if (warp == 2) {
+            float v = __ldcg(a.v + size_t(kvh) * DIM + col0 + lane);
+            if (a.v_bias != nullptr) v = __fadd_rn(v, a.v_bias[size_t(kvh) * DIM + col0 + lane]);
+            v_new[lane] = __float2half_rn(v);
+        }
+        __syncthreads();
+        const f32x2 one2 = pack2(one, one);
+        const ulonglong2* q2 = reinterpret_cast<const ulonglong2*>(q_row + half * 8);
+        for (uint32_t p0 = 0; p0 < cnt; p0 += kSumThreads / 2 * POS) {
+            if (p0 != 0) load_k(p0);
+            f32x2 part[POS][4];
+#pragma unroll
+            for (int j = 0; j < POS; ++j) {
+                if (p0 + in_cta + j * (kSumThreads / 2) == cnt - 1) {  // the token's own row, as the cache holds it
+#pragma unroll
+                    for (int s = 0; s < kSteps; ++s) {
+                        __half2 hv[4];
+#pragma unroll
+                        for (int k = 0; k < 4; ++k) hv[k] = __floats2half2_rn(k_new[s * 16 + half * 8 + 2 * k], k_new[s * 16 + half * 8 + 2 * k + 1]);
+                        raw[j][s] = *reinterpret_cast<const uint4*>(hv);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < 4; ++k) part[j][k] = 0ull;
+            }
+#pragma unroll
+            for (int s = 0; s < kSteps; ++s) {
+                const ulonglong2 q0 = q2[s * 4], q1 = q2[s * 4 + 1];
+                const f32x2 qv[4] = {q0.x, q0.y, q1.x, q1.y};
+#pragma unroll
+                for (int j = 0; j < POS; ++j) {
+                    const __half2* hv = reinterpret_cast<const __half2*>(&raw[j][s]);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float2 f = __half22float2(hv[k]);
+                        part[j][k] = fma2(mul2(qv[k], pack2(f.x, f.y)), one2, part[j][k]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int j = 0; j < POS; ++j) {
+                float sum = 0.0f;
+                auto add_parts = [&] {
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        float x, y;
+                        unpack2(part[j][k], x, y);
+                        sum = __fadd_rn(__fadd_rn(sum, x), y);
+                    }
+                };
+                add_parts();
+                sum = __shfl_sync(0xffffffffu, sum, lane & 15);  // the upper half-warp goes on from its partner's sum of the first eight
+                const uint32_t i = p0 + in_cta + j * (kSumThreads / 2);
+                if (half == 1 && i < cnt) {
+                    add_parts();
+                    const float v = __fmul_rn(sum, a.scale);
+                    ps[i] = v;
+                    m = fmaxf(m, v);
+                }
+            }
+        }
+    }
 
     // ---- softmax (src/kernels_f32.cpp:275-284): e = expf(s - max), f64 sum, p = e * float(1 / sum) ----
     const float* s = a.scores + size_t(h) * a.max_context + start;
-    float m = -INFINITY;
-    for (uint32_t p0 = tid; p0 < cnt; p0 += 8 * kSumThreads) {  // eight loads in flight
+    if constexpr (!kScores) for (uint32_t p0 = tid; p0 < cnt; p0 += 8 * kSumThreads) {  // eight loads in flight
         float v[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) v[u] = p0 + u * kSumThreads < cnt ? __ldcg(s + p0 + u * kSumThreads) : -INFINITY;
@@ -253,7 +346,7 @@ __global__ void __launch_bounds__(kSumThreads, 1) decode_sum_kernel(const DecAtt
     // ---- weighted sum ----
     const uint32_t chunks = (cnt + kTile - 1) / kTile;
     if (producer < kProducers) {
-        if ((cnt - 1) / kTile + 1 < kDepth) {  // a short context: the own row belongs to a tile requested above
+        if (!kScores && (cnt - 1) / kTile + 1 < kDepth) {  // a short context: the own row belongs to a tile requested above
             request((cnt - 1) / kTile, cnt - 1, cnt);
             asm volatile("cp.async.commit_group;" ::: "memory");
             asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -261,7 +354,7 @@ __global__ void __launch_bounds__(kSumThreads, 1) decode_sum_kernel(const DecAtt
 #pragma unroll 1
         for (uint32_t c = 0; c < chunks; ++c) {
             const uint32_t b = c & 1, dp = lane & 15, pg = lane >> 4;  // this lane: values 2 dp, 2 dp + 1 of positions 4 pg .. 4 pg + 3
-            request(c + kDepth - 1, 0, cnt);
+            request(c + kDepth - 1, 0, kScores ? cnt - 1 : cnt);
             asm volatile("cp.async.commit_group;" ::: "memory");
             asm volatile("cp.async.wait_group %0;" ::"n"(kDepth - 1) : "memory");
             __syncwarp();  // tile c's pieces of this warp have landed
@@ -271,7 +364,10 @@ __global__ void __launch_bounds__(kSumThreads, 1) decode_sum_kernel(const DecAtt
             for (uint32_t i = 0; i < kItems; ++i) {
                 const unsigned char* at = piece_at(c, i) + pg * 5 * 64 + dp * 4;
 #pragma unroll
-                for (int j = 0; j < 4; ++j) v[i][j] = *reinterpret_cast<const uint32_t*>(at + j * 64);
+                for (int j = 0; j < 4; ++j) {
+                    v[i][j] = *reinterpret_cast<const uint32_t*>(at + j * 64);
+                    if (kScores && c * kTile + (i * kProducers + producer) * 8 + pg * 4 + j == cnt - 1) v[i][j] = *reinterpret_cast<const uint32_t*>(v_new + 2 * dp);
+                }
                 pr[i] = *reinterpret_cast<const float4*>(ps + min(c * kTile + (i * kProducers + producer) * 8 + pg * 4, ps_floats - 4));
             }
             if (c >= 2) tile_sync(3 + b);  // the chains are done with this buffer's previous tile
@@ -371,14 +467,25 @@ size_t sum_smem(uint32_t positions) { return size_t((positions + 3) & ~3u) * 4 +
 
 bool attn_decode_fits(uint32_t dim, uint32_t positions) { return (dim == 64 || dim == 128 || dim == 256) && sum_smem(positions) <= 200 * 1024; }
 
-void launch_attn_decode(const DecAttnParams& a, uint32_t window, cudaStream_t s) {
-    if (a.dim == 64) launch_scores<64>(a, a.max_context, s);
-    else if (a.dim == 128) launch_scores<128>(a, a.max_context, s);
-    else launch_scores<256>(a, a.max_context, s);
+template <int DIM>
+static void launch_sum(const DecAttnParams& a, uint32_t window, cudaStream_t s) {
     static DeviceOnce once;
-    if (once.first()) BK_CUDA(cudaFuncSetAttribute(decode_sum_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    if (once.first()) BK_CUDA(cudaFuncSetAttribute(decode_sum_kernel<DIM>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     const uint32_t positions = window != 0 ? std::min(window, a.max_context) : a.max_context;
-    launch_dependent(decode_sum_kernel, dim3(a.heads * (a.dim / 32)), dim3(kSumThreads), sum_smem(positions), s, a, window, (positions + 3) & ~3u);
+    launch_dependent(decode_sum_kernel<DIM>, dim3(a.heads * (a.dim / 32)), dim3(kSumThreads), sum_smem(positions), s, a, window, (positions + 3) & ~3u, 1.0f);
+}
+
+int launch_attn_decode(const DecAttnParams& a, uint32_t window, bool fused, cudaStream_t s) {
+    if (fused && a.dim == 64) launch_sum<64>(a, window, s);
+    else if (fused && a.dim == 128) launch_sum<128>(a, window, s);
+    else {
+        if (a.dim == 64) launch_scores<64>(a, a.max_context, s);
+        else if (a.dim == 128) launch_scores<128>(a, a.max_context, s);
+        else launch_scores<256>(a, a.max_context, s);
+        launch_sum<0>(a, window, s);
+        return 2;
+    }
+    return 1;
 }
 
 }  // namespace bk

@@ -390,7 +390,7 @@ bool dec_attention_fits(uint32_t max_context, uint32_t heads, uint32_t dim, uint
     return dec_attn_out_smem(max_context, dec_attn_slice_width(heads, dim, sms)) <= 200 * 1024;
 }
 
-void launch_dec_attention(const RopeArgs& r, const AttnArgs& at, uint32_t sms, cudaStream_t s) {
+int launch_dec_attention(const RopeArgs& r, const AttnArgs& at, bool fused, uint32_t sms, cudaStream_t s) {
     DecAttnParams a{};
     a.q = r.q; a.k = r.k; a.v = r.v; a.q_norm = r.q_norm; a.k_norm = r.k_norm; a.rope = r.rope;
     a.q_bias = r.q_bias; a.k_bias = r.k_bias; a.v_bias = r.v_bias;
@@ -401,8 +401,7 @@ void launch_dec_attention(const RopeArgs& r, const AttnArgs& at, uint32_t sms, c
     const uint32_t group = a.heads / a.kv_heads;
     if (a.dim % 16 != 0 || a.dim > 256) throw CudaError("cuda: head size must be a multiple of 16 up to 256");
     if (chain_mode() != 0 && !relaxed("attention") && attn_decode_fits(a.dim, at.window != 0 ? std::min(at.window, a.max_context) : a.max_context)) {
-        launch_attn_decode(a, at.window, s);
-        return;
+        return launch_attn_decode(a, at.window, fused, s);
     }
     if (at.window != 0) throw CudaError("cuda: a sliding-window layer needs the kernels of attn_decode.cu for single tokens");
     // Contexts whose probabilities do not fit beside that kernel's tiles (and BRISK_CUDA_CHAIN=0, for comparison): a slice of a
@@ -432,7 +431,7 @@ void launch_dec_attention(const RopeArgs& r, const AttnArgs& at, uint32_t sms, c
         dec_attn_flash_kernel<<<dim3(a.heads, kFlashSplits), 128, 0, s>>>(a, partial);
         dec_attn_combine_kernel<<<a.heads, 128, 0, s>>>(a, partial);
         BK_CUDA(cudaGetLastError());
-        return;
+        return 3;
     }
     a.slice_width = dec_attn_slice_width(a.heads, a.dim, sms);
     const size_t smem2 = dec_attn_out_smem(a.max_context, a.slice_width);
@@ -440,6 +439,7 @@ void launch_dec_attention(const RopeArgs& r, const AttnArgs& at, uint32_t sms, c
     if (smem2 > 40 * 1024 && once.first()) BK_CUDA(cudaFuncSetAttribute(dec_attn_out_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     if (smem2 > 200 * 1024) throw CudaError("cuda: context too long for the single-token attention kernel");
     launch_pdl(dec_attn_out_kernel, dim3(a.heads, a.dim / a.slice_width), dim3(256), smem2, s, a);
+    return 2;
 }
 
 }  // namespace bk

@@ -151,7 +151,8 @@ bool launch_dec_multiply_two(const MatTarget* first, int count1, const MatTarget
                              uint32_t cols, uint32_t sms, cudaStream_t s);
 // Attention of the single new token: per-head norm + RoPE of q and the new k, f16 K/V store, scores, softmax and weighted sum.
 // Takes the same argument structs as the batched kernels (n is 1).
-void launch_dec_attention(const RopeArgs& r, const AttnArgs& at, uint32_t sms, cudaStream_t s);
+// fused: as one kernel where the geometry allows it; the number of kernels launched is returned.
+int launch_dec_attention(const RopeArgs& r, const AttnArgs& at, bool fused, uint32_t sms, cudaStream_t s);
 // Whether a context of max_context positions fits the shared memory of that attention's weighted-sum kernel.
 bool dec_attention_fits(uint32_t max_context, uint32_t heads, uint32_t dim, uint32_t sms);
 

@@ -187,11 +187,15 @@ struct Session {
     uint64_t position = 0;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
-    cudaGraphExec_t step_graph = nullptr;
-    uint64_t step_graph_nodes = 0;
+    // The captured single-token step, in two forms: [1] for contexts in which the fused attention kernel is the faster one.
+    cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
+    uint64_t step_graph_nodes[2] = {0, 0};
+    bool fused_attention = false;  // the form of the single-token step being run or captured
+    uint64_t layer_bytes = 0;      // of the layers' matrices
     // The persistent all-layer kernel of the single-token step (step.cu), when the model is within what it covers.
     StepPlan step_plan;
     bool step_enabled = false;
+    bool step_forced = false;  // BRISK_CUDA_STEP=force: the persistent kernel whatever was measured
     // One launch per token (token.cu): embedding, layers, head and arg-max in one kernel, where the model allows it.
     TokenPlan token_plan;
     bool token_enabled = false;
@@ -275,11 +279,17 @@ struct Session {
         stats.h2d_bytes += bytes;
     }
 
+    void drop_step_graphs() {
+        for (cudaGraphExec_t& g : step_graph) {
+            if (g) cudaGraphExecDestroy(g);
+            g = nullptr;
+        }
+    }
+
     ~Session() {
         if (stream) cudaStreamSynchronize(stream);
         // A graph that captured collectives keeps the communicator busy: release it before the communicator.
-        if (step_graph) cudaGraphExecDestroy(step_graph);
-        step_graph = nullptr;
+        drop_step_graphs();
         if (comm != nullptr && Nccl::get().ok()) Nccl::get().CommDestroy(comm);
         for (void* m : peer_mapped) cudaIpcCloseMemHandle(m);
         for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
@@ -417,6 +427,7 @@ struct Session {
         else head = upload_matrix(m.output.data != nullptr ? m.output : m.token_embd, "output.weight", vocab, hidden, staging, r * vocab_l, vocab_l);
         output_norm = upload_vector(m.output_norm, hidden, "output_norm.weight", true);
         layers.resize(n_layers);
+        const uint64_t before_layers = weight_bytes;
         for (uint32_t l = 0; l < n_layers; ++l) {
             const brisk_cuda_layer& s = m.layers[l];
             Layer& d = layers[l];
@@ -447,6 +458,7 @@ struct Session {
             if (d.no_rope) unrotated_layers = true;
             if (d.attn_post_norm || d.ffn_post_norm || d.slides) variant_layers = true;
         }
+        layer_bytes = weight_bytes - before_layers;
         if (gelu || embedding_scale != 1.0f || final_softcap != 0.0f) variant_layers = true;
         if (head_dim > 128) variant_layers = true;  // the persistent kernel takes heads of 64 and 128
         if (rope_dim != head_dim) variant_layers = true;  // ... and rotates whole heads
@@ -610,6 +622,7 @@ struct Session {
             }
         }
         const std::string token_why = why;
+        step_forced = env != nullptr && std::strcmp(env, "force") == 0;
         step_enabled = step_plan.build(args, sh, sms, stream, why);
         step_note = step_enabled ? "on: " + step_plan.description() : "off: " + why;
         if (!token_why.empty()) step_note += " (one launch per token: " + token_why + ")";
@@ -740,10 +753,7 @@ struct Session {
         }
         peer_table.alloc(table.size() * sizeof(uint2*));
         BK_CUDA(cudaMemcpy(peer_table.p, table.data(), table.size() * sizeof(uint2*), cudaMemcpyHostToDevice));
-        if (step_graph) {  // a captured step holds all-gathers: capture again with the peer exchange
-            cudaGraphExecDestroy(step_graph);
-            step_graph = nullptr;
-        }
+        drop_step_graphs();  // a captured step holds all-gathers: capture again with the peer exchange
         peer_on = true;
     }
 
@@ -828,8 +838,7 @@ struct Session {
             {
                 Scope sc(this, PH_ATTENTION);
                 if (single) {
-                    launch_dec_attention(r, at, sms, stream);
-                    launches += 2;
+                    launches += launch_dec_attention(r, at, fused_attention, sms, stream);
                 } else {
                     launch_qk_norm_rope_store(r, stream);
                     launch_attention(at, stream);
@@ -964,8 +973,8 @@ struct Session {
     }
     bool step_active() const { return (step_enabled || token_enabled) && !profiling; }
     bool token_active() const { return token_enabled && !profiling; }
-    void forward_decode() {
-        if (!step_active()) {
+    void forward_decode(bool persistent) {
+        if (!persistent) {
             run_layers(1, LAST_LOGITS, uint32_t(max_context), true);
             return;
         }
@@ -1036,14 +1045,15 @@ struct Session {
         return on && !token_enabled && step_plan.graph_safe();
     }
 
-    void build_step_graph() {
-        if (step_graph != nullptr || (flags & BRISK_CUDA_FLAG_NO_GRAPH) || (step_active() && !step_in_graph())) return;
+    // Captures the present form of the step, if it is to be replayed and has not been captured yet.
+    void build_step_graph(bool persistent) {
+        if (step_graph[fused_attention] != nullptr || (flags & BRISK_CUDA_FLAG_NO_GRAPH) || (persistent && !step_in_graph())) return;
         const uint64_t before = launches;
         cudaGraph_t graph = nullptr;
         BK_CUDA(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
         capturing = true;
         try {
-            forward_decode();
+            forward_decode(persistent);
         } catch (...) {
             capturing = false;
             cudaStreamEndCapture(stream, &graph);
@@ -1052,27 +1062,38 @@ struct Session {
         }
         capturing = false;
         BK_CUDA(cudaStreamEndCapture(stream, &graph));
-        step_graph_nodes = launches - before;
+        step_graph_nodes[fused_attention] = launches - before;
         launches = before;
-        const cudaError_t e = cudaGraphInstantiate(&step_graph, graph, 0);
+        const cudaError_t e = cudaGraphInstantiate(&step_graph[fused_attention], graph, 0);
         cudaGraphDestroy(graph);
         BK_CUDA(e);
     }
 
-    void step_on_device() {  // one token whose id is *d_tokens() at *d_position()
+    // Up to 512 visible positions the attention of a single token is one kernel (attn_decode.cu; its K rows are requested ahead
+    // of the projections: 0.6B shape at 181 positions 719 -> 661 us a token, at 520 - a second, late round of rows - 757 ->
+    // 790). With it one kernel per operation is also faster than the persistent kernel (727), which keeps the models whose
+    // layers stay in L2: there the two differ by 2-5 % (2 layers 58.9 and 57.4, 6 layers 150 and 143 us a token).
+    bool takes_fused_attention(uint64_t visible) const {
+        return visible <= 512 && head_dim <= 128 && rope_dim == head_dim && chain_mode() != 0 && attn_decode_fits(head_dim, uint32_t(max_context));
+    }
+    static constexpr uint64_t kLayersInL2 = uint64_t(100) << 20;
+
+    void step_on_device(uint64_t visible) {  // one token whose id is *d_tokens() at *d_position() = visible - 1
+        fused_attention = takes_fused_attention(visible);
+        const bool persistent = step_active() && (token_enabled || step_forced || !fused_attention || layer_bytes <= kLayersInL2);
         if (!single_kernels()) batched = true;
         // The fused weighted sum keeps a head's probabilities of the whole context in shared memory; past that the batched
         // kernels, which have no such limit, take single tokens too.
-        const bool too_long = !step_active() && !variant_layers &&
+        const bool too_long = !persistent && !variant_layers &&
                               !dec_attention_fits(uint32_t(max_context), heads_l, head_dim, sms);
         if ((flags & BRISK_CUDA_FLAG_NO_MEGAKERNEL) || too_long) {
             forward(1, LAST_LOGITS, uint32_t(max_context));  // the batched kernels, one token
-        } else if ((flags & BRISK_CUDA_FLAG_NO_GRAPH) || profiling || (step_active() && !step_in_graph())) {
-            forward_decode();
+        } else if ((flags & BRISK_CUDA_FLAG_NO_GRAPH) || profiling || (persistent && !step_in_graph())) {
+            forward_decode(persistent);
         } else {
-            build_step_graph();
-            BK_CUDA(cudaGraphLaunch(step_graph, stream));
-            launches += step_graph_nodes;
+            build_step_graph(persistent);
+            BK_CUDA(cudaGraphLaunch(step_graph[fused_attention], stream));
+            launches += step_graph_nodes[fused_attention];
         }
     }
 
@@ -1107,7 +1128,7 @@ struct Session {
             const uint32_t cnt = uint32_t(std::min<uint64_t>(kMaxBatch, n - begin));
             if (begin != 0) BK_CUDA(cudaStreamSynchronize(stream));  // the staging buffer is reused; calls end synchronised
             upload_inputs(tokens + begin, cnt);
-            if (cnt == 1 && (!all || n == 1)) step_on_device();  // one token: its one row of logits is all there is, with or without `all`
+            if (cnt == 1 && (!all || n == 1)) step_on_device(position + 1);  // one token: its one row of logits is all there is, with or without `all`
             else forward(cnt, all ? ALL_LOGITS : begin + cnt == n ? LAST_LOGITS : NO_LOGITS, uint32_t(position + cnt));
             position += cnt;
         }
@@ -1217,12 +1238,11 @@ struct Session {
             logit_history.alloc(steps * vocab * sizeof(float));
         }
         upload_inputs(&first, 1);
-        build_step_graph();
         BK_CUDA(cudaEventRecord(ev0, stream));
         const bool fused_pick = token_active() && !(flags & BRISK_CUDA_FLAG_NO_MEGAKERNEL);
         for (uint64_t i = 0; i < steps; ++i) {
             advance_on_device = fused_pick;
-            step_on_device();
+            step_on_device(position + i + 1);
             advance_on_device = false;
             if (out_logits != nullptr) {
                 BK_CUDA(cudaMemcpyAsync(logit_history.as<float>() + i * vocab, logits_b.p, size_t(vocab) * sizeof(float), cudaMemcpyDeviceToDevice, stream));

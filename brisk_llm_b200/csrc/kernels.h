@@ -130,14 +130,12 @@ struct AttnArgs {
 };
 size_t attn_scratch_floats(uint32_t n, uint32_t heads, uint32_t max_context);
 void launch_attention(const AttnArgs& a, cudaStream_t s);
-// Weighted sum for a few tokens (attn_chain.cu): a.scores holds their probabilities. One CTA per (token, one or
-// two query heads, slice of the head), chain warps and product warps; same results as the kernels above.
-bool attn_chain_fits(uint32_t n, uint32_t heads, uint32_t kv_heads, uint32_t dim, uint32_t max_visible, uint32_t sms);
+// Weighted sum for a few tokens (attn_chain.cu): a.scores holds their probabilities. A warp per (token, query head) and 32
+// values; same results as the kernels above.
 void launch_attn_chain(const AttnArgs& a, uint32_t sms, cudaStream_t s);
 constexpr uint32_t kChainMaxTokens = 24;      // more tokens than this share V rows through the tiled kernel instead
 // BRISK_CUDA_CHAIN: 0 never (nor the single-token kernel of attn_decode.cu), 1 wherever it fits, unset: 2..kChainMaxTokens tokens.
 int chain_mode();
-unsigned int* attn_chain_error_word();        // non-zero on the device after a launch whose wait for a bulk copy ran out
 
 // ---- fused single-token step (decode.cu) -------------------------------------------------------------------------
 // One multiply of the decode step: every CTA rebuilds the activation row in shared memory (x, optionally RMS-normed with

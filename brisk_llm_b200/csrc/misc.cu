@@ -340,7 +340,7 @@ void launch_attention(const AttnArgs& a, cudaStream_t s) {
     launch_attn_scores(a, sms, s);
     launch_attn_softmax(a, sms, s);
     const int mode = chain_mode();
-    if (mode != 0 && (a.n <= kChainMaxTokens || mode == 1) && attn_chain_fits(a.n, a.heads, a.kv_heads, a.dim, a.max_visible, sms)) launch_attn_chain(a, sms, s);
+    if (mode != 0 && (a.n <= kChainMaxTokens || mode == 1)) launch_attn_chain(a, sms, s);
     else launch_attn_weighted(a, sms, s);
 }
 

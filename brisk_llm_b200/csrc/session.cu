@@ -206,7 +206,6 @@ struct Session {
     std::vector<void*> peer_mapped;              // what cudaIpcOpenMemHandle returned (closed with the session)
     bool peer_on = false;
     unsigned int* gemm_tc_error_dev = nullptr;
-    unsigned int* chain_error_dev = nullptr;  // the few-token attention kernel's error word (a device symbol)
     unsigned int* step_error_host = nullptr;  // pinned copy of the kernel's barrier-timeout word
     uint64_t persistent_steps = 0;
     uint64_t launches = 0;  // kernels launched by the current call
@@ -564,9 +563,8 @@ struct Session {
         BK_CUDA(cudaMallocHost(&topk_host, 2 * kMaxTopK * sizeof(int32_t)));
         score_dev.alloc(kMaxBatch * sizeof(double));
         BK_CUDA(cudaMallocHost(&score_host, kMaxBatch * sizeof(double)));
-        BK_CUDA(cudaMallocHost(&step_error_host, 4 * sizeof(unsigned int)));  // [0] the persistent kernel's word, [1] the peer exchange's, [2] the few-token attention's
+        BK_CUDA(cudaMallocHost(&step_error_host, 4 * sizeof(unsigned int)));  // [0] the persistent kernel's word, [1] the peer exchange's
         step_error_host[0] = step_error_host[1] = step_error_host[2] = step_error_host[3] = 0;  // [3]: the tcgen05 prompt multiply's
-        chain_error_dev = attn_chain_error_word();
         gemm_tc_error_dev = gemm_tc_error_word();
         BK_CUDA(cudaStreamSynchronize(stream));
         plan_step();
@@ -998,10 +996,9 @@ struct Session {
     }
     // After the call's final synchronisation: did a barrier wait of the persistent kernel run out?
     void queue_step_check() {
-        // The few-token attention and the tcgen05 multiply have bounded waits: their error words, read with the results of a call
-        // that may have run them. (A word is a copy of its own, about 2 us at the end of every call.)
+        // The tcgen05 multiply has bounded waits: its error word, read with the results of a call that may have run it. (A word is
+        // a copy of its own, about 2 us at the end of every call.)
         if (batched) {
-            BK_CUDA(cudaMemcpyAsync(step_error_host + 2, chain_error_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
             BK_CUDA(cudaMemcpyAsync(step_error_host + 3, gemm_tc_error_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
         }
         if (peer_on) BK_CUDA(cudaMemcpyAsync(step_error_host + 1, peer_state.as<unsigned int>() + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
@@ -1018,11 +1015,6 @@ struct Session {
             step_error_host[1] = 0;
             BK_CUDA(cudaMemsetAsync(peer_state.as<unsigned int>() + 1, 0, sizeof(unsigned int), stream));
             throw CudaError("cuda: a tensor-parallel peer did not deliver its share of an exchange in time; the results of this call are invalid");
-        }
-        if (step_error_host[2] != 0) {
-            step_error_host[2] = 0;
-            BK_CUDA(cudaMemsetAsync(chain_error_dev, 0, sizeof(unsigned int), stream));
-            throw CudaError("cuda: a bulk copy of the few-token attention kernel did not complete in time; the results of this call are invalid");
         }
         if ((step_enabled || token_enabled) && *step_error_host != 0) {
             *step_error_host = 0;

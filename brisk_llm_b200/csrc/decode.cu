@@ -143,13 +143,18 @@ void dispatch_dec(DecMatParams& p, bool pair, uint32_t sms, cudaStream_t s) {
     if (relaxed("rowsum")) div4 = false;
     if (div4 && !heavy && rows / 4 >= enough) rw = 4;
     else if (div2 && rows / 2 >= enough) rw = 2;
+    if constexpr (!heavy) {
+        if (rw == 4) {
+            if (pair) launch_dec_one<F, 4, true>(p, sms, s);
+            else launch_dec_one<F, 4, false>(p, sms, s);
+            return;
+        }
+    }
     if (pair) {
-        if (rw == 4) launch_dec_one<F, 4, true>(p, sms, s);
-        else if (rw == 2) launch_dec_one<F, 2, true>(p, sms, s);
+        if (rw == 2) launch_dec_one<F, 2, true>(p, sms, s);
         else launch_dec_one<F, 1, true>(p, sms, s);
     } else {
-        if (rw == 4) launch_dec_one<F, 4, false>(p, sms, s);
-        else if (rw == 2) launch_dec_one<F, 2, false>(p, sms, s);
+        if (rw == 2) launch_dec_one<F, 2, false>(p, sms, s);
         else launch_dec_one<F, 1, false>(p, sms, s);
     }
 }

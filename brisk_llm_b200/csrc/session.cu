@@ -196,6 +196,7 @@ struct Session {
     StepPlan step_plan;
     bool step_enabled = false;
     bool step_forced = false;  // BRISK_CUDA_STEP=force: the persistent kernel whatever was measured
+    bool step_graph_wanted = false;  // BRISK_CUDA_STEP_GRAPH=1, see step_in_graph()
     // One launch per token (token.cu): embedding, layers, head and arg-max in one kernel, where the model allows it.
     TokenPlan token_plan;
     bool token_enabled = false;
@@ -621,6 +622,8 @@ struct Session {
         }
         const std::string token_why = why;
         step_forced = env != nullptr && std::strcmp(env, "force") == 0;
+        const char* graph_env = std::getenv("BRISK_CUDA_STEP_GRAPH");
+        step_graph_wanted = graph_env != nullptr && std::atoi(graph_env) != 0;
         step_enabled = step_plan.build(args, sh, sms, stream, why);
         step_note = step_enabled ? "on: " + step_plan.description() : "off: " + why;
         if (!token_why.empty()) step_note += " (one launch per token: " + token_why + ")";
@@ -983,7 +986,6 @@ struct Session {
             }
             token_plan.launch(stream, advance_on_device);
             ++launches;
-            ++persistent_steps;
             return;
         }
         // embedding | all layers in one persistent kernel | output head
@@ -992,9 +994,9 @@ struct Session {
         MatTarget target{head, logits_b.as<float>(), vocab};
         launch_dec_multiply(&target, 1, hidden_b.as<float>(), output_norm, eps, hidden, EPI_STORE, sms, stream, nullptr);
         launches += 3;
-        ++persistent_steps;
     }
-    // After the call's final synchronisation: did a barrier wait of the persistent kernel run out?
+    // After the call's final synchronisation: did a wait of the persistent kernel run out? Asked after every call that ran it,
+    // enqueued or replayed from a graph (step_on_device counts both).
     void queue_step_check() {
         // The tcgen05 multiply has bounded waits: its error word, read with the results of a call that may have run it. (A word is
         // a copy of its own, about 2 us at the end of every call.)
@@ -1021,6 +1023,7 @@ struct Session {
             if (token_enabled) token_plan.rearm(stream);
             else step_plan.rearm(stream);
             step_enabled = token_enabled = false;  // later steps take the per-operation kernels
+            drop_step_graphs();                    // ... also where a graph holds the persistent kernel
             step_note = "off: a grid barrier timed out";
             throw CudaError("cuda: a grid barrier of the single-token kernel timed out; the results of this call are invalid");
         }
@@ -1029,13 +1032,7 @@ struct Session {
     // Three launches per token gain little from a graph; BRISK_CUDA_STEP_GRAPH=1 captures them all the same - unless the
     // kernel exchanges tagged pairs: its tags are a launch parameter that must change with every token, and a replayed
     // graph would launch with the tags of the token it was captured for.
-    bool step_in_graph() const {
-        static const bool on = [] {
-            const char* env = std::getenv("BRISK_CUDA_STEP_GRAPH");
-            return env != nullptr && std::atoi(env) != 0;
-        }();
-        return on && !token_enabled && step_plan.graph_safe();
-    }
+    bool step_in_graph() const { return step_graph_wanted && !token_enabled && step_plan.graph_safe(); }
 
     // Captures the present form of the step, if it is to be replayed and has not been captured yet.
     void build_step_graph(bool persistent) {
@@ -1080,7 +1077,10 @@ struct Session {
                               !dec_attention_fits(uint32_t(max_context), heads_l, head_dim, sms);
         if ((flags & BRISK_CUDA_FLAG_NO_MEGAKERNEL) || too_long) {
             forward(1, LAST_LOGITS, uint32_t(max_context));  // the batched kernels, one token
-        } else if ((flags & BRISK_CUDA_FLAG_NO_GRAPH) || profiling || (persistent && !step_in_graph())) {
+            return;
+        }
+        if (persistent) ++persistent_steps;
+        if ((flags & BRISK_CUDA_FLAG_NO_GRAPH) || profiling || (persistent && !step_in_graph())) {
             forward_decode(persistent);
         } else {
             build_step_graph(persistent);

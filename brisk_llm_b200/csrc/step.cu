@@ -757,14 +757,15 @@ bool StepPlan::build(const std::vector<StepLayerArgs>& layers, const StepShared&
     impl_->plain_hidden = shared.hidden;
     impl_->hidden_size = shared.hidden_size;
     impl_->tags_per_launch = uint32_t(descs.size()) * 6 + 2;
+    // BRISK_CUDA_TEST_POLL_TIMEOUT=1 (tests only): the second layer's first multiply waits for a tag nobody writes and every
+    // wait gives up after 64 re-reads - the kernel ends at once with the error word set, and the host must raise, keep the
+    // position and carry on with the per-operation kernels. Every access stays in bounds; nothing faults or hangs. The barrier
+    // form has the word set from the start instead, as a barrier that ran out leaves it.
+    const char* env = std::getenv("BRISK_CUDA_TEST_POLL_TIMEOUT");
+    const bool inject = env != nullptr && std::strcmp(env, "1") == 0;
     {
-        // BRISK_CUDA_TEST_POLL_TIMEOUT=1 (tests only): the second layer's first multiply waits for a tag nobody writes and every
-        // wait gives up after 64 re-reads - the kernel ends at once with the error word set, and the host must raise, keep the
-        // position and carry on with the per-operation kernels. Every access stays in bounds; nothing faults or hangs.
-        const char* env = std::getenv("BRISK_CUDA_TEST_POLL_TIMEOUT");
-        const bool inject = tagged && env != nullptr && std::strcmp(env, "1") == 0;
-        impl_->fault_layer = inject ? std::min<uint32_t>(1u, uint32_t(descs.size()) - 1) : 0xffffffffu;
-        const uint32_t limit = inject ? 64u : kPollLimitDefault;
+        impl_->fault_layer = inject && tagged ? std::min<uint32_t>(1u, uint32_t(descs.size()) - 1) : 0xffffffffu;
+        const uint32_t limit = inject && tagged ? 64u : kPollLimitDefault;
         BK_CUDA(cudaMemcpyToSymbolAsync(c_poll_limit, &limit, sizeof(limit), 0, cudaMemcpyHostToDevice, s));
     }
     impl_->n_layers = uint32_t(descs.size());
@@ -775,6 +776,7 @@ bool StepPlan::build(const std::vector<StepLayerArgs>& layers, const StepShared&
     BK_CUDA(cudaMalloc(&impl_->sync_dev, 64));
     BK_CUDA(cudaMemcpyAsync(impl_->layers_dev, descs.data(), descs.size() * sizeof(StepLayerDesc), cudaMemcpyHostToDevice, s));
     BK_CUDA(cudaMemsetAsync(impl_->sync_dev, 0, 64, s));
+    if (inject && !tagged) BK_CUDA(cudaMemsetAsync(impl_->sync_dev + 2, 1, sizeof(unsigned int), s));
     BK_CUDA(cudaStreamSynchronize(s));  // descs goes out of scope
     char text[96];
     std::snprintf(text, sizeof text, "%s, rows per warp %d/%d/%d/%d, %u CTAs, %zu KB shared", tagged ? "tagged exchange" : "grid barriers", pick->rw[0],

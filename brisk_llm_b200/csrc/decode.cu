@@ -391,8 +391,11 @@ bool launch_dec_multiply_two(const MatTarget* first, int count1, const MatTarget
     return true;
 }
 
+// The kernels of attn_decode.cu run wherever `positions` (the context, or a sliding layer's window) fit them.
+static bool attn_decode_runs(uint32_t dim, uint32_t positions) { return chain_mode() != 0 && !relaxed("attention") && attn_decode_fits(dim, positions); }
+
 bool dec_attention_fits(uint32_t max_context, uint32_t heads, uint32_t dim, uint32_t sms) {
-    return dec_attn_out_smem(max_context, dec_attn_slice_width(heads, dim, sms)) <= 200 * 1024;
+    return attn_decode_runs(dim, max_context) || dec_attn_out_smem(max_context, dec_attn_slice_width(heads, dim, sms)) <= 200 * 1024;
 }
 
 int launch_dec_attention(const RopeArgs& r, const AttnArgs& at, bool fused, uint32_t sms, cudaStream_t s) {
@@ -405,7 +408,7 @@ int launch_dec_attention(const RopeArgs& r, const AttnArgs& at, bool fused, uint
     a.pdl = pdl_mode();
     const uint32_t group = a.heads / a.kv_heads;
     if (a.dim % 16 != 0 || a.dim > 256) throw CudaError("cuda: head size must be a multiple of 16 up to 256");
-    if (chain_mode() != 0 && !relaxed("attention") && attn_decode_fits(a.dim, at.window != 0 ? std::min(at.window, a.max_context) : a.max_context)) {
+    if (attn_decode_runs(a.dim, at.window != 0 ? std::min(at.window, a.max_context) : a.max_context)) {
         return launch_attn_decode(a, at.window, fused, s);
     }
     if (at.window != 0) throw CudaError("cuda: a sliding-window layer needs the kernels of attn_decode.cu for single tokens");

@@ -151,7 +151,8 @@ bool launch_dec_multiply_two(const MatTarget* first, int count1, const MatTarget
 // Takes the same argument structs as the batched kernels (n is 1).
 // fused: as one kernel where the geometry allows it; the number of kernels launched is returned.
 int launch_dec_attention(const RopeArgs& r, const AttnArgs& at, bool fused, uint32_t sms, cudaStream_t s);
-// Whether a context of max_context positions fits the shared memory of that attention's weighted-sum kernel.
+// Whether a context of max_context positions fits the shared memory of the weighted-sum kernel that would run: 33792 positions
+// for attn_decode.cu's (heads of 64 to 256), else 26496 or 38848 (slices of 32 or 16 values, see dec_attn_slice_width).
 bool dec_attention_fits(uint32_t max_context, uint32_t heads, uint32_t dim, uint32_t sms);
 
 // ---- the single-token step of all layers as one persistent kernel (step.cu) -------------------------------------

@@ -1164,7 +1164,7 @@ struct Session {
                 check_tokens(tokens + good, cnt, true);
             } catch (...) {
                 position = before;
-                if (good > 0) score(tokens, good, good);
+                if (good > 0) score(tokens, good, 0);
                 throw;
             }
             good += cnt;
@@ -1173,9 +1173,8 @@ struct Session {
         return score(tokens, n, n - 1);
     }
 
-    // Appends n tokens and returns the summed log-probability of tokens[1 .. rows]; rows < n unless only the appending matters.
+    // Appends n tokens and returns the summed log-probability of tokens[1 .. rows], rows < n; rows = 0 appends only (no head).
     double score(const int32_t* tokens, uint64_t n, uint64_t rows) {
-        rows = std::min<uint64_t>(rows, n - 1);
         begin_call();
         BK_CUDA(cudaEventRecord(ev0, stream));
         double total = 0.0;

@@ -25,3 +25,20 @@ def test_log_likelihood_is_the_log_softmax_of_the_rows(n, chunk):
         with pytest.raises(RuntimeError, match="out of range"):
             s.log_likelihood(bad, chunk)
         assert s.position() == (n - 1) // chunk * chunk
+
+
+def test_an_error_of_a_later_chunk_scores_nothing():
+    """The chunks before the error are appended without the output head: no log-probability leaves the device, and the sequence
+    goes on as if they had been evaluated."""
+    spec = synth.tiny(synth.QWEN3_0_6B, layers=1, vocab=777, context=600)
+    toks = synth.random_tokens(spec, 130, seed=1)
+    bad = np.append(toks, np.int32(spec.vocab))
+    with engine.CudaSession(synth.generate(spec, seed=3)) as s:
+        s.eval(toks[:128])
+        want = s.eval(toks[128:])
+        s.rollback(0)
+        with pytest.raises(RuntimeError, match="out of range"):
+            s.log_likelihood(bad, 64)
+        assert s.position() == 128
+        assert s.stats()["d2h_bytes"] == 0
+        assert np.array_equal(s.eval(toks[128:]), want)

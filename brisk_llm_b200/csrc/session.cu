@@ -1059,17 +1059,21 @@ struct Session {
     }
 
     // Up to 512 visible positions the attention of a single token is one kernel (attn_decode.cu; its K rows are requested ahead
-    // of the projections: 0.6B shape at 181 positions 719 -> 661 us a token, at 520 - a second, late round of rows - 757 ->
-    // 790). With it one kernel per operation is also faster than the persistent kernel (727), which keeps the models whose
-    // layers stay in L2: there the two differ by 2-5 % (2 layers 58.9 and 57.4, 6 layers 150 and 143 us a token).
+    // of the projections: 0.6B shape, one kernel per operation, at 181 positions 719 -> 661 us a token, at 520 - a second, late
+    // round of rows - 757 -> 790).
     bool takes_fused_attention(uint64_t visible) const {
         return visible <= 512 && head_dim <= 128 && rope_dim == head_dim && chain_mode() != 0 && attn_decode_fits(head_dim, uint32_t(max_context));
     }
-    static constexpr uint64_t kLayersInL2 = uint64_t(100) << 20;
+    // With the fused attention one kernel per operation also beats the persistent kernel, until the positions eat the gain up.
+    // Persistent / per operation, us a token at 64, 256 and 440 positions: 4 layers of the 0.6B shape (35 MB) 99/97, 104/105,
+    // 109/114; 11 layers (97 MB) 261/244, 274/265, 280/288; 12 (106 MB) 283/264, 298/287, 304/311; 28 (248 MB) 643/598, 672/652,
+    // 697/715. The ratio is the same from 8 layers on (1.06-1.08, 1.03-1.04, 0.97): nothing in it marks this line, it is not the
+    // L2's. It keeps models of few layers, where the whole difference is 17 us at most, on one path at every position.
+    static constexpr uint64_t kFewLayers = uint64_t(100) << 20;
 
     void step_on_device(uint64_t visible) {  // one token whose id is *d_tokens() at *d_position() = visible - 1
         fused_attention = takes_fused_attention(visible);
-        const bool persistent = step_active() && (token_enabled || step_forced || !fused_attention || layer_bytes <= kLayersInL2);
+        const bool persistent = step_active() && (token_enabled || step_forced || !fused_attention || layer_bytes <= kFewLayers);
         if (!single_kernels()) batched = true;
         // The fused weighted sum keeps a head's probabilities of the whole context in shared memory; past that the batched
         // kernels, which have no such limit, take single tokens too.

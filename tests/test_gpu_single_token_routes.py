@@ -55,3 +55,25 @@ def test_long_sessions_keep_the_single_token_kernels(context, fits):
             for t in toks[at:at + 2]:
                 assert np.array_equal(s.eval([t]), general.eval([t])), s.position()
                 assert (s.stats()["kernel_launches"] == usual) == fits
+
+
+@pytest.mark.parametrize("layers", [11, 12])
+def test_the_switch_at_512_positions(layers):
+    """Layers past 100 MB (12 of this shape; 11 stay below): one kernel per operation up to 512 positions, the persistent
+    kernel from there on, in one call and between calls; smaller models stay persistent."""
+    spec = synth.tiny(synth.QWEN3_0_6B, layers=layers, vocab=512, context=640)
+    model = synth.perturb_norms(synth.generate(spec, seed=5, share_layers=True))
+    toks = synth.random_tokens(spec, 512, seed=6)
+    with engine.CudaSession(model) as s, engine.CudaSession(model, flags=abi.FLAG_NO_MEGAKERNEL) as general:
+        for session in (s, general):
+            session.eval(toks[:509])
+        for at in range(509, 512):
+            assert np.array_equal(s.eval(toks[at:at + 1]), general.eval(toks[at:at + 1]))
+            assert s.stats()["persistent_steps"] == (1 if layers < 12 else 0)
+        for session in (s, general):
+            session.rollback(506)
+        ids, logits = s.generate_greedy(7, 10, want_logits=True)  # the tokens at 512 and later see more than 512 positions
+        assert s.stats()["persistent_steps"] == (10 if layers < 12 else 4)
+        want_ids, want = general.generate_greedy(7, 10, want_logits=True)
+        assert np.array_equal(ids, want_ids) and np.array_equal(logits, want)
+        assert np.array_equal(s.eval([3]), general.eval([3])) and s.stats()["persistent_steps"] == 1

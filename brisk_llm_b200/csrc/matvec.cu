@@ -1,4 +1,4 @@
-// Streaming multiply: a few token rows (1..8) against whole weight matrices, HBM-bound.
+// Streaming multiply: a few token rows (1..8; the super-block formats: 1) against whole weight matrices, HBM-bound.
 //
 // One warp owns RW consecutive weight rows and walks their 16-byte units with lane stride, so each
 // load instruction of a warp covers 512 contiguous bytes of a row and every lane keeps RW independent
@@ -137,6 +137,7 @@ void launch_one(const Params& p, uint32_t groups, cudaStream_t s) {
 
 // Rows per warp: as many as keep one lane per chain (<= 32 chains) and divide every target's row count.
 //   1 token : 8 | 4 | 1        2-4 tokens: 4 | 1        5-8 tokens: 4 (pair: 2) | 1
+// The super-block formats go to gemm_k.cu from 2 tokens on, whatever their row length.
 template <class F, bool PAIR>
 void dispatch_tile(Params& p, cudaStream_t s) {
     auto divides = [&](uint32_t rw) {
@@ -159,6 +160,8 @@ void dispatch_tile(Params& p, cudaStream_t s) {
         if (!heavy && divides(8)) launch_one<F, 1, 8, PAIR>(p, groups_for(8), s);
         else if (divides(4)) launch_one<F, 1, 4, PAIR>(p, groups_for(4), s);
         else launch_one<F, 1, 1, PAIR>(p, groups_for(1), s);
+    } else if constexpr (std::is_same_v<F, FQ4_K> || std::is_same_v<F, FQ5_K> || std::is_same_v<F, FQ6_K> || std::is_same_v<F, FTQ2_0>) {
+        throw CudaError("cuda: the streaming multiply takes one token of the super-block formats");
     } else if (p.ntok <= 4) {
         if (divides(4)) launch_one<F, 4, 4, PAIR>(p, groups_for(4), s);
         else launch_one<F, 4, 1, PAIR>(p, groups_for(1), s);

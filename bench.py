@@ -11,7 +11,8 @@ runs an independent replica (batch-1 decode of one sequence has nothing to shard
 After the headline the same run times the one configuration that does shard - the Mistral-7B-shaped Q4_0 model,
 8192-token prompt + 512 greedy steps - tensor-parallel over all N ranks (N = 1: on the one GPU) and reports it in the
 `tensor_parallel` object, so the 1 -> N scaling of that configuration can be read from the per-N lines.
-`--impl reference` times the reference's own CPU engine on the host cores instead.
+`--impl reference` times the reference's own CPU engine on the host cores instead: the library `make -C oracle ref` builds
+from a reference checkout. Without it the line says so; nothing else stands in.
 """
 from __future__ import annotations
 
@@ -223,6 +224,12 @@ def cpu_sample_sizes(spec, prompt, decode):
 def run_reference_arm(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
+        return
+    sys.path.insert(0, os.path.join(ROOT, "tests"))
+    import helpers as H
+    if not H.have_ref():
+        print(json.dumps({"impl": "reference", "unavailable": "the reference engine is a C++ project that has to be built from a checkout "
+                          "(make -C oracle ref); there is none here and no prebuilt oracle/_ref"}), flush=True)
         return
     spec, prompt, decode = workload_for(args)
     model = synth.generate(spec, seed=0, share_layers=spec.layers * spec.hidden * spec.ffn > 1e9)

@@ -211,3 +211,22 @@ def test_bench_helpers_follow_the_workload():
     s.t0 = now + 2.0
     fallback = s.stop()
     assert fallback["samples"] == 2 and fallback["reasons"] == ["sw_power_cap"] and "warm-up" in fallback["window"]
+
+
+def test_reference_arm_without_the_reference_says_unavailable(monkeypatch, capsys):
+    """--impl reference runs the reference's engine or nothing: where it is not built, one line says so and no model, kernel or
+    checker of this repository stands in."""
+    import importlib.util
+    import json
+    spec_ = importlib.util.spec_from_file_location("bench_module", os.path.join(H.ROOT, "bench.py"))
+    bench = importlib.util.module_from_spec(spec_)
+    spec_.loader.exec_module(bench)
+
+    def never(*args, **kwargs):
+        raise AssertionError("the reference arm went on without the reference")
+    monkeypatch.setattr(H, "have_ref", lambda: False)
+    monkeypatch.setattr(bench, "cpu_engine", never)
+    monkeypatch.setattr("sys.argv", ["bench.py", "--impl", "reference", "--steps", "2", "--warmup", "1"])
+    bench.main()
+    line = json.loads(capsys.readouterr().out)
+    assert line["impl"] == "reference" and line["unavailable"] and "value" not in line

@@ -22,6 +22,7 @@
 #include "attn_decode.h"
 #include "decode_body.cuh"
 #include "exact_math.h"
+#include "packed.cuh"
 #include "pdl.cuh"
 
 namespace bk {
@@ -36,13 +37,6 @@ constexpr uint32_t kPieceBytes = 9 * 64;                // a staged piece: rows 
 constexpr uint32_t kRingBytes = kDepth * kPieces * kPieceBytes;
 
 constexpr uint32_t kTile = kTileFloats / 32, kBatch = 32;  // positions per tile, and that a chain lane loads ahead
-
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-// the packed sum: an addition the assembler does not contract with the multiplication before it (see attn_prompt.cu)
-__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) { f32x2 r; asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c)); return r; }
 
 template <int DIM>
 __global__ void __launch_bounds__(kScoreThreads, 2) decode_scores_kernel(const DecAttnParams a, float one) {

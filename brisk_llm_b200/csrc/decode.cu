@@ -16,12 +16,10 @@
 
 #include "attn_decode.h"
 #include "decode_body.cuh"
+#include "pdl.cuh"
 
 namespace bk {
 namespace {
-
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // How the step's kernels overlap: 2 (default) = programmatic dependent launch, dependents released after a kernel's
 // prologue, so that only the next kernel runs ahead: its CTAs are resident with their first weights (or K rows and V tiles)
@@ -44,28 +42,18 @@ void launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, c
         BK_CUDA(cudaGetLastError());
         return;
     }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    BK_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
+    launch_dependent(kernel, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
 // ---- multiply ---------------------------------------------------------------------------------------------------
 struct PdlGate {  // the gate of the one-kernel-per-operation path: programmatic dependent launch, or nothing
     int pdl;
     __device__ __forceinline__ void wait() {
-        if (pdl == 1) pdl_launch_dependents();
-        pdl_wait();
+        if (pdl == 1) release_next();
+        wait_for_previous();
     }
     __device__ __forceinline__ void prologue_done() {
-        if (pdl == 2) pdl_launch_dependents();
+        if (pdl == 2) release_next();
     }
 };
 
@@ -163,8 +151,8 @@ void dispatch_dec(DecMatParams& p, bool pair, uint32_t sms, cudaStream_t s) {
 template <int GROUP, int DIM>
 __global__ void __launch_bounds__(128) dec_attn_scores_kernel(const DecAttnParams a) {
     extern __shared__ float sm[];  // q heads [GROUP][DIM] | new k [DIM]
-    if (a.pdl != 0) pdl_launch_dependents();
-    pdl_wait();
+    if (a.pdl != 0) release_next();
+    wait_for_previous();
     constexpr uint32_t dim = DIM;
     const uint32_t kvh = blockIdx.y;
     const uint32_t pos = *a.position, visible = pos + 1;
@@ -243,8 +231,8 @@ __global__ void __launch_bounds__(128) dec_attn_scores_kernel(const DecAttnParam
 struct PdlGateEarly {  // releases the dependents as soon as the kernel runs
     int pdl;
     __device__ __forceinline__ void wait() {
-        if (pdl != 0) pdl_launch_dependents();
-        pdl_wait();
+        if (pdl != 0) release_next();
+        wait_for_previous();
     }
 };
 

@@ -23,6 +23,7 @@
 // full issue, against ~140 for the same arithmetic behind mma.sync fragments (gemm.cu), which also spends issue slots on
 // fragment loads and on the MMAs themselves.
 #include "kernels.h"
+#include "packed.cuh"
 
 namespace bk {
 namespace {
@@ -120,16 +121,6 @@ __device__ __forceinline__ void tmem_ld_nowait(uint32_t taddr, uint32_t (&v)[kEC
         : "r"(taddr)
         : "memory");
 }
-// Two f32 operations per instruction (packed f32x2, IEEE round-to-nearest in each half: the same results as two scalar
-// instructions - measured on 4 M random operands). The epilogue is bound by its f32 instruction count. NOT used for the
-// final addition: a mul.rn.f32x2 whose only use is an add.rn.f32x2 gets contracted into a fused multiply-add by the
-// assembler (measured: 36 % of the results change, with or without -fmad=false), and the reference does not fuse.
-using f32x2 = unsigned long long;
-__device__ __forceinline__ f32x2 pack2(float a, float b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b)); return r; }
-__device__ __forceinline__ f32x2 pack2(uint32_t a, uint32_t b) { f32x2 r; asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "r"(a), "r"(b)); return r; }
-__device__ __forceinline__ void unpack2(f32x2 v, float& a, float& b) { asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v)); }
-__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b) { f32x2 r; asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
-__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) { f32x2 r; asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b)); return r; }
 
 // four nibbles 0..15, one per byte -> four signed bytes (nibble - 8): no borrow can cross a byte once bit 7 is set
 __device__ __forceinline__ uint32_t recentre(uint32_t nibbles) { return ((nibbles | 0x80808080u) - 0x08080808u) ^ 0x80808080u; }

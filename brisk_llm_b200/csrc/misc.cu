@@ -14,28 +14,10 @@
 namespace bk {
 namespace {
 
-// No-op unless the kernel was launched as a programmatic dependent of its predecessor (the decode step does that).
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <class... Params, class... Args>
-void launch_pdl(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args&&... args) {
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = grid;
-    cfg.blockDim = block;
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr{};
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-    BK_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
-}
-
 // ---- embedding: one token row of the embedding matrix, decoded exactly like the reference's dequantize_*
 // (src/quant.cpp:196-307, :565-578; embedding_row, src/model.cpp:27-70), read from the repacked planes. ----
 __global__ void embed_kernel(const DevMatrix m, const int32_t* tokens, float* __restrict__ hidden) {
-    pdl_wait();
+    wait_for_previous();
     const uint32_t t = blockIdx.x;
     uint32_t row = uint32_t(tokens[t]);
     if (row >= m.rows) row = 0;  // the host checks ids it is given; an id chosen on the device is checked where it is chosen, this is the last guard
@@ -227,7 +209,7 @@ __device__ __forceinline__ void better(float& v, int32_t& i, float ov, int32_t o
 }
 
 __global__ void __launch_bounds__(256) argmax_stage1(const float* logits, uint32_t vocab, float* pv, int32_t* pi) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");  // no-op unless launched as a programmatic dependent
+    wait_for_previous();
     const uint32_t row = blockIdx.y;
     const float* x = logits + size_t(row) * vocab;
     float v = -INFINITY;
@@ -255,7 +237,7 @@ __global__ void __launch_bounds__(256) argmax_stage1(const float* logits, uint32
 // an id inside the vocabulary, whatever the logits hold.
 __global__ void __launch_bounds__(256) argmax_stage2(const float* pv, const int32_t* pi, const float* logits, uint32_t vocab, int32_t* out,
                                                      int32_t* token_slot, uint32_t* position, int32_t* history, uint32_t* history_len) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    wait_for_previous();
     const uint32_t row = blockIdx.x;
     float v = -INFINITY;
     int32_t idx = 0x7fffffff;
@@ -310,7 +292,7 @@ void launch_tp_unpack(const float* gathered, float* dst, uint32_t n, uint32_t ro
 }
 
 void launch_embed(const DevMatrix& embd, const int32_t* tokens_dev, uint32_t n, float* hidden, cudaStream_t s) {
-    launch_pdl(embed_kernel, dim3(n), dim3(128), 0, s, embd, tokens_dev, hidden);
+    launch_dependent(embed_kernel, dim3(n), dim3(128), 0, s, embd, tokens_dev, hidden);
 }
 
 void launch_qk_norm_rope_store(const RopeArgs& a, cudaStream_t s) {
@@ -356,8 +338,8 @@ void launch_argmax(const float* logits, uint32_t vocab, uint32_t n, int32_t* out
 
 void launch_argmax_advance(const float* logits, uint32_t vocab, int32_t* out_token, float* scratch_val, int32_t* scratch_idx,
                            int32_t* token_slot, uint32_t* position, int32_t* history, uint32_t* history_len, cudaStream_t s) {
-    launch_pdl(argmax_stage1, dim3(kArgmaxBlocks, 1), dim3(256), 0, s, logits, vocab, scratch_val, scratch_idx);
-    launch_pdl(argmax_stage2, dim3(1), dim3(256), 0, s, (const float*)scratch_val, (const int32_t*)scratch_idx, logits, vocab, out_token, token_slot,
+    launch_dependent(argmax_stage1, dim3(kArgmaxBlocks, 1), dim3(256), 0, s, logits, vocab, scratch_val, scratch_idx);
+    launch_dependent(argmax_stage2, dim3(1), dim3(256), 0, s, (const float*)scratch_val, (const int32_t*)scratch_idx, logits, vocab, out_token, token_slot,
                position, history, history_len);
 }
 

@@ -1,9 +1,10 @@
-// Programmatic dependent launch of the batched kernels. A kernel started with launch_dependent() becomes resident while the
-// one before it drains; it may read constants (weights) at once, everything else only behind wait_for_previous(), and
-// lets the next kernel start with release_next() some time after it has waited itself - so nothing runs ahead of results
-// that are more than one kernel away. Short kernels release at once, long ones when their main loop is done; CTAs that
-// wait beside a running kernel for long slow it down (prompts of 512 to 800 tokens: 5-18 % between the two). What it saves
-// is the gap between two kernels, 1-2 us, of which a layer of a short prompt has twelve.
+// Programmatic dependent launch of the batched and the single-token kernels (those of decode.cu: see pdl_mode() there). A kernel
+// started with launch_dependent() becomes resident while the one before it drains; it may read constants (weights) at once,
+// everything else only behind wait_for_previous(), and lets the next kernel start with release_next() some time after it
+// has waited itself - so nothing runs ahead of results that are more than one kernel away. Short kernels release at once,
+// long ones when their main loop is done; CTAs that wait beside a running kernel for long slow it down (prompts of 512 to
+// 800 tokens: 5-18 % between the two). What it saves is the gap between two kernels, 1-2 us, of which a layer of a short
+// prompt has twelve.
 #pragma once
 
 #include <utility>
@@ -13,6 +14,7 @@
 namespace bk {
 
 #ifdef __CUDACC__
+// No-ops in a kernel that was launched in plain stream order.
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void release_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -1,5 +1,5 @@
-// Attention of the single new token in two kernels, bit-identical to the CPU engine's (src/model.cpp:1022-1093; the orders
-// of the float operations are those of attn_prompt.cu). Both are launched with programmatic dependent launch and request
+// Attention of the single new token in two kernels, or one up to 512 positions, bit-identical to the CPU engine's (src/model.cpp:1022-1093; the orders
+// of the float operations are those of attn_prompt.cu). They are launched with programmatic dependent launch and request
 // the K rows and V tiles of earlier positions before the results they depend on are complete.
 //
 //   scores  a CTA takes 256 positions of one K/V head and all of its query heads: per-head norm and RoPE of q (and, where the

@@ -1,4 +1,4 @@
-// Fused kernels of the single-token step (batch-1 decode), five per layer:
+// Fused kernels of the single-token step (batch-1 decode), five or (attention in two kernels) six per layer:
 //
 //   multiply   norm+quantise prologue -> q/k/v | o (+residual) | gate,up (+activation) | down (+residual) | head
 //   attention  norm, RoPE, cache store, scores, softmax and position-ordered weighted sum: attn_decode.cu (or, past the

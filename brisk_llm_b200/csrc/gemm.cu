@@ -25,8 +25,8 @@
 // fragments, small ones fill the GPU; the rule is at pick_tile). Weights, activations and their scales come through a ring
 // of cp.async stages of four blocks. Row pitches carry 16 bytes of padding: fragment reads are conflict-free. For a
 // gate/up pair half of a warp's rows are gate rows and half the up rows at the same place, and the activation is applied
-// in the epilogue. Measured: 4096 x 14336 Q4_0 at 512 tokens 282 -> 225 us (134 TMAC/s), 1024 x 3072 25 -> 19 us; at 9
-// tokens 43 -> 30 us (and 14336 x 4096 35 -> 23 us) against a kernel whose warps split a stage and add terms up through
+// in the epilogue. Measured: 4096 x 14336 Q4_0 at 512 tokens 282 -> 225 us (134 TMAC/s), 1024 x 3072 25 -> 21 us; at 9
+// tokens 43 -> 24 us (and 14336 x 4096 35 -> 17 us) against a kernel whose warps split a stage and add terms up through
 // shared memory.
 #include <algorithm>
 #include <cstdlib>
@@ -393,7 +393,8 @@ uint32_t sm_count() {
 
 bool gemm_tc_supports(int type, uint32_t cols);  // gemm_tc.cu: the same arithmetic on tcgen05 / tensor memory
 void launch_gemm_tc(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s);
-// BRISK_CUDA_GEMM=tc / mma picks the prompt GEMM of Q4_0 / Q8_0 matrices (read at every call); unset: kGemmTcDefault
+// BRISK_CUDA_GEMM=tc / mma picks the prompt GEMM of Q4_0 / Q8_0 matrices (read at every call); unset: kGemmTcDefault. Measured,
+// 512 tokens, us here / gemm_tc.cu: 1024 x 3072 Q4_0 21 / 37, 2048 x 8192 76 / 91, 4096 x 14336 228 / 296, Q8_0 240 / 317.
 constexpr bool kGemmTcDefault = false;
 static bool gemm_tc_on() {
     const char* env = std::getenv("BRISK_CUDA_GEMM");

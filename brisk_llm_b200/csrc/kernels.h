@@ -134,7 +134,7 @@ void launch_attention(const AttnArgs& a, cudaStream_t s);
 // values; same results as the kernels above.
 void launch_attn_chain(const AttnArgs& a, uint32_t sms, cudaStream_t s);
 constexpr uint32_t kChainMaxTokens = 24;      // more tokens than this share V rows through the tiled kernel instead
-// BRISK_CUDA_CHAIN: 0 never (nor the single-token kernel of attn_decode.cu), 1 wherever it fits, unset: 2..kChainMaxTokens tokens.
+// BRISK_CUDA_CHAIN: 0 never (nor the single-token kernel of attn_decode.cu), 1 wherever it fits, unset: up to kChainMaxTokens tokens.
 int chain_mode();
 
 // ---- fused single-token step (decode.cu) -------------------------------------------------------------------------

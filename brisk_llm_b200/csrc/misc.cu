@@ -1,5 +1,5 @@
-// Per-token vector kernels of the token loop: embedding lookup, per-head norm + RoPE + K/V cache write,
-// split-position attention with a combine pass, and the greedy arg-max that keeps decoding on the device.
+// Per-token vector kernels of the token loop: embedding lookup, per-head norm + RoPE + K/V cache write, and the greedy
+// arg-max that keeps decoding on the device; the choice among the batched attention kernels.
 #include <cstdio>
 #include <mutex>
 #include <string>

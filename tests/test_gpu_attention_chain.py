@@ -1,9 +1,10 @@
-"""The chained softmax + weighted-sum kernel (csrc/attn_chain.cu) against the kernels it stands in for.
+"""The chained weighted-sum kernels against the kernels they stand in for: csrc/attn_chain.cu for few tokens (a speculative
+verify step of 1 + 8 tokens, a short eval_all; a single token only where the batched kernels are made to take it) and
+csrc/attn_decode.cu for single tokens.
 
-It takes the attention of few tokens (a speculative verify step of 1 + 8 tokens, a short eval_all) and of single tokens at long
-contexts. The float operations and their order are the reference's (src/kernels_f32.cpp:265-284), as in the other attention
-kernels, so logits must be identical bits whichever kernel ran; the oracle is the arbiter for one of the families.
-BRISK_CUDA_CHAIN=0 keeps the older kernels, =1 takes the chained kernel wherever it fits.
+The float operations and their order are the reference's (src/kernels_f32.cpp:265-284), as in the other attention kernels, so
+logits must be identical bits whichever kernel ran; the oracle is the arbiter for one of the families. BRISK_CUDA_CHAIN=0
+keeps the older kernels, =1 takes the chained kernels wherever they fit.
 """
 import numpy as np
 import pytest

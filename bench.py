@@ -310,7 +310,7 @@ def tensor_parallel_section(engine, torch, dist, rank, local, world, max_over_ra
 
 
 def run_speculative(args):
-    """configs[4]'s second workload: 4 sequences of the Mistral-7B-shaped model, each an 8192-token prompt, then 512 tokens
+    """The speculative-verify workload: 4 sequences of the Mistral-7B-shaped model, each an 8192-token prompt, then 512 tokens
     settled by lookup-draft speculative decoding with D drafted tokens per verify step (Speculator + LookupDrafter,
     brisk-llm src/speculative.cpp:45-118: a verify step is eval_all(1 + drafts) and a rollback). The four sessions are
     stepped round-robin from one host thread, every call with host buffers (the logits of all 1 + D rows come back)."""

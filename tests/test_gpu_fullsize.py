@@ -91,14 +91,14 @@ def run_workload(spec, prompt_len, steps, scored, exact, share_layers=False):
 
 
 def test_qwen3_0_6b_q4_0_exactly_as_benchmarked():
-    """configs[0], the model and workload of the headline number: 512-token prompt + 128 greedy steps, context 2048."""
+    """The model and workload of the headline number: 512-token prompt + 128 greedy steps, context 2048."""
     from dataclasses import replace
     spec = replace(synth.PRESETS["qwen3-0.6b-q4_0"], context=2048)
     run_workload(spec, 512, 128, scored=130, exact=True)
 
 
 def test_llama_3_2_1b_q4_k_m_full_depth():
-    """configs[2] at full depth and vocabulary (16 layers, 128 256 ids, Q4_K with Q6_K V/down/embedding, llama3 rope
+    """The Llama-3.2-1B shape at full depth and vocabulary (16 layers, 128 256 ids, Q4_K with Q6_K V/down/embedding, llama3 rope
     frequency scaling; every layer reuses layer 0's seeded weights - quantising sixteen distinct layers in numpy takes two
     minutes); prompt shortened from 1024 to 160 tokens and the greedy run from 256 to 24 steps."""
     from dataclasses import replace
@@ -107,7 +107,7 @@ def test_llama_3_2_1b_q4_k_m_full_depth():
 
 
 def test_bitnet_2b_tq2_0_full_depth():
-    """configs[3] at full depth and vocabulary (30 layers, ternary TQ2_0 matrices, sub-norms, squared-ReLU gate, F16
+    """The BitNet-2B4T shape at full depth and vocabulary (30 layers, ternary TQ2_0 matrices, sub-norms, squared-ReLU gate, F16
     embedding/head; every layer reuses layer 0's seeded weights); prompt shortened from 512 to 96 tokens and the greedy run
     from 256 to 16 steps."""
     from dataclasses import replace
@@ -116,7 +116,7 @@ def test_bitnet_2b_tq2_0_full_depth():
 
 
 def test_mistral_7b_q4_0_full_depth_one_gpu():
-    """configs[4] on one GPU at full depth and vocabulary (32 layers of the real widths, untied Q4_0 head; every layer
+    """The Mistral-7B shape on one GPU at full depth and vocabulary (32 layers of the real widths, untied Q4_0 head; every layer
     reuses layer 0's seeded weights, as the benchmark draws them); prompt shortened from 8192 to 80 tokens and the
     greedy run from 512 to 8 steps."""
     from dataclasses import replace
@@ -132,7 +132,7 @@ SWEEP_SHAPES = ((1024, 3072), (2048, 8192), (4096, 14336), (14336, 4096))
 @pytest.mark.parametrize("rows,cols", SWEEP_SHAPES, ids=lambda v: str(v))
 @pytest.mark.parametrize("fmt", SWEEP_FORMATS, ids=lambda f: F.NAMES[f])
 def test_kernel_sweep_grid_bit_for_bit(fmt, rows, cols):
-    """every format at every shape, activations ~N(0,1) at 1, 4 and 512 tokens, against the oracle's
+    """The kernel sweep: every format at every shape, activations ~N(0,1) at 1, 4 and 512 tokens, against the oracle's
     restatement of the reference's matvec/matmul (src/kernels.cpp:13-30, :129-163) - bit for bit. 512 tokens of the
     two largest shapes is about a second of CPU each."""
     os.environ.setdefault("BRISK_ORACLE_THREADS", str(os.cpu_count() or 1))

@@ -401,7 +401,7 @@ static bool gemm_tc_on() {
     return env == nullptr ? kGemmTcDefault : std::strcmp(env, "tc") == 0;
 }
 bool gemm_k_supports(int type);  // gemm_k.cu: the 256-value super-block formats
-void launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t sms, cudaStream_t s);
+bool launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t sms, cudaStream_t s);
 
 // From 2 tokens on: Q4_0 / Q8_0 rows of a multiple of 4 blocks (128 values), and the super-block formats.
 static bool gemm_supports(int type, uint32_t cols, uint32_t n) {
@@ -415,9 +415,7 @@ int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t
     }
     const int type = targets[0].m.type;
     if (type != T_Q4_0 && type != T_Q8_0) {
-        if (pair) return 0;
-        launch_gemm_k(targets, count, act, n, epi, sm_count(), s);
-        return 1;
+        return launch_gemm_k(targets, count, act, n, epi, sm_count(), s) ? 1 : 0;
     }
     if (!pair && n >= 32 && gemm_tc_on() && gemm_tc_supports(type, targets[0].m.cols)) {
         for (int i = 0; i < count; ++i) launch_gemm_tc(targets[i], act, n, epi, s);

@@ -1,4 +1,5 @@
-// Prompt multiply on int8 tensor cores for the 256-value super-block formats (Q4_K, Q5_K, Q6_K, TQ2_0) against Q8_K
+// Multiply of a few to some hundred tokens (and, with few rows, more; gemm_k_tc.cu takes the rest) on int8 tensor cores for the
+// 256-value super-block formats (Q4_K, Q5_K, Q6_K, TQ2_0) against Q8_K
 // activations, with the reference's integer arithmetic and float order (src/quant.cpp:500-596):
 //
 //   TQ2_0  acc   = sum over the super-block of q*x            (8 MMAs of k = 32 chained in int32)
@@ -497,14 +498,19 @@ KTile tile_of(uint64_t alone, uint64_t shared) {
 }
 
 // The tile whose busiest SM is done first, as in gemm.cu; 800 ns for what a CTA does besides its super-blocks. The other types'
-// figures are the same within their common factor. Measured, Q4_K: 2048 x 8192 at 9 tokens 65 (128 x 64 tiles) / 25 (64 x 16)
-// / 7.9 us (16 x 16, split), 14336 x 4096 at 9 tokens 80 / 20 / 24, 2048 x 2048 at 512 tokens 18.8 / 30 / -.
+// figures are the same within their common factor. Measured, Q4_K: 2048 x 8192 at 9 tokens 25 (64 x 16 tiles) / 7.9 us (16 x 16,
+// split), 14336 x 4096 at 9 tokens 20 / 24.
+//
+// False: the tensor-memory kernel (gemm_k_tc.cu) is estimated to be done sooner (than other_ns), and nothing was launched. It takes tiles of 128
+// rows and needs about 3.5 us around its super-blocks, so few rows or tokens stay here (2048 x 2048 Q4_K at 128 tokens 9.6 us
+// here, 12.2 there; 14336 x 4096 at 64 tokens 34 and 21).
 template <int TYPE>
-void launch_type(KParams& p, uint32_t sms, cudaStream_t s) {
+bool launch_type(KParams& p, uint64_t other_ns, bool ask_only, uint32_t sms, cudaStream_t s) {
     static const KTile tiles[] = {
-        tile_of<TYPE, 2, 4, 4, 2, 1, 2, 1>(2000, 2000), tile_of<TYPE, 1, 4, 4, 2, 1, 2, 2>(1250, 1060), tile_of<TYPE, 1, 2, 4, 1, 1, 4, 4>(770, 540),
+        tile_of<TYPE, 1, 4, 4, 2, 1, 2, 2>(1250, 1060), tile_of<TYPE, 1, 2, 4, 1, 1, 4, 4>(770, 540),
         tile_of<TYPE, 1, 2, 1, 1, 8, 2, 1>(210, 230), tile_of<TYPE, 1, 1, 1, 1, 4, 3, 3>(200, 137),
     };
+    constexpr uint64_t kPercent = TYPE == T_Q4_K ? 100 : TYPE == T_Q5_K ? 120 : TYPE == T_Q6_K ? 170 : 75;  // of Q4_K's figures
     static DeviceOnce once;
     if (once.first()) {
         for (const KTile& tile : tiles) BK_CUDA(cudaFuncSetAttribute(tile.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile.smem)));
@@ -523,19 +529,35 @@ void launch_type(KParams& p, uint32_t sms, cudaStream_t s) {
             best = cost;
         }
     }
+    if (other_ns < best * kPercent / 100) return false;
+    if (ask_only) return true;
     uint32_t row_tiles = 0;
     for (int i = 0; i < p.count; ++i) {
         p.first_tile[i] = row_tiles;
         row_tiles += (p.m[i].rows + pick->rows - 1) / pick->rows;
     }
     launch_dependent(pick->kernel, dim3(row_tiles, (p.n + pick->tokens - 1) / pick->tokens), dim3(pick->threads), pick->smem, s, p);
+    return true;
 }
 
 }  // namespace
 
+// gemm_k_tc.cu: the multiply in tensor memory, and what it is expected to take
+void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t sms, cudaStream_t s);
+uint64_t gemm_k_tc_ns(const MatTarget* targets, int count, uint32_t n, bool pair, uint32_t sms);
+
 bool gemm_k_supports(int type) { return type == T_Q4_K || type == T_Q5_K || type == T_Q6_K || type == T_TQ2_0; }
 
-void launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t sms, cudaStream_t s) {
+// False, nothing launched: a gate/up pair that the caller multiplies separately.
+bool launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t sms, cudaStream_t s) {
+    const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
+    uint64_t other_ns = gemm_k_tc_ns(targets, count, n, pair, sms);
+    if (pair) {
+        // Here the activation is a launch of its own (a 3 us launch, 22 us for 512 x 8192 values): the tensor-memory kernel applies it
+        // as it stores. The two matrices are asked about as the caller would send them.
+        const uint64_t activation_ns = 3000 + uint64_t(n) * targets[0].m.rows / 220;
+        other_ns = other_ns > activation_ns ? other_ns - activation_ns : 0;
+    }
     KParams p{};
     for (int i = 0; i < count; ++i) {
         p.m[i] = targets[i].m;
@@ -546,13 +568,17 @@ void launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint3
     p.n = n;
     p.count = count;
     p.epi = int(epi);
+    bool here = false;
     switch (targets[0].m.type) {
-        case T_Q4_K: launch_type<T_Q4_K>(p, sms, s); break;
-        case T_Q5_K: launch_type<T_Q5_K>(p, sms, s); break;
-        case T_Q6_K: launch_type<T_Q6_K>(p, sms, s); break;
-        case T_TQ2_0: launch_type<T_TQ2_0>(p, sms, s); break;
+        case T_Q4_K: here = launch_type<T_Q4_K>(p, other_ns, pair, sms, s); break;
+        case T_Q5_K: here = launch_type<T_Q5_K>(p, other_ns, pair, sms, s); break;
+        case T_Q6_K: here = launch_type<T_Q6_K>(p, other_ns, pair, sms, s); break;
+        case T_TQ2_0: here = launch_type<T_TQ2_0>(p, other_ns, pair, sms, s); break;
         default: throw CudaError("cuda: no super-block tensor kernel for this type");
     }
+    if (here) return !pair;
+    launch_gemm_k_tc(targets, count, act, n, epi, sms, s);
+    return true;
 }
 
 }  // namespace bk

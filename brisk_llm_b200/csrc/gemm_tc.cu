@@ -25,6 +25,7 @@
 // registers a thread (380 us against 296).
 #include "kernels.h"
 #include "packed.cuh"
+#include "tc.cuh"
 
 namespace bk {
 namespace {
@@ -37,8 +38,6 @@ constexpr int kThreads = kLoaders + kEpilogue + 32;   // loaders (warps 0-3) | e
 constexpr int kMmaWarp = (kLoaders + kEpilogue) / 32;
 constexpr uint32_t kATile = kTM * 32, kBTile = kTN * 32;                                     // one block's operand tiles, bytes
 constexpr uint32_t kStageBytes = kCB * (kATile + kBTile) + kTM * kCB * 2 + kTN * kCB * 4;   // + f16 weight scales + f32 token scales
-constexpr long long kWaitCycles = 2000000000ll;  // about a second: a wait that lasts this long has failed
-constexpr uint32_t kTmemCols = 512;
 
 __device__ unsigned int g_gemm_tc_error;
 
@@ -59,35 +58,6 @@ struct TcParams {
     int epi;
 };
 
-__device__ __forceinline__ uint32_t saddr(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
-__device__ __forceinline__ void mbar_init(uint64_t* b, uint32_t count) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(saddr(b)), "r"(count) : "memory");
-}
-__device__ __forceinline__ void mbar_arrive(uint64_t* b) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(saddr(b)) : "memory"); }
-__device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
-    uint32_t ok;
-    asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(saddr(b)), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Bounded: should a wait run out, the error word is set, `dead` makes this thread's later waits return at once, and the
-// kernel ends (with garbage) and still frees its tensor memory.
-__device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity, bool& dead) {
-    if (dead || mbar_try_wait(b, parity)) return;
-    const long long start = clock64();
-    while (!mbar_try_wait(b, parity)) {
-        if (clock64() - start > kWaitCycles) {  // bounded in time, not in tries: one try may itself sleep for a while
-            atomicOr(&g_gemm_tc_error, 1u);
-            dead = true;
-            return;
-        }
-    }
-}
-
-// K-major operand tile without swizzle: core matrices of 8 rows x 16 bytes; `lbo` bytes between the two 16-byte halves of
-// K, `sbo` bytes between groups of 8 rows. Bit 46: the descriptor version of this architecture.
-__device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo, uint32_t sbo) {
-    return uint64_t((addr >> 4) & 0x3FFF) | (uint64_t((lbo >> 4) & 0x3FFF) << 16) | (uint64_t((sbo >> 4) & 0x3FFF) << 32) | (1ull << 46);
-}
 // s32 accumulator, s8 x s8, both operands K-major, N = 64, M = 128
 constexpr uint32_t kInstrDesc = (2u << 4) | (1u << 7) | (1u << 10) | (uint32_t(kTN >> 3) << 17) | (uint32_t(kTM >> 4) << 24);
 
@@ -108,10 +78,6 @@ __device__ __forceinline__ void tmem_preset(uint32_t taddr) {
         ::"r"(taddr), "r"(kMagicBits)
         : "memory");
 }
-__device__ __forceinline__ void mma_commit(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(saddr(bar)) : "memory");
-}
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_ld_nowait(uint32_t taddr, uint32_t (&v)[kEC]) {
     static_assert(kEC == 32, "the load below (and the preset above) is the x32 form");
     asm volatile(
@@ -185,7 +151,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
         auto fill = [&](const Regs& g, uint32_t c) {
             const uint32_t s = c % kStages, round = c / kStages;
             const long long t_w = TC_CLOCK();
-            if (round > 0) mbar_wait(&stage_free[s], (round - 1) & 1, dead);
+            if (round > 0) mbar_wait(&stage_free[s], (round - 1) & 1, dead, &g_gemm_tc_error);
             if (warp == 0) TC_ADD(0, t_w);
             const long long t_f = TC_CLOCK();
             unsigned char* st = smem + size_t(s) * kStageBytes;
@@ -249,10 +215,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
             for (uint32_t c = 0; c < chunks; ++c) {
                 const uint32_t s = c % kStages, set = c & 1;
                 const long long t_a = TC_CLOCK();
-                mbar_wait(&full[s], (c / kStages) & 1, dead);
+                mbar_wait(&full[s], (c / kStages) & 1, dead, &g_gemm_tc_error);
                 TC_ADD(2, t_a);
                 const long long t_b = TC_CLOCK();
-                mbar_wait(&set_free[set], (c >> 1) & 1, dead);  // use u of a set waits for its u-th release; the 0th is the epilogue's preset
+                mbar_wait(&set_free[set], (c >> 1) & 1, dead, &g_gemm_tc_error);  // use u of a set waits for its u-th release; the 0th is the epilogue's preset
                 TC_ADD(3, t_b);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a0 = saddr(smem + size_t(s) * kStageBytes), b0 = a0 + kCB * kATile;
@@ -284,7 +250,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
         for (uint32_t c = 0; c < chunks; ++c) {
             const uint32_t s = c % kStages, set = c & 1;
             const long long t_e = TC_CLOCK();
-            mbar_wait(&set_full[set], (c >> 1) & 1, dead);
+            mbar_wait(&set_full[set], (c >> 1) & 1, dead, &g_gemm_tc_error);
             if (ew == 0) TC_ADD(4, t_e);
             const long long t_g = TC_CLOCK();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");

@@ -67,8 +67,8 @@ void launch_tp_peer_exchange(uint2* const* bufs_dev, uint32_t* epoch, unsigned i
 
 // ---- batched multiply on the int8 tensor path (gemm.cu) ----------------------------------------
 // Same contract as launch_matvec; returns the number of kernels launched, 0 when these types, shapes or token counts have
-// no tensor kernel (the caller then uses launch_matvec). The super-block formats have none for the pair epilogues: the
-// caller multiplies gate and up separately and runs launch_gate_mul.
+// no tensor kernel (the caller then uses launch_matvec). The super-block formats have one for the pair epilogues where there are
+// rows and tokens enough (gemm_k_tc.cu); elsewhere the caller multiplies gate and up separately and runs launch_gate_mul.
 int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s);
 // The Q4_0 / Q8_0 prompt multiply on tcgen05 / tensor memory (gemm_tc.cu; BRISK_CUDA_GEMM=tc): its waits are bounded, and this
 // word is non-zero on the device after a launch whose wait ran out.

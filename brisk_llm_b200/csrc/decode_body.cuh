@@ -623,6 +623,48 @@ __device__ __forceinline__ void warp_head_load(const float* src, const float* bi
     }
 }
 
+// This lane's norm weights and (cos, sin) values of a head: constants, to be asked for ahead of the values they meet. Behind them,
+// one after the other, the three loads are three trips to L2.
+template <int VPL>
+struct HeadConstants {
+    float norm[VPL], turn[VPL];
+};
+template <int VPL>
+__device__ __forceinline__ void warp_head_constants(const float* norm, const float* rope, int neox, HeadConstants<VPL>& c) {
+    const uint32_t lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 0; k < VPL; ++k) c.norm[k] = norm != nullptr ? norm[neox ? lane + 32 * k : VPL * lane + k] : 1.0f;
+#pragma unroll
+    for (int k = 0; k < VPL / 2; ++k) {
+        const uint32_t pair = neox ? lane + 32 * k : VPL / 2 * lane + k;
+        c.turn[2 * k] = rope[2 * pair];
+        c.turn[2 * k + 1] = rope[2 * pair + 1];
+    }
+}
+
+template <int VPL, bool NEOX>
+__device__ __forceinline__ void warp_head_finish(float (&v)[VPL], bool normed, const HeadConstants<VPL>& c, float eps, float* dst) {
+    const uint32_t lane = threadIdx.x & 31;
+    if (normed) {
+        double part = 0.0;
+#pragma unroll
+        for (int k = 0; k < VPL; ++k) part += double(__fmul_rn(v[k], v[k]));
+        part = warp_sum(part);
+        const float mean = float(part * (1.0 / (VPL * 32)));  // a power of two: the division's result
+        const float scale = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(mean, eps)));
+#pragma unroll
+        for (int k = 0; k < VPL; ++k) v[k] = __fmul_rn(__fmul_rn(v[k], scale), c.norm[k]);
+    }
+#pragma unroll
+    for (int k = 0; k < VPL / 2; ++k) {
+        // pair (a, b): NeoX -> registers k and k + VPL/2 (elements i, i + dim/2); adjacent -> registers 2k, 2k+1 (elements 2i, 2i+1)
+        const int ra = NEOX ? k : 2 * k, rb = NEOX ? k + VPL / 2 : 2 * k + 1;
+        const uint32_t ia = NEOX ? lane + 32 * ra : VPL * lane + ra, ib = NEOX ? lane + 32 * rb : VPL * lane + rb;
+        const float x0 = v[ra], x1 = v[rb];
+        dst[ia] = __fsub_rn(__fmul_rn(x0, c.turn[2 * k]), __fmul_rn(x1, c.turn[2 * k + 1]));
+        dst[ib] = __fadd_rn(__fmul_rn(x0, c.turn[2 * k + 1]), __fmul_rn(x1, c.turn[2 * k]));
+    }
+}
 template <int VPL, bool NEOX>
 __device__ __forceinline__ void warp_head_norm_rope(float (&v)[VPL], const float* norm, const float* rope, float eps, float* dst) {
     constexpr uint32_t dim = VPL * 32;
@@ -655,6 +697,18 @@ __device__ __forceinline__ void warp_norm_rope_head_impl(const float* src, const
     float v[VPL];
     warp_head_load<VPL, NEOX>(src, bias, v);
     warp_head_norm_rope<VPL, NEOX>(v, norm, rope, eps, dst);
+}
+
+template <int VPL>
+__device__ __forceinline__ void warp_norm_rope_head(const float* src, const float* bias, bool normed, const HeadConstants<VPL>& c, float eps, int neox, float* dst) {
+    float v[VPL];
+    if (neox) {
+        warp_head_load<VPL, true>(src, bias, v);
+        warp_head_finish<VPL, true>(v, normed, c, eps, dst);
+    } else {
+        warp_head_load<VPL, false>(src, bias, v);
+        warp_head_finish<VPL, false>(v, normed, c, eps, dst);
+    }
 }
 
 template <int VPL>

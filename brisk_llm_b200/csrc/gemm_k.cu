@@ -487,18 +487,20 @@ __global__ void __launch_bounds__(WR * WT * KS * 32, RESIDENT) gemm_k_kernel(con
 
 struct KTile {
     uint32_t rows, tokens, split, threads, resident, smem;
-    uint64_t alone, shared;  // ns of a super-block (Q4_K): of one CTA by itself, and per CTA of a full SM
+    uint64_t alone, shared;  // ns of a super-block of Q4_K: of one CTA by itself, and per CTA of a full SM
+    uint64_t percent;        // of them that this type takes
     void (*kernel)(KParams);
 };
 
 template <int TYPE, int MI, int NI, int WR, int WT, int KS, int STAGES, int RESIDENT>
-KTile tile_of(uint64_t alone, uint64_t shared) {
+KTile tile_of(uint64_t alone, uint64_t shared, uint64_t q5_k, uint64_t q6_k, uint64_t tq2_0) {
     const uint32_t stages = KS * STAGES * KStage<TYPE, 16 * MI * WR, 8 * NI * WT>::kBytes, terms = KS > 1 ? 2 * KS * MI * NI * 128 * 4 : 0;
-    return KTile{16 * MI * WR, 8 * NI * WT, KS, WR * WT * KS * 32, RESIDENT, stages + terms, alone, shared, gemm_k_kernel<TYPE, MI, NI, WR, WT, KS, STAGES, RESIDENT>};
+    const uint64_t percent = TYPE == T_Q4_K ? 100 : TYPE == T_Q5_K ? q5_k : TYPE == T_Q6_K ? q6_k : tq2_0;
+    return KTile{16 * MI * WR, 8 * NI * WT, KS, WR * WT * KS * 32, RESIDENT, stages + terms, alone, shared, percent,
+                 gemm_k_kernel<TYPE, MI, NI, WR, WT, KS, STAGES, RESIDENT>};
 }
 
-// The tile whose busiest SM is done first, as in gemm.cu; 800 ns for what a CTA does besides its super-blocks. The other types'
-// figures are the same within their common factor. Measured, Q4_K: 2048 x 8192 at 9 tokens 25 (64 x 16 tiles) / 7.9 us (16 x 16,
+// The tile whose busiest SM is done first, as in gemm.cu; 800 ns for what a CTA does besides its super-blocks. Measured, Q4_K: 2048 x 8192 at 9 tokens 25 (64 x 16 tiles) / 7.9 us (16 x 16,
 // split), 14336 x 4096 at 9 tokens 20 / 24.
 //
 // False: the tensor-memory kernel (gemm_k_tc.cu) is estimated to be done sooner (than other_ns), and nothing was launched. It takes tiles of 128
@@ -507,10 +509,9 @@ KTile tile_of(uint64_t alone, uint64_t shared) {
 template <int TYPE>
 bool launch_type(KParams& p, uint64_t other_ns, bool ask_only, uint32_t sms, cudaStream_t s) {
     static const KTile tiles[] = {
-        tile_of<TYPE, 1, 4, 4, 2, 1, 2, 2>(1250, 1060), tile_of<TYPE, 1, 2, 4, 1, 1, 4, 4>(770, 540),
-        tile_of<TYPE, 1, 2, 1, 1, 8, 2, 1>(210, 230), tile_of<TYPE, 1, 1, 1, 1, 4, 3, 3>(200, 137),
+        tile_of<TYPE, 1, 4, 4, 2, 1, 2, 2>(1250, 1060, 122, 172, 74), tile_of<TYPE, 1, 2, 4, 1, 1, 4, 4>(770, 540, 125, 143, 65),
+        tile_of<TYPE, 1, 2, 1, 1, 8, 2, 1>(210, 230, 118, 137, 85), tile_of<TYPE, 1, 1, 1, 1, 4, 3, 3>(200, 137, 110, 135, 85),
     };
-    constexpr uint64_t kPercent = TYPE == T_Q4_K ? 100 : TYPE == T_Q5_K ? 120 : TYPE == T_Q6_K ? 170 : 75;  // of Q4_K's figures
     static DeviceOnce once;
     if (once.first()) {
         for (const KTile& tile : tiles) BK_CUDA(cudaFuncSetAttribute(tile.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile.smem)));
@@ -529,7 +530,7 @@ bool launch_type(KParams& p, uint64_t other_ns, bool ask_only, uint32_t sms, cud
             best = cost;
         }
     }
-    if (other_ns < best * kPercent / 100) return false;
+    if (other_ns < best * pick->percent / 100) return false;
     if (ask_only) return true;
     uint32_t row_tiles = 0;
     for (int i = 0; i < p.count; ++i) {

@@ -483,29 +483,34 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
             const uint32_t row_tile = tile / p.tok_tiles, tok_base = tile % p.tok_tiles * (kTokens * NT);
             const int target = target_of(row_tile);
             if (tile + gridDim.x >= p.tiles) release_next();
-            const uint32_t row_base = (row_tile - p.first_tile[target]) * (PAIR ? kRows / 2 : kRows) + quarter * 32 + g;
-            if constexpr (PAIR) {  // the up rows' sums to the warps that hold the gate rows
+            // (a pair: lanes 0 - 15 of a quarter's gate rows are finished there, 16 - 31 on the up side)
+            const uint32_t row_base = (row_tile - p.first_tile[target]) * (PAIR ? kRows / 2 : kRows) + (PAIR ? (quarter & 1) * 32 + (quarter >> 1) * 16 : quarter * 32) + g;
+            if constexpr (PAIR) {
+                // Gate rows are with quarters 0 and 1, the same up rows with 2 and 3. Each side sends the other half of its sums and
+                // applies the activation to the rest: sums 0 .. 7 of a token half stay on the gate side, 8 .. 15 go to the up side.
                 f32x2* exchange = reinterpret_cast<f32x2*>(minimums + 4 * S::kMn) + part * 64 + (quarter & 1) * 32 + lane;
+                const bool up_side = quarter >= 2;
 #pragma unroll
                 for (int nt = 0; nt < NT; ++nt) {
-                    if (quarter >= 2) {
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) exchange[k * 128] = acc[nt][k >> 3][(k >> 1) & 3][k & 1];
+                    for (int k = 0; k < 8; ++k) {
+                        const f32x2 low = acc[nt][0][(k >> 1) & 3][k & 1], high = acc[nt][1][(k >> 1) & 3][k & 1];
+                        exchange[(up_side ? k : 8 + k) * 128] = up_side ? low : high;
                     }
                     asm volatile("bar.sync 2, 256;" ::: "memory");
-                    if (quarter < 2) {
 #pragma unroll
-                        for (int k = 0; k < 16; ++k) {
-                            f32x2& gate = acc[nt][k >> 3][(k >> 1) & 3][k & 1];
-                            float g0, g1, u0, u1;
-                            unpack2(gate, g0, g1);
-                            unpack2(exchange[k * 128], u0, u1);
-                            gate = p.epi == EPI_SILU_MUL ? pack2(silu_mul(g0, u0), silu_mul(g1, u1)) : pack2(relu2_mul(g0, u0), relu2_mul(g1, u1));
+                    for (int k = 0; k < 8; ++k) {
+                        const f32x2 mine2 = up_side ? acc[nt][1][(k >> 1) & 3][k & 1] : acc[nt][0][(k >> 1) & 3][k & 1], other2 = exchange[(up_side ? 8 + k : k) * 128];
+                        float g0, g1, u0, u1;
+                        unpack2(up_side ? other2 : mine2, g0, g1);
+                        unpack2(up_side ? mine2 : other2, u0, u1);
+                        if (tok_base + nt * 64 + part * 32 + (k >> 1) * 8 < p.n) {  // of these eight tokens, some exist
+                            acc[nt][0][(k >> 1) & 3][k & 1] =
+                                p.epi == EPI_SILU_MUL ? pack2(silu_mul(g0, u0), silu_mul(g1, u1)) : pack2(relu2_mul(g0, u0), relu2_mul(g1, u1));
                         }
                     }
                     asm volatile("bar.sync 2, 256;" ::: "memory");  // the exchange may be overwritten
                 }
-                if (quarter >= 2) continue;
             }
             float* const out = p.out[target];
             const uint32_t rows = p.m[target].rows, ldo = p.ldo[target];
@@ -519,7 +524,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
                         if (tok >= p.n) continue;
                         float* o = out + size_t(tok) * ldo;
 #pragma unroll
-                        for (int h = 0; h < 2; ++h)
+                        for (int h = 0; h < (PAIR ? 1 : 2); ++h)
 #pragma unroll
                             for (int r = 0; r < 2; ++r) {
                                 const uint32_t row = row_base + h * 16 + r * 8;
@@ -593,7 +598,8 @@ CUtensorMap tensor_map(const void* base, uint64_t row_bytes, uint64_t rows, uint
 }
 
 // ns that `count` targets (a pair: gate and up) take with tiles of 64 `halves` tokens: the busiest SM's tiles one after the other.
-// Measured: ns of a super-block in either tile, and 3.5 us before the first and after the last.
+// Measured: ns of a super-block in either tile, 1.2 us of activation for every 64 tokens of a pair's tile, and 5 us before the first
+// and after the last (3.5 where the same multiply is repeated; among other kernels its start overlaps less of theirs).
 static uint64_t tile_ns(const MatTarget* targets, int count, uint32_t n, bool pair, int halves, uint32_t sms) {
     const int type = targets[0].m.type;
     const uint64_t one = type == T_Q4_K ? 1020 : type == T_Q5_K ? 1070 : type == T_Q6_K ? 1130 : 610;
@@ -601,7 +607,7 @@ static uint64_t tile_ns(const MatTarget* targets, int count, uint32_t n, bool pa
     uint64_t tiles = 0;
     for (int i = 0; i < (pair ? 1 : count); ++i) tiles += (targets[i].m.rows + (pair ? kRows / 2 : kRows) - 1) / (pair ? kRows / 2 : kRows);
     tiles *= (n + kTokens * halves - 1) / (kTokens * halves);
-    return (tiles + sms - 1) / sms * targets[0].m.blocks * (halves == 2 ? two : one) + 3500;
+    return (tiles + sms - 1) / sms * (targets[0].m.blocks * (halves == 2 ? two : one) + (pair ? 1200 * halves : 0)) + 5000;
 }
 
 uint64_t gemm_k_tc_ns(const MatTarget* targets, int count, uint32_t n, bool pair, uint32_t sms) {

@@ -1064,16 +1064,17 @@ struct Session {
     bool takes_fused_attention(uint64_t visible) const {
         return visible <= 512 && head_dim <= 128 && rope_dim == head_dim && chain_mode() != 0 && attn_decode_fits(head_dim, uint32_t(max_context));
     }
-    // With the fused attention one kernel per operation also beats the persistent kernel, until the positions eat the gain up.
-    // Persistent / per operation, us a token at 64, 256 and 440 positions: 4 layers of the 0.6B shape (35 MB) 99/97, 104/105,
-    // 109/114; 11 layers (97 MB) 261/244, 274/265, 280/288; 12 (106 MB) 283/264, 298/287, 304/311; 28 (248 MB) 643/598, 672/652,
-    // 697/715. The ratio is the same from 8 layers on (1.06-1.08, 1.03-1.04, 0.97): nothing in it marks this line, it is not the
-    // L2's. It keeps models of few layers, where the whole difference is 17 us at most, on one path at every position.
-    static constexpr uint64_t kFewLayers = uint64_t(100) << 20;
+    // One kernel per operation also beats the persistent kernel, at every depth and position. Persistent / per operation, us a token
+    // at 181, 440, 530, 1024 and 2000 positions: 4 layers of the 0.6B shape (35 MB) 125/111, 129/125, 134/130, 145/138, 170/150;
+    // 12 layers (106 MB) 315/270, 323/311, 336/325, 378/352, 462/390; 28 (248 MB) 683/589, 727/690, 757/724, 853/788, 1019/869. What
+    // the persistent kernel keeps are small models at short contexts, where that is 7 to 45 us a token: those of up to kFewLayers at
+    // up to 1024 positions, and from 513 on those of up to kSomeLayers.
+    static constexpr uint64_t kFewLayers = uint64_t(100) << 20, kSomeLayers = uint64_t(160) << 20;
+    bool takes_persistent(uint64_t visible) const { return visible <= 1024 && layer_bytes <= (visible <= 512 ? kFewLayers : kSomeLayers); }
 
     void step_on_device(uint64_t visible) {  // one token whose id is *d_tokens() at *d_position() = visible - 1
         fused_attention = takes_fused_attention(visible);
-        const bool persistent = step_active() && (token_enabled || step_forced || !fused_attention || layer_bytes <= kFewLayers);
+        const bool persistent = step_active() && (token_enabled || step_forced || takes_persistent(visible));
         if (!single_kernels()) batched = true;
         // The fused weighted sum keeps a head's probabilities of the whole context in shared memory; past that the batched
         // kernels, which have no such limit, take single tokens too.

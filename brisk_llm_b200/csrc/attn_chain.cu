@@ -18,6 +18,7 @@
 // scheduler waits out every load.
 #include "kernels.h"
 #include "pdl.cuh"
+#include "rowops.cuh"
 
 namespace bk {
 namespace {
@@ -28,6 +29,7 @@ struct ChainParams {
     const float* probs;    // [n][heads][max_context]
     const __half* v_cache; // [kv][max_context][dim]
     float* out;            // [n][heads * dim]
+    DevActMut quant;       // where q0 is set: the same as Q8_0 planes
     const uint32_t* position;
     uint32_t n, heads, kv_heads, dim, max_context, window;
 };
@@ -43,7 +45,9 @@ __global__ void __launch_bounds__(ROWS * 32) attn_chain_kernel(const ChainParams
     const uint32_t r0 = blockIdx.z * ROWS, last = min(r0 + ROWS, rows) - 1, row = min(r0 + warp, last);  // a warp past the last row repeats it
     const uint32_t token = row / group, h = kvh * group + row % group;
     wait_for_previous();
-    release_next();
+    // Where the rows end in planes, the multiply that takes them starts when the chains are done; released here, its CTAs would sit
+    // beside these for the whole walk.
+    if (a.quant.q0 == nullptr) release_next();
     const uint32_t position = *a.position;
     // a sliding-window layer attends to the last `window` positions only (src/model.cpp:1084-1091)
     auto start_of = [&](uint32_t visible) { return a.window != 0 && visible > a.window ? visible - a.window : 0u; };
@@ -128,10 +132,33 @@ __global__ void __launch_bounds__(ROWS * 32) attn_chain_kernel(const ChainParams
             }
             i += batches * kBatch;
         }
-        for (; i < hi; ++i) add(p[i], v[i * 32]);
+        if (i < hi) {  // fewer than a batch: the rest of it adds -0.0, which changes nothing
+            load(i, v0, p0);
+            const uint32_t left = hi - i;
+            const float pv[kBatch] = {p0[0].x, p0[0].y, p0[0].z, p0[0].w, p0[1].x, p0[1].y, p0[1].z, p0[1].w, p0[2].x, p0[2].y, p0[2].z, p0[2].w, p0[3].x, p0[3].y, p0[3].z, p0[3].w};
+#pragma unroll
+            for (uint32_t u = 0; u < kBatch; ++u) {
+                const float product = __fmul_rn(pv[u], __half2float(v0[u]));
+                acc = __fadd_rn(acc, u < left ? product : -0.0f);
+            }
+        }
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (r0 + warp <= last) a.out[(size_t(token) * a.heads + h) * a.dim + col0 + lane] = acc;
+    if (a.quant.q0 != nullptr) release_next();
+    const size_t at = (size_t(token) * a.heads + h) * a.dim + col0;
+    if (r0 + warp <= last) a.out[at + lane] = acc;
+    if (a.quant.q0 != nullptr) {  // the warp's 32 values are a block of the next multiply's input
+        int sum;
+        float d;
+        const int q = warp_quantize_q8_0(acc, d, sum);
+        if (r0 + warp <= last) {
+            a.quant.q0[at + lane] = int8_t(q);
+            if (lane == 0) {
+                a.quant.d0[at / 32] = d;
+                a.quant.s0[at / 32] = sum;
+            }
+        }
+    }
 }
 
 template <int ROWS>
@@ -144,7 +171,7 @@ void launch_rows(const ChainParams& p, uint32_t groups, cudaStream_t s) {
 // a.scores holds the probabilities of the n tokens (rows of max_context floats); a.out receives the attended rows.
 void launch_attn_chain(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
     ChainParams p{};
-    p.probs = a.scores; p.v_cache = a.v_cache; p.out = a.out; p.position = a.position;
+    p.probs = a.scores; p.v_cache = a.v_cache; p.out = a.out; p.quant = a.quant; p.position = a.position;
     p.n = a.n; p.heads = a.heads; p.kv_heads = a.kv_heads; p.dim = a.dim; p.max_context = a.max_context; p.window = a.window;
     const uint32_t rows = a.n * (a.heads / a.kv_heads);
     // The rows a CTA takes: whichever leaves the busiest SM with fewer warps, the more of them on a tie (less V traffic).

@@ -312,6 +312,11 @@ void launch_attn_scores(const AttnArgs& a, uint32_t sms, cudaStream_t s);
 void launch_attn_softmax(const AttnArgs& a, uint32_t sms, cudaStream_t s);
 void launch_attn_weighted(const AttnArgs& a, uint32_t sms, cudaStream_t s);
 
+bool attention_takes_chain(uint32_t n) {
+    const int mode = chain_mode();
+    return mode != 0 && (n <= kChainMaxTokens || mode == 1);
+}
+
 void launch_attention(const AttnArgs& a, cudaStream_t s) {
     if ((a.dim != 64 && a.dim != 128 && a.dim != 256) || a.heads / a.kv_heads > 8) throw CudaError("cuda: attention takes head sizes 64, 128 and 256 and at most 8 query heads per K/V head");
     static const uint32_t sms = [] {
@@ -321,8 +326,7 @@ void launch_attention(const AttnArgs& a, cudaStream_t s) {
     }();
     launch_attn_scores(a, sms, s);
     launch_attn_softmax(a, sms, s);
-    const int mode = chain_mode();
-    if (mode != 0 && (a.n <= kChainMaxTokens || mode == 1)) launch_attn_chain(a, sms, s);
+    if (attention_takes_chain(a.n)) launch_attn_chain(a, sms, s);
     else launch_attn_weighted(a, sms, s);
 }
 

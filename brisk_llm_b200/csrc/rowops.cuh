@@ -94,6 +94,22 @@ __device__ __forceinline__ uint2 quad_quantize_q8_0(const float (&v)[8], float& 
     return make_uint2(packed[0], packed[1]);
 }
 
+// One Q8_0 block by one warp, a value a lane: the lane's quantised value; the block's scale (rounded to f16) and sum in every lane.
+__device__ __forceinline__ int warp_quantize_q8_0(float v, float& d, int& sum) {
+    float amax = fabsf(v);
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    amax = fmaxf(0.0f, amax);
+    const float dd = __fdiv_rn(amax, 127.0f);
+    const float inv = dd != 0.0f ? __fdiv_rn(1.0f, dd) : 0.0f;
+    const int q = __float2int_rn(__fmul_rn(v, inv));
+    sum = q;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    d = __half2float(__float2half_rn(dd));
+    return q;
+}
+
 // One Q8_K super-block by one warp: lane l holds values 8l .. 8l + 7. `qk` and `bs` are this lane's own places (its values, the
 // sums of 16 its pair of lanes forms), `dk` the super-block's.
 __device__ __forceinline__ void warp_quantize_q8_k(const float (&vals)[8], int8_t* qk, float* dk, int16_t* bs) {

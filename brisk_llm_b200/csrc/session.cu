@@ -786,8 +786,9 @@ struct Session {
         uint32_t slot = 0;
 
         // out = W x (optionally RMS-normed, then quantised) for one group of targets sharing the input.
-        auto apply = [&](std::vector<MatTarget> targets, const float* x, uint32_t ldx, const float* w, uint32_t cols, Epilogue epi, uint32_t count = 0) {
-            if (count == 0) count = n;
+        // ready: the input as Q8_0 planes, where the kernel before has made them.
+        auto apply = [&](std::vector<MatTarget> targets, const float* x, uint32_t ldx, const float* w, uint32_t cols, Epilogue epi, const DevActMut* ready = nullptr) {
+            const uint32_t count = n;
             if (single) {
                 unsigned long long* t = tr ? tr + 8 * (slot++ % 512) : nullptr;
                 if (epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL) {
@@ -807,6 +808,13 @@ struct Session {
                     ++launches;
                     targets.swap(rest);
                 }
+                return;
+            }
+            if (ready != nullptr) {
+                DevActMut a = *ready;
+                a.f32 = nullptr;
+                a.cols = cols;
+                multiply(std::move(targets), a.view(), count, epi);
                 return;
             }
             Needs nd;
@@ -836,6 +844,15 @@ struct Session {
             at.scores = partial.as<float>(); at.position = d_position();
             at.n = n; at.heads = heads_l; at.kv_heads = kv_heads_l; at.dim = head_dim; at.max_context = uint32_t(max_context);
             at.max_visible = max_visible; at.scale = attn_scale; at.window = L.slides ? sliding_window : 0;
+            // The output projection of a few tokens takes the attended rows as Q8_0 planes, with no norm between: the chains end in
+            // them, a launch less. us a pass, quantised by its own launch / by the chains: 0.6B shape Q4_0 at 2, 9, 23 tokens 1104/1075,
+            // 1220/1178, 1315/1296, Q8_0 verifying 9 after 700 positions 1889/1861, Gemma 1B shape at 9 and 23 1675/1648, 1827/1797,
+            // 1B Llama shape (4.2 M weights) at 23 1094/1087. The 7B shape (16.8 M) loses more by its projection's late start than the
+            // launch gives: 23 tokens 4341/4453, 23 after 500 positions 5208/5442, 9 after 2064 4469/4506 (2 to 16 tokens win).
+            const bool planes = !single && !tp && L.attn_sub_norm == nullptr && block_elems(L.o.type) == 32 &&
+                uint64_t(hidden) * q_dim <= kPlanesMaxWeights && attention_takes_chain(n);
+            const DevActMut* attended_planes = planes ? &act : nullptr;
+            if (planes) at.quant = act;
             {
                 Scope sc(this, PH_ATTENTION);
                 if (single) {
@@ -875,10 +892,10 @@ struct Session {
             } else {
                 Scope sc(this, PH_ATTN_OUT);
                 if (L.attn_post_norm) {
-                    apply({{L.o, proj_b.as<float>(), hidden}}, attended, q_dim, L.attn_sub_norm, q_dim, EPI_STORE);
+                    apply({{L.o, proj_b.as<float>(), hidden}}, attended, q_dim, L.attn_sub_norm, q_dim, EPI_STORE, attended_planes);
                     post_norm_add(L.attn_post_norm);
                 } else {
-                    apply({{L.o, hid, hidden}}, attended, q_dim, L.attn_sub_norm, q_dim, EPI_ADD);
+                    apply({{L.o, hid, hidden}}, attended, q_dim, L.attn_sub_norm, q_dim, EPI_ADD, attended_planes);
                 }
             }
 
@@ -1069,6 +1086,7 @@ struct Session {
     // 12 layers (106 MB) 315/270, 323/311, 336/325, 378/352, 462/390; 28 (248 MB) 683/589, 727/690, 757/724, 853/788, 1019/869. What
     // the persistent kernel keeps are small models at short contexts, where that is 7 to 45 us a token: those of up to kFewLayers at
     // up to 1024 positions, and from 513 on those of up to kSomeLayers.
+    static constexpr uint64_t kPlanesMaxWeights = uint64_t(8) << 20;  // measured where it is used
     static constexpr uint64_t kFewLayers = uint64_t(100) << 20, kSomeLayers = uint64_t(160) << 20;
     bool takes_persistent(uint64_t visible) const { return visible <= 1024 && layer_bytes <= (visible <= 512 ? kFewLayers : kSomeLayers); }
 

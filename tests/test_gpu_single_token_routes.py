@@ -77,3 +77,24 @@ def test_the_switch_at_512_positions(layers):
         want_ids, want = general.generate_greedy(7, 10, want_logits=True)
         assert np.array_equal(ids, want_ids) and np.array_equal(logits, want)
         assert np.array_equal(s.eval([3]), general.eval([3])) and s.stats()["persistent_steps"] == 1
+
+
+@pytest.mark.parametrize("layers,before,after", [(2, 1, 0), (18, 1, 0), (19, 0, 0)])
+def test_the_switch_at_1024_positions(layers, before, after):
+    """The persistent kernel's upper lines: layers past 160 MB (19 of this shape; 18 stay below) leave it past 512 positions too,
+    and no model takes it past 1024 visible ones."""
+    spec = synth.tiny(synth.QWEN3_0_6B, layers=layers, vocab=512, context=1152)
+    model = synth.perturb_norms(synth.generate(spec, seed=8, share_layers=True))
+    toks = synth.random_tokens(spec, 1026, seed=9)
+    with engine.CudaSession(model) as s, engine.CudaSession(model, flags=abi.FLAG_NO_MEGAKERNEL) as general:
+        for session in (s, general):
+            session.eval(toks[:1022])
+        for at in range(1022, 1026):
+            assert np.array_equal(s.eval(toks[at:at + 1]), general.eval(toks[at:at + 1]))
+            assert s.stats()["persistent_steps"] == (before if at + 1 <= 1024 else after), at
+        for session in (s, general):
+            session.rollback(1021)
+        ids, logits = s.generate_greedy(7, 5, want_logits=True)  # one call over the line
+        assert s.stats()["persistent_steps"] == 3 * before + 2 * after
+        want_ids, want = general.generate_greedy(7, 5, want_logits=True)
+        assert np.array_equal(ids, want_ids) and np.array_equal(logits, want)

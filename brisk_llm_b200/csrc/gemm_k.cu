@@ -16,7 +16,8 @@
 // Bound: integer multiply-adds and the shared-memory reads that feed them, not the tensor pipe. So what depends on the token
 // alone is worked out once per super-block when the stage is filled - sum(x) for TQ2_0, -32 * bsum[g] for Q6_K, where it is
 // the C operand of the group's MMA, and for Q4_K / Q5_K the sums of 32 as two 6-bit digits, so that two k = 16 MMAs against
-// the row's eight minimums replace eight multiply-adds per output. Measured: prompts of 777 tokens, ternary 2B shape
+// the row's eight minimums replace eight multiply-adds per output. Measured (before gemm_k_tc.cu took
+// prompts of these sizes): 777 tokens, ternary 2B shape
 // 30.0 -> 27.1 ms, Q5_K_M 1B shape (its Q5_K matrices went through the streaming kernel) 119.7 -> 18.6 ms; 1023 tokens of
 // the Q4_K_M 1B shape 21.5 -> 20.0 ms.
 // Tiling as in gemm.cu: the tile is picked from rows, tokens and row length (launch_type); stages of one super-block come

@@ -3,7 +3,7 @@
 //
 // A sub-block's scale is an integer, and so is weighted = sum of scale[sb] * q * x over a super-block: what an MMA per sub-block
 // and a scale-and-add per output on the CUDA cores compute is one contraction of length 256 over the products scale * q. Those
-// take 10 to 14 bits, so they go in as two 8-bit digits, p = 256 high + low, low unsigned: 16 MMAs of k = 32 accumulate the two
+// take 10 to 14 bits, so they go in as two 8-bit digits (Q6_K: p = 256 high + low, Q4_K and Q5_K: 8 high + low): 16 MMAs of k = 32 accumulate the two
 // digit sums of a super-block in tensor memory, and an output meets the CUDA cores once per 256 values instead of once per 32
 // (Q6_K: 16). The minimums of Q4_K / Q5_K times the sums of 16 activations are exact in f16, and their sum (below 2^24) in the
 // MMA's f32: one MMA of kind::f16 gives float(offsets) itself. Ternary weights need one digit and no scales.
@@ -23,8 +23,8 @@
 //
 // Measured, 512 tokens, us against the tiles of gemm_k.cu: 14336 x 4096 Q4_K 228 -> 111, Q5_K 269 -> 120, Q6_K 364 -> 118, TQ2_0
 // 168 -> 74; 2048 x 8192 Q4_K 67 -> 36, Q6_K 118 -> 41. Bound: not the MMAs (16 of 32 cycles each, plus one, in the 1900 cycles a
-// super-block and 64 tokens take; 1400 in tiles of 128) but the hand-overs around them. A wait on an mbarrier costs about 140
-// cycles even when it is long complete, and the tensor memory beside two sets of accumulators holds the digits of one super-block
+// super-block and 64 tokens take; 1400 in tiles of 128) but the hand-overs around them. A wait on an mbarrier costs 71
+// cycles even when it is long complete (111 where lanes wait for several), and the tensor memory beside two sets of accumulators holds the digits of one super-block
 // only: with neither arithmetic nor MMAs the same hand-overs take 900 cycles. Tiles of 128 tokens, one expansion for two sets,
 // are the better ones where they fill the GPU.
 #include <algorithm>

@@ -42,8 +42,8 @@ __device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity, bool& de
     }
 }
 
-// A warp waits for several barriers at once, lanes first .. end - 1 for one each: a wait costs about 140 cycles even where the
-// barrier is long complete.
+// A warp waits for several barriers at once, lanes first .. end - 1 for one each: even where the barriers are long
+// complete one wait costs 71 cycles, several at once 111.
 __device__ __forceinline__ void mbar_wait_all(uint64_t* mine, uint32_t parity, uint32_t first, uint32_t end, bool& dead, unsigned int* error) {
     const uint32_t lane = threadIdx.x & 31;
     const bool waits = lane >= first && lane < end;

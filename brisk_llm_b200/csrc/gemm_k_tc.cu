@@ -614,7 +614,7 @@ uint64_t gemm_k_tc_ns(const MatTarget* targets, int count, uint32_t n, bool pair
     return std::min(tile_ns(targets, count, n, pair, 1, sms), tile_ns(targets, count, n, pair, 2, sms));
 }
 
-void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t sms, cudaStream_t s) {
+void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, uint32_t sms, cudaStream_t s) {
     KtParams p{};
     for (int i = 0; i < count; ++i) {
         p.m[i] = targets[i].m;
@@ -626,7 +626,7 @@ void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, ui
     p.count = count;
     p.epi = int(epi);
     p.one = 1.0f;
-    p.error = gemm_tc_error_word();
+    p.error = wait_error;
     const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
     const int halves = tile_ns(targets, count, n, pair, 2, sms) < tile_ns(targets, count, n, pair, 1, sms) ? 2 : 1;
     switch (targets[0].m.type) {

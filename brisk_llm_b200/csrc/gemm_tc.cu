@@ -39,8 +39,6 @@ constexpr int kMmaWarp = (kLoaders + kEpilogue) / 32;
 constexpr uint32_t kATile = kTM * 32, kBTile = kTN * 32;                                     // one block's operand tiles, bytes
 constexpr uint32_t kStageBytes = kCB * (kATile + kBTile) + kTM * kCB * 2 + kTN * kCB * 4;   // + f16 weight scales + f32 token scales
 
-__device__ unsigned int g_gemm_tc_error;
-
 #ifdef BK_TC_TRACE  // development aid: cycles CTA (0,0) spends waiting, by role - never compiled into the library
 __device__ unsigned long long g_tc_trace[16];
 #define TC_CLOCK() clock64()
@@ -56,6 +54,7 @@ struct TcParams {
     float* out;
     uint32_t ldo, n;
     int epi;
+    unsigned int* error;
 };
 
 // s32 accumulator, s8 x s8, both operands K-major, N = 64, M = 128
@@ -151,7 +150,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
         auto fill = [&](const Regs& g, uint32_t c) {
             const uint32_t s = c % kStages, round = c / kStages;
             const long long t_w = TC_CLOCK();
-            if (round > 0) mbar_wait(&stage_free[s], (round - 1) & 1, dead, &g_gemm_tc_error);
+            if (round > 0) mbar_wait(&stage_free[s], (round - 1) & 1, dead, p.error);
             if (warp == 0) TC_ADD(0, t_w);
             const long long t_f = TC_CLOCK();
             unsigned char* st = smem + size_t(s) * kStageBytes;
@@ -215,10 +214,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
             for (uint32_t c = 0; c < chunks; ++c) {
                 const uint32_t s = c % kStages, set = c & 1;
                 const long long t_a = TC_CLOCK();
-                mbar_wait(&full[s], (c / kStages) & 1, dead, &g_gemm_tc_error);
+                mbar_wait(&full[s], (c / kStages) & 1, dead, p.error);
                 TC_ADD(2, t_a);
                 const long long t_b = TC_CLOCK();
-                mbar_wait(&set_free[set], (c >> 1) & 1, dead, &g_gemm_tc_error);  // use u of a set waits for its u-th release; the 0th is the epilogue's preset
+                mbar_wait(&set_free[set], (c >> 1) & 1, dead, p.error);  // use u of a set waits for its u-th release; the 0th is the epilogue's preset
                 TC_ADD(3, t_b);
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 const uint32_t a0 = saddr(smem + size_t(s) * kStageBytes), b0 = a0 + kCB * kATile;
@@ -250,7 +249,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
         for (uint32_t c = 0; c < chunks; ++c) {
             const uint32_t s = c % kStages, set = c & 1;
             const long long t_e = TC_CLOCK();
-            mbar_wait(&set_full[set], (c >> 1) & 1, dead, &g_gemm_tc_error);
+            mbar_wait(&set_full[set], (c >> 1) & 1, dead, p.error);
             if (ew == 0) TC_ADD(4, t_e);
             const long long t_g = TC_CLOCK();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -336,17 +335,11 @@ void launch_tile(const TcParams& p, cudaStream_t s) {
 
 }  // namespace
 
-unsigned int* gemm_tc_error_word() {
-    unsigned int* p = nullptr;
-    BK_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_gemm_tc_error));
-    return p;
-}
-
 bool gemm_tc_supports(int type, uint32_t cols) { return (type == T_Q4_0 || type == T_Q8_0) && cols % 128 == 0; }
 
 // out = weights x activations (EPI_STORE / EPI_ADD) for one Q4_0 / Q8_0 target on the tcgen05 path.
-void launch_gemm_tc(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s) {
-    const TcParams p{tg.m, act, tg.out, tg.ldo, n, int(epi)};
+void launch_gemm_tc(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, cudaStream_t s) {
+    const TcParams p{tg.m, act, tg.out, tg.ldo, n, int(epi), wait_error};
     if (tg.m.type == T_Q4_0) launch_tile<16>(p, s);
     else launch_tile<32>(p, s);
 }

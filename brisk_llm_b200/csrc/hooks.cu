@@ -38,13 +38,28 @@ struct ActBuffers {
     }
 };
 
+// The word that a bounded wait of a multiply sets: read it behind the multiplies that were given it.
+struct WaitError {
+    Buf word{sizeof(unsigned int)};
+    WaitError() {
+        const unsigned int start = bk::tc_error_at_start();
+        BK_CUDA(cudaMemcpy(word.p, &start, sizeof start, cudaMemcpyHostToDevice));
+    }
+    unsigned int* get() const { return word.as<unsigned int>(); }
+    void check() const {
+        unsigned int set = 0;
+        BK_CUDA(cudaMemcpy(&set, word.p, sizeof set, cudaMemcpyDeviceToHost));
+        if (set != 0) throw bk::CudaError("cuda: a wait inside a multiply in tensor memory ran out; its result is invalid");
+    }
+};
+
 // The multiply the session would run for n tokens: the fused single-token kernel (which quantises x itself), the
 // tensor-core kernel where the format has one for n tokens, the streaming kernel otherwise.
-void multiply(const bk::DevMatrix& m, float* out, const float* x, const bk::DevAct& a, uint32_t n, uint32_t sms, cudaStream_t s) {
+void multiply(const bk::DevMatrix& m, float* out, const float* x, const bk::DevAct& a, uint32_t n, const WaitError& word, uint32_t sms, cudaStream_t s) {
     bk::MatTarget t{m, out, m.rows};
     if (n == 1) {
         bk::launch_dec_multiply(&t, 1, x, nullptr, 0.0f, m.cols, bk::EPI_STORE, sms, s);
-    } else if (bk::launch_gemm(&t, 1, a, n, bk::EPI_STORE, s) == 0) {
+    } else if (bk::launch_gemm(&t, 1, a, n, bk::EPI_STORE, word.get(), s) == 0) {
         bk::launch_matvec(&t, 1, a, n, bk::EPI_STORE, s);
     }
 }
@@ -80,7 +95,9 @@ int brisk_cuda_matmul(int32_t type, const void* w, uint64_t rows, uint64_t cols,
         bk::DevActMut a = ab.act;
         if (!f) a.f32 = nullptr;
         bk::launch_norm_quant(xd.as<float>(), uint32_t(cols), nullptr, 0.0f, uint32_t(n), uint32_t(cols), a, !k && !f, k, nullptr);
-        multiply(m, od.as<float>(), xd.as<float>(), ab.act.view(), uint32_t(n), sm_count(), nullptr);
+        const WaitError word;
+        multiply(m, od.as<float>(), xd.as<float>(), ab.act.view(), uint32_t(n), word, sm_count(), nullptr);
+        word.check();
         BK_CUDA(cudaMemcpy(out, od.p, n * rows * 4, cudaMemcpyDeviceToHost));
         return 0;
     } catch (const std::exception& e) {
@@ -116,18 +133,20 @@ int brisk_cuda_matmul_seconds(int32_t type, const void* w, uint64_t rows, uint64
         const bool k = bk::takes_q8_k(type), f = type == bk::T_F16 || type == bk::T_F32;
         bk::launch_norm_quant(xd.as<float>(), uint32_t(cols), nullptr, 0.0f, uint32_t(n), uint32_t(cols), ab.act, !k && !f, k, nullptr);
         const uint32_t sms = sm_count();
-        for (uint32_t i = 0; i < 3; ++i) multiply(ms[i % copies], od.as<float>(), xd.as<float>(), ab.act.view(), uint32_t(n), sms, nullptr);
+        const WaitError word;
+        for (uint32_t i = 0; i < 3; ++i) multiply(ms[i % copies], od.as<float>(), xd.as<float>(), ab.act.view(), uint32_t(n), word, sms, nullptr);
         cudaEvent_t e0, e1;
         BK_CUDA(cudaEventCreate(&e0));
         BK_CUDA(cudaEventCreate(&e1));
         BK_CUDA(cudaEventRecord(e0, nullptr));
-        for (uint32_t i = 0; i < iterations; ++i) multiply(ms[i % copies], od.as<float>(), xd.as<float>(), ab.act.view(), uint32_t(n), sms, nullptr);
+        for (uint32_t i = 0; i < iterations; ++i) multiply(ms[i % copies], od.as<float>(), xd.as<float>(), ab.act.view(), uint32_t(n), word, sms, nullptr);
         BK_CUDA(cudaEventRecord(e1, nullptr));
         BK_CUDA(cudaEventSynchronize(e1));
         float ms_total = 0;
         BK_CUDA(cudaEventElapsedTime(&ms_total, e0, e1));
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
+        word.check();
         *seconds = double(ms_total) * 1e-3 / iterations;
         return 0;
     } catch (const std::exception& e) {

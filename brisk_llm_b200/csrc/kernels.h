@@ -69,10 +69,12 @@ void launch_tp_peer_exchange(uint2* const* bufs_dev, uint32_t* epoch, unsigned i
 // Same contract as launch_matvec; returns the number of kernels launched, 0 when these types, shapes or token counts have
 // no tensor kernel (the caller then uses launch_matvec). The super-block formats have one for the pair epilogues where there are
 // rows and tokens enough (gemm_k_tc.cu); elsewhere the caller multiplies gate and up separately and runs launch_gate_mul.
-int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, cudaStream_t s);
-// The Q4_0 / Q8_0 prompt multiply on tcgen05 / tensor memory (gemm_tc.cu; BRISK_CUDA_GEMM=tc): its waits are bounded, and this
-// word is non-zero on the device after a launch whose wait ran out.
-unsigned int* gemm_tc_error_word();
+// The kernels in tensor memory (gemm_k_tc.cu, and gemm_tc.cu: BRISK_CUDA_GEMM=tc) have bounded waits: `wait_error`, a word of the
+// caller's in device memory, is non-zero after a launch whose wait ran out. It belongs to one caller: read and cleared by several, one
+// would take the other's garbage for results.
+int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, cudaStream_t s);
+// BRISK_CUDA_TEST_TC_TIMEOUT=1 (tests only): the word of whoever asks is set from the start, as a wait that ran out leaves it.
+unsigned int tc_error_at_start();
 // The activation after separate gate and up multiplies. mode 0: gate[i] = silu(gate[i]) * up[i]; 1: max(gate[i],0)^2 * up[i];
 // 2: tanh-GELU(gate[i]) * up[i] (gelu_mul_f32, src/kernels_f32.cpp:291-296), its tanh corrected by tanh_table (see
 // build_tanh_table) when one is given.

@@ -206,7 +206,7 @@ struct Session {
     DevBuffer peer_buf, peer_table, peer_state;  // peer_state: [0] the next tag, [1] the error word
     std::vector<void*> peer_mapped;              // what cudaIpcOpenMemHandle returned (closed with the session)
     bool peer_on = false;
-    unsigned int* gemm_tc_error_dev = nullptr;
+    DevBuffer tc_error;  // set by a wait of this session's multiplies in tensor memory that ran out
     unsigned int* step_error_host = nullptr;  // pinned copy of the kernel's barrier-timeout word
     uint64_t persistent_steps = 0;
     uint64_t launches = 0;  // kernels launched by the current call
@@ -565,8 +565,10 @@ struct Session {
         score_dev.alloc(kMaxBatch * sizeof(double));
         BK_CUDA(cudaMallocHost(&score_host, kMaxBatch * sizeof(double)));
         BK_CUDA(cudaMallocHost(&step_error_host, 4 * sizeof(unsigned int)));  // [0] the persistent kernel's word, [1] the peer exchange's
-        step_error_host[0] = step_error_host[1] = step_error_host[2] = step_error_host[3] = 0;  // [3]: the tcgen05 prompt multiply's
-        gemm_tc_error_dev = gemm_tc_error_word();
+        step_error_host[0] = step_error_host[1] = step_error_host[2] = step_error_host[3] = 0;  // [3]: that of the multiplies in tensor memory
+        tc_error.alloc(sizeof(unsigned int));
+        const unsigned int tc_start = tc_error_at_start();
+        BK_CUDA(cudaMemcpyAsync(tc_error.p, &tc_start, sizeof tc_start, cudaMemcpyHostToDevice, stream));
         BK_CUDA(cudaStreamSynchronize(stream));
         plan_step();
         stats.weight_bytes = weight_bytes;
@@ -653,13 +655,13 @@ struct Session {
     // batches go to the tensor-core kernel where the type has one.
     void multiply(std::vector<MatTarget> targets, const DevAct& a, uint32_t n, Epilogue epi) {
         if (epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL) {
-            if (const int ran = launch_gemm(targets.data(), int(targets.size()), a, n, epi, stream)) {
+            if (const int ran = launch_gemm(targets.data(), int(targets.size()), a, n, epi, tc_error.as<unsigned int>(), stream)) {
                 launches += ran;
                 return;
             }
             // formats whose tensor kernel has no fused activation: gate and up as two multiplies, then the activation elementwise
             const MatTarget both[2] = {{targets[0].m, targets[0].out, targets[0].ldo}, {targets[1].m, up_b.as<float>(), targets[0].ldo}};
-            if (const int ran = launch_gemm(both, 2, a, n, EPI_STORE, stream)) {
+            if (const int ran = launch_gemm(both, 2, a, n, EPI_STORE, tc_error.as<unsigned int>(), stream)) {
                 launch_gate_mul(targets[0].out, up_b.as<float>(), size_t(n) * targets[0].ldo, epi == EPI_RELU2_MUL, stream);
                 launches += ran + 1;
                 return;
@@ -671,7 +673,7 @@ struct Session {
         while (!targets.empty()) {
             std::vector<MatTarget> same, rest;
             for (const MatTarget& t : targets) (t.m.type == targets[0].m.type ? same : rest).push_back(t);
-            if (const int ran = launch_gemm(same.data(), int(same.size()), a, n, epi, stream)) {
+            if (const int ran = launch_gemm(same.data(), int(same.size()), a, n, epi, tc_error.as<unsigned int>(), stream)) {
                 launches += ran;
             } else {
                 launch_matvec(same.data(), int(same.size()), a, n, epi, stream);
@@ -1018,7 +1020,7 @@ struct Session {
         // The tcgen05 multiply has bounded waits: its error word, read with the results of a call that may have run it. (A word is
         // a copy of its own, about 2 us at the end of every call.)
         if (batched) {
-            BK_CUDA(cudaMemcpyAsync(step_error_host + 3, gemm_tc_error_dev, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
+            BK_CUDA(cudaMemcpyAsync(step_error_host + 3, tc_error.p, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
         }
         if (peer_on) BK_CUDA(cudaMemcpyAsync(step_error_host + 1, peer_state.as<unsigned int>() + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
         if (token_enabled && persistent_steps != 0) BK_CUDA(cudaMemcpyAsync(step_error_host, token_plan.error_word(), sizeof(unsigned int), cudaMemcpyDeviceToHost, stream));
@@ -1027,8 +1029,8 @@ struct Session {
     void finish_step_check() {
         if (step_error_host[3] != 0) {
             step_error_host[3] = 0;
-            BK_CUDA(cudaMemsetAsync(gemm_tc_error_dev, 0, sizeof(unsigned int), stream));
-            throw CudaError("cuda: a wait inside the tcgen05 prompt multiply ran out; the results of this call are invalid");
+            BK_CUDA(cudaMemsetAsync(tc_error.p, 0, sizeof(unsigned int), stream));
+            throw CudaError("cuda: a wait inside a multiply in tensor memory ran out; the results of this call are invalid");
         }
         if (step_error_host[1] != 0) {
             step_error_host[1] = 0;

@@ -12,8 +12,6 @@ namespace bk {
 // as wide as the box, none for 16). Rows past the last arrive as zeros.
 CUtensorMap tensor_map(const void* base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows);
 
-unsigned int* gemm_tc_error_word();  // the current device's: set by a wait that ran out, read by the session after a call
-
 #ifdef __CUDACC__
 constexpr long long kTcWaitCycles = 2000000000ll;  // about a second: a wait that lasts this long has failed
 constexpr uint32_t kTmemCols = 512;

@@ -169,10 +169,11 @@ void launch_rows(const ChainParams& p, uint32_t groups, cudaStream_t s) {
 }  // namespace
 
 // a.scores holds the probabilities of the n tokens (rows of max_context floats); a.out receives the attended rows.
-void launch_attn_chain(const AttnArgs& a, uint32_t sms, cudaStream_t s) {
+void launch_attn_chain(const AttnArgs& a, const DevActMut* planes, uint32_t sms, cudaStream_t s) {
     ChainParams p{};
-    p.probs = a.scores; p.v_cache = a.v_cache; p.out = a.out; p.quant = a.quant; p.position = a.position;
+    p.probs = a.scores; p.v_cache = a.v_cache; p.out = a.out; p.position = a.position;
     p.n = a.n; p.heads = a.heads; p.kv_heads = a.kv_heads; p.dim = a.dim; p.max_context = a.max_context; p.window = a.window;
+    if (planes != nullptr) p.quant = *planes;
     const uint32_t rows = a.n * (a.heads / a.kv_heads);
     // The rows a CTA takes: whichever leaves the busiest SM with fewer warps, the more of them on a tie (less V traffic).
     auto groups = [&](uint32_t per_cta) { return (rows + per_cta - 1) / per_cta; };

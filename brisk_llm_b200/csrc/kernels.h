@@ -129,13 +129,15 @@ struct AttnArgs {
     uint32_t max_visible;  // host-side upper bound of position + n (sizes the grid)
     float scale;
     uint32_t window = 0;   // sliding-window layer: a token attends to its last `window` positions only (0: to all)
-    DevActMut quant{};     // where attention_takes_chain(n) and quant.q0 is set, the attended rows go there as Q8_0 planes too
 };
 size_t attn_scratch_floats(uint32_t n, uint32_t heads, uint32_t max_context);
-void launch_attention(const AttnArgs& a, cudaStream_t s);
+static_assert(sizeof(AttnArgs) == 80, "a parameter of the prompt attention's kernels: see launch_attention");
+// planes: where attention_takes_chain(n), the attended rows go there as Q8_0 planes too. Not a member of AttnArgs: the prompt kernels
+// take that as their parameter, and with 64 bytes more of it attn_weighted_kernel ran 26.7 us instead of 25.7 (333 tokens, 0.6B shape).
+void launch_attention(const AttnArgs& a, const DevActMut* planes, cudaStream_t s);
 // Weighted sum for a few tokens (attn_chain.cu): a.scores holds their probabilities. A warp per (token, query head) and 32
 // values; same results as the kernels above.
-void launch_attn_chain(const AttnArgs& a, uint32_t sms, cudaStream_t s);
+void launch_attn_chain(const AttnArgs& a, const DevActMut* planes, uint32_t sms, cudaStream_t s);
 bool attention_takes_chain(uint32_t n);       // whether launch_attention ends with it
 constexpr uint32_t kChainMaxTokens = 24;      // more tokens than this share V rows through the tiled kernel instead
 // BRISK_CUDA_CHAIN: 0 never (nor the single-token kernel of attn_decode.cu), 1 wherever it fits, unset: up to kChainMaxTokens tokens.

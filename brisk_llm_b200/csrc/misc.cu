@@ -317,7 +317,7 @@ bool attention_takes_chain(uint32_t n) {
     return mode != 0 && (n <= kChainMaxTokens || mode == 1);
 }
 
-void launch_attention(const AttnArgs& a, cudaStream_t s) {
+void launch_attention(const AttnArgs& a, const DevActMut* planes, cudaStream_t s) {
     if ((a.dim != 64 && a.dim != 128 && a.dim != 256) || a.heads / a.kv_heads > 8) throw CudaError("cuda: attention takes head sizes 64, 128 and 256 and at most 8 query heads per K/V head");
     static const uint32_t sms = [] {
         int dev = 0, count = 148;
@@ -326,7 +326,7 @@ void launch_attention(const AttnArgs& a, cudaStream_t s) {
     }();
     launch_attn_scores(a, sms, s);
     launch_attn_softmax(a, sms, s);
-    if (attention_takes_chain(a.n)) launch_attn_chain(a, sms, s);
+    if (attention_takes_chain(a.n)) launch_attn_chain(a, planes, sms, s);
     else launch_attn_weighted(a, sms, s);
 }
 

@@ -854,14 +854,13 @@ struct Session {
             const bool planes = !single && !tp && L.attn_sub_norm == nullptr && block_elems(L.o.type) == 32 &&
                 uint64_t(hidden) * q_dim <= kPlanesMaxWeights && attention_takes_chain(n);
             const DevActMut* attended_planes = planes ? &act : nullptr;
-            if (planes) at.quant = act;
             {
                 Scope sc(this, PH_ATTENTION);
                 if (single) {
                     launches += launch_dec_attention(r, at, fused_attention, sms, stream);
                 } else {
                     launch_qk_norm_rope_store(r, stream);
-                    launch_attention(at, stream);
+                    launch_attention(at, attended_planes, stream);
                     launches += 4;
                 }
             }

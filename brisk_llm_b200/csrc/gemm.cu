@@ -392,7 +392,7 @@ uint32_t sm_count() {
 }  // namespace
 
 bool gemm_tc_supports(int type, uint32_t cols);  // gemm_tc.cu: the same arithmetic on tcgen05 / tensor memory
-void launch_gemm_tc(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, cudaStream_t s);
+void launch_gemm_tc(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, cudaStream_t s);
 // BRISK_CUDA_GEMM=tc / mma picks the prompt GEMM of Q4_0 / Q8_0 matrices (read at every call); unset: kGemmTcDefault. Measured,
 // 512 tokens, us here / gemm_tc.cu: 1024 x 3072 Q4_0 21 / 37, 2048 x 8192 76 / 91, 4096 x 14336 228 / 296, Q8_0 240 / 317.
 constexpr bool kGemmTcDefault = false;
@@ -401,29 +401,39 @@ static bool gemm_tc_on() {
     return env == nullptr ? kGemmTcDefault : std::strcmp(env, "tc") == 0;
 }
 bool gemm_k_supports(int type);  // gemm_k.cu: the 256-value super-block formats
-bool launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, uint32_t sms, cudaStream_t s);
+bool launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, uint32_t sms, cudaStream_t s);
 
 // From 2 tokens on: Q4_0 / Q8_0 rows of a multiple of 4 blocks (128 values), and the super-block formats.
 static bool gemm_supports(int type, uint32_t cols, uint32_t n) {
     return n >= 2 && (type == T_Q4_0 || type == T_Q8_0 ? cols % (32 * KB) == 0 : gemm_k_supports(type));
 }
 
-unsigned int tc_error_at_start() {
+WaitBound wait_bound(unsigned int* word_on_device, cudaStream_t s) {
     const char* env = std::getenv("BRISK_CUDA_TEST_TC_TIMEOUT");
-    return env != nullptr && std::strcmp(env, "1") == 0 ? 1u : 0u;
+    const int test = env != nullptr ? std::atoi(env) : 0;
+    const unsigned int start = test == 1 ? 1u : 0u;
+    BK_CUDA(cudaMemcpyAsync(word_on_device, &start, sizeof start, cudaMemcpyHostToDevice, s));
+    BK_CUDA(cudaStreamSynchronize(s));
+    WaitBound bound;
+    bound.error = word_on_device;
+    if (test >= 2) {
+        bound.cycles = 100000;
+        bound.withheld = uint32_t(test - 2);
+    }
+    return bound;
 }
 
-int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, cudaStream_t s) {
+int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, cudaStream_t s) {
     const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
     for (int i = 0; i < count; ++i) {
         if (!gemm_supports(targets[i].m.type, targets[i].m.cols, n)) return 0;
     }
     const int type = targets[0].m.type;
     if (type != T_Q4_0 && type != T_Q8_0) {
-        return launch_gemm_k(targets, count, act, n, epi, wait_error, sm_count(), s) ? 1 : 0;
+        return launch_gemm_k(targets, count, act, n, epi, bound, sm_count(), s) ? 1 : 0;
     }
     if (!pair && n >= 32 && gemm_tc_on() && gemm_tc_supports(type, targets[0].m.cols)) {
-        for (int i = 0; i < count; ++i) launch_gemm_tc(targets[i], act, n, epi, wait_error, s);
+        for (int i = 0; i < count; ++i) launch_gemm_tc(targets[i], act, n, epi, bound, s);
         return count;
     }
     GemmParams p{};

@@ -545,13 +545,13 @@ bool launch_type(KParams& p, uint64_t other_ns, bool ask_only, uint32_t sms, cud
 }  // namespace
 
 // gemm_k_tc.cu: the multiply in tensor memory, and what it is expected to take
-void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, uint32_t sms, cudaStream_t s);
+void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, uint32_t sms, cudaStream_t s);
 uint64_t gemm_k_tc_ns(const MatTarget* targets, int count, uint32_t n, bool pair, uint32_t sms);
 
 bool gemm_k_supports(int type) { return type == T_Q4_K || type == T_Q5_K || type == T_Q6_K || type == T_TQ2_0; }
 
 // False, nothing launched: a gate/up pair that the caller multiplies separately.
-bool launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, uint32_t sms, cudaStream_t s) {
+bool launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, uint32_t sms, cudaStream_t s) {
     const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
     uint64_t other_ns = gemm_k_tc_ns(targets, count, n, pair, sms);
     if (pair) {
@@ -579,7 +579,7 @@ bool launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint3
         default: throw CudaError("cuda: no super-block tensor kernel for this type");
     }
     if (here) return !pair;
-    launch_gemm_k_tc(targets, count, act, n, epi, wait_error, sms, s);
+    launch_gemm_k_tc(targets, count, act, n, epi, bound, sms, s);
     return true;
 }
 

@@ -9,7 +9,7 @@
 // MMA's f32: one MMA of kind::f16 gives float(offsets) itself. Ternary weights need one digit and no scales.
 //
 // CTA tile: 128 weight rows (of one matrix, or 64 gate and 64 up rows) x 64 or 128 tokens, a CTA per SM that walks tiles until
-// none are left; the roles run ahead of one another across tiles and meet only at mbarriers (bounded waits, error word):
+// none are left; the roles run ahead of one another across tiles and meet only at mbarriers (bounded waits, error word: tc.cuh):
 //
 //   8 loader warps    thread = row = tensor-memory lane, a half super-block each: quants times scales four or two at a time, the digits
 //                     in registers until the MMAs of the half before are done, then into tensor memory as the A operand. (In
@@ -72,7 +72,7 @@ struct KtParams {
     uint32_t n, tok_tiles, tiles;
     int count, epi;
     float one;
-    unsigned int* error;
+    WaitBound bound;
 };
 
 // Four products of 16 bits, in even and odd bytes' order -> the four low bytes and the four high bytes.
@@ -161,7 +161,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
     using S = Shape<TYPE, NT>;
     extern __shared__ unsigned char smem_raw[];
     __shared__ __align__(8) uint64_t a_full[2], a_free[2], d_full[2], d_free[2], w_full[kSlots], w_free[kSlots], b_full[kSlots], b_free[kSlots];
-    __shared__ uint32_t tmem_slot;
+    __shared__ __align__(8) uint64_t drained;
+    __shared__ uint32_t tmem_slot, stored;
     unsigned char* const weights = smem_raw + (1024 - saddr(smem_raw) % 1024) % 1024;  // swizzled tiles lie on 1024-byte boundaries
     unsigned char* const slots = weights + kSlots * S::kWSlot;
     unsigned char* const minimums = slots + kSlots * S::kSlot;  // of the rows, as an f16 operand, for four super-blocks
@@ -182,6 +183,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
             mbar_init(&b_full[i], kHelpWarps);  // two warps that store, one copy
             mbar_init(&b_free[i], 1 + kEpiWarps);
         }
+        mbar_init(&drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {  // all 512 columns: one CTA per SM
@@ -192,7 +194,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = *reinterpret_cast<volatile uint32_t*>(&tmem_slot);
-    bool dead = false;
+    bool dead = false;  // a wait of this lane gave up
+    auto report = [&] { atomicOr(p.bound.error, 1u); };
+    // Of a thread that asked for copies or MMAs: the barriers on which they are counted, and how often.
+    uint64_t* asked_on = &drained;
+    uint32_t asked = 0;
 
     auto target_of = [&](uint32_t row_tile) {
         int target = 0;
@@ -218,7 +224,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
         const uint32_t h = warp >> 2, r = (warp & 3) * 32 + lane, ta = tmem + (((warp & 3) * 32) << 16) + kACol + h * 64;
         for (uint32_t it = 0; it < total; ++it) {
             const uint32_t w = it % kSlots;
-            mbar_wait(&w_full[w], (it / kSlots) & 1, dead, p.error);
+            mbar_wait(&w_full[w], (it / kSlots) & 1, dead, p.bound.cycles);
             uint32_t lo[32], hi[32];
             expand_half<TYPE, S>(weights + w * S::kWSlot, r, h, lo, hi);
             if constexpr (S::kMins) {  // this half's four minimums, each twice: for the sums of 16 on either side of a sub-block.
@@ -234,7 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
                 *reinterpret_cast<uint4*>(minimums + (it & 3) * S::kMn + h * (kRows * 16) + r * 16) = make_uint4(v[0], v[1], v[2], v[3]);
                 async_proxy_fence();
             }
-            if (it > 0) mbar_wait(&a_free[h], (it - 1) & 1, dead, p.error);
+            if (it > 0) mbar_wait(&a_free[h], (it - 1) & 1, dead, p.bound.cycles);
             __syncwarp();
             tc_fence_after();
             tmem_st16(ta, *reinterpret_cast<const uint32_t(*)[16]>(lo));
@@ -246,26 +252,29 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) {
+            if (lane == 0 && !dead) {
                 mbar_arrive(&a_full[h]);
                 mbar_arrive(&w_free[w]);
             }
         }
+        if (dead) report();
     } else if (warp >= kHelpWarp) {
         // ---- helpers ----
         // One warp copies: weights by TMA. The other two: a thread has two rows' d, two runs of eight sums and a token's scale,
         // loaded a super-block ahead; their first thread asks for the activations.
         Walk at{blockIdx.x, 0};
+        const bool leader = elect_one();
         if (warp == kHelpWarp) {
-            const bool leader = elect_one();
-            for (uint32_t it = 0; it < total; ++it, at.next(nsb)) {
+            asked_on = w_full;
+            for (uint32_t it = 0; it < total && it != p.bound.withheld; ++it, at.next(nsb)) {
                 const uint32_t w = it % kSlots;
-                if (it >= kSlots) mbar_wait(&w_free[w], (it / kSlots - 1) & 1, dead, p.error);
+                if (it >= kSlots) mbar_wait(&w_free[w], (it / kSlots - 1) & 1, dead, p.bound.cycles);
                 __syncwarp();
                 const uint32_t row_tile = at.tile / p.tok_tiles;
                 const int target = target_of(row_tile);
                 const uint32_t row = (row_tile - p.first_tile[target]) * (PAIR ? kRows / 2 : kRows);
-                if (leader) {
+                if (leader && !dead) {
+                    ++asked;
                     mbar_expect(&w_full[w], S::kWSlot);
 #pragma unroll
                     for (uint32_t half = 0; half < 2; ++half) {
@@ -331,10 +340,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
             fetch_tokens();
             for (uint32_t it = 0; it < total; ++it) {
                 const uint32_t b = it % kSlots;
-                if (it >= kSlots) mbar_wait(&b_free[b], (it / kSlots - 1) & 1, dead, p.error);
-                unsigned char* bslot = slots + b * S::kSlot;
+                if (it >= kSlots) mbar_wait(&b_free[b], (it / kSlots - 1) & 1, dead, p.bound.cycles);
                 __syncwarp();
-                if (warp == kHelpWarp + 1 && elect_one()) {
+                unsigned char* bslot = slots + b * S::kSlot;
+                if (warp == kHelpWarp + 1 && leader && !dead) {
                     mbar_expect(&b_full[b], S::kB);
                     const uint32_t y = at.tile % p.tok_tiles * (kTokens * NT);
 #pragma unroll
@@ -362,7 +371,10 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
                 }
                 if (S::kMins) async_proxy_fence();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(&b_full[b]);
+                if (leader && !dead) {
+                    mbar_arrive(&b_full[b]);
+                    ++asked;
+                }
                 const bool new_tile = at.next(nsb);
                 if (it + 1 < total) {
                     if (new_tile) enter_tile();
@@ -370,46 +382,69 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
                     fetch_tokens();
                 }
             }
+            // A slot is full once both warps have arrived. Should the other one have given up first, its arrivals are made here.
+            if (warp != kHelpWarp + 1 && leader) stored = asked;
+            __syncwarp();
+            asm volatile("bar.sync 3, 64;" ::: "memory");
+            if (warp == kHelpWarp + 1) {
+                asked_on = b_full;
+                if (leader) for (uint32_t i = *reinterpret_cast<volatile uint32_t*>(&stored); i < asked; ++i) mbar_arrive(&b_full[i % kSlots]);
+            } else {
+                asked = 0;
+            }
         }
+        if (dead) report();
     } else if (warp == kMmaWarp) {
         // ---- MMAs: one elected lane ----
         constexpr uint32_t kLow = instr_i8(TYPE == T_TQ2_0, kTokens), kHigh = instr_i8(TYPE == T_Q6_K, kTokens);
         const bool leader = elect_one();
-        for (uint32_t it = 0; it < total; ++it) {
-            const uint32_t b = it % kSlots, base = saddr(slots + b * S::kSlot);
+        auto issue = [&] {
+            for (uint32_t it = 0; it < total; ++it) {
+                const uint32_t b = it % kSlots, base = saddr(slots + b * S::kSlot);
 #pragma unroll
-            for (uint32_t nt = 0; nt < NT; ++nt) {
-                const uint32_t i = it * NT + nt, set = i & 1, d = tmem + set * S::kSet;
-                const uint64_t bd = smem_desc_swizzled(base + nt * (kTokens * 256));
-                // a free set of accumulators (from the third use on), the activations, the first half's digits
-                mbar_wait_all(lane == 0 ? &d_free[set] : lane == 1 ? &a_full[0] : &b_full[b], lane == 0 ? ((i >> 1) - 1) & 1 : lane == 1 ? it & 1 : (it / kSlots) & 1, i >= 2 ? 0 : 1,
-                              nt == 0 ? 3 : 1, dead, p.error);
+                for (uint32_t nt = 0; nt < NT; ++nt) {
+                    const uint32_t i = it * NT + nt, set = i & 1, d = tmem + set * S::kSet;
+                    const uint64_t bd = smem_desc_swizzled(base + nt * (kTokens * 256));
+                    // a free set of accumulators (from the third use on), the activations, the first half's digits
+                    if (!mbar_wait_all(lane == 0 ? &d_free[set] : lane == 1 ? &a_full[0] : &b_full[b], lane == 0 ? ((i >> 1) - 1) & 1 : lane == 1 ? it & 1 : (it / kSlots) & 1, i >= 2 ? 0 : 1,
+                                       nt == 0 ? 3 : 1, p.bound.cycles)) {
+                        if (lane == 0) report();
+                        return;
+                    }
 #pragma unroll
-                for (uint32_t h = 0; h < 2; ++h) {
-                    if (nt == 0 && h == 1) {
-                        mbar_wait(&a_full[1], it & 1, dead, p.error);
+                    for (uint32_t h = 0; h < 2; ++h) {
+                        if (nt == 0 && h == 1) {
+                            mbar_wait(&a_full[1], it & 1, dead, p.bound.cycles);
+                            __syncwarp();
+                        }
+                        tc_fence_after();
+                        // (Where the wait for the digits gave up, these MMAs run on what is there, and the next wait ends the walk: asking
+                        // here as well took 0.2 % of a Q4_K prompt, 1.7 % of a ternary one.)
+                        if (leader) {
+                            asked = 1;
+                            if (S::kMins && h == 1) {
+                                mma_f16_ss(d + 2 * kTokens, smem_desc(saddr(minimums + (it & 3) * S::kMn), kRows * 16, 128),
+                                           smem_desc(base + S::kB + nt * (kTokens * 32), kTokens * 16, 128), instr_f16(kTokens));
+                            }
+#pragma unroll
+                            for (uint32_t j = 0; j < 4; ++j) {
+                                const uint32_t a = tmem + kACol + h * 64 + j * 8;
+                                mma_i8_ts(d, a, bd + (h * (kTokens * 128) + j * 32) / 16, kLow, h + j != 0);
+                                if (S::kDigits == 2) mma_i8_ts(d + kTokens, a + 32, bd + (h * (kTokens * 128) + j * 32) / 16, kHigh, h + j != 0);
+                            }
+                            if (nt + 1 == NT) mma_commit(&a_free[h]);
+                            if (h == 1) mma_commit(&d_full[set]);
+                            if (h == 1 && nt + 1 == NT) mma_commit(&b_free[b]);
+                        }
                         __syncwarp();
                     }
-                    tc_fence_after();
-                    if (leader) {
-                        if (S::kMins && h == 1) {
-                            mma_f16_ss(d + 2 * kTokens, smem_desc(saddr(minimums + (it & 3) * S::kMn), kRows * 16, 128),
-                                       smem_desc(base + S::kB + nt * (kTokens * 32), kTokens * 16, 128), instr_f16(kTokens));
-                        }
-#pragma unroll
-                        for (uint32_t j = 0; j < 4; ++j) {
-                            const uint32_t a = tmem + kACol + h * 64 + j * 8;
-                            mma_i8_ts(d, a, bd + (h * (kTokens * 128) + j * 32) / 16, kLow, h + j != 0);
-                            if (S::kDigits == 2) mma_i8_ts(d + kTokens, a + 32, bd + (h * (kTokens * 128) + j * 32) / 16, kHigh, h + j != 0);
-                        }
-                        if (nt + 1 == NT) mma_commit(&a_free[h]);
-                        if (h == 1) mma_commit(&d_full[set]);
-                        if (h == 1 && nt + 1 == NT) mma_commit(&b_free[b]);
-                    }
-                    __syncwarp();
                 }
             }
-        }
+        };
+        issue();
+        if (dead) report();
+        // One commit behind all others: the MMAs, and the arrivals of the last commits (which nobody else waits for), are through.
+        if (asked != 0) mma_commit(&drained);
     } else {
         // ---- epilogue ----
         const uint32_t quarter = warp & 3, part = (warp - kLoadWarps) >> 2;  // tensor-memory lanes 32 quarter .., token columns 32 part ..
@@ -418,124 +453,139 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_kt_kernel(const __grid_const
         const f32x2 one2 = pack2(p.one, p.one), minus2 = pack2(-p.one, -p.one);
         wait_for_previous();
         uint32_t it = 0;
-        for (uint32_t tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
-            f32x2 acc[NT][2][4][2];  // [tokens 64 ..][16 lanes][8 columns][lane g / g + 8]
+        auto finish = [&] {
+            for (uint32_t tile = blockIdx.x; tile < p.tiles; tile += gridDim.x) {
+                f32x2 acc[NT][2][4][2];  // [tokens 64 ..][16 lanes][8 columns][lane g / g + 8]
 #pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
+                for (int nt = 0; nt < NT; ++nt)
 #pragma unroll
-                for (int h = 0; h < 2; ++h)
+                    for (int h = 0; h < 2; ++h)
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) acc[nt][h][c][0] = acc[nt][h][c][1] = 0ull;
-            for (uint32_t sb = 0; sb < nsb; ++sb, ++it) {
-                const uint32_t b = it % kSlots;
-                const unsigned char* bslot = slots + b * S::kSlot;
-                const float2* dw = reinterpret_cast<const float2*>(bslot + S::kB + S::kSums + S::kXd) + quarter * 32 + g;
-                float2 rs[2][2];
+                        for (int c = 0; c < 4; ++c) acc[nt][h][c][0] = acc[nt][h][c][1] = 0ull;
+                for (uint32_t sb = 0; sb < nsb; ++sb, ++it) {
+                    const uint32_t b = it % kSlots;
+                    const unsigned char* bslot = slots + b * S::kSlot;
+                    const float2* dw = reinterpret_cast<const float2*>(bslot + S::kB + S::kSums + S::kXd) + quarter * 32 + g;
+                    float2 rs[2][2];
 #pragma unroll
-                for (uint32_t nt = 0; nt < NT; ++nt) {
-                    const uint32_t i = it * NT + nt, set = i & 1, at = mine + set * S::kSet;
-                    // the accumulators and the scales
-                    mbar_wait_all(lane == 0 ? &d_full[set] : &b_full[b], lane == 0 ? (i >> 1) & 1 : (it / kSlots) & 1, 0, nt == 0 ? 2 : 1, dead, p.error);
-                    tc_fence_after();
-                    const f32x2* xd = reinterpret_cast<const f32x2*>(bslot + S::kB + S::kSums) + nt * 32 + part * 16 + t;
-                    if (nt == 0) {
-#pragma unroll
-                        for (int h = 0; h < 2; ++h) {
-                            rs[h][0] = dw[h * 16];
-                            rs[h][1] = dw[h * 16 + 8];
+                    for (uint32_t nt = 0; nt < NT; ++nt) {
+                        const uint32_t i = it * NT + nt, set = i & 1, at = mine + set * S::kSet;
+                        // the accumulators and the scales
+                        if (!mbar_wait_all(lane == 0 ? &d_full[set] : &b_full[b], lane == 0 ? (i >> 1) & 1 : (it / kSlots) & 1, 0, nt == 0 ? 2 : 1, p.bound.cycles)) {
+                            if (lane == 0) report();
+                            if (PAIR) {  // the warps of a pair meet at barriers: twice for every tile and half of its tokens
+                                for (uint32_t left = tile; left < p.tiles; left += gridDim.x) {
+                                    for (int k = 0; k < 2 * NT; ++k) asm volatile("bar.sync 2, 256;" ::: "memory");
+                                }
+                            }
+                            return;
                         }
-                    }
-                    f32x2 xs[4];
+                        tc_fence_after();
+                        const f32x2* xd = reinterpret_cast<const f32x2*>(bslot + S::kB + S::kSums) + nt * 32 + part * 16 + t;
+                        if (nt == 0) {
 #pragma unroll
-                    for (int c = 0; c < 4; ++c) xs[c] = xd[c * 4];
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {  // 16 lanes x 8 columns at a time
-                        const int h = k >> 2, c = k & 3;
-                        const uint32_t from = at + (uint32_t(h * 16) << 16) + c * 8;
-                        uint32_t low[4], high[4], off[4];
-                        tmem_ld_frag1(from, low);
-                        if (S::kDigits == 2) tmem_ld_frag1(from + kTokens, high);
-                        if (S::kMins) tmem_ld_frag1(from + 2 * kTokens, off);
-                        tmem_wait_ld();
-                        if (k == 7) {
-                            tc_fence_before();
-                            __syncwarp();
-                            if (lane == 0) {
-                                mbar_arrive(&d_free[set]);
-                                if (nt + 1 == NT) mbar_arrive(&b_free[b]);  // the scales are in registers
+                            for (int h = 0; h < 2; ++h) {
+                                rs[h][0] = dw[h * 16];
+                                rs[h][1] = dw[h * 16 + 8];
                             }
                         }
+                        f32x2 xs[4];
 #pragma unroll
-                        for (int r = 0; r < 2; ++r) {
-                            auto joined = [&](int e) { return float(int(S::kDigits == 2 ? (high[2 * r + e] << S::kDigitBits) + low[2 * r + e] : low[2 * r + e])); };
-                            const f32x2 sum2 = pack2(joined(0), joined(1)), dw2 = pack2(rs[h][r].x, rs[h][r].x);
-                            f32x2 term;
-                            if constexpr (S::kMins) {  // x.d * (d * weighted - dmin * offsets)
-                                term = mul2(xs[c], fma2(mul2(pack2(rs[h][r].y, rs[h][r].y), pack2(off[2 * r], off[2 * r + 1])), minus2, mul2(dw2, sum2)));
-                            } else {  // (x.d * d) * weighted
-                                term = mul2(mul2(xs[c], dw2), sum2);
+                        for (int c = 0; c < 4; ++c) xs[c] = xd[c * 4];
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {  // 16 lanes x 8 columns at a time
+                            const int h = k >> 2, c = k & 3;
+                            const uint32_t from = at + (uint32_t(h * 16) << 16) + c * 8;
+                            uint32_t low[4], high[4], off[4];
+                            tmem_ld_frag1(from, low);
+                            if (S::kDigits == 2) tmem_ld_frag1(from + kTokens, high);
+                            if (S::kMins) tmem_ld_frag1(from + 2 * kTokens, off);
+                            tmem_wait_ld();
+                            if (k == 7) {
+                                tc_fence_before();
+                                __syncwarp();
+                                if (lane == 0) {
+                                    mbar_arrive(&d_free[set]);
+                                    if (nt + 1 == NT) mbar_arrive(&b_free[b]);  // the scales are in registers
+                                }
                             }
-                            acc[nt][h][c][r] = fma2(term, one2, acc[nt][h][c][r]);
-                        }
-                    }
-                }
-            }
-            const uint32_t row_tile = tile / p.tok_tiles, tok_base = tile % p.tok_tiles * (kTokens * NT);
-            const int target = target_of(row_tile);
-            if (tile + gridDim.x >= p.tiles) release_next();
-            // (a pair: lanes 0 - 15 of a quarter's gate rows are finished there, 16 - 31 on the up side)
-            const uint32_t row_base = (row_tile - p.first_tile[target]) * (PAIR ? kRows / 2 : kRows) + (PAIR ? (quarter & 1) * 32 + (quarter >> 1) * 16 : quarter * 32) + g;
-            if constexpr (PAIR) {
-                // Gate rows are with quarters 0 and 1, the same up rows with 2 and 3. Each side sends the other half of its sums and
-                // applies the activation to the rest: sums 0 .. 7 of a token half stay on the gate side, 8 .. 15 go to the up side.
-                f32x2* exchange = reinterpret_cast<f32x2*>(minimums + 4 * S::kMn) + part * 64 + (quarter & 1) * 32 + lane;
-                const bool up_side = quarter >= 2;
-#pragma unroll
-                for (int nt = 0; nt < NT; ++nt) {
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const f32x2 low = acc[nt][0][(k >> 1) & 3][k & 1], high = acc[nt][1][(k >> 1) & 3][k & 1];
-                        exchange[(up_side ? k : 8 + k) * 128] = up_side ? low : high;
-                    }
-                    asm volatile("bar.sync 2, 256;" ::: "memory");
-#pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const f32x2 mine2 = up_side ? acc[nt][1][(k >> 1) & 3][k & 1] : acc[nt][0][(k >> 1) & 3][k & 1], other2 = exchange[(up_side ? 8 + k : k) * 128];
-                        float g0, g1, u0, u1;
-                        unpack2(up_side ? other2 : mine2, g0, g1);
-                        unpack2(up_side ? mine2 : other2, u0, u1);
-                        if (tok_base + nt * 64 + part * 32 + (k >> 1) * 8 < p.n) {  // of these eight tokens, some exist
-                            acc[nt][0][(k >> 1) & 3][k & 1] =
-                                p.epi == EPI_SILU_MUL ? pack2(silu_mul(g0, u0), silu_mul(g1, u1)) : pack2(relu2_mul(g0, u0), relu2_mul(g1, u1));
-                        }
-                    }
-                    asm volatile("bar.sync 2, 256;" ::: "memory");  // the exchange may be overwritten
-                }
-            }
-            float* const out = p.out[target];
-            const uint32_t rows = p.m[target].rows, ldo = p.ldo[target];
-#pragma unroll
-            for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-                for (int c = 0; c < 4; ++c)
-#pragma unroll
-                    for (int e = 0; e < 2; ++e) {
-                        const uint32_t tok = tok_base + nt * 64 + part * 32 + c * 8 + 2 * t + e;
-                        if (tok >= p.n) continue;
-                        float* o = out + size_t(tok) * ldo;
-#pragma unroll
-                        for (int h = 0; h < (PAIR ? 1 : 2); ++h)
 #pragma unroll
                             for (int r = 0; r < 2; ++r) {
-                                const uint32_t row = row_base + h * 16 + r * 8;
-                                float x, y;
-                                unpack2(acc[nt][h][c][r], x, y);
-                                const float value = e == 0 ? x : y;
-                                if (row < rows) o[row] = p.epi == EPI_ADD ? __fadd_rn(o[row], value) : value;
+                                auto joined = [&](int e) { return float(int(S::kDigits == 2 ? (high[2 * r + e] << S::kDigitBits) + low[2 * r + e] : low[2 * r + e])); };
+                                const f32x2 sum2 = pack2(joined(0), joined(1)), dw2 = pack2(rs[h][r].x, rs[h][r].x);
+                                f32x2 term;
+                                if constexpr (S::kMins) {  // x.d * (d * weighted - dmin * offsets)
+                                    term = mul2(xs[c], fma2(mul2(pack2(rs[h][r].y, rs[h][r].y), pack2(off[2 * r], off[2 * r + 1])), minus2, mul2(dw2, sum2)));
+                                } else {  // (x.d * d) * weighted
+                                    term = mul2(mul2(xs[c], dw2), sum2);
+                                }
+                                acc[nt][h][c][r] = fma2(term, one2, acc[nt][h][c][r]);
                             }
+                        }
                     }
-        }
+                }
+                const uint32_t row_tile = tile / p.tok_tiles, tok_base = tile % p.tok_tiles * (kTokens * NT);
+                const int target = target_of(row_tile);
+                if (tile + gridDim.x >= p.tiles) release_next();
+                // (a pair: lanes 0 - 15 of a quarter's gate rows are finished there, 16 - 31 on the up side)
+                const uint32_t row_base = (row_tile - p.first_tile[target]) * (PAIR ? kRows / 2 : kRows) + (PAIR ? (quarter & 1) * 32 + (quarter >> 1) * 16 : quarter * 32) + g;
+                if constexpr (PAIR) {
+                    // Gate rows are with quarters 0 and 1, the same up rows with 2 and 3. Each side sends the other half of its sums and
+                    // applies the activation to the rest: sums 0 .. 7 of a token half stay on the gate side, 8 .. 15 go to the up side.
+                    f32x2* exchange = reinterpret_cast<f32x2*>(minimums + 4 * S::kMn) + part * 64 + (quarter & 1) * 32 + lane;
+                    const bool up_side = quarter >= 2;
+                    __syncwarp();
+#pragma unroll
+                    for (int nt = 0; nt < NT; ++nt) {
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            const f32x2 low = acc[nt][0][(k >> 1) & 3][k & 1], high = acc[nt][1][(k >> 1) & 3][k & 1];
+                            exchange[(up_side ? k : 8 + k) * 128] = up_side ? low : high;
+                        }
+                        asm volatile("bar.sync 2, 256;" ::: "memory");
+#pragma unroll
+                        for (int k = 0; k < 8; ++k) {
+                            const f32x2 mine2 = up_side ? acc[nt][1][(k >> 1) & 3][k & 1] : acc[nt][0][(k >> 1) & 3][k & 1], other2 = exchange[(up_side ? 8 + k : k) * 128];
+                            float g0, g1, u0, u1;
+                            unpack2(up_side ? other2 : mine2, g0, g1);
+                            unpack2(up_side ? mine2 : other2, u0, u1);
+                            if (tok_base + nt * 64 + part * 32 + (k >> 1) * 8 < p.n) {  // of these eight tokens, some exist
+                                acc[nt][0][(k >> 1) & 3][k & 1] =
+                                    p.epi == EPI_SILU_MUL ? pack2(silu_mul(g0, u0), silu_mul(g1, u1)) : pack2(relu2_mul(g0, u0), relu2_mul(g1, u1));
+                            }
+                        }
+                        asm volatile("bar.sync 2, 256;" ::: "memory");  // the exchange may be overwritten
+                    }
+                }
+                float* const out = p.out[target];
+                const uint32_t rows = p.m[target].rows, ldo = p.ldo[target];
+#pragma unroll
+                for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+                    for (int c = 0; c < 4; ++c)
+#pragma unroll
+                        for (int e = 0; e < 2; ++e) {
+                            const uint32_t tok = tok_base + nt * 64 + part * 32 + c * 8 + 2 * t + e;
+                            if (tok >= p.n) continue;
+                            float* o = out + size_t(tok) * ldo;
+#pragma unroll
+                            for (int h = 0; h < (PAIR ? 1 : 2); ++h)
+#pragma unroll
+                                for (int r = 0; r < 2; ++r) {
+                                    const uint32_t row = row_base + h * 16 + r * 8;
+                                    float x, y;
+                                    unpack2(acc[nt][h][c][r], x, y);
+                                    const float value = e == 0 ? x : y;
+                                    if (row < rows) o[row] = p.epi == EPI_ADD ? __fadd_rn(o[row], value) : value;
+                                }
+                        }
+            }
+        };
+        finish();
     }
+    // Copies are complete by now unless a wait gave up; MMAs and their commits' arrivals in any case only behind this.
+    for (uint32_t i = asked < kSlots ? 0 : asked - kSlots; i < asked; ++i) mbar_drain(&asked_on[i % kSlots], (i / kSlots) & 1);
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
     if (warp == kMmaWarp) {
@@ -614,7 +664,7 @@ uint64_t gemm_k_tc_ns(const MatTarget* targets, int count, uint32_t n, bool pair
     return std::min(tile_ns(targets, count, n, pair, 1, sms), tile_ns(targets, count, n, pair, 2, sms));
 }
 
-void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, uint32_t sms, cudaStream_t s) {
+void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, uint32_t sms, cudaStream_t s) {
     KtParams p{};
     for (int i = 0; i < count; ++i) {
         p.m[i] = targets[i].m;
@@ -626,7 +676,7 @@ void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, ui
     p.count = count;
     p.epi = int(epi);
     p.one = 1.0f;
-    p.error = wait_error;
+    p.bound = bound;
     const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
     const int halves = tile_ns(targets, count, n, pair, 2, sms) < tile_ns(targets, count, n, pair, 1, sms) ? 2 : 1;
     switch (targets[0].m.type) {

@@ -54,7 +54,7 @@ struct TcParams {
     float* out;
     uint32_t ldo, n;
     int epi;
-    unsigned int* error;
+    WaitBound bound;
 };
 
 // s32 accumulator, s8 x s8, both operands K-major, N = 64, M = 128
@@ -95,6 +95,7 @@ template <int WBYTES>
 __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) {
     extern __shared__ __align__(128) unsigned char smem[];
     __shared__ __align__(8) uint64_t full[kStages], stage_free[kStages], set_full[2], set_free[2];
+    __shared__ __align__(8) uint64_t drained;
     __shared__ uint32_t tmem_slot;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t row_base = blockIdx.x * kTM, tok_base = blockIdx.y * kTN;
@@ -109,6 +110,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
             mbar_init(&set_full[s], 1);
             mbar_init(&set_free[s], kEpilogue / 32);
         }
+        mbar_init(&drained, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {  // the MMA warp owns the tensor memory: all 512 columns (one CTA per SM)
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(&tmem_slot);
-    bool dead = false;
+    bool dead = false;  // a wait of this lane gave up
 
     // (Tried: 16 epilogue warps of 16 columns for more warps per scheduler. 21 warps leave 80 registers a thread, the loaders
     // spill, and setmaxnreg cannot help - it only moves registers inside what the CTA was launched with, so raising the
@@ -150,7 +152,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
         auto fill = [&](const Regs& g, uint32_t c) {
             const uint32_t s = c % kStages, round = c / kStages;
             const long long t_w = TC_CLOCK();
-            if (round > 0) mbar_wait(&stage_free[s], (round - 1) & 1, dead, p.error);
+            if (round > 0) mbar_wait(&stage_free[s], (round - 1) & 1, dead, p.bound.cycles);
+            if (c == p.bound.withheld) dead = true;
             if (warp == 0) TC_ADD(0, t_w);
             const long long t_f = TC_CLOCK();
             unsigned char* st = smem + size_t(s) * kStageBytes;
@@ -193,7 +196,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
             }
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");  // the tensor core reads these stores through the async proxy
             __syncwarp();
-            if (lane == 0) mbar_arrive(&full[s]);
+            if (lane == 0 && !dead) mbar_arrive(&full[s]);
             if (warp == 0) TC_ADD(1, t_f);
         };
         // two register sets, two chunks ahead of the stores: a chunk's loads have two stage times to arrive
@@ -209,17 +212,21 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
             }
         }
     } else if (warp == kMmaWarp) {
-        // ---- MMA issue: one thread ----
-        if (lane == 0) {
-            for (uint32_t c = 0; c < chunks; ++c) {
-                const uint32_t s = c % kStages, set = c & 1;
-                const long long t_a = TC_CLOCK();
-                mbar_wait(&full[s], (c / kStages) & 1, dead, p.error);
-                TC_ADD(2, t_a);
-                const long long t_b = TC_CLOCK();
-                mbar_wait(&set_free[set], (c >> 1) & 1, dead, p.error);  // use u of a set waits for its u-th release; the 0th is the epilogue's preset
-                TC_ADD(3, t_b);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        // ---- MMA issue: one elected thread ----
+        const bool leader = elect_one();
+        bool issued = false;  // the leader's
+        for (uint32_t c = 0; c < chunks; ++c) {
+            const uint32_t s = c % kStages, set = c & 1;
+            const long long t_a = TC_CLOCK();
+            mbar_wait(&full[s], (c / kStages) & 1, dead, p.bound.cycles);
+            TC_ADD(2, t_a);
+            const long long t_b = TC_CLOCK();
+            mbar_wait(&set_free[set], (c >> 1) & 1, dead, p.bound.cycles);  // use u of a set waits for its u-th release; the 0th is the epilogue's preset
+            TC_ADD(3, t_b);
+            __syncwarp();
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (leader && !dead) {
+                issued = true;
                 const uint32_t a0 = saddr(smem + size_t(s) * kStageBytes), b0 = a0 + kCB * kATile;
 #pragma unroll
                 for (int b = 0; b < kCB; ++b) {
@@ -227,6 +234,11 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
                 }
                 mma_commit(&set_full[set]);
             }
+            __syncwarp();
+        }
+        if (issued) {  // a commit behind all others: nothing of the MMAs outlives the CTA
+            mma_commit(&drained);
+            mbar_drain(&drained, 0);
         }
     } else {
         // ---- epilogue: thread = (row, 32 tokens) ----
@@ -249,7 +261,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
         for (uint32_t c = 0; c < chunks; ++c) {
             const uint32_t s = c % kStages, set = c & 1;
             const long long t_e = TC_CLOCK();
-            mbar_wait(&set_full[set], (c >> 1) & 1, dead, p.error);
+            mbar_wait(&set_full[set], (c >> 1) & 1, dead, p.bound.cycles);
+            __syncwarp();
             if (ew == 0) TC_ADD(4, t_e);
             const long long t_g = TC_CLOCK();
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -297,14 +310,14 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");  // the presets have landed
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) {
+            if (lane == 0 && !dead) {
                 mbar_arrive(&set_free[set]);
                 mbar_arrive(&stage_free[s]);
             }
             if (ew == 0) TC_ADD(5, t_g);
         }
         const uint32_t row = row_base + r;
-        if (row < p.m.rows) {
+        if (!dead && row < p.m.rows) {
 #pragma unroll
             for (int j = 0; j < kEC; ++j) {
                 const float value = acc[j];
@@ -316,6 +329,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_tc_kernel(const TcParams p) 
             }
         }
     }
+    if (dead) atomicOr(p.bound.error, 1u);
+    __syncwarp();
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == kMmaWarp) {
@@ -338,8 +353,8 @@ void launch_tile(const TcParams& p, cudaStream_t s) {
 bool gemm_tc_supports(int type, uint32_t cols) { return (type == T_Q4_0 || type == T_Q8_0) && cols % 128 == 0; }
 
 // out = weights x activations (EPI_STORE / EPI_ADD) for one Q4_0 / Q8_0 target on the tcgen05 path.
-void launch_gemm_tc(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, cudaStream_t s) {
-    const TcParams p{tg.m, act, tg.out, tg.ldo, n, int(epi), wait_error};
+void launch_gemm_tc(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, cudaStream_t s) {
+    const TcParams p{tg.m, act, tg.out, tg.ldo, n, int(epi), bound};
     if (tg.m.type == T_Q4_0) launch_tile<16>(p, s);
     else launch_tile<32>(p, s);
 }

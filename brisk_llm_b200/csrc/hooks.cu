@@ -41,11 +41,7 @@ struct ActBuffers {
 // The word that a bounded wait of a multiply sets: read it behind the multiplies that were given it.
 struct WaitError {
     Buf word{sizeof(unsigned int)};
-    WaitError() {
-        const unsigned int start = bk::tc_error_at_start();
-        BK_CUDA(cudaMemcpy(word.p, &start, sizeof start, cudaMemcpyHostToDevice));
-    }
-    unsigned int* get() const { return word.as<unsigned int>(); }
+    bk::WaitBound bound = bk::wait_bound(word.as<unsigned int>(), nullptr);
     void check() const {
         unsigned int set = 0;
         BK_CUDA(cudaMemcpy(&set, word.p, sizeof set, cudaMemcpyDeviceToHost));
@@ -59,7 +55,7 @@ void multiply(const bk::DevMatrix& m, float* out, const float* x, const bk::DevA
     bk::MatTarget t{m, out, m.rows};
     if (n == 1) {
         bk::launch_dec_multiply(&t, 1, x, nullptr, 0.0f, m.cols, bk::EPI_STORE, sms, s);
-    } else if (bk::launch_gemm(&t, 1, a, n, bk::EPI_STORE, word.get(), s) == 0) {
+    } else if (bk::launch_gemm(&t, 1, a, n, bk::EPI_STORE, word.bound, s) == 0) {
         bk::launch_matvec(&t, 1, a, n, bk::EPI_STORE, s);
     }
 }

@@ -65,16 +65,25 @@ constexpr uint32_t kPeerSlotPairs = 65536;
 void launch_tp_peer_exchange(uint2* const* bufs_dev, uint32_t* epoch, unsigned int* error, uint32_t tp, uint32_t rank, uint32_t slot_pairs,
                              const float* local, float* dst, uint32_t rows_l, bool add, cudaStream_t s);
 
+// ---- bounded waits of the kernels in tensor memory (gemm_k_tc.cu, and gemm_tc.cu: BRISK_CUDA_GEMM=tc) ----
+constexpr long long kTcWaitCycles = 2000000000ll;  // about a second: a wait that lasts this long has failed
+// `error`, a word of the caller's in device memory, is non-zero after a launch with a wait that ran out. It belongs to one caller: read
+// and cleared by several, one would take the other's garbage for results.
+struct WaitBound {
+    unsigned int* error = nullptr;
+    long long cycles = kTcWaitCycles;
+    uint32_t withheld = 0xffffffffu;  // tests only: the step of a CTA's walk whose weights are never brought
+};
+// BRISK_CUDA_TEST_TC_TIMEOUT (tests only), for the bounds made while it is set. 1: the word is set from the start, as a wait that ran
+// out leaves it. 2 + k: the weights of step k are withheld, and the waits for them run out after 50 us. Every access stays in bounds and
+// every wait ends; nothing faults or hangs.
+WaitBound wait_bound(unsigned int* word_on_device, cudaStream_t s);
+
 // ---- batched multiply on the int8 tensor path (gemm.cu) ----------------------------------------
 // Same contract as launch_matvec; returns the number of kernels launched, 0 when these types, shapes or token counts have
 // no tensor kernel (the caller then uses launch_matvec). The super-block formats have one for the pair epilogues where there are
 // rows and tokens enough (gemm_k_tc.cu); elsewhere the caller multiplies gate and up separately and runs launch_gate_mul.
-// The kernels in tensor memory (gemm_k_tc.cu, and gemm_tc.cu: BRISK_CUDA_GEMM=tc) have bounded waits: `wait_error`, a word of the
-// caller's in device memory, is non-zero after a launch whose wait ran out. It belongs to one caller: read and cleared by several, one
-// would take the other's garbage for results.
-int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, unsigned int* wait_error, cudaStream_t s);
-// BRISK_CUDA_TEST_TC_TIMEOUT=1 (tests only): the word of whoever asks is set from the start, as a wait that ran out leaves it.
-unsigned int tc_error_at_start();
+int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, cudaStream_t s);
 // The activation after separate gate and up multiplies. mode 0: gate[i] = silu(gate[i]) * up[i]; 1: max(gate[i],0)^2 * up[i];
 // 2: tanh-GELU(gate[i]) * up[i] (gelu_mul_f32, src/kernels_f32.cpp:291-296), its tanh corrected by tanh_table (see
 // build_tanh_table) when one is given.

@@ -207,6 +207,7 @@ struct Session {
     std::vector<void*> peer_mapped;              // what cudaIpcOpenMemHandle returned (closed with the session)
     bool peer_on = false;
     DevBuffer tc_error;  // set by a wait of this session's multiplies in tensor memory that ran out
+    WaitBound tc_bound;
     unsigned int* step_error_host = nullptr;  // pinned copy of the kernel's barrier-timeout word
     uint64_t persistent_steps = 0;
     uint64_t launches = 0;  // kernels launched by the current call
@@ -567,8 +568,7 @@ struct Session {
         BK_CUDA(cudaMallocHost(&step_error_host, 4 * sizeof(unsigned int)));  // [0] the persistent kernel's word, [1] the peer exchange's
         step_error_host[0] = step_error_host[1] = step_error_host[2] = step_error_host[3] = 0;  // [3]: that of the multiplies in tensor memory
         tc_error.alloc(sizeof(unsigned int));
-        const unsigned int tc_start = tc_error_at_start();
-        BK_CUDA(cudaMemcpyAsync(tc_error.p, &tc_start, sizeof tc_start, cudaMemcpyHostToDevice, stream));
+        tc_bound = wait_bound(tc_error.as<unsigned int>(), stream);
         BK_CUDA(cudaStreamSynchronize(stream));
         plan_step();
         stats.weight_bytes = weight_bytes;
@@ -655,13 +655,13 @@ struct Session {
     // batches go to the tensor-core kernel where the type has one.
     void multiply(std::vector<MatTarget> targets, const DevAct& a, uint32_t n, Epilogue epi) {
         if (epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL) {
-            if (const int ran = launch_gemm(targets.data(), int(targets.size()), a, n, epi, tc_error.as<unsigned int>(), stream)) {
+            if (const int ran = launch_gemm(targets.data(), int(targets.size()), a, n, epi, tc_bound, stream)) {
                 launches += ran;
                 return;
             }
             // formats whose tensor kernel has no fused activation: gate and up as two multiplies, then the activation elementwise
             const MatTarget both[2] = {{targets[0].m, targets[0].out, targets[0].ldo}, {targets[1].m, up_b.as<float>(), targets[0].ldo}};
-            if (const int ran = launch_gemm(both, 2, a, n, EPI_STORE, tc_error.as<unsigned int>(), stream)) {
+            if (const int ran = launch_gemm(both, 2, a, n, EPI_STORE, tc_bound, stream)) {
                 launch_gate_mul(targets[0].out, up_b.as<float>(), size_t(n) * targets[0].ldo, epi == EPI_RELU2_MUL, stream);
                 launches += ran + 1;
                 return;
@@ -673,7 +673,7 @@ struct Session {
         while (!targets.empty()) {
             std::vector<MatTarget> same, rest;
             for (const MatTarget& t : targets) (t.m.type == targets[0].m.type ? same : rest).push_back(t);
-            if (const int ran = launch_gemm(same.data(), int(same.size()), a, n, epi, tc_error.as<unsigned int>(), stream)) {
+            if (const int ran = launch_gemm(same.data(), int(same.size()), a, n, epi, tc_bound, stream)) {
                 launches += ran;
             } else {
                 launch_matvec(same.data(), int(same.size()), a, n, epi, stream);

@@ -4,7 +4,7 @@
 
 #include <cuda.h>
 
-#include "common.cuh"
+#include "kernels.h"
 
 namespace bk {
 
@@ -13,7 +13,6 @@ namespace bk {
 CUtensorMap tensor_map(const void* base, uint64_t row_bytes, uint64_t rows, uint32_t box_bytes, uint32_t box_rows);
 
 #ifdef __CUDACC__
-constexpr long long kTcWaitCycles = 2000000000ll;  // about a second: a wait that lasts this long has failed
 constexpr uint32_t kTmemCols = 512;
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return uint32_t(__cvta_generic_to_shared(p)); }
@@ -26,36 +25,49 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
     asm volatile("{\n.reg .pred p;\nmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}" : "=r"(ok) : "r"(saddr(b)), "r"(parity) : "memory");
     return ok != 0;
 }
-// Bounded: should a wait run out, the error word is set, `dead` makes this thread's later waits return at once, and the
-// kernel ends (with garbage) and still frees its tensor memory.
-__device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity, bool& dead, unsigned int* error) {
+// The waits of a kernel's warps are bounded: one that lasts longer than `limit` cycles gives up, and whoever gave up says so in the error
+// word at the kernel's end. What follows a wait that gave up:
+//   - No copy is asked for any more: one into a slot whose last is still on its way overdraws the slot's barrier. Nobody arrives whose
+//     own wait did not succeed, so that the waits of others give up in turn.
+//   - What had been asked for is waited for at the kernel's end (mbar_drain): copies, MMAs and commits that outlive their CTA write into
+//     shared and tensor memory that is another's by then.
+//   - A warp stays together. Lanes that went on where others gave up would meet those at no vote and no barrier again.
+//
+// By every lane of a warp for itself: `dead` where it gave up, at which its later waits return at once; all go on to the same end. A
+// __syncwarp follows: behind waits of single lanes even a vote does not bring the warp together again, and .sync.aligned instructions
+// (tcgen05.ld, tcgen05.st) that lanes reach apart have ended in an illegal memory access.
+__device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity, bool& dead, long long limit) {
     if (dead || mbar_try_wait(b, parity)) return;
     const long long start = clock64();
     while (!mbar_try_wait(b, parity)) {
-        if (clock64() - start > kTcWaitCycles) {  // bounded in time, not in tries: one try may itself sleep for a while
-            atomicOr(error, 1u);
+        if (clock64() - start > limit) {  // bounded in time, not in tries: one try may itself sleep for a while
             dead = true;
             return;
         }
     }
 }
-
 // A warp waits for several barriers at once, lanes first .. end - 1 for one each: even where the barriers are long
-// complete one wait costs 71 cycles, several at once 111.
-__device__ __forceinline__ void mbar_wait_all(uint64_t* mine, uint32_t parity, uint32_t first, uint32_t end, bool& dead, unsigned int* error) {
+// complete one wait costs 71 cycles, several at once 111. Every try is voted on, so that all lanes have one answer. False: gave up.
+__device__ __forceinline__ bool mbar_wait_all(uint64_t* mine, uint32_t parity, uint32_t first, uint32_t end, long long limit) {
     const uint32_t lane = threadIdx.x & 31;
     const bool waits = lane >= first && lane < end;
-    if (!dead && !__all_sync(0xffffffffu, !waits || mbar_try_wait(mine, parity))) {
+    bool done = __all_sync(0xffffffffu, !waits || mbar_try_wait(mine, parity));
+    if (!done) {
         const long long start = clock64();
-        while (!__all_sync(0xffffffffu, !waits || mbar_try_wait(mine, parity))) {
-            if (__any_sync(0xffffffffu, clock64() - start > kTcWaitCycles)) {
-                atomicOr(error, 1u);
-                dead = true;
-                break;
-            }
-        }
+        do {
+            done = __all_sync(0xffffffffu, !waits || mbar_try_wait(mine, parity));
+        } while (!done && !__any_sync(0xffffffffu, clock64() - start > limit));
     }
     __syncwarp();
+    return done;
+}
+// At the kernel's end, for what is sure to complete: a copy or a commit that was issued. (A second is far more than
+// either can take; it is there so that nothing waits without an end.)
+__device__ __forceinline__ void mbar_drain(uint64_t* b, uint32_t parity) {
+    const long long start = clock64();
+    while (!mbar_try_wait(b, parity)) {
+        if (clock64() - start > kTcWaitCycles) break;
+    }
 }
 
 // K-major operand tile without swizzle: core matrices of 8 rows x 16 bytes; `lbo` bytes between the two 16-byte halves of

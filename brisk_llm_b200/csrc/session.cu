@@ -764,8 +764,10 @@ struct Session {
     // (windows, 256-wide heads) needs a context that fits them.
     bool single_kernels() const {
         if (!variant_layers) return true;
-        return rope_dim == head_dim && chain_mode() != 0 && attn_decode_fits(head_dim, uint32_t(max_context));
+        return rope_dim == head_dim && attn_decode_runs();
     }
+    // Whether the kernels of attn_decode.cu take single tokens: contexts up to 33 792 positions, unless switched off.
+    bool attn_decode_runs() const { return chain_mode() != 0 && attn_decode_fits(head_dim, uint32_t(max_context)); }
 
     // The layers of one batch. n tokens are in d_tokens(), their first position in d_position(); max_visible bounds
     // position + n. single = true takes the fused single-token kernels (n == 1).
@@ -1080,7 +1082,7 @@ struct Session {
     // of the projections: 0.6B shape, one kernel per operation, at 181 positions 719 -> 661 us a token, at 520 - a second, late
     // round of rows - 757 -> 790).
     bool takes_fused_attention(uint64_t visible) const {
-        return visible <= 512 && head_dim <= 128 && rope_dim == head_dim && chain_mode() != 0 && attn_decode_fits(head_dim, uint32_t(max_context));
+        return visible <= 512 && head_dim <= 128 && rope_dim == head_dim && attn_decode_runs();
     }
     // One kernel per operation also beats the persistent kernel, at every depth and position. Persistent / per operation, us a token
     // at 181, 440, 530, 1024 and 2000 positions: 4 layers of the 0.6B shape (35 MB) 125/111, 129/125, 134/130, 145/138, 170/150;
@@ -1088,8 +1090,16 @@ struct Session {
     // the persistent kernel keeps are small models at short contexts, where that is 7 to 45 us a token: those of up to kFewLayers at
     // up to 1024 positions, and from 513 on those of up to kSomeLayers.
     static constexpr uint64_t kPlanesMaxWeights = uint64_t(8) << 20;  // measured where it is used
-    static constexpr uint64_t kFewLayers = uint64_t(100) << 20, kSomeLayers = uint64_t(160) << 20;
-    bool takes_persistent(uint64_t visible) const { return visible <= 1024 && layer_bytes <= (visible <= 512 ? kFewLayers : kSomeLayers); }
+    static constexpr uint64_t kFewLayers = uint64_t(100) << 20, kSomeLayers = uint64_t(160) << 20, kOlderAttention = 2500;
+    // All of that holds beside the attention of attn_decode.cu. A context too long for it (a session opened at a distributed model's own
+    // 40 960 positions) leaves the other side to the older attention kernels or, longer still, to the batched path. Persistent / older
+    // kernels, opened at 36 000: 28 layers at 200, 2000, 3000 and 8000 positions 685/722, 1019/1041, 1231/1214, 2244/2065, 4 layers at
+    // 200, 2000 and 4000 127/129, 169/174, 236/226. Persistent / batched path, opened at 40 960: 28 layers at 200, 2000 and 30 000
+    // 695/1316, 1036/1826, 6585/8972, 4 layers at 200 and 16 000 127/210, 591/799.
+    bool takes_persistent(uint64_t visible) const {
+        if (!attn_decode_runs()) return visible <= kOlderAttention || !dec_attention_fits(uint32_t(max_context), heads_l, head_dim, sms);
+        return visible <= 1024 && layer_bytes <= (visible <= 512 ? kFewLayers : kSomeLayers);
+    }
 
     void step_on_device(uint64_t visible) {  // one token whose id is *d_tokens() at *d_position() = visible - 1
         fused_attention = takes_fused_attention(visible);

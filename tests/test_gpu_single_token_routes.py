@@ -57,6 +57,28 @@ def test_long_sessions_keep_the_single_token_kernels(context, fits):
                 assert (s.stats()["kernel_launches"] == usual) == fits
 
 
+@pytest.mark.parametrize("layers,context,positions", [
+    (2, 40960, {300: 1, 1100: 1, 2600: 1}),          # the other side would be the batched path
+    (19, 40960, {20: 1}),                            # ... for layers past 160 MB too
+    (2, 36000, {300: 1, 2499: 1, 2500: 0, 2501: 0}),  # the older attention kernels, faster from 2501 visible positions on
+])
+def test_contexts_too_long_for_the_single_token_attention(layers, context, positions):
+    """Past 33 792 positions the kernels of csrc/attn_decode.cu do not run, and what was measured with them decides nothing. (0.6B files
+    state 40 960 positions, and a session takes what the file states.)"""
+    spec = synth.tiny(synth.QWEN3_0_6B, layers=layers, vocab=512, context=context)
+    model = synth.perturb_norms(synth.generate(spec, seed=10, share_layers=True))
+    toks = synth.random_tokens(spec, 2600, seed=11)
+    with engine.CudaSession(model) as s, engine.CudaSession(model, flags=abi.FLAG_NO_MEGAKERNEL) as general:
+        for at, persistent in positions.items():
+            for session in (s, general):
+                if session.position() < at:
+                    session.eval(toks[session.position():at])
+            assert np.array_equal(s.eval([5]), general.eval([5])), at
+            assert s.stats()["persistent_steps"] == persistent, at
+            for session in (s, general):
+                session.rollback(at)
+
+
 @pytest.mark.parametrize("layers", [11, 12])
 def test_the_switch_at_512_positions(layers):
     """Layers past 100 MB (12 of this shape; 11 stay below): one kernel per operation up to 512 positions, the persistent

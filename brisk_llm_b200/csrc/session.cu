@@ -626,8 +626,12 @@ struct Session {
         step_forced = env != nullptr && std::strcmp(env, "force") == 0;
         const char* graph_env = std::getenv("BRISK_CUDA_STEP_GRAPH");
         step_graph_wanted = graph_env != nullptr && std::atoi(graph_env) != 0;
-        step_enabled = step_plan.build(args, sh, sms, stream, why);
-        step_note = step_enabled ? "on: " + step_plan.description() : "off: " + why;
+        if (!step_forced && attn_decode_runs() && layer_bytes > kSomeLayers) {  // no token would take it: see takes_persistent
+            why = "layers of " + std::to_string(layer_bytes >> 20) + " MB take one kernel per operation, which is faster there";
+        } else {
+            step_enabled = step_plan.build(args, sh, sms, stream, why);
+        }
+        step_note = step_enabled ? "on: " + step_plan.description() + persistent_range() : "off: " + why;
         if (!token_why.empty()) step_note += " (one launch per token: " + token_why + ")";
         if (step_enabled && tracing) step_plan.set_trace(trace.as<unsigned long long>());
     }
@@ -1099,6 +1103,13 @@ struct Session {
     bool takes_persistent(uint64_t visible) const {
         if (!attn_decode_runs()) return visible <= kOlderAttention || !dec_attention_fits(uint32_t(max_context), heads_l, head_dim, sms);
         return visible <= 1024 && layer_bytes <= (visible <= 512 ? kFewLayers : kSomeLayers);
+    }
+
+    std::string persistent_range() const {  // of visible positions, as takes_persistent has it
+        if (step_forced) return "";
+        if (attn_decode_runs()) return layer_bytes <= kFewLayers ? ", up to 1024 positions" : ", from 513 to 1024 positions";
+        if (!dec_attention_fits(uint32_t(max_context), heads_l, head_dim, sms)) return "";
+        return ", up to " + std::to_string(kOlderAttention) + " positions";
     }
 
     void step_on_device(uint64_t visible) {  // one token whose id is *d_tokens() at *d_position() = visible - 1

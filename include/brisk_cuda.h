@@ -264,8 +264,9 @@ int brisk_cuda_argmax_static(const float* logits, uint32_t vocab, uint32_t rows,
                              size_t errlen);
 
 /* How single-token steps run in this session, as text: "persistent step kernel on: <configuration>" or
- * "persistent step kernel off: <reason>" (tensor parallel, flags, a model outside what the kernel covers, a barrier
- * that timed out earlier). No reference counterpart; benchmarks record it next to their numbers. */
+ * "persistent step kernel off: <reason>" (tensor parallel, flags, a model outside what the kernel covers or whose tokens
+ * are all faster without it, a barrier that timed out earlier). The configuration ends with the positions at which tokens
+ * take the kernel, where that is not all of them. No reference counterpart; benchmarks record it next to their numbers. */
 int brisk_cuda_step_path(brisk_cuda_session* session, char* text, size_t len);
 
 /* Per-phase device time, the counterpart of Session::profile() / BRISK_PROFILE (src/model.h:242-245,

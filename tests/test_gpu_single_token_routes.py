@@ -79,6 +79,19 @@ def test_contexts_too_long_for_the_single_token_attention(layers, context, posit
                 session.rollback(at)
 
 
+@pytest.mark.parametrize("layers,context,says", [(2, 640, "kernel on: tagged exchange"), (2, 640, ", up to 1024 positions"), (12, 640, ", from 513 to 1024 positions"),
+                                                 (19, 640, "kernel off: layers of 16"), (19, 40960, "kernel on: tagged exchange"), (2, 36000, ", up to 2500 positions")])
+def test_the_step_path_names_what_runs(layers, context, says):
+    """Where no token of a session takes the persistent kernel it is not built, and the session says so."""
+    spec = synth.tiny(synth.QWEN3_0_6B, layers=layers, vocab=512, context=context)
+    with engine.CudaSession(synth.generate(spec, seed=12, share_layers=True)) as s:
+        path = s.step_path()
+        assert says in path, path
+        s.eval(synth.random_tokens(spec, 513, seed=13))
+        s.eval([1])
+        assert s.stats()["persistent_steps"] == (0 if "off" in path else 1)
+
+
 @pytest.mark.parametrize("layers", [11, 12])
 def test_the_switch_at_512_positions(layers):
     """Layers past 100 MB (12 of this shape; 11 stay below): one kernel per operation up to 512 positions, the persistent

@@ -853,12 +853,15 @@ struct Session {
             at.n = n; at.heads = heads_l; at.kv_heads = kv_heads_l; at.dim = head_dim; at.max_context = uint32_t(max_context);
             at.max_visible = max_visible; at.scale = attn_scale; at.window = L.slides ? sliding_window : 0;
             // The output projection of a few tokens takes the attended rows as Q8_0 planes, with no norm between: the chains end in
-            // them, a launch less. us a pass, quantised by its own launch / by the chains: 0.6B shape Q4_0 at 2, 9, 23 tokens 1104/1075,
-            // 1220/1178, 1315/1296, Q8_0 verifying 9 after 700 positions 1889/1861, Gemma 1B shape at 9 and 23 1675/1648, 1827/1797,
-            // 1B Llama shape (4.2 M weights) at 23 1094/1087. The 7B shape (16.8 M) loses more by its projection's late start than the
-            // launch gives: 23 tokens 4341/4453, 23 after 500 positions 5208/5442, 9 after 2064 4469/4506 (2 to 16 tokens win).
+            // them, a launch less, but the projection starts later: its CTAs would sit beside the chains for the whole walk. Measured after
+            // 0, 500 and 2064 positions, us a pass, quantised by its own launch / by the chains. One token tile of the projection (up to 16
+            // tokens): 1.2 to 9.4 M weights 1 to 4 % faster at all of 2, 4, 9, 12, 16 tokens (0.6B shape 9 tokens 1137/1098, 3072 x 3072 16
+            // tokens 1254/1222), 12.8 and 16.8 M 0.5 to 8 % (16 tokens 1442/1417 and 1779/1645), 26 M even (2 tokens 1708/1715, 16
+            // 2473/2467), 67 M likewise. Two tiles: up to 4.2 M 1 to 3 % faster (0.6B shape 23 tokens 1246/1209, 1B Llama shape 992/976; at
+            // 2064 positions of the 0.6B shape Q4_0 up to 7 % slower, Q8_0 1 % faster), from 6.6 M on either way with the tokens: 2560 x
+            // 2560 at 17 and 23 1159/1262, 1295/1274, 4096 x 4096 2286/2210, 2186/2236.
             const bool planes = !single && !tp && L.attn_sub_norm == nullptr && block_elems(L.o.type) == 32 &&
-                uint64_t(hidden) * q_dim <= kPlanesMaxWeights && attention_takes_chain(n);
+                uint64_t(hidden) * q_dim <= (n <= 16 ? kPlanesOneTile : kPlanesTwoTiles) && attention_takes_chain(n);
             const DevActMut* attended_planes = planes ? &act : nullptr;
             {
                 Scope sc(this, PH_ATTENTION);
@@ -1093,7 +1096,7 @@ struct Session {
     // 12 layers (106 MB) 315/270, 323/311, 336/325, 378/352, 462/390; 28 (248 MB) 683/589, 727/690, 757/724, 853/788, 1019/869. What
     // the persistent kernel keeps are small models at short contexts, where that is 7 to 45 us a token: those of up to kFewLayers at
     // up to 1024 positions, and from 513 on those of up to kSomeLayers.
-    static constexpr uint64_t kPlanesMaxWeights = uint64_t(8) << 20;  // measured where it is used
+    static constexpr uint64_t kPlanesOneTile = uint64_t(20) << 20, kPlanesTwoTiles = uint64_t(5) << 20;  // weights; measured where they are used
     static constexpr uint64_t kFewLayers = uint64_t(100) << 20, kSomeLayers = uint64_t(160) << 20, kOlderAttention = 2500;
     // All of that holds beside the attention of attn_decode.cu. A context too long for it (a session opened at a distributed model's own
     // 40 960 positions) leaves the other side to the older attention kernels or, longer still, to the batched path. Persistent / older

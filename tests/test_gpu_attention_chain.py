@@ -14,6 +14,26 @@ from brisk_llm_b200 import abi, engine, synth
 
 pytestmark = pytest.mark.gpu
 
+# (hidden = heads x 128, tokens from which the output projection's input is quantised by a launch of its own)
+@pytest.mark.parametrize("hidden,first", [(2048, 25), (2560, 17), (4096, 17), (5120, 2)])
+def test_where_the_chains_end_in_planes(hidden, first):
+    """The attended rows of few tokens as 8-bit planes from the chains, a launch a layer less, on both sides of the lines by the weights
+    of the output projection and by its token tiles: the oracle's bits either way."""
+    spec = synth.tiny(synth.MISTRAL_7B, layers=1, vocab=512, context=128, hidden=hidden, heads=hidden // 128, kv_heads=hidden // 512, ffn=512)
+    model = synth.perturb_norms(synth.generate(spec, seed=hidden))
+    toks = synth.random_tokens(spec, 24, seed=43)
+    oracle = H.OracleSession(model)
+    launches = {}
+    with engine.CudaSession(model) as s:
+        for n in (2, 16, 17, 24):
+            s.rollback(0)
+            got = s.eval(toks[:n])
+            launches[n] = s.stats()["kernel_launches"]
+            oracle.rollback(0)
+            assert np.array_equal(got, oracle.eval(toks[:n])), n
+    assert launches == {n: 15 if n >= first else 14 for n in launches}
+
+
 FAMILIES = [
     ("qwen3", synth.tiny(synth.QWEN3_0_6B, layers=2, vocab=512, context=2048)),      # 128-wide heads, 2 per K/V head
     ("llama", synth.tiny(synth.LLAMA_3_2_1B, layers=2, vocab=512, context=2048)),    # 64-wide heads, 4 per K/V head

@@ -491,6 +491,7 @@ struct KTile {
     uint64_t alone, shared;  // ns of a super-block of Q4_K: of one CTA by itself, and per CTA of a full SM
     uint64_t percent;        // of them that this type takes
     void (*kernel)(KParams);
+    mutable DeviceOnce allowed{};  // its shared memory
 };
 
 template <int TYPE, int MI, int NI, int WR, int WT, int KS, int STAGES, int RESIDENT>
@@ -501,85 +502,91 @@ KTile tile_of(uint64_t alone, uint64_t shared, uint64_t q5_k, uint64_t q6_k, uin
                  gemm_k_kernel<TYPE, MI, NI, WR, WT, KS, STAGES, RESIDENT>};
 }
 
-// The tile whose busiest SM is done first, as in gemm.cu; 800 ns for what a CTA does besides its super-blocks. Measured, Q4_K: 2048 x 8192 at 9 tokens 25 (64 x 16 tiles) / 7.9 us (16 x 16,
-// split), 14336 x 4096 at 9 tokens 20 / 24.
-//
-// False: the tensor-memory kernel (gemm_k_tc.cu) is estimated to be done sooner (than other_ns), and nothing was launched. It takes tiles of 128
-// rows and needs about 3.5 us around its super-blocks, so few rows or tokens stay here (2048 x 2048 Q4_K at 128 tokens 9.6 us
-// here, 12.2 there; 14336 x 4096 at 64 tokens 34 and 21).
+// The tile whose busiest SM is done first, as in gemm.cu, and its time in ns; 800 ns for what a CTA does besides its super-blocks.
+// Measured, Q4_K: 2048 x 8192 at 9 tokens 25 (64 x 16 tiles) / 7.9 us (16 x 16, split), 14336 x 4096 at 9 tokens 20 / 24.
 template <int TYPE>
-bool launch_type(KParams& p, uint64_t other_ns, bool ask_only, uint32_t sms, cudaStream_t s) {
+const KTile& fastest_tile(const MatTarget* targets, int count, uint32_t n, uint32_t sms, uint64_t& ns) {
     static const KTile tiles[] = {
         tile_of<TYPE, 1, 4, 4, 2, 1, 2, 2>(1250, 1060, 122, 172, 74), tile_of<TYPE, 1, 2, 4, 1, 1, 4, 4>(770, 540, 125, 143, 65),
         tile_of<TYPE, 1, 2, 1, 1, 8, 2, 1>(210, 230, 118, 137, 85), tile_of<TYPE, 1, 1, 1, 1, 4, 3, 3>(200, 137, 110, 135, 85),
     };
-    static DeviceOnce once;
-    if (once.first()) {
-        for (const KTile& tile : tiles) BK_CUDA(cudaFuncSetAttribute(tile.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile.smem)));
-    }
     const KTile* pick = nullptr;
     uint64_t best = 0;
     for (const KTile& tile : tiles) {
         uint64_t ctas = 0;
-        for (int i = 0; i < p.count; ++i) ctas += (p.m[i].rows + tile.rows - 1) / tile.rows;
-        ctas *= (p.n + tile.tokens - 1) / tile.tokens;
+        for (int i = 0; i < count; ++i) ctas += (targets[i].m.rows + tile.rows - 1) / tile.rows;
+        ctas *= (n + tile.tokens - 1) / tile.tokens;
         const uint64_t per_sm = (ctas + sms - 1) / sms, rounds = (per_sm + tile.resident - 1) / tile.resident;
-        const uint64_t blocks = (p.m[0].blocks + tile.split - 1) / tile.split * tile.split;
+        const uint64_t blocks = (targets[0].m.blocks + tile.split - 1) / tile.split * tile.split;
         const uint64_t cost = std::max(rounds * (tile.alone * blocks + 800), per_sm * tile.shared * blocks);
         if (pick == nullptr || cost < best) {
             pick = &tile;
             best = cost;
         }
     }
-    if (other_ns < best * pick->percent / 100) return false;
-    if (ask_only) return true;
-    uint32_t row_tiles = 0;
-    for (int i = 0; i < p.count; ++i) {
-        p.first_tile[i] = row_tiles;
-        row_tiles += (p.m[i].rows + pick->rows - 1) / pick->rows;
+    ns = best * pick->percent / 100;
+    return *pick;
+}
+
+const KTile& fastest_tile(const MatTarget* targets, int count, uint32_t n, uint32_t sms, uint64_t& ns) {
+    switch (targets[0].m.type) {
+        case T_Q4_K: return fastest_tile<T_Q4_K>(targets, count, n, sms, ns);
+        case T_Q5_K: return fastest_tile<T_Q5_K>(targets, count, n, sms, ns);
+        case T_Q6_K: return fastest_tile<T_Q6_K>(targets, count, n, sms, ns);
+        case T_TQ2_0: return fastest_tile<T_TQ2_0>(targets, count, n, sms, ns);
+        default: throw CudaError("cuda: no super-block tensor kernel for this type");
     }
-    launch_dependent(pick->kernel, dim3(row_tiles, (p.n + pick->tokens - 1) / pick->tokens), dim3(pick->threads), pick->smem, s, p);
-    return true;
 }
 
 }  // namespace
 
-// gemm_k_tc.cu: the multiply in tensor memory, and what it is expected to take
-void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, uint32_t sms, cudaStream_t s);
-uint64_t gemm_k_tc_ns(const MatTarget* targets, int count, uint32_t n, bool pair, uint32_t sms);
+// gemm_k_tc.cu: the multiply in tensor memory, in tiles of `tokens` tokens, what it is expected to take and with which tile
+void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t tokens, const WaitBound& bound, uint32_t sms, cudaStream_t s);
+uint64_t gemm_k_tc_ns(const MatTarget* targets, int count, uint32_t n, bool pair, uint32_t sms, uint32_t& tokens);
 
 bool gemm_k_supports(int type) { return type == T_Q4_K || type == T_Q5_K || type == T_Q6_K || type == T_TQ2_0; }
 
-// False, nothing launched: a gate/up pair that the caller multiplies separately.
-bool launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, uint32_t sms, cudaStream_t s) {
-    const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
-    uint64_t other_ns = gemm_k_tc_ns(targets, count, n, pair, sms);
+// The kernel in tensor memory takes tiles of 128 rows and needs about 5 us around its super-blocks, so few rows or tokens stay here
+// (2048 x 2048 Q4_K at 128 tokens 9.6 us here, 12.2 there; 14336 x 4096 at 64 tokens 34 and 21): whichever is estimated to be done sooner.
+uint32_t super_block_tokens(const MatTarget* targets, int count, uint32_t n, bool pair, uint32_t sms) {
+    uint64_t here_ns = 0;
+    fastest_tile(targets, count, n, sms, here_ns);
+    uint32_t tokens = 0;
+    uint64_t there_ns = gemm_k_tc_ns(targets, count, n, pair, sms, tokens);
     if (pair) {
         // Here the activation is a launch of its own (a 3 us launch, 22 us for 512 x 8192 values): the tensor-memory kernel applies it
         // as it stores. The two matrices are asked about as the caller would send them.
         const uint64_t activation_ns = 3000 + uint64_t(n) * targets[0].m.rows / 220;
-        other_ns = other_ns > activation_ns ? other_ns - activation_ns : 0;
+        there_ns = there_ns > activation_ns ? there_ns - activation_ns : 0;
     }
+    return there_ns < here_ns ? tokens : 0;
+}
+
+// False, nothing launched: a gate/up pair that the caller multiplies separately.
+bool launch_gemm_k(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, uint32_t sms, cudaStream_t s) {
+    const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
+    if (const uint32_t tokens = super_block_tokens(targets, count, n, pair, sms)) {
+        launch_gemm_k_tc(targets, count, act, n, epi, tokens, bound, sms, s);
+        return true;
+    }
+    if (pair) return false;
     KParams p{};
+    uint64_t ns = 0;
+    const KTile& tile = fastest_tile(targets, count, n, sms, ns);
+    uint32_t row_tiles = 0;
     for (int i = 0; i < count; ++i) {
         p.m[i] = targets[i].m;
         p.out[i] = targets[i].out;
         p.ldo[i] = targets[i].ldo;
+        p.first_tile[i] = row_tiles;
+        row_tiles += (p.m[i].rows + tile.rows - 1) / tile.rows;
     }
     p.act = act;
     p.n = n;
     p.count = count;
     p.epi = int(epi);
-    bool here = false;
-    switch (targets[0].m.type) {
-        case T_Q4_K: here = launch_type<T_Q4_K>(p, other_ns, pair, sms, s); break;
-        case T_Q5_K: here = launch_type<T_Q5_K>(p, other_ns, pair, sms, s); break;
-        case T_Q6_K: here = launch_type<T_Q6_K>(p, other_ns, pair, sms, s); break;
-        case T_TQ2_0: here = launch_type<T_TQ2_0>(p, other_ns, pair, sms, s); break;
-        default: throw CudaError("cuda: no super-block tensor kernel for this type");
-    }
-    if (here) return !pair;
-    launch_gemm_k_tc(targets, count, act, n, epi, bound, sms, s);
+    if (tile.allowed.first()) BK_CUDA(cudaFuncSetAttribute(tile.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(tile.smem)));
+    launch_dependent(tile.kernel, dim3(row_tiles, (n + tile.tokens - 1) / tile.tokens), dim3(tile.threads), tile.smem, s, p);
     return true;
 }
 

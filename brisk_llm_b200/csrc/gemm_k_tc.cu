@@ -660,11 +660,13 @@ static uint64_t tile_ns(const MatTarget* targets, int count, uint32_t n, bool pa
     return (tiles + sms - 1) / sms * (targets[0].m.blocks * (halves == 2 ? two : one) + (pair ? 1200 * halves : 0)) + 5000;
 }
 
-uint64_t gemm_k_tc_ns(const MatTarget* targets, int count, uint32_t n, bool pair, uint32_t sms) {
-    return std::min(tile_ns(targets, count, n, pair, 1, sms), tile_ns(targets, count, n, pair, 2, sms));
+uint64_t gemm_k_tc_ns(const MatTarget* targets, int count, uint32_t n, bool pair, uint32_t sms, uint32_t& tokens) {
+    const uint64_t one = tile_ns(targets, count, n, pair, 1, sms), two = tile_ns(targets, count, n, pair, 2, sms);
+    tokens = two < one ? 2 * kTokens : kTokens;
+    return std::min(one, two);
 }
 
-void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, uint32_t sms, cudaStream_t s) {
+void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, uint32_t tokens, const WaitBound& bound, uint32_t sms, cudaStream_t s) {
     KtParams p{};
     for (int i = 0; i < count; ++i) {
         p.m[i] = targets[i].m;
@@ -678,7 +680,7 @@ void launch_gemm_k_tc(const MatTarget* targets, int count, const DevAct& act, ui
     p.one = 1.0f;
     p.bound = bound;
     const bool pair = epi == EPI_SILU_MUL || epi == EPI_RELU2_MUL;
-    const int halves = tile_ns(targets, count, n, pair, 2, sms) < tile_ns(targets, count, n, pair, 1, sms) ? 2 : 1;
+    const int halves = int(tokens / kTokens);
     switch (targets[0].m.type) {
         case T_Q4_K: launch_type<T_Q4_K>(p, pair, halves, sms, s); break;
         case T_Q5_K: launch_type<T_Q5_K>(p, pair, halves, sms, s); break;

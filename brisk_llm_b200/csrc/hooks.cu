@@ -151,4 +151,17 @@ int brisk_cuda_matmul_seconds(int32_t type, const void* w, uint64_t rows, uint64
     }
 }
 
+// Not part of the header: the tokens of the tile (64 or 128) in which gemm_k_tc.cu multiplies `count` matrices of a super-block format by n
+// tokens on a GPU of `sms` SMs, 0 where gemm_k.cu does. Host arithmetic, for the tests of those kernels.
+uint32_t brisk_cuda_super_block_tokens(int32_t type, const uint32_t* rows, uint32_t count, uint32_t cols, uint32_t n, int32_t pair, uint32_t sms) {
+    bk::MatTarget targets[3]{};
+    if (count > 3) count = 3;
+    for (uint32_t i = 0; i < count; ++i) {
+        targets[i].m.type = type;
+        targets[i].m.rows = rows[i];
+        targets[i].m.blocks = cols / 256;
+    }
+    return bk::super_block_tokens(targets, int(count), n, pair != 0, sms);
+}
+
 }  // extern "C"

@@ -84,6 +84,8 @@ WaitBound wait_bound(unsigned int* word_on_device, cudaStream_t s);
 // no tensor kernel (the caller then uses launch_matvec). The super-block formats have one for the pair epilogues where there are
 // rows and tokens enough (gemm_k_tc.cu); elsewhere the caller multiplies gate and up separately and runs launch_gate_mul.
 int launch_gemm(const MatTarget* targets, int count, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, cudaStream_t s);
+// The tokens of gemm_k_tc.cu's tile for this multiply of a super-block format (pair: gate and up with the activation), 0: gemm_k.cu's.
+uint32_t super_block_tokens(const MatTarget* targets, int count, uint32_t n, bool pair, uint32_t sms);
 // The activation after separate gate and up multiplies. mode 0: gate[i] = silu(gate[i]) * up[i]; 1: max(gate[i],0)^2 * up[i];
 // 2: tanh-GELU(gate[i]) * up[i] (gelu_mul_f32, src/kernels_f32.cpp:291-296), its tanh corrected by tanh_table (see
 // build_tanh_table) when one is given.

@@ -168,10 +168,11 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
     return ok != 0;
 }
 // Bounded: a bulk copy from valid memory always completes; if it does not within the limit the error word is set and the
-// caller goes on (with garbage), so the kernel still ends.
+// caller goes on (with garbage), so the kernel still ends. Not given up because a poll of results ran out, as polls are: the copy has been
+// asked for and comes, and a caller that went on would ask for the next one over it, or end before it.
 __device__ __noinline__ void mbar_wait(uint64_t* b, uint32_t parity, unsigned int* error) {
     for (uint32_t spin = 0; !mbar_try_wait(b, parity); ++spin) {
-        if (spin == kMbarLimit || poll_abandoned(spin, error)) {
+        if (spin == kMbarLimit) {
             poll_failed(error);
             return;
         }

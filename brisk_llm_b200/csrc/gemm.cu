@@ -394,7 +394,7 @@ uint32_t sm_count() {
 bool gemm_tc_supports(int type, uint32_t cols);  // gemm_tc.cu: the same arithmetic on tcgen05 / tensor memory
 void launch_gemm_tc(const MatTarget& tg, const DevAct& act, uint32_t n, Epilogue epi, const WaitBound& bound, cudaStream_t s);
 // BRISK_CUDA_GEMM=tc / mma picks the prompt GEMM of Q4_0 / Q8_0 matrices (read at every call); unset: kGemmTcDefault. Measured,
-// 512 tokens, us here / gemm_tc.cu: 1024 x 3072 Q4_0 21 / 37, 2048 x 8192 76 / 91, 4096 x 14336 228 / 296, Q8_0 240 / 317.
+// 512 tokens, us here / gemm_tc.cu: 1024 x 3072 Q4_0 21 / 37, 2048 x 8192 76 / 89, 4096 x 14336 228 / 287, Q8_0 241 / 322.
 constexpr bool kGemmTcDefault = false;
 static bool gemm_tc_on() {
     const char* env = std::getenv("BRISK_CUDA_GEMM");

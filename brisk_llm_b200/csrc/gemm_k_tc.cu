@@ -21,12 +21,13 @@
 //   8 epilogue warps  per super-block: accumulators as mma-style fragments (4 rows x 8 tokens a thread, so that a scale read
 //                     from shared memory meets 4 or 8 outputs), the digits joined, one conversion, the reference's roundings
 //
-// Measured, 512 tokens, us against the tiles of gemm_k.cu: 14336 x 4096 Q4_K 228 -> 111, Q5_K 269 -> 120, Q6_K 364 -> 118, TQ2_0
-// 168 -> 74; 2048 x 8192 Q4_K 67 -> 36, Q6_K 118 -> 41. Bound: not the MMAs (16 of 32 cycles each, plus one, in the 1900 cycles a
-// super-block and 64 tokens take; 1400 in tiles of 128) but the hand-overs around them. A wait on an mbarrier costs 71
-// cycles even when it is long complete (111 where lanes wait for several), and the tensor memory beside two sets of accumulators holds the digits of one super-block
-// only: with neither arithmetic nor MMAs the same hand-overs take 900 cycles. Tiles of 128 tokens, one expansion for two sets,
-// are the better ones where they fill the GPU.
+// Measured, 512 tokens, us against the tiles of gemm_k.cu: 14336 x 4096 Q4_K 228 -> 108, Q5_K 269 -> 114, Q6_K 364 -> 115, TQ2_0
+// 168 -> 72; 2048 x 8192 Q4_K 67 -> 36, Q6_K 118 -> 42. Bound: not the MMAs (16 of 32 cycles each, plus one, in the 1900 cycles a
+// super-block and 64 tokens take; 1400 in tiles of 128; the tensor pipe is active 11 to 26 % of the time, the issue slots 30 to 57)
+// but the hand-overs around them. By cycle stamps in a copy of the kernel a wait on an mbarrier costs 71 cycles even when it is long
+// complete (111 where lanes wait for several), and with neither arithmetic nor MMAs the same hand-overs take 900 cycles: the tensor
+// memory beside two sets of accumulators holds the digits of one super-block only. Tiles of 128 tokens, one expansion for two
+// sets, are the better ones where they fill the GPU.
 #include <algorithm>
 
 #include "formats.cuh"

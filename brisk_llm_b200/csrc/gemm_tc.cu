@@ -20,9 +20,9 @@
 //
 // Loaders, MMA and epilogue meet only at mbarriers (stage full / stage free / set full / set free); every wait is bounded
 // and ends in an error word. The epilogue is the bound: 5 f32-pipe instructions per (row, token, block) is ~215 TMAC/s at
-// full issue; measured, 4096 x 14336 Q4_0 at 512 tokens, it reaches 102. gemm.cu, with three instructions of the f32 pipe a
+// full issue; measured, 4096 x 14336 Q4_0 at 512 tokens, it reaches 105. gemm.cu, with three instructions of the f32 pipe a
 // term, reaches 132 behind mma.sync fragments and is the default; its arithmetic in this kernel's epilogue spilled at 128
-// registers a thread (380 us against 296).
+// registers a thread (380 us against 296 then).
 #include "kernels.h"
 #include "packed.cuh"
 #include "tc.cuh"

@@ -3,8 +3,8 @@
 // everything else only behind wait_for_previous(), and lets the next kernel start with release_next() some time after it
 // has waited itself - so nothing runs ahead of results that are more than one kernel away. Short kernels release at once,
 // long ones when their main loop is done; CTAs that wait beside a running kernel for long slow it down (prompts of 512 to
-// 800 tokens: 5-18 % between the two). What it saves is the gap between two kernels, 1-2 us, of which a layer of a short
-// prompt has twelve.
+// 800 tokens: 5-18 % between the two). What it saves is the gap between two kernels, 1-2 us, of which a layer of a
+// prompt has twelve, one of a few tokens eleven.
 #pragma once
 
 #include <utility>

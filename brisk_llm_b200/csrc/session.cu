@@ -627,7 +627,7 @@ struct Session {
         const char* graph_env = std::getenv("BRISK_CUDA_STEP_GRAPH");
         step_graph_wanted = graph_env != nullptr && std::atoi(graph_env) != 0;
         if (!step_forced && attn_decode_runs() && layer_bytes > kSomeLayers) {  // no token would take it: see takes_persistent
-            why = "layers of " + std::to_string(layer_bytes >> 20) + " MB take one kernel per operation, which is faster there";
+            why = "layers of " + std::to_string(layer_bytes >> 20) + " MiB take one kernel per operation, which is faster there";
         } else {
             step_enabled = step_plan.build(args, sh, sms, stream, why);
         }
@@ -1093,9 +1093,10 @@ struct Session {
     }
     // One kernel per operation also beats the persistent kernel, at every depth and position. Persistent / per operation, us a token
     // at 181, 440, 530, 1024 and 2000 positions: 4 layers of the 0.6B shape (35 MB) 125/111, 129/125, 134/130, 145/138, 170/150;
-    // 12 layers (106 MB) 315/270, 323/311, 336/325, 378/352, 462/390; 28 (248 MB) 683/589, 727/690, 757/724, 853/788, 1019/869. What
-    // the persistent kernel keeps are small models at short contexts, where that is 7 to 45 us a token: those of up to kFewLayers at
-    // up to 1024 positions, and from 513 on those of up to kSomeLayers.
+    // 12 layers (106 MB) 315/270, 323/311, 336/325, 378/352, 462/390; 28 (248 MB) 683/589, 727/690, 757/724, 853/788, 1019/869. So no
+    // line between the two is one where they cross. These bound what the persistent kernel still takes until it is taught the other's
+    // attention or goes: models of up to kFewLayers at up to 1024 positions, and from 513 on those of up to kSomeLayers. That costs them 4 us
+    // a token (4 layers at 440 or 530 positions) to about 40 (11 layers at 181).
     static constexpr uint64_t kPlanesOneTile = uint64_t(20) << 20, kPlanesTwoTiles = uint64_t(5) << 20;  // weights; measured where they are used
     static constexpr uint64_t kFewLayers = uint64_t(100) << 20, kSomeLayers = uint64_t(160) << 20, kOlderAttention = 2500;
     // All of that holds beside the attention of attn_decode.cu. A context too long for it (a session opened at a distributed model's own

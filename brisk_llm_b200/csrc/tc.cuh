@@ -34,7 +34,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* b, uint32_t parity) {
 //   - A warp stays together. Lanes that went on where others gave up would meet those at no vote and no barrier again.
 //
 // By every lane of a warp for itself: `dead` where it gave up, at which its later waits return at once; all go on to the same end. A
-// __syncwarp follows: behind waits of single lanes even a vote does not bring the warp together again, and .sync.aligned instructions
+// __syncwarp follows: behind waits of single lanes even a vote need not bring the warp together again, and .sync.aligned instructions
 // (tcgen05.ld, tcgen05.st) that lanes reach apart have ended in an illegal memory access.
 __device__ __forceinline__ void mbar_wait(uint64_t* b, uint32_t parity, bool& dead, long long limit) {
     if (dead || mbar_try_wait(b, parity)) return;
